@@ -201,14 +201,13 @@ QSES_API int qses_autotune(qses_context *ctx, const qses_params *p, const qses_f
  * shape.  Same codes for all. */
 QSES_API int qses_set_field_shape(qses_context *ctx, int shape);
 /* Fixes the smoothing launch shape of ctx: threads 512 or 1024 per slab CTA, slab size
- * aimed at (>= 256 vertices), cache_flags bit 0 = prefetch successors' neighbour lists into
- * L1 instead of L2, bit 1 = neighbour positions through L1, bit 2 = keep the positions in
- * persisting L2 lines during the pass (a window on the context's stream, cleared after it),
- * bit 3 = each slab's own positions in shared memory (slabs of at most 8192 vertices),
- * bit 4 = two vertex updates per worker warp (16 lanes each), bit 5 = four (8 lanes each;
- * not with bit 4); wave_vertices = most vertices per slab-kernel launch (0 = the whole mesh in one launch;
- * otherwise sequential waves); threads = 0 returns to the tuned/default shape.
- * Every shape gives the same mesh. */
+ * aimed at (>= 256 vertices; slabs hold at most 11 904), cache_flags bit 2 = keep the
+ * positions in persisting L2 lines during the pass (a window on the context's stream, cleared
+ * after it); bits 0, 1, 3, 4 and 5 (not 4 and 5 together) are accepted and without effect: a
+ * slab's positions are in shared memory and a worker warp takes a second vertex whenever more
+ * are ready than warps; wave_vertices = most vertices per slab-kernel launch (0 = the whole
+ * mesh in one launch; otherwise sequential waves); threads = 0 returns to the tuned/default
+ * shape.  Every shape gives the same mesh. */
 QSES_API int qses_set_smoothing_shape(qses_context *ctx, int threads, unsigned target, unsigned cache_flags,
                                       unsigned wave_vertices);
 /* Sets the process-wide smoothing shape (as qses_set_smoothing_shape, no waves) for every
@@ -277,12 +276,11 @@ QSES_API int qses_last_launch_count(qses_context *ctx);
  * pre-filter count so it can start while the smoothing pass runs). */
 QSES_API unsigned long long qses_last_download_bytes(qses_context *ctx);
 /* Smoothing diagnostics of the last call: [0] slabs, [1] vertices per slab, [2] most
- * boundary polls of one slab, [3] slabs that did not finish, [4] clock cycles spent in
- * vertex updates, [5] in releasing successors, [6] vertices updated, [7] cycles until a
- * vertex's neighbour ids arrived, [8] then until their positions arrived, [9] in the
- * position store and its fence (summed over warps); [2]-[9] are counted on calls
- * made with profiling on (qses_set_profiling) and are 0 otherwise.  Returns the number of
- * values written. */
+ * boundary polls of one slab, [3] slabs that did not finish, [6] vertices updated (summed
+ * over passes); [2], [3] and [6] are counted on calls made with profiling on
+ * (qses_set_profiling) and are 0 otherwise.  [4], [5] and [7]-[9] held clock cycles of parts of
+ * an update; clock reads lengthen the dependency chain, so they are no longer taken and read 0.
+ * Returns the number of values written. */
 QSES_API int qses_diagnostics(qses_context *ctx, unsigned long long *out, int max);
 
 /* Host timeline of the last pipeline run on ctx (ms; for a batch call, its last batch):

@@ -726,7 +726,7 @@ QSES_API int qses_autotune_batch(qses_context *ctx, const qses_request *reqs, un
     }
     ctx->gs_force = qses::GsShape{0, 0, 0, 0};
     if (rc) return rc;
-    if (nv > 0) qses::gs_shape_record((unsigned)std::min<unsigned long long>(nv, 152ull * qses::kGsSlabMaxVerts), true, best);
+    if (nv > 0) qses::gs_shape_record((unsigned)std::min<unsigned long long>(nv, 0xffffffffull), true, best);
     if (threads_out) *threads_out = best.threads;
     if (target_out) *target_out = best.target;
     if (flags_out) *flags_out = best.flags;
@@ -788,15 +788,19 @@ QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int
     if (!ctx || !kernel_status || spin_cycles < 1000000ll || spin_cycles > 4000000000ll) return QSES_ERR_INVALID_ARG;
     *kernel_status = 0;
     cudaSetDevice(ctx->device);
-    // Vertices 0-1 (slab 0) and 2-3 (slab 1), lists 0:{1} 1:{0} 2:{3} 3:{2}.  Vertex 2 is
-    // marked as waiting for one lower-slab hand-off (remote count 1, +1 in its counter) that
-    // no vertex ever sends, so slab 1 cannot finish and its boundary warp's wait runs out.
+    // Vertices 0-1 (slab 0) and 2-3 (slab 1), lists 0:{1 1} 1:{0 0} 2:{3 3} 3:{2 2}.  Vertex 2 is
+    // marked as waiting for one release from a lower slab (byte 2 of ext, bit 7 and one count in
+    // its word) that no vertex ever sends, so slab 1 cannot finish and its receivers' wait runs
+    // out.
     const unsigned table_h[6] = {2, 0, 2, 4, 0, 1};  // Q, bounds (qcap + 1 = 3), order
     const uint2 start_h[5] = {{0, 0}, {1, 0}, {2, 0}, {3, 0}, {4, 0}};
-    const unsigned nbr_h[4] = {1, 0, 3, 2};
-    const unsigned short cnt_h[4] = {0, 1, 1, 1};
-    const int remote_h[4] = {0, 0, 1, 0};
-    const uint2 home_h[4] = {{0, 0}, {0, 0}, {1, 2}, {1, 2}};
+    const unsigned nbr_h[8] = {1, 1, 0, 0, 3, 3, 2, 2};
+    const unsigned word_h[4] = {0x200, 0x201, 0x281, 0x201};  // one pair of entries
+    unsigned pack_h[4][16];  // records; past the end: smax; bit 30: higher, bit 29: named before
+    for (int v = 0; v < 4; v++)
+        for (int e = 0; e < 16; e++)
+            pack_h[v][e] = e > 1 ? 2u : v & 1 ? (e ? 0x20000000u : 0u) : (e ? 0x60000001u : 0x40000001u);
+    const unsigned char ext_h[4] = {0, 0, 1, 0};
     const float4 pos_h[4] = {{0, 0, 0, 0}, {1, 0, 0, 0}, {0, 1, 0, 0}, {0, 0, 1, 0}};
     char *d = nullptr;
     const size_t bytes = 4096;
@@ -804,25 +808,25 @@ QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int
         cudaGetLastError();
         return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "wait-limit check buffers");
     }
-    unsigned *table = (unsigned *)d, *nbr = (unsigned *)(d + 256), *inbox = (unsigned *)(d + 512),
-             *tails = (unsigned *)(d + 768);
-    uint2 *start = (uint2 *)(d + 1024), *home = (uint2 *)(d + 1280);
-    unsigned short *cnt = (unsigned short *)(d + 1536);
-    int *remote = (int *)(d + 1792), *err = (int *)(d + 2048);
+    unsigned *table = (unsigned *)d, *nbr = (unsigned *)(d + 256), *next_slab = (unsigned *)(d + 768);
+    uint2 *start = (uint2 *)(d + 1024);
+    unsigned *word0 = (unsigned *)(d + 1536);
+    uint4 *pack = (uint4 *)(d + 2560);
+    unsigned *ext = (unsigned *)(d + 1792);
+    int *err = (int *)(d + 2048);
     float4 *pos = (float4 *)(d + 2304);
     cudaStream_t s = ctx->stream;
     cudaError_t e = cudaMemsetAsync(d, 0, bytes, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(inbox, 0xff, 256, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(table, table_h, sizeof(table_h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(start, start_h, sizeof(start_h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(nbr, nbr_h, sizeof(nbr_h), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, cnt_h, sizeof(cnt_h), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(remote, remote_h, sizeof(remote_h), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(home, home_h, sizeof(home_h), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(word0, word_h, sizeof(word_h), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pack, pack_h, sizeof(pack_h), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ext, ext_h, sizeof(ext_h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(pos, pos_h, sizeof(pos_h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = qses::launch_gs_slab(pos, 0, 4, 2, table, 2, tails + 2, home, 2, 512, 0, 0, start, nbr, cnt, remote, inbox,
-                                 tails, err, spin_cycles, nullptr, s);
+        e = qses::launch_gs_slab(pos, 0, 4, 2, table, 2, next_slab, 2, 512, start, nbr, word0, pack, ext, 1u, err,
+                                 spin_cycles, nullptr, s);
     int h_err = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

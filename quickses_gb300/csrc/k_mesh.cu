@@ -9,9 +9,8 @@
 //  k_weld_*       unique quantised positions in lexicographic order (CudaSurf.cu:444-457)
 //  k_closest      closest atom per welded vertex (closestAtomPerVertex, Kernels.cu:547-604)
 //  k_tri_*        drop triangles with a repeated index (CudaSurf.cu:820-829)
-//  k_csr_* / k_gs_setup  neighbour lists in triangle order (getNeighboorsVertices,
-//                 SmoothMesh.cpp:45-123) and the per-vertex dependency counts and slab homes
-//                 of the Gauss-Seidel dataflow (k_smooth.cu)
+//  k_csr_*        neighbour lists in triangle order (getNeighboorsVertices,
+//                 SmoothMesh.cpp:45-123) for the Gauss-Seidel dataflow (k_smooth.cu)
 #include <cfloat>
 #include <cstdlib>
 #include <cstring>
@@ -575,10 +574,7 @@ __global__ void k_tri_compact_batch(QBatch b, const unsigned *__restrict__ tri, 
 // Neighbour lists without a sort.  count: occurrences of each vertex among the 3T triangle
 // corners (start[v].x, later scanned); scatter: each corner q is written into its vertex's
 // range at a position taken with an atomic (start[v].y, zero after the scan), so the order
-// within a range is arbitrary; sortfill: one thread per vertex sorts its range by corner
-// index, which restores triangle order exactly (the order getNeighboorsVertices appends
-// in, SmoothMesh.cpp:45-66), writes the two other corners of each triangle to the list, and
-// doubles the offset (two entries per occurrence).
+// within a range is arbitrary (k_gs_lists sorts it).
 __global__ void k_csr_count(const unsigned *__restrict__ tri, size_t n3, uint2 *__restrict__ start) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n3) atomicAdd(&start[tri[q]].x, 1u);
@@ -591,93 +587,6 @@ __global__ void k_csr_scatter(const unsigned *__restrict__ tri, size_t n3, uint2
     const unsigned v = tri[q];
     const unsigned k = atomicAdd(&start[v].y, 1u);
     occ[start[v].x + k] = (unsigned)q;
-}
-
-// 12 resident CTAs per SM (at most 42 registers) instead of 9: the kernel waits on scattered
-// triangle reads, so more warps in flight hide them
-__global__ void __launch_bounds__(128, 12) k_csr_sortfill(const unsigned *__restrict__ tri, unsigned *__restrict__ occ, size_t n3, unsigned nv,
-                               uint2 *__restrict__ start, unsigned *__restrict__ nbr) {
-    const unsigned v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v > nv) return;
-    if (v == nv) {
-        start[nv] = make_uint2(2u * (unsigned)n3, 0u);
-        return;
-    }
-    const uint2 st = start[v];
-    const unsigned o = st.x, n = st.y;  // offset, occurrences
-    constexpr unsigned kReg = 16;
-    if (n <= kReg) {
-        unsigned r[kReg];
-#pragma unroll
-        for (unsigned i = 0; i < kReg; i++) r[i] = i < n ? occ[o + i] : 0xffffffffu;
-        // insertion sort in registers (n is small: ~6 incident triangles per vertex)
-#pragma unroll
-        for (unsigned i = 1; i < kReg; i++) {
-#pragma unroll
-            for (unsigned j = i; j > 0; j--) {
-                const unsigned a = r[j - 1], b = r[j];
-                r[j - 1] = min(a, b);
-                r[j] = max(a, b);
-            }
-        }
-#pragma unroll
-        for (unsigned i = 0; i < kReg; i++) {
-            if (i < n) {
-                const unsigned q = r[i], t = q / 3u, c = q - 3u * t;
-                const unsigned a = tri[3ull * t], b = tri[3ull * t + 1], d = tri[3ull * t + 2];
-                nbr[2ull * (o + i)] = c == 0 ? b : a;
-                nbr[2ull * (o + i) + 1] = c == 2 ? b : d;
-            }
-        }
-    } else {
-        // rare high-degree vertex: insertion sort in place in global memory
-        for (unsigned i = 1; i < n; i++) {
-            const unsigned x = occ[o + i];
-            unsigned j = i;
-            while (j > 0 && occ[o + j - 1] > x) {
-                occ[o + j] = occ[o + j - 1];
-                j--;
-            }
-            occ[o + j] = x;
-        }
-        for (unsigned i = 0; i < n; i++) {
-            const unsigned q = occ[o + i], t = q / 3u, c = q - 3u * t;
-            const unsigned a = tri[3ull * t], b = tri[3ull * t + 1], d = tri[3ull * t + 2];
-            nbr[2ull * (o + i)] = c == 0 ? b : a;
-            nbr[2ull * (o + i) + 1] = c == 2 ? b : d;
-        }
-    }
-    start[v] = make_uint2(2u * o, 0u);
-}
-
-// Per vertex: lower-id neighbour entries inside its slab (+1 if any lie in lower slabs),
-// the count of entries in lower slabs, and its home: slab id and the slab's first vertex.
-// Vertices [v0, v1) form the slabs of the table (Q, then Q + 1 bounds in id order).
-// Neighbours below v0 belong to waves that finished before this one (final values);
-// neighbours at or above v1 are read before their update.
-__global__ void k_gs_setup(const uint2 *__restrict__ start, const unsigned *__restrict__ nbr, unsigned v0,
-                           unsigned v1, const unsigned *__restrict__ table, unsigned short *__restrict__ cnt_local,
-                           int *__restrict__ remote, uint2 *__restrict__ home) {
-    unsigned v = v0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= v1) return;
-    const unsigned Q = __ldg(table);
-    const unsigned *bnd = table + 1;
-    unsigned lo = 0, hi = Q;  // bnd[lo] <= v < bnd[hi]
-    while (hi - lo > 1) {
-        const unsigned mid = (lo + hi) >> 1;
-        if (__ldg(bnd + mid) <= v) lo = mid; else hi = mid;
-    }
-    const unsigned a = __ldg(bnd + lo);
-    unsigned loc = 0, rem = 0;
-    for (unsigned e = start[v].x; e < start[v + 1].x; e++) {
-        const unsigned u = nbr[e];
-        if (u < v && u >= v0) {  // below v0: an earlier wave, already final
-            if (u >= a) loc++; else rem++;
-        }
-    }
-    cnt_local[v] = (unsigned short)min(loc + (rem ? 1u : 0u), 65535u);
-    remote[v] = (int)rem;
-    home[v] = make_uint2(lo, a);
 }
 
 __global__ void k_to_float4(const float *__restrict__ v3, unsigned nv, float4 *__restrict__ v4) {
@@ -779,14 +688,6 @@ void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, cudaStream_t
 }
 void launch_csr_scatter(const unsigned *tri, size_t n3, uint2 *start, unsigned *occ, cudaStream_t s) {
     k_csr_scatter<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, start, occ);
-}
-void launch_csr_sortfill(const unsigned *tri, unsigned *occ, size_t n3, unsigned nv, uint2 *start, unsigned *nbr,
-                         cudaStream_t s) {
-    k_csr_sortfill<<<nblk((size_t)nv + 1, 128), 128, 0, s>>>(tri, occ, n3, nv, start, nbr);
-}
-void launch_gs_setup(const uint2 *start, const unsigned *nbr, unsigned v0, unsigned v1, const unsigned *table,
-                     unsigned short *cnt_local, int *remote, uint2 *home, cudaStream_t s) {
-    k_gs_setup<<<nblk(v1 - v0, 256), 256, 0, s>>>(start, nbr, v0, v1, table, cnt_local, remote, home);
 }
 void launch_to_float4(const float *v3, unsigned nv, float4 *v4, cudaStream_t s) {
     k_to_float4<<<nblk(nv, 256), 256, 0, s>>>(v3, nv, v4);

@@ -1,7 +1,6 @@
 // Exact Gauss-Seidel Laplacian smoothing (SmoothMesh.cpp:45-123) as a dataflow over slabs of
 // vertex ids: a vertex is updated once every lower-id neighbour has been, exactly as the
 // sequential loop would see them.  Persistent CTAs take the slabs from a device work queue.
-#include <cstdlib>
 #include <cstring>
 
 #include "device_common.cuh"
@@ -10,577 +9,650 @@
 
 namespace qses {
 
-__device__ __forceinline__ int atom_sub_acq_rel(int *p, int v) {
-    int old;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(-v) : "memory");
+// Slab-partitioned Gauss-Seidel pass.  Vertex ids are split into contiguous slabs; every
+// dependency edge goes from a lower to a higher id, so a chain of updates crosses each slab
+// boundary at most once.  Inside a slab a vertex is one 16-byte record in shared memory - its
+// position and a word with its readiness counter and its list's length - so that a chain step is
+// one shared-memory gather, the sum, and one atomic per successor that returns all the next step
+// needs.  L2 is touched only for the neighbour list (one 64-byte line, asked for while its
+// vertex's lower neighbours are updated) and for neighbours in other slabs.
+//
+// What bounds it: the chain of dependent updates (5 332 levels on the 3 540 000-vertex mesh of
+// 50 000 atoms at 0.2 A), not bytes.  Measured on GB300 with one chain of updates in one slab, a
+// step takes 700 cycles - of them the gather, the rows and the sum in list order ~240, position
+// store and fence 35, the successors' atomics 45, choosing and fetching the next ~150 - 1 050
+// with a neighbour in another slab, and 500 more when the next vertex goes to another warp.  Per
+// level a whole pass took 1.86 us with a warp per vertex, counters in shared memory and positions
+// and lists in L2, and takes 1.0 us (9.89 -> 5.3 ms; 0.94 -> 0.41 ms on 30 000 vertices; 4.1 ->
+// 1.7 ms on a batch of 16 molecules).  A slab's SM is saturated at ~43 cycles per vertex.
+constexpr int kGsThreadsMax = 1024;
+constexpr int kGsRecvWarps = 2;  // warps that watch the lower slabs' releases
+constexpr unsigned kGsRow = 36;  // floats per component of a warp's row (32 used; offset banks)
+
+// Shared-memory layout of a slab of at most smax vertices (bytes).
+struct GsSmem {
+    unsigned rec, pend, ring, bytes;
+};
+__host__ __device__ constexpr GsSmem gs_smem(unsigned smax) {
+    GsSmem L{};
+    L.rec = 0;                                       // records, and one of -0 that past-the-end entries read
+    L.pend = L.rec + 16 * (smax + 1);                // 1 bit per vertex: waits for lower slabs
+    L.ring = L.pend + 4 * ((smax + 62) / 32 + 1);    // 16-bit slab offsets of ready vertices
+    L.bytes = (L.ring + 2 * (smax + 32) + 15) & ~15u;  // + one slot per warp past the last vertex
+    return L;
+}
+static_assert(gs_smem(kGsSlabCap).bytes + 15 * 1024 <= 227 * 1024, "a slab's state fits a CTA");
+
+// A record's word, built by k_gs_lists: bits 0-6 readiness counter (lower neighbours to come),
+// bit 7 one of them is in a lower slab, bit 8 the list has more than 16 entries.  Lists of up to 16
+// entries are at 16 v in the packed table, past-the-end entries naming record smax; bits 9-12 are
+// their length in pairs.  Longer lists are in the neighbour table: bits 9-14 their length in
+// pairs, bits 15-31 the offset in pairs from the slab's first entry, or kGsLost in bits 9-14 if
+// either does not fit (the offsets table has both).
+constexpr unsigned kGsPend = 0x80u, kGsLong = 0x100u, kGsLost = 63u;
+__device__ __forceinline__ unsigned gs_first(unsigned word) { return (word >> 15) * 2u; }
+__device__ __forceinline__ unsigned gs_len(unsigned word) { return ((word >> 9) & 63u) * 2u; }
+
+// List entries.  Bit 31: in another slab; bit 30: higher id than the list's vertex; bit 29: no
+// release (in a later wave, or named by an earlier entry of the list).  Below: the record (bit 31
+// clear) or the vertex id.
+constexpr unsigned kGsSucc = 2u, kGsFar = 6u;  // the top three bits of a successor here / in a higher slab
+
+__device__ __forceinline__ void fence_cta() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+
+// A vertex position with its pass stamp in w, read and written as one 16-byte access: the
+// stamp tells a reader whether the position is this pass's, so no fence orders the two.
+__device__ __forceinline__ float4 ld_pos(const float4 *p) {
+    float4 q;
+    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
+                 "ld.relaxed.gpu.global.b128 t, [%4];\n\t"
+                 "mov.b128 {lo, hi}, t;\n\tmov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+                 : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w)
+                 : "l"(p)
+                 : "memory");
+    return q;
+}
+__device__ __forceinline__ void ld_pos_if(float4 &q, const float4 *p, bool go) {
+    asm volatile("{\n\t.reg .pred g;\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\tsetp.ne.u32 g, %5, 0;\n\t"
+                 "mov.b64 lo, {%0, %1};\n\tmov.b64 hi, {%2, %3};\n\tmov.b128 t, {lo, hi};\n\t"
+                 "@g ld.relaxed.gpu.global.b128 t, [%4];\n\t"
+                 "mov.b128 {lo, hi}, t;\n\tmov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+                 : "+f"(q.x), "+f"(q.y), "+f"(q.z), "+f"(q.w)
+                 : "l"(p), "r"((unsigned)go)
+                 : "memory");
+}
+__device__ __forceinline__ void st_pos(float4 *p, float4 q, bool go = true) {
+    asm volatile("{\n\t.reg .pred g;\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\tsetp.ne.u32 g, %5, 0;\n\t"
+                 "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 t, {lo, hi};\n\t"
+                 "@g st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "f"(q.x), "f"(q.y), "f"(q.z), "f"(q.w), "r"((unsigned)go)
+                 : "memory");
+}
+
+// A record's position (its word may be counted down at the same time: a relaxed access).
+__device__ __forceinline__ float4 ld_rec(unsigned p) {
+    float4 q;
+    asm volatile("ld.relaxed.cta.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(p) : "memory");
+    return q;
+}
+__device__ __forceinline__ float ld_comp(unsigned p) {
+    float x;
+    asm volatile("ld.relaxed.cta.shared.f32 %0, [%1];" : "=f"(x) : "r"(p) : "memory");
+    return x;
+}
+__device__ __forceinline__ void st_comp(unsigned p, float x, bool go) {
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g st.relaxed.cta.shared.f32 [%0], %1;\n\t}" ::"r"(p), "f"(x),
+                 "r"((unsigned)go) : "memory");
+}
+// Counts the record at p down if `go`; the word before (0 if not).
+__device__ __forceinline__ unsigned dec_rec(unsigned p, bool go) {
+    unsigned old;
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\tmov.u32 %0, 0;\n\t"
+                 "@g atom.relaxed.cta.shared.add.u32 %0, [%1], -1;\n\t}"
+                 : "=&r"(old) : "r"(p + 12u), "r"((unsigned)go) : "memory");
     return old;
 }
 
-// Slab-partitioned Gauss-Seidel pass.  Vertex ids are split into P contiguous slabs, one
-// persistent CTA each.  Every dependency edge goes from a lower to a higher id, so a chain
-// of updates crosses each slab boundary at most once: readiness inside a slab is tracked
-// with shared-memory counters and a ring of ready vertices, and only boundary edges go
-// through global memory (an acquire/release counter per vertex and a per-slab inbox).
-// Each vertex is still computed exactly as the sequential loop would.
-constexpr int kGsSlabMaxSmem = 200 * 1024;  // dynamic part: offsets, packed counters, ring: 8 B/vertex
-                                            // (+ 16 B/vertex of positions with kGsSmemPos)
-__host__ __device__ constexpr size_t gs_spos_offset(unsigned smax) {
-    return ((4ull * (smax + 1) + 4ull * ((smax + 1) / 2) + 2ull * smax) + 15) & ~(size_t)15;
+// Asks for the sectors of a neighbour list without a register or a wait: an asynchronous copy
+// of one word per sector into scratch that nobody reads (prefetch.global.L1 brings nothing into
+// L1 on this GPU, and a plain load would be waited for by the next fence).
+__device__ __forceinline__ void touch_l1(unsigned scratch, const unsigned *p, bool go) {
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g cp.async.ca.shared.global [%0], [%1], 4;\n\t}" ::"r"(scratch),
+                 "l"(p), "r"((unsigned)go) : "memory");
 }
 
-// Two 16-bit readiness counters per shared word; returns the counter value before the
-// decrement.  Counters never go below zero, so no borrow crosses into the other half.
-__device__ __forceinline__ unsigned dec16(unsigned *w, unsigned k) {
-    const unsigned sh = 16u * (k & 1u);
-    return (atomicSub(&w[k >> 1], 1u << sh) >> sh) & 0xffffu;
+__device__ __forceinline__ void red_ext(unsigned *ext, unsigned u, bool go) {
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g red.relaxed.gpu.global.add.u32 [%0], %1;\n\t}" ::"l"(ext + (u >> 2)),
+                 "r"(0u - (1u << (8u * (u & 3u)))), "r"((unsigned)go) : "memory");
+}
+// This lane's entry of a list (what past-the-end entries read otherwise).
+__device__ __forceinline__ unsigned ld_entry(const unsigned *p, bool go, unsigned other) {
+    unsigned x = other;
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g ld.global.nc.u32 %0, [%1];\n\t}" : "+r"(x) : "l"(p), "r"((unsigned)go));
+    return x;
 }
 
-__device__ __forceinline__ void ring_push16(volatile unsigned short *ring, unsigned *tail, unsigned off) {
-    const unsigned k = atomicAdd(tail, 1u);
-    ring[k] = (unsigned short)off;  // each vertex enters the ring once: no wrap-around
+// s / n for a whole n in [1, 126] with rn = 1/n correctly rounded: one multiplication and one
+// correction by the exact residual give the correctly rounded quotient (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990; checked for every
+// mantissa and every n up to 1 024) unless the quotient is subnormal (gs_tiny: it may be).
+__device__ __forceinline__ float gs_div(float s, float n, float rn) {
+    const float q = __fmul_rn(s, rn);
+    return __fmaf_rn(__fmaf_rn(-q, n, s), rn, q);
+}
+__device__ __forceinline__ bool gs_tiny(float s) {  // 0 < |s| < 2^-100 (zero wraps round)
+    return 2u * __float_as_uint(s) - 1u < 2u * 0x0d800000u - 1u;
 }
 
-constexpr unsigned kGsOutbox = 1024;  // shared-memory queue of cross-slab releases
-
-__device__ __forceinline__ void prefetch_l2(const void *p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+// The slab's ready vertices: a ring in shared memory.  An idle warp takes the next ticket and
+// watches the ring's slot of that number, so a vertex goes to the warp that has waited longest
+// without any of them contending for it.
+struct __align__(16) GsQueue {
+    unsigned ticket, tail, done, stop;
+};
+__device__ __forceinline__ uint2 ld_queue(unsigned p) {  // ticket, tail
+    uint2 x;
+    asm volatile("ld.relaxed.cta.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x.x), "=r"(x.y) : "r"(p) : "memory");
+    return x;
 }
-__device__ __forceinline__ void prefetch_l1(const void *p) {
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+constexpr unsigned kGsEmpty = 0xffffu, kGsQuit = 0xfffeu;  // ring slots that hold no slab offset
+
+// Each vertex enters the ring at most once: no wrap-around.  In two halves, so that a step can do
+// other work between taking the slot and filling it; predicated, as a branch would end its block.
+__device__ __forceinline__ unsigned gs_slot(unsigned tail, bool go) {
+    unsigned t = 0;
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g atom.relaxed.cta.shared.add.u32 %0, [%1], 1;\n\t}"
+                 : "+r"(t) : "r"(tail), "r"((unsigned)go) : "memory");
+    return t;
+}
+__device__ __forceinline__ void gs_fill(unsigned ring, unsigned slot, unsigned k, bool go) {
+    asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g st.relaxed.cta.shared.u16 [%0], %1;\n\t}" ::"r"(ring + 2 * slot),
+                 "h"((unsigned short)k), "r"((unsigned)go) : "memory");
+}
+__device__ __forceinline__ void gs_push(unsigned tail, unsigned ring, unsigned k, bool go) {
+    gs_fill(ring, gs_slot(tail, go), k, go);
+}
+
+__device__ __forceinline__ float add4(float s, float4 q) {
+    return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, q.x), q.y), q.z), q.w);
 }
 
 // Persistent CTAs take the wave's slabs from a counter, in the table's order (a slab only
 // waits for slabs taken before it, by CTAs that were running when they took them, so every
-// wait ends without a co-residency guarantee).  Per slab,
-// warp 0 takes boundary arrivals from lower slabs, warp 1 sends this slab's cross-slab
-// releases (GPU-scope atomics, off the workers' critical path), the other warps update
-// vertices.  Table: Q, the Q + 1 slab bounds in id order (qcap + 1 slots), then the Q slab ids
-// in the order they are taken.
-template <int kGsT, unsigned kFlags>
-__global__ void __launch_bounds__(kGsT, kGsT <= 512 ? 2 : 1) k_gs_flow(float4 *pos4, unsigned v0, unsigned nv, unsigned smax,
-                                                  const unsigned *__restrict__ table, unsigned qcap,
-                                                  unsigned *next_slab, const uint2 *__restrict__ home,
-                                                  const uint2 *__restrict__ start, const unsigned *__restrict__ nbr,
-                                                  const unsigned short *__restrict__ cnt_local, int *remote,
-                                                  unsigned *inbox, unsigned *inbox_tail, int *err,
-                                                  long long spin_cycles, unsigned long long *stats,
-                                                  unsigned idle_ns_max, unsigned hot_warps) {
-    extern __shared__ unsigned s_dyn[];
-    __shared__ unsigned s_head, s_tail, s_done, s_stop, s_ob_head, s_ob_tail, s_slab;
-    __shared__ unsigned s_ob[kGsOutbox];
-    // Per worker warp: one row of neighbour positions, summed in list order by lane 0 (of
-    // each lane group): one shared-memory round trip, then a chain of adds in registers,
-    // instead of a shuffle per entry.
-    __shared__ float4 s_stage[kGsT / 32][32];
-    unsigned *st = s_dyn;                                        // len + 1 CSR offsets of the slab
-    unsigned *cnt = s_dyn + (smax + 1);                          // (len + 1) / 2 words: packed counters
-    volatile unsigned short *ring = (volatile unsigned short *)(cnt + (smax + 1) / 2);  // slab offsets
-    // kGsSmemPos: the slab's positions (old until a vertex updates, then new), so neighbours
-    // inside the slab are read from shared memory; others from global memory as before
-    constexpr bool kSP = (kFlags & kGsSmemPos) != 0;
-    // lanes per vertex update: 32 (one vertex per worker warp), or 16 / 8 with kGsPair /
-    // kGsQuad (2 / 4 ready vertices per worker warp, one lane group each)
-    constexpr unsigned kLanes = (kFlags & kGsQuad) ? 8u : (kFlags & kGsPair) ? 16u : 32u;
-    float4 *spos = (float4 *)((char *)s_dyn + gs_spos_offset(smax));
-    volatile unsigned *ob = s_ob;
+// wait ends without a co-residency guarantee).  Per slab the first two warps watch the release
+// counters that lower slabs decrement (ext, one byte per vertex: neighbour entries in lower
+// slabs still to come), the other warps update vertices.
+// Table: Q, the Q + 1 slab bounds in id order (qcap + 1 slots), then the Q slab ids in the
+// order they are taken.
+__global__ void __launch_bounds__(kGsThreadsMax, 1)
+    k_gs_flow(float4 *pos4, unsigned v0, unsigned nv, unsigned smax, const unsigned *__restrict__ table, unsigned qcap,
+              unsigned *next_slab, const uint2 *__restrict__ start, const unsigned *__restrict__ nbr,
+              const unsigned *__restrict__ word0, const unsigned *__restrict__ pack, unsigned *ext, unsigned stamp, int *err,
+              long long spin_cycles, unsigned long long *stats) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ GsQueue s_q;
+    __shared__ unsigned s_slab;
+    // Per worker warp: the neighbours' coordinates, one row per component, summed in list order
+    __shared__ __align__(16) float s_row[kGsThreadsMax / 32][3 * kGsRow];
+    __shared__ unsigned s_void[32];  // target of touch_l1
+    __shared__ float2 s_rcp[16];  // a packed list's length in pairs -> length, its reciprocal
+    const GsSmem L = gs_smem(smax);
+    float4 *rec = (float4 *)(s_dyn + L.rec);
+    unsigned *pend = (unsigned *)(s_dyn + L.pend);
+    volatile unsigned short *ring = (volatile unsigned short *)(s_dyn + L.ring);
+    const unsigned rec_s = (unsigned)__cvta_generic_to_shared(rec), ring_s = (unsigned)__cvta_generic_to_shared(s_dyn + L.ring);
+    const unsigned queue_s = (unsigned)__cvta_generic_to_shared(&s_q), tail_s = queue_s + 4;
+    const unsigned T = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned Q = min(__ldg(table), qcap);
     const unsigned *bnd = table + 1, *order = table + 2 + qcap;
-    const unsigned lane = threadIdx.x & 31;
-    // longest sleep of this warp when idle: the first hot_warps worker warps poll the ring
-    // every 64 ns at most, so a vertex pushed there is picked up without waiting for a
-    // warp that backed off to idle_ns_max
-    const unsigned idle_cap = (threadIdx.x >> 5) < 2u + hot_warps ? min(64u, idle_ns_max) : idle_ns_max;
-    unsigned long long cyc_update = 0, cyc_release = 0, nproc = 0, polls = 0, cyc_ids = 0, cyc_pos = 0, cyc_fence = 0;
-    if (threadIdx.x == 0) s_stop = 0;
-    for (;;) {
+    volatile unsigned *v_done = &s_q.done, *v_stop = &s_q.stop;
+    const float fstamp = __uint_as_float(stamp);
+    const unsigned v_scratch = (unsigned)__cvta_generic_to_shared(&s_void[lane]);
+    unsigned long long polls = 0;
     if (threadIdx.x == 0) {
-        const unsigned k = atomicAdd(next_slab, 1u);
-        s_slab = (k < Q && !s_stop) ? __ldg(order + k) : 0xffffffffu;
-        s_head = 0; s_tail = 0; s_done = 0; s_ob_head = 0; s_ob_tail = 0;
+        s_q.stop = 0;
+        rec[smax] = make_float4(-0.0f, -0.0f, -0.0f, 0.0f);
     }
-    __syncthreads();
-    const unsigned p = s_slab;
-    if (p >= Q) break;  // uniform per CTA: no slab left (or an error stopped this CTA)
-    const unsigned a = __ldg(bnd + p), b = __ldg(bnd + p + 1), len = b - a;
-    if (a < v0 || b > nv || b <= a || len > smax) {  // uniform: a malformed table entry
-        if (threadIdx.x == 0) raise_error(err, QSES_ERR_INTERNAL);
-        break;
-    }
-    unsigned *box = inbox + (a - v0);                            // boundary arrivals from lower slabs
-    for (unsigned k = threadIdx.x; k < kGsOutbox; k += kGsT) s_ob[k] = 0xffffffffu;
-    for (unsigned k = threadIdx.x; k <= len; k += kGsT) st[k] = start[a + k].x;
-    for (unsigned k = threadIdx.x; k < len; k += kGsT) ring[k] = 0xffffu;
-    if (kSP)
-        for (unsigned k = threadIdx.x; k < len; k += kGsT) spos[k] = __ldcg(pos4 + a + k);
-    for (unsigned k = threadIdx.x; 2 * k < len; k += kGsT) {
-        const unsigned lo = cnt_local[a + 2 * k], hi = 2 * k + 1 < len ? cnt_local[a + 2 * k + 1] : 0u;
-        cnt[k] = lo | (hi << 16);
-    }
-    __syncthreads();
-    for (unsigned k = threadIdx.x; k < len; k += kGsT)
-        if (cnt_local[a + k] == 0) ring_push16(ring, &s_tail, k);
-    __syncthreads();
+    if (threadIdx.x < 16) s_rcp[threadIdx.x] = make_float2(2.0f * threadIdx.x, __frcp_rn(2.0f * threadIdx.x));
+    for (;;) {
+        if (threadIdx.x == 0) {
+            const unsigned k = atomicAdd(next_slab, 1u);
+            s_slab = (k < Q && !s_q.stop) ? __ldg(order + k) : 0xffffffffu;
+            s_q.ticket = 0; s_q.tail = 0; s_q.done = 0;
+        }
+        __syncthreads();
+        const unsigned p = s_slab;
+        if (p >= Q) break;  // uniform per CTA: no slab left (or an error stopped this CTA)
+        const unsigned a = __ldg(bnd + p), b = __ldg(bnd + p + 1), len = b - a;
+        if (a < v0 || b > nv || b <= a || len > smax) {  // uniform: a malformed table entry
+            if (threadIdx.x == 0) raise_error(err, QSES_ERR_INTERNAL);
+            break;
+        }
+        const unsigned a32 = a & ~31u, nword = (b - a32 + 31) / 32;  // words of ext bytes and pend bits
+        const unsigned *list = nbr + 2 * (size_t)start[a].x;
+        const unsigned *packs = pack + 16 * (size_t)a;
+        for (unsigned k = threadIdx.x; k < len; k += T) {
+            float4 q = ld_pos(pos4 + a + k);
+            q.w = __uint_as_float(word0[a + k] & ~kGsPend);
+            rec[k] = q;
+        }
+        for (unsigned k = threadIdx.x; k < len + 32; k += T) ring[k] = kGsEmpty;
+        for (unsigned w = warp; w < nword; w += T / 32) {
+            const unsigned v = a32 + 32 * w + lane;
+            const unsigned m = __ballot_sync(0xffffffffu, v >= a && v < b && (word0[v] & kGsPend));
+            if (lane == 0) pend[w] = m;
+        }
+        __syncthreads();
+        for (unsigned k = threadIdx.x; k < len; k += T)
+            gs_push(tail_s, ring_s, k, (word0[a + k] & 0x7fu) == 0);
+        __syncthreads();
 
-    if (threadIdx.x < 32) {
-        // Warp 0 only takes boundary arrivals (the last lower-slab dependency of a vertex
-        // finished); it never updates vertices, so arrivals are never stuck behind a chain.
-        if (lane == 0) {
-            unsigned seen = 0, done_seen = 0;
+        if (warp < kGsRecvWarps) {
+            // Receivers never update vertices, so arrivals are never stuck behind a chain.  A lane
+            // watches 32 vertices at a time: the bytes of those still waiting; a byte at zero means
+            // that every neighbour in a lower slab has been updated.
+            unsigned idle_ns = 0, done_seen = 0;
             long long last = clock64();
             for (;;) {
-                if (*(volatile unsigned *)&s_done >= len || *(volatile unsigned *)&s_stop) break;
-                const unsigned tail = min(ld_acquire_u32(inbox_tail + p), len);
+                const unsigned d = *v_done;
+                if (__any_sync(0xffffffffu, d >= len || *v_stop)) break;
                 polls++;
-                for (unsigned k = seen; k < tail; k++) {
-                    unsigned u = 0xffffffffu;
-                    for (unsigned it = 0; it < (1u << 20) && u == 0xffffffffu; it++) u = ld_acquire_u32(box + k);
-                    if (u < a || u >= b) {
-                        raise_error(err, u == 0xffffffffu ? QSES_ERR_TIMEOUT : QSES_ERR_INTERNAL);
-                        s_stop = 1;
-                        break;
+                bool any = false, left = false;
+                for (unsigned w = warp * 32 + lane; w < nword; w += 32 * kGsRecvWarps) {
+                    const unsigned m = pend[w];
+                    if (!m) continue;
+                    const unsigned *e = ext + (a32 >> 2) + 8 * w;
+                    unsigned x[8], zero = 0;
+                    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "l"(e) : "memory");
+                    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]) : "l"(e + 4) : "memory");
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        // 0x80 in each zero byte, then one bit per byte (the products do not overlap)
+                        const unsigned z = ~(((x[j] & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x[j] | 0x7f7f7f7fu);
+                        zero |= ((((z >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * j);
                     }
-                    __threadfence_block();
-                    if (dec16(cnt, u - a) == 1u) ring_push16(ring, &s_tail, u - a);
+                    unsigned now = zero & m;
+                    pend[w] = m & ~now;
+                    left |= (m & ~now) != 0;
+                    any |= now != 0;
+                    for (; now; now &= now - 1) {
+                        const unsigned k = a32 + 32 * w + (__ffs(now) - 1) - a;
+                        const bool go = (dec_rec(rec_s + 16 * k, true) & 0x7fu) == 1u;
+                        fence_cta();  // the neighbours' positions before the ring entry
+                        gs_push(tail_s, ring_s, k, go);
+                    }
                 }
+                any = __any_sync(0xffffffffu, any);
+                left = __any_sync(0xffffffffu, left);
+                if (!left) break;  // nobody here waits for a lower slab any more
                 const long long now = clock64();
-                const unsigned d = *(volatile unsigned *)&s_done;
-                if (tail != seen || d != done_seen) last = now;
-                seen = tail;
+                if (any || d != done_seen) last = now;
                 done_seen = d;
                 if (now - last > spin_cycles) {
-                    raise_error(err, QSES_ERR_TIMEOUT);
-                    s_stop = 1;
-                }
-                if (tail == seen) __nanosleep(20);
-            }
-        }
-    } else if (threadIdx.x < 64) {
-        // Warp 1 sends cross-slab releases queued by the workers, up to 32 at a time.  A
-        // worker queues an entry after its position store and a CTA-scope fence; the fence
-        // here plus the GPU-scope acq_rel atomic carry that store to the receiving slab.
-        unsigned head = 0;
-        for (;;) {
-            const unsigned tail = *(volatile unsigned *)&s_ob_tail;
-            const unsigned count = min(tail - head, 32u);
-            if (count == 0) {
-                if (*(volatile unsigned *)&s_stop) break;
-                if (*(volatile unsigned *)&s_done >= len) {
-                    __threadfence_block();
-                    if (*(volatile unsigned *)&s_ob_tail == head) break;  // every worker is done
-                    continue;
-                }
-                __nanosleep(20);
-                continue;
-            }
-            if (lane < count) {
-                volatile unsigned *slot = ob + (head + lane) % kGsOutbox;
-                unsigned u = 0xffffffffu;
-                for (unsigned it = 0; it < (1u << 20) && u == 0xffffffffu; it++) u = *slot;  // reserved slot
-                if (u == 0xffffffffu || u < b || u >= nv) {
-                    raise_error(err, u == 0xffffffffu ? QSES_ERR_TIMEOUT : QSES_ERR_INTERNAL);
-                    s_stop = 1;
-                } else {
-                    *slot = 0xffffffffu;
-                    __threadfence_block();
-                    const uint2 h = __ldg(home + u);  // u's slab and its first vertex (constant)
-                    if (atom_sub_acq_rel(remote + u, 1) == 1) {
-                        // last lower-slab dependency of u: hand u to its slab
-                        const unsigned k = atomicAdd(inbox_tail + h.x, 1u);
-                        if (k < smax && h.x < Q) st_release_u32(inbox + (h.y - v0) + k, u);
-                    }
-                }
-            }
-            head += count;
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence_block();
-                *(volatile unsigned *)&s_ob_head = head;  // slots before head are free again
-            }
-        }
-    } else if constexpr (kLanes == 32) {
-        // Worker warps: one vertex per warp; lanes fetch neighbours in parallel.  An idle
-        // worker backs off (32 ns doubling up to idle_ns_max, 1 us by default): a hot polling loop of up to
-        // 30 warps would take issue slots and shared-memory bandwidth from the warps on the
-        // critical path.
-        unsigned idle_ns = 0;
-        for (;;) {
-            unsigned v = 0xffffffffu, quit = 0;
-            if (lane == 0) {
-                const unsigned h = *(volatile unsigned *)&s_head, t = *(volatile unsigned *)&s_tail;
-                if (h < t && atomicCAS(&s_head, h, h + 1) == h) {
-                    unsigned off = 0xffffu;
-                    for (unsigned it = 0; it < (1u << 20) && off == 0xffffu; it++) off = ring[h];  // reserved slot
-                    if (off == 0xffffu) {
-                        raise_error(err, QSES_ERR_TIMEOUT);
-                        s_stop = 1;
-                    } else {
-                        v = a + off;
-                    }
-                } else if (h >= t) {
-                    quit = (*(volatile unsigned *)&s_done >= len) || *(volatile unsigned *)&s_stop;
-                }
-            }
-            v = __shfl_sync(0xffffffffu, v, 0);
-            quit = __shfl_sync(0xffffffffu, quit, 0);
-            if (quit) break;
-            if (v == 0xffffffffu) {
-                idle_ns = idle_ns ? min(2 * idle_ns, idle_cap) : 32u;
-                __nanosleep(idle_ns);
-                continue;
-            }
-            idle_ns = 0;
-            // Neighbour ids of the vertex this warp continues with, loaded as soon as the
-            // release picked it (the lists are constant, so the early load is always valid).
-            unsigned pre_v = 0xffffffffu, pre_id = 0u;
-            while (v != 0xffffffffu) {  // follow the chain of vertices this warp releases
-                __threadfence_block();
-                const long long c0 = clock64();
-                const unsigned e0 = st[v - a], e1 = st[v - a + 1];
-                float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-                unsigned first_id = v;
-                for (unsigned base = e0; base < e1; base += 32) {
-                    const unsigned m = min(32u, e1 - base);
-                    const unsigned id = (base == e0 && pre_v == v) ? pre_id
-                                                                  : (lane < m ? __ldg(nbr + base + lane) : v);
-                    if (base == e0) first_id = id;
-                    long long ca = 0;
-                    if (stats && base == e0) {  // diagnostics: when the ids have arrived (the mov waits for them)
-                        unsigned t;
-                        asm volatile("mov.b32 %0, %1;" : "=r"(t) : "r"(id));
-                        ca = clock64();
-                        cyc_ids += ca - c0 + (t & 0u);
-                    }
-                    // Weak loads either way: the CTA- and GPU-scope acquires above order them.
-                    float4 q;
-                    if (kSP && id - a < len) q = spos[id - a];
-                    else q = (kFlags & kGsL1Positions) ? pos4[id] : __ldcg(pos4 + id);
-                    if (stats && base == e0) {  // ... and their positions
-                        float t;
-                        asm volatile("mov.b32 %0, %1;" : "=f"(t) : "f"(q.x));
-                        cyc_pos += clock64() - ca + (t != t ? 1 : 0);
-                    }
-                    // strictly in neighbour-list order, by lane 0 from the warp's row
-                    float4 *row = s_stage[threadIdx.x >> 5];
-                    if (lane < m) row[lane] = q;
-                    __syncwarp();
                     if (lane == 0) {
-#pragma unroll 4
-                        for (unsigned k = 0; k < m; k++) {
-                            const float4 p = row[k];
-                            sx = __fadd_rn(sx, p.x);
-                            sy = __fadd_rn(sy, p.y);
-                            sz = __fadd_rn(sz, p.z);
-                        }
+                        raise_error(err, QSES_ERR_TIMEOUT);
+                        *v_stop = 1;
                     }
-                    __syncwarp();  // the row is rewritten by the next chunk or vertex
+                    break;
                 }
-                const float n = (float)(int)(e1 - e0);
-                if (lane == 0) {
-                    const float4 np = make_float4(__fdiv_rn(sx, n), __fdiv_rn(sy, n), __fdiv_rn(sz, n), 0.0f);
-                    long long cs = 0;
-                    if (stats) {  // diagnostics: the store and its fence (the movs wait for the sums)
-                        float t0, t1, t2;
-                        asm volatile("mov.b32 %0, %3; mov.b32 %1, %4; mov.b32 %2, %5;"
-                                     : "=f"(t0), "=f"(t1), "=f"(t2) : "f"(np.x), "f"(np.y), "f"(np.z));
-                        cs = clock64() + (t0 != t0 || t1 != t1 || t2 != t2 ? 1 : 0);
-                    }
-                    if (kSP) spos[v - a] = np;
-                    __stcg(pos4 + v, np);
-                    // Successors in this slab read the new position after a CTA-scope
-                    // acquire; successors in higher slabs get it through the sender warp.
-                    __threadfence_block();
-                    if (stats) cyc_fence += clock64() - cs;
-                }
-                const long long c1 = clock64();
-                __syncwarp();
-                // Release: one lane per neighbour entry.
-                unsigned next = 0xffffffffu;
-                for (unsigned base = e0; base < e1; base += 32) {
-                    const unsigned m = min(32u, e1 - base);
-                    const unsigned u = lane < m ? (base == e0 ? first_id : __ldg(nbr + base + lane)) : 0u;
-                    // successors at or above nv (the wave's end) belong to a later wave, which
-                    // starts after this one has finished: nothing to release for them
-                    const bool higher = lane < m && u > v && u < nv;
-                    const bool remote_edge = higher && u >= b;
-                    bool ready = false;
-                    if (higher) {
-                        if (!remote_edge) {
-                            // u's list, needed when u runs
-                            if (kFlags & kGsL1Prefetch) prefetch_l1(nbr + st[u - a]);
-                            else prefetch_l2(nbr + st[u - a]);
-                            ready = dec16(cnt, u - a) == 1u;
-                        } else {
-                            const unsigned k = atomicAdd(&s_ob_tail, 1u);
-                            unsigned it = 0;
-                            for (; it < (1u << 22) && k - *(volatile unsigned *)&s_ob_head >= kGsOutbox; it++)
-                                __nanosleep(32);
-                            if (k - *(volatile unsigned *)&s_ob_head >= kGsOutbox) {
-                                raise_error(err, QSES_ERR_TIMEOUT);
-                                s_stop = 1;
-                            } else {
-                                __threadfence_block();  // release: the position store before the entry
-                                ob[k % kGsOutbox] = u;
-                            }
-                        }
-                    }
-                    unsigned mask = __ballot_sync(0xffffffffu, ready);
-                    if (mask && next == 0xffffffffu) {
-                        const unsigned f = __ffs(mask) - 1;
-                        next = __shfl_sync(0xffffffffu, u, f);  // continue with it directly
-                        mask &= ~(1u << f);
-                        const unsigned ne0 = st[next - a], nm = min(32u, st[next - a + 1] - ne0);
-                        pre_id = lane < nm ? __ldg(nbr + ne0 + lane) : next;
-                        pre_v = next;
-                    }
-                    if ((mask >> lane) & 1u) ring_push16(ring, &s_tail, u - a);
-                }
-                __syncwarp();  // queued releases precede the done count the sender checks
-                if (lane == 0) atomicAdd(&s_done, 1u);
-                v = next;
-                const long long c2 = clock64();
-                cyc_update += c1 - c0;
-                cyc_release += c2 - c1;
-                nproc++;
+                idle_ns = any ? 0u : min(idle_ns + 20u, 200u);
+                if (idle_ns) __nanosleep(idle_ns);
             }
-        }
-    } else {
-        // Worker warps of 32 / kLanes lane groups.  Ready vertices never depend on one another
-        // (a vertex is ready only once every lower-id neighbour has been updated), so the
-        // groups of a warp update different ready vertices in the same instructions; each
-        // group keeps its vertex's in-order sum (shuffles of width kLanes) and follows the
-        // chain of vertices it releases, and a group without a vertex takes one from the
-        // ring at the top of each step.
-        constexpr unsigned kGroups = 32u / kLanes;
-        constexpr unsigned kLow = (1u << kLanes) - 1u;
-        constexpr unsigned kLeaders = kGroups == 2 ? 0x00010001u : 0x01010101u;  // lane 0 of each group
-        const unsigned gl = lane % kLanes, g0 = lane - gl;  // lane in the group, the group's lane 0
-        unsigned idle_ns = 0;
-        unsigned v = 0xffffffffu;  // this group's vertex
-        unsigned pre_v = 0xffffffffu, pre_id[2] = {0u, 0u};
-        for (;;) {
-            const unsigned empty = __ballot_sync(0xffffffffu, gl == 0 && v == 0xffffffffu);
-            if (empty) {
-                unsigned got = 0, h0 = 0, quit = 0;
-                if (lane == 0) {
-                    const unsigned h = *(volatile unsigned *)&s_head, t = *(volatile unsigned *)&s_tail;
-                    if (h < t) {
-                        const unsigned k = min((unsigned)__popc(empty), t - h);
-                        if (atomicCAS(&s_head, h, h + k) == h) {
-                            got = k;
-                            h0 = h;
-                        }
-                    } else if (empty == kLeaders) {  // no group has a vertex
-                        quit = (*(volatile unsigned *)&s_done >= len) || *(volatile unsigned *)&s_stop;
-                    }
-                }
-                got = __shfl_sync(0xffffffffu, got, 0);
-                h0 = __shfl_sync(0xffffffffu, h0, 0);
-                if (__shfl_sync(0xffffffffu, quit, 0)) break;
-                if (gl == 0 && v == 0xffffffffu) {
-                    const unsigned r = __popc(empty & ((1u << lane) - 1u));  // empty groups before this one
-                    if (r < got) {
-                        unsigned off = 0xffffu;
-                        for (unsigned it = 0; it < (1u << 20) && off == 0xffffu; it++) off = ring[h0 + r];  // reserved slot
-                        if (off == 0xffffu) {
+            // The workers' own wait for a vertex ends with the slab or an error; it is watched here
+            // once no arrival is expected any more.
+            if (warp == 0) {
+                long long since = clock64();
+                unsigned seen = *v_done;
+                while (true) {
+                    const unsigned d = *v_done;
+                    if (__any_sync(0xffffffffu, d >= len || *v_stop)) break;
+                    const long long now = clock64();
+                    if (d != seen) since = now;
+                    seen = d;
+                    if (now - since > spin_cycles) {
+                        if (lane == 0) {
                             raise_error(err, QSES_ERR_TIMEOUT);
-                            s_stop = 1;
-                        } else {
-                            v = a + off;
+                            *v_stop = 1;
                         }
+                        break;
                     }
+                    __nanosleep(500);
                 }
-                v = __shfl_sync(0xffffffffu, v, g0);
             }
-            const unsigned busy = __ballot_sync(0xffffffffu, gl == 0 && v != 0xffffffffu);
-            if (!busy) {
-                idle_ns = idle_ns ? min(2 * idle_ns, idle_cap) : 32u;
-                __nanosleep(idle_ns);
-                continue;
-            }
-            idle_ns = 0;
-            __threadfence_block();
-            const long long c0 = clock64();
-            const bool act = v != 0xffffffffu;
-            const unsigned e0 = act ? st[v - a] : 0u, nlen = act ? st[v - a + 1] - e0 : 0u;
-            const unsigned maxlen = __reduce_max_sync(0xffffffffu, nlen);
-            // Rounds of two chunks of kLanes entries: both chunks' ids, then both chunks'
-            // positions are in flight before the in-order sum (lists of up to 2 kLanes
-            // entries take one round trip for each, as a whole warp's 32 lanes do).
-            float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-            unsigned first_id[2] = {0u, 0u};
-            for (unsigned r0 = 0; r0 < maxlen; r0 += 2 * kLanes) {
-                unsigned id[2];
-                float4 q[2];
-#pragma unroll
-                for (unsigned j = 0; j < 2; j++) {
-                    const unsigned o = r0 + j * kLanes + gl;
-                    id[j] = o >= nlen ? 0u : (r0 == 0 && pre_v == v) ? pre_id[j] : __ldg(nbr + e0 + o);
-                }
-#pragma unroll
-                for (unsigned j = 0; j < 2; j++) {
-                    // weak loads: the CTA- and GPU-scope acquires order them; lanes past the
-                    // list load nothing (their slots are not summed)
-                    q[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (r0 + j * kLanes + gl < nlen) {
-                        if (kSP && id[j] - a < len) q[j] = spos[id[j] - a];
-                        else q[j] = (kFlags & kGsL1Positions) ? pos4[id[j]] : __ldcg(pos4 + id[j]);
+        } else {
+            // Worker warps: a vertex per half warp, and on along the chain of vertices it releases.
+            // The second half is in use only while more vertices are ready than warps wait for: 28
+            // chains in a slab take 1 210 cycles a step on 14 warps that pair them, 1 850 on 28 that do
+            // not (the shared-memory pipe is the limit, and a pair shares its instructions).  `i`,
+            // `word` and `act` are a half's vertex at hand and whether there is one, `code` the lane's
+            // entry of its list.
+            float *row = s_row[warp];
+            const unsigned hl = lane & 15u, half = lane & 16u;
+            const float4 *crow = (const float4 *)(row + kGsRow * min(hl, 2u) + half);  // lanes past 2 repeat z
+            const unsigned comp = rec_s + 4 * min(hl, 2u);
+            unsigned i = smax, word = 0, code = smax, done = 0;
+            bool act = false;
+            // The step of the halves' vertices: sums, divisions, positions, then their successors of this
+            // slab counted down; one that a half makes ready is its next vertex, others go to the ring.
+            // The lists of all successors are asked for, for the steps that run them.  Halves that
+            // `odd` says need more (a position still on its way, a quotient that may be subnormal)
+            // release nothing and keep their vertex.  No branch: the step is one basic block (a branch
+            // in it, taken or not, cost it 80-110 cycles), with predicated accesses instead.
+            auto step = [&](bool &odd, bool &surplus) {
+                const float2 fr = s_rcp[(word >> 9) & 15u];
+                float4 q = ld_rec(rec_s + 16 * min(code & 0x1fffffffu, smax));
+                touch_l1(v_scratch, packs + 16 * (code & 0xffffu) + ((code >> 29) & 1u) * 8, (code >> 30) == 1u);
+                const uint2 qt = ld_queue(queue_s);
+                // Neighbours in other slabs: positions of this pass below (a release may overtake its
+                // position), of the last one above.
+                ld_pos_if(q, pos4 + (code & 0x1fffffffu), (int)code < 0);
+                const bool stale = (code >> 30) == 2u && __float_as_uint(q.w) != stamp;
+                row[lane] = q.x; row[kGsRow + lane] = q.y; row[2 * kGsRow + lane] = q.z;
+                __syncwarp();
+                // Strictly in list order; entries past the list are -0: adding them changes no sum.
+                const float4 q0 = crow[0], q1 = crow[1], q2 = crow[2], q3 = crow[3];
+                const float sum = add4(add4(add4(add4(0.0f, q0), q1), q2), q3);
+                odd = ((__ballot_sync(0xffffffffu, stale || gs_tiny(sum)) >> half) & 0xffffu) != 0u;
+                st_comp(comp + 16 * i, gs_div(sum, fr.x, fr.y), hl < 3 && act && !odd);
+                __syncwarp();
+                fence_cta();  // release: the position before the counters
+                const unsigned k = code & 0xffffu, old = dec_rec(rec_s + 16 * k, (code >> 29) == kGsSucc && !odd);
+                const bool now = (old & 0x7fu) == 1u;
+                const unsigned ready = (__ballot_sync(0xffffffffu, now) >> half) & 0xffffu;
+                // Successors in higher slabs (none that belong to a later wave, which starts after this
+                // one): the position for all, then their counters.
+                const bool far = (code >> 29) == kGsFar && !odd;
+                float4 r = ld_rec(rec_s + 16 * i);
+                fence_cta();  // acquire: the next vertex's other neighbours
+                const unsigned f = (31u - __clz(ready)) + half;
+                const unsigned slot = gs_slot(tail_s, now && lane != f);
+                const unsigned ni = __shfl_sync(0xffffffffu, k, f), nw = __shfl_sync(0xffffffffu, old, f);
+                r.w = fstamp;
+                st_pos(pos4 + a + i, r, far);  // every such lane the same
+                red_ext(ext, code & 0x1fffffffu, far);
+                done += act && !odd ? 1u : 0u;
+                act = act && (odd || ready);
+                i = ready ? ni : i;
+                word = ready ? nw : word;
+                code = ld_entry(packs + 16 * i + hl, act && !odd && !(word & kGsLong), odd ? code : smax);
+                gs_fill(ring_s, slot, k, now && lane != f);
+                surplus = !act && (int)(qt.y - qt.x) > 0;  // more vertices ready than warps wait for, and a half free
+            };
+            for (;;) {
+                // Nothing at hand: wait for a vertex (the ring's slot of this warp's ticket).
+                unsigned t = 0;
+                if (lane == 0) t = atomicAdd(&s_q.ticket, 1u);
+                t = min(__shfl_sync(0xffffffffu, t, 0), len + 31);
+                unsigned got;
+                for (unsigned it = 1;; it++) {
+                    got = ring[t];
+                    if (got != kGsEmpty) break;
+                    if ((it & 63u) == 0 && (*v_stop || *v_done >= len)) {
+                        got = kGsQuit;
+                        break;
                     }
+                    // the warps next in line look all the time, the others leave them the issue slots
+                    if ((int)(t - *(volatile unsigned *)&s_q.tail) >= 4) __nanosleep(100);
                 }
-                if (r0 == 0) {
-                    first_id[0] = id[0];
-                    first_id[1] = id[1];
+                if (got == kGsQuit) break;
+                if (half == 0) {
+                    act = true;
+                    i = got;
                 }
-                // strictly in neighbour-list order, by each group's lane 0 from the warp's row
-                // (a group's entries sit in its own kLanes slots)
-                float4 *row = s_stage[threadIdx.x >> 5];
-#pragma unroll
-                for (unsigned j = 0; j < 2; j++) {
-                    if (r0 + j * kLanes >= maxlen) break;  // uniform: no group has entries here
-                    row[lane] = q[j];
-                    __syncwarp();
-                    const unsigned o0 = r0 + j * kLanes;
-                    if (gl == 0 && o0 < nlen) {
-                        const unsigned cj = min(kLanes, nlen - o0);
-#pragma unroll 4
-                        for (unsigned k = 0; k < cj; k++) {
-                            const float4 p = row[g0 + k];
-                            sx = __fadd_rn(sx, p.x);
-                            sy = __fadd_rn(sy, p.y);
-                            sz = __fadd_rn(sz, p.z);
-                        }
+                done = 0;
+                bool fresh = half == 0;  // the vertex at hand comes from the ring
+                for (;;) {
+                    fence_cta();  // acquire: the neighbours' positions behind the vertex
+                    if (fresh) word = *(volatile unsigned *)&rec[i].w;
+                    code = ld_entry(packs + 16 * i + hl, fresh && !(word & kGsLong), code);
+                    bool odd = false, surplus = false;
+                    if (!__any_sync(0xffffffffu, act && (word & kGsLong))) {
+                        do {
+                            step(odd, surplus);
+                        } while (__ballot_sync(0xffffffffu, act) &&
+                                 !__any_sync(0xffffffffu, surplus || odd || (act && (word & kGsLong))));
                     }
-                    __syncwarp();  // the row is rewritten by the next chunk or vertex
-                }
-            }
-            if (act && gl == 0) {
-                const float n = (float)(int)nlen;
-                const float4 np = make_float4(__fdiv_rn(sx, n), __fdiv_rn(sy, n), __fdiv_rn(sz, n), 0.0f);
-                if (kSP) spos[v - a] = np;
-                __stcg(pos4 + v, np);
-                __threadfence_block();
-            }
-            const long long c1 = clock64();
-            __syncwarp();
-            // Release: one lane per neighbour entry of the group's vertex.
-            unsigned next = 0xffffffffu;
-            for (unsigned r0 = 0; r0 < maxlen; r0 += 2 * kLanes) {
-#pragma unroll
-                for (unsigned j = 0; j < 2; j++) {
-                    if (r0 + j * kLanes >= maxlen) break;  // uniform
-                    const unsigned o = r0 + j * kLanes + gl;
-                    const unsigned u = o < nlen ? (r0 == 0 ? first_id[j] : __ldg(nbr + e0 + o)) : 0u;
-                    const bool higher = o < nlen && u > v && u < nv;
-                    const bool remote_edge = higher && u >= b;
-                    bool ready = false;
-                    if (higher) {
-                        if (!remote_edge) {
-                            if (kFlags & kGsL1Prefetch) prefetch_l1(nbr + st[u - a]);
-                            else prefetch_l2(nbr + st[u - a]);
-                            ready = dec16(cnt, u - a) == 1u;
-                        } else {
-                            const unsigned k = atomicAdd(&s_ob_tail, 1u);
-                            unsigned it = 0;
-                            for (; it < (1u << 22) && k - *(volatile unsigned *)&s_ob_head >= kGsOutbox; it++)
-                                __nanosleep(32);
-                            if (k - *(volatile unsigned *)&s_ob_head >= kGsOutbox) {
-                                raise_error(err, QSES_ERR_TIMEOUT);
-                                s_stop = 1;
-                            } else {
-                                __threadfence_block();  // release: the position store before the entry
-                                ob[k % kGsOutbox] = u;
+                    // A half at a time: long lists and odd vertices, without haste and by the whole warp.
+                    for (unsigned h = 0; h < 32; h += 16) {
+                        if (!__shfl_sync(0xffffffffu, (unsigned)(act && (odd || (word & kGsLong))), h)) continue;
+                        const unsigned vi = __shfl_sync(0xffffffffu, i, h), vw = __shfl_sync(0xffffffffu, word, h);
+                        unsigned n = gs_len(vw);
+                        const unsigned *ids = packs + 16 * vi;
+                        if (vw & kGsLong) {
+                            ids = list + gs_first(vw);
+                            if (n == 2 * kGsLost) {  // the list is where the offsets table says
+                                const unsigned e = start[a + vi].x;
+                                ids = nbr + 2 * (size_t)e;
+                                n = 2 * (start[a + vi + 1].x - e);
                             }
                         }
+                        float sum = 0.0f;
+                        unsigned first = smax;
+                        for (unsigned base = 0; base < n; base += 32) {
+                            const unsigned cd = ld_entry(ids + base + lane, base + lane < n, smax);
+                            if (base == 0) first = cd;
+                            float4 q = ld_rec(rec_s + 16 * min(cd & 0x1fffffffu, smax));
+                            const float4 *up = pos4 + (cd & 0x1fffffffu);
+                            ld_pos_if(q, up, (int)cd < 0);
+                            for (unsigned it = 0;; it++) {
+                                const bool stale = (cd >> 30) == 2u && __float_as_uint(q.w) != stamp;
+                                if (!__any_sync(0xffffffffu, stale)) break;
+                                if (it == (1u << 20)) {
+                                    if (lane == 0) raise_error(err, QSES_ERR_TIMEOUT);
+                                    *v_stop = 1;
+                                    break;
+                                }
+                                ld_pos_if(q, up, stale);
+                            }
+                            __syncwarp();  // the rows are rewritten
+                            row[lane] = q.x; row[kGsRow + lane] = q.y; row[2 * kGsRow + lane] = q.z;
+                            __syncwarp();
+                            const float4 *all = (const float4 *)(row + kGsRow * min(hl, 2u));
+                            for (int j = 0; j < 8; j++) sum = add4(sum, all[j]);
+                        }
+                        st_comp(comp + 16 * vi, __fdiv_rn(sum, (float)(int)n), lane < 3);
+                        __syncwarp();
+                        fence_cta();  // release: the position before the counters
+                        float4 r = ld_rec(rec_s + 16 * vi);
+                        r.w = fstamp;
+                        unsigned next = kGsEmpty, nw = 0;
+                        for (unsigned base = 0; base < n; base += 32) {
+                            const unsigned cd = base == 0 ? first : ld_entry(ids + base + lane, base + lane < n, smax);
+                            const unsigned k = cd & 0xffffu, old = dec_rec(rec_s + 16 * k, (cd >> 29) == kGsSucc);
+                            const bool now = (old & 0x7fu) == 1u;
+                            const unsigned ready = __ballot_sync(0xffffffffu, now);
+                            fence_cta();
+                            unsigned f = 32;
+                            if (ready && next == kGsEmpty) {
+                                f = __ffs(ready) - 1;
+                                next = __shfl_sync(0xffffffffu, k, f);
+                                nw = __shfl_sync(0xffffffffu, old, f);
+                            }
+                            gs_push(tail_s, ring_s, k, now && lane != f);
+                            st_pos(pos4 + a + vi, r, (cd >> 29) == kGsFar);
+                            red_ext(ext, cd & 0x1fffffffu, (cd >> 29) == kGsFar);
+                        }
+                        if (half == h) {
+                            done++;
+                            act = next != kGsEmpty;
+                            i = act ? next : i;
+                            word = act ? nw : word;
+                            code = ld_entry(packs + 16 * i + hl, act && !(word & kGsLong), smax);
+                        }
                     }
-                    unsigned gm = (__ballot_sync(0xffffffffu, ready) >> g0) & kLow;  // this group's ready lanes
-                    const bool take = gm != 0 && next == 0xffffffffu;
-                    const unsigned f = take ? __ffs(gm) - 1 : 0u;
-                    const unsigned cand = __shfl_sync(0xffffffffu, u, g0 + f);
-                    if (take) {  // continue with it directly; its first two chunks of ids load now
-                        next = cand;
-                        gm &= ~(1u << f);
-                        const unsigned ne0 = st[next - a], nn = st[next - a + 1] - ne0;
-                        pre_id[0] = gl < nn ? __ldg(nbr + ne0 + gl) : 0u;
-                        pre_id[1] = kLanes + gl < nn ? __ldg(nbr + ne0 + kLanes + gl) : 0u;
-                        pre_v = next;
+                    // A free half takes a vertex that no warp waits for.
+                    fresh = false;
+                    const unsigned free = __ballot_sync(0xffffffffu, surplus && !act);
+                    if (free) {
+                        unsigned x = kGsEmpty;
+                        const unsigned src = __ffs(free) - 1;  // one half at a time
+                        if (lane == src) {
+                            // a ticket only if its slot is sure to be filled
+                            unsigned tk = *(volatile unsigned *)&s_q.ticket;
+                            if ((int)(*(volatile unsigned *)&s_q.tail - tk) > 0 && atomicCAS(&s_q.ticket, tk, tk + 1) == tk)
+                            {
+                                for (unsigned it = 0; it < (1u << 20) && x == kGsEmpty; it++) x = ring[tk];
+                                if (x == kGsEmpty) {
+                                    raise_error(err, QSES_ERR_TIMEOUT);
+                                    *v_stop = 1;
+                                }
+                            }
+                        }
+                        x = __shfl_sync(0xffffffffu, x, src);
+                        if (x != kGsEmpty && x != kGsQuit && half == (src & 16u)) {
+                            act = fresh = true;
+                            i = x;
+                        }
                     }
-                    if ((gm >> gl) & 1u) ring_push16(ring, &s_tail, u - a);
+                    if (!__any_sync(0xffffffffu, act)) break;
                 }
+                done = __reduce_add_sync(0xffffffffu, hl == 0 ? done : 0u);
+                if (stats && lane == 0) atomicAdd(stats + 4, (unsigned long long)done);
+                done = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(&s_q.done, done) + done : 0u, 0);
+                if (done >= len) ring[*(volatile unsigned *)&s_q.tail + lane] = kGsQuit;  // the slab is done: so are the waiting warps
             }
-            __syncwarp();  // queued releases precede the done count the sender checks
-            if (lane == 0) atomicAdd(&s_done, (unsigned)__popc(busy));
-            v = next;
-            const long long c2 = clock64();
-            cyc_update += c1 - c0;
-            cyc_release += c2 - c1;
-            nproc += __popc(busy);
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
-    }
-    __syncthreads();
-    if (stats && threadIdx.x == 0 && s_done < len) atomicAdd(stats + 1, 1ull);  // unfinished slabs
+        __syncthreads();
+        if (*v_done >= len) {
+            // the whole slab: its positions to the later waves, passes and the result
+            for (unsigned k = threadIdx.x; k < len; k += T) {
+                float4 q = rec[k];
+                q.w = fstamp;
+                st_pos(pos4 + a + k, q);
+            }
+        } else if (stats && threadIdx.x == 0) {
+            atomicAdd(stats + 1, 1ull);  // unfinished slabs
+        }
+        __syncthreads();
     }  // next slab
-    if (stats) {  // diagnostics: polls (max), update cycles, release cycles, vertices
-        if (threadIdx.x == 0) atomicMax(stats, polls);
-        if (lane == 0 && nproc) {
-            atomicAdd(stats + 2, cyc_update);
-            atomicAdd(stats + 3, cyc_release);
-            atomicAdd(stats + 4, nproc);
-            atomicAdd(stats + 5, cyc_ids);
-            atomicAdd(stats + 6, cyc_pos);
-            atomicAdd(stats + 7, cyc_fence);
-        }
+    if (stats && threadIdx.x == 0) atomicMax(stats, polls);
+}
+
+// Neighbour lists without a sort of all corners: occ holds each vertex's triangle corners in any
+// order (k_csr_scatter); sorting a vertex's few restores triangle order exactly (the order
+// getNeighboorsVertices appends in, SmoothMesh.cpp:45-66), and each adds the two other corners of
+// its triangle.  Then the vertex's word (counting only distinct lower neighbours), its list in the
+// form the pass reads, and the count of neighbours in lower slabs.  Vertices [v0, v1) form the
+// slabs of the table (Q, then Q + 1 bounds in id order).  Neighbours below v0 belong to waves that
+// finished before this one (final values); neighbours at or above v1 are read before their update.
+__global__ void __launch_bounds__(128) k_gs_lists(const unsigned *__restrict__ tri, unsigned *__restrict__ occ,
+                                                  const uint2 *__restrict__ start, unsigned *__restrict__ nbr, unsigned v0,
+                                                  unsigned v1, unsigned smax, const unsigned *__restrict__ table,
+                                                  unsigned *__restrict__ word0, uint4 *__restrict__ pack,
+                                                  unsigned char *__restrict__ ext, int *err) {
+    const unsigned v = v0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= v1) return;
+    const unsigned *bnd = table + 1;
+    unsigned lo = 0, hi = __ldg(table);  // bnd[lo] <= v < bnd[hi]
+    while (hi - lo > 1) {
+        const unsigned mid = (lo + hi) >> 1;
+        if (__ldg(bnd + mid) <= v) lo = mid; else hi = mid;
     }
+    const unsigned a = __ldg(bnd + lo), b = __ldg(bnd + lo + 1);
+    const unsigned o0 = start[v].x, m = start[v + 1].x - o0;  // occurrences
+    unsigned loc = 0, rem = 0, w;
+    // An entry in the pass's form; `again`: an earlier one names the same vertex.
+    auto take = [&](unsigned u, bool again) {
+        const bool here = u >= a && u < b;
+        if (u < v && u >= v0 && !again) {  // below v0: an earlier wave, already final
+            if (here) loc++; else rem++;
+        }
+        return (here ? u - a : u | 0x80000000u) | (u > v ? 0x40000000u : 0u) | (again || u >= v1 ? 0x20000000u : 0u);
+    };
+    if (m <= 8) {
+        unsigned r[8];
+#pragma unroll
+        for (unsigned i = 0; i < 8; i++) r[i] = i < m ? occ[o0 + i] : 0xffffffffu;
+#pragma unroll
+        for (unsigned i = 1; i < 8; i++) {
+#pragma unroll
+            for (unsigned j = i; j > 0; j--) {
+                const unsigned x = r[j - 1], y = r[j];
+                r[j - 1] = min(x, y);
+                r[j] = max(x, y);
+            }
+        }
+        unsigned id[16];
+#pragma unroll
+        for (unsigned i = 0; i < 8; i++) {
+            id[2 * i] = id[2 * i + 1] = 0xffffffffu;
+            if (i < m) {
+                const unsigned t = r[i] / 3u, c = r[i] - 3u * t;
+                const unsigned x = tri[3ull * t], y = tri[3ull * t + 1], z = tri[3ull * t + 2];
+                id[2 * i] = c == 0 ? y : x;
+                id[2 * i + 1] = c == 2 ? y : z;
+            }
+        }
+        unsigned code[16];
+#pragma unroll
+        for (unsigned i = 0; i < 16; i++) {
+            bool again = false;
+#pragma unroll
+            for (unsigned j = 0; j < i; j++) again |= id[j] == id[i];
+            code[i] = i < 2 * m ? take(id[i], again) : smax;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            pack[4 * (size_t)v + j] = make_uint4(code[4 * j], code[4 * j + 1], code[4 * j + 2], code[4 * j + 3]);
+        w = m << 9;
+    } else {
+        // insertion sort in place in global memory
+        for (unsigned i = 1; i < m; i++) {
+            const unsigned x = occ[o0 + i];
+            unsigned j = i;
+            while (j > 0 && occ[o0 + j - 1] > x) {
+                occ[o0 + j] = occ[o0 + j - 1];
+                j--;
+            }
+            occ[o0 + j] = x;
+        }
+        unsigned *list = nbr + 2 * (size_t)o0;
+        for (unsigned i = 0; i < m; i++) {
+            const unsigned q = occ[o0 + i], t = q / 3u, c = q - 3u * t;
+            const unsigned x = tri[3ull * t], y = tri[3ull * t + 1], z = tri[3ull * t + 2];
+            list[2 * i] = c == 0 ? y : x;
+            list[2 * i + 1] = c == 2 ? y : z;
+        }
+        for (unsigned i = 2 * m; i-- > 0;) {  // from the end: the entries before are still ids
+            const unsigned u = list[i];
+            bool again = false;
+            for (unsigned j = 0; j < i; j++) again |= list[j] == u;
+            list[i] = take(u, again);
+        }
+        const unsigned o = o0 - start[a].x;
+        w = kGsLong | (o < (1u << 17) && m < kGsLost ? m << 9 | o << 15 : kGsLost << 9);
+    }
+    // A vertex is the weld of edges around one grid corner, so its distinct neighbours lie on the
+    // 54 edges of 8 cells: both counts stay below their fields.
+    if (rem > 255u || loc > 0x7eu) raise_error(err, QSES_ERR_INTERNAL);
+    word0[v] = w | (loc + (rem ? 1u + kGsPend : 0u));
+    ext[v] = (unsigned char)rem;
 }
 
 // ------------------------------------------------------------ launchers
 
-size_t gs_slab_smem(unsigned S, unsigned flags) {
-    return (flags & kGsSmemPos) ? gs_spos_offset(S) + 16ull * S + 16 : 4ull * (S + 1) + 4ull * ((S + 1) / 2) + 2ull * S + 16;
+void launch_gs_lists(const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
+                     unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext, int *err,
+                     cudaStream_t s) {
+    k_gs_lists<<<(v1 - v0 + 127) / 128, 128, 0, s>>>(tri, occ, start, nbr, v0, v1, smax, table, word0, pack, ext, err);
 }
-template <int T, unsigned M>
-static constexpr const void *gs_fn(unsigned c) {
-    return c == 0 ? (const void *)k_gs_flow<T, M | 0> : c == 1 ? (const void *)k_gs_flow<T, M | 1>
-         : c == 2 ? (const void *)k_gs_flow<T, M | 2> : c == 3 ? (const void *)k_gs_flow<T, M | 3>
-         : c == 4 ? (const void *)k_gs_flow<T, M | 8> : c == 5 ? (const void *)k_gs_flow<T, M | 9>
-         : c == 6 ? (const void *)k_gs_flow<T, M | 10> : (const void *)k_gs_flow<T, M | 11>;
-}
-// The kernel instance for a launch shape: threads, lanes per vertex and the cache flags
-// (bits 0, 1, 3; bit 2 is host-side only).
-static const void *gs_flow_fn(int threads, unsigned flags) {
-    const unsigned c = (flags & 3u) | ((flags & kGsSmemPos) ? 4u : 0u);
-    const unsigned mode = (flags & kGsQuad) ? 2u : (flags & kGsPair) ? 1u : 0u;
-    if (threads >= 1024)
-        return mode == 2 ? gs_fn<1024, kGsQuad>(c) : mode == 1 ? gs_fn<1024, kGsPair>(c) : gs_fn<1024, 0>(c);
-    return mode == 2 ? gs_fn<512, kGsQuad>(c) : mode == 1 ? gs_fn<512, kGsPair>(c) : gs_fn<512, 0>(c);
-}
+
+size_t gs_slab_smem(unsigned S) { return gs_smem(S).bytes; }
+
 cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax, const unsigned *table,
-                           unsigned qcap, unsigned *next_slab, const uint2 *home, int P, int threads, unsigned flags,
-                           unsigned hot_warps, const uint2 *start, const unsigned *nbr,
-                           const unsigned short *cnt_local, int *remote,
-                           unsigned *inbox, unsigned *inbox_tail, int *err, long long spin_cycles,
-                           unsigned long long *stats, cudaStream_t s) {
-    if (smax == 0 || smax > kGsSlabMaxVerts || ((flags & kGsSmemPos) && smax > kGsSmemPosMaxVerts) ||
-        !gs_flags_valid(flags))
-        return cudaErrorInvalidValue;
-    size_t smem = gs_slab_smem(smax, flags);
-    if (smem > (size_t)kGsSlabMaxSmem) return cudaErrorInvalidValue;
-    const void *fn = gs_flow_fn(threads, flags);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGsSlabMaxSmem);
-    // longest sleep of an idle worker warp (ns); QSES_GS_IDLE_NS overrides it
-    static const unsigned idle_ns_max = [] {
-        const char *e = getenv("QSES_GS_IDLE_NS");
-        const long v = e ? strtol(e, nullptr, 10) : 0;
-        return v >= 32 && v <= 100000 ? (unsigned)v : 1024u;
-    }();
-    // worker warps that stay hot; QSES_GS_HOT_WARPS (0-30) overrides the caller's count
-    static const int hot_env = [] {
-        const char *e = getenv("QSES_GS_HOT_WARPS");
-        const long v = e ? strtol(e, nullptr, 10) : -1;
-        return v >= 0 && v <= 30 ? (int)v : -1;
-    }();
-    unsigned idle = idle_ns_max, hot = hot_env >= 0 ? (unsigned)hot_env : hot_warps;
-    void *args[] = {&pos,    &v0,    &nv,          &smax,  (void *)&table, &qcap,         &next_slab,
-                    (void *)&home, (void *)&start, (void *)&nbr, (void *)&cnt_local, &remote, &inbox,
-                    &inbox_tail, &err, &spin_cycles, &stats, &idle, &hot};
+                           unsigned qcap, unsigned *next_slab, int P, int threads,
+                           const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
+                           unsigned stamp, int *err, long long spin_cycles, unsigned long long *stats, cudaStream_t s) {
+    if (smax == 0 || smax > kGsSlabCap) return cudaErrorInvalidValue;
+    const size_t smem = gs_slab_smem(smax);
+    const void *fn = (const void *)k_gs_flow;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs_slab_smem(kGsSlabCap));
+    void *args[] = {&pos, &v0, &nv, &smax, (void *)&table, &qcap, &next_slab, (void *)&start, (void *)&nbr,
+                    (void *)&word0, (void *)&pack, &ext, &stamp, &err, &spin_cycles, &stats};
     // A cooperative launch: every CTA resident from the start.  (A plain launch would also be
     // safe - a CTA only waits for slabs taken before its own, by CTAs that were running when
     // they took them - but its CTAs can then take the SMs the side stream's kernels wait for.)
@@ -610,11 +682,11 @@ void gs_l2_window(int device, cudaStream_t s, const void *p, size_t bytes) {
     cudaGetLastError();  // the window is a hint: a refusal leaves the results unchanged
 }
 
-int gs_slab_max_blocks(int device, unsigned S, int threads, unsigned flags) {
-    const void *fn = gs_flow_fn(threads, flags);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGsSlabMaxSmem);
+int gs_slab_max_blocks(int device, unsigned S, int threads) {
+    const void *fn = (const void *)k_gs_flow;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs_slab_smem(kGsSlabCap));
     int per_sm = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads >= 1024 ? 1024 : 512, gs_slab_smem(S, flags));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads >= 1024 ? 1024 : 512, gs_slab_smem(S));
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     return per_sm * sms;
 }

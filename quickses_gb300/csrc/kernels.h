@@ -32,60 +32,55 @@ void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *
 void launch_tri_flags(const unsigned *tri, unsigned nt, uint2 *flags, cudaStream_t s);
 void launch_tri_compact(const unsigned *tri, unsigned nt, const uint2 *excl, unsigned *out, cudaStream_t s);
 // Neighbour lists by counting: start (nv + 1 entries, zeroed) -> counts -> (scan) -> corner
-// occurrences scattered per vertex into occ (n3) -> sorted per vertex and expanded into nbr
-// (2 n3), start[v].x = list offset.
+// occurrences scattered per vertex into occ (n3), in any order.
 void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, cudaStream_t s);
 void launch_csr_scatter(const unsigned *tri, size_t n3, uint2 *start, unsigned *occ, cudaStream_t s);
-void launch_csr_sortfill(const unsigned *tri, unsigned *occ, size_t n3, unsigned nv, uint2 *start, unsigned *nbr,
-                         cudaStream_t s);
 // Slab table of one Gauss-Seidel wave (device words): [0] Q slabs, [1, Q + 2) their bounds in
 // id order (qcap + 1 slots), [qcap + 2, qcap + 2 + Q) the slab ids in the order CTAs take them.
 inline size_t gs_table_words(unsigned qcap) { return 2ull * qcap + 2; }
-void launch_gs_setup(const uint2 *start, const unsigned *nbr, unsigned v0, unsigned v1, const unsigned *table,
-                     unsigned short *cnt_local, int *remote, uint2 *home, cudaStream_t s);
-size_t gs_slab_smem(unsigned S, unsigned flags);
+// The pass's lists from the occurrences: word0, pack (64 B) per vertex, lists of more than 16
+// entries in nbr (2 n3) at twice the vertex's offset (k_smooth.cu); ext: one byte per vertex, the
+// neighbours in lower slabs still to come.
+void launch_gs_lists(const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
+                     unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext, int *err,
+                     cudaStream_t s);
+size_t gs_slab_smem(unsigned S);
 void launch_to_float4(const float *v3, unsigned nv, float4 *v4, cudaStream_t s);
 void launch_from_float4(const float4 *v4, unsigned nv, float *v3, cudaStream_t s);
 // One Gauss-Seidel pass over vertices [v0, nv) in the table's slabs (each at most smax
-// vertices), taken by P persistent CTAs from *next_slab (zeroed, like inbox_tail's qcap
-// counters).  threads: 512 or 1024 per slab CTA.
+// vertices), taken by P persistent CTAs from *next_slab (zeroed).  stamp: written to w of every
+// position updated (another value than any position holds before the pass).  threads: 512 or
+// 1024 per slab CTA.
 cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax, const unsigned *table,
-                           unsigned qcap, unsigned *next_slab, const uint2 *home, int P, int threads, unsigned flags,
-                           unsigned hot_warps, const uint2 *start, const unsigned *nbr,
-                           const unsigned short *cnt_local, int *remote,
-                           unsigned *inbox, unsigned *inbox_tail, int *err, long long spin_cycles,
-                           unsigned long long *stats, cudaStream_t s);
-int gs_slab_max_blocks(int device, unsigned S, int threads, unsigned flags);
+                           unsigned qcap, unsigned *next_slab, int P, int threads,
+                           const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
+                           unsigned stamp, int *err, long long spin_cycles, unsigned long long *stats, cudaStream_t s);
+int gs_slab_max_blocks(int device, unsigned S, int threads);
 
 // Gauss-Seidel launch shape: threads per slab CTA and the slab size aimed at (vertices);
-// the result does not depend on it, only the time does.
+// the result does not depend on it, only the time does.  The cache flags name policies of an
+// earlier kernel that read positions through L2; the records in shared memory leave them nothing
+// to choose, so they are accepted and, but for kGsPersistL2, without effect on a pass
+// (gs_plan_for still splits by kGsSmemPos when no cap is given).
 struct GsShape {
     int threads = 512;
     unsigned target = 16384;
-    unsigned flags = 0;  // kGsL1Prefetch | kGsL1Positions | kGsPersistL2 | kGsSmemPos | kGsPair / kGsQuad
+    unsigned flags = 0;
     unsigned wave = 0;   // most vertices per slab-kernel launch (0: all that fit on the GPU)
-    unsigned hot = 0;    // worker warps per CTA whose idle sleeps stay short (same results)
+    unsigned cap = 0;    // largest slab (0: 8192 with kGsSmemPos, else 25 000)
 };
-// Hot worker warps of single-molecule passes: 12 of 30 polling the ready ring every 64 ns
-// at most took the 50 000-atom pass from 10.42-10.44 to 10.27-10.29 ms (0: 15.72-15.74 ms
-// per call, 12: 15.51); all 30 hot was slower (16.0 ms); batches are faster with none.
-constexpr unsigned kGsHotWarpsSingle = 12;
-// Cache policies of the smoothing kernel (same results, different memory paths):
-constexpr unsigned kGsL1Prefetch = 1;   // prefetch a successor's neighbour list into L1, not L2
-constexpr unsigned kGsL1Positions = 2;  // neighbour positions through L1 (default: L2 only)
 constexpr unsigned kGsPersistL2 = 4;    // host side: keep the positions in persisting L2 lines
-constexpr unsigned kGsSmemPos = 8;      // the slab's own positions in shared memory (slabs <= 8192)
+constexpr unsigned kGsSmemPos = 8;
 constexpr unsigned kGsSmemPosMaxVerts = 8192;
-// Lanes per vertex update (same results): 32 by default; 16 with kGsPair (two ready vertices
-// per worker warp), 8 with kGsQuad (four).
 constexpr unsigned kGsPair = 16;
 constexpr unsigned kGsQuad = 32;
 inline bool gs_flags_valid(unsigned f) { return f < 64 && (f & (kGsPair | kGsQuad)) != (kGsPair | kGsQuad); }
 // Sets (bytes > 0) or clears the stream's L2 persistence window over [p, p + bytes); the
 // set-aside is this process's context limit, restored when the window is cleared.
 void gs_l2_window(int device, cudaStream_t s, const void *p, size_t bytes);
-// Tuned shape for a mesh of nv vertices (batch = waves of many molecules), or the default.
-GsShape gs_shape(unsigned nv, bool batch);
+// Tuned shape for a mesh of nv vertices (batch: many molecules), or the default; biggest: the
+// vertices of the largest molecule.
+GsShape gs_shape(unsigned nv, bool batch, unsigned biggest);
 void gs_shape_record(unsigned nv, bool batch, GsShape s);
 void gs_shape_record_all(bool batch, GsShape s);  // every mesh-size class
 int gs_shape_candidates(GsShape *out, int max);
@@ -94,6 +89,8 @@ int edt_shape(int G);
 void edt_shape_record(int G, int shape);
 constexpr int kEdtShapes = 4;
 constexpr unsigned kGsSlabMaxVerts = 25000;
+constexpr unsigned kGsSlabCap = 11904;  // vertices whose state fits a CTA's shared memory (18 B each)
+constexpr unsigned kGsSlabTwo = 5376;   // ... fits twice into an SM's
 
 // ---- batch forms (QBatch: per-molecule grids and offsets in device memory)
 void launch_atom_hash_batch(const QBatch &b, const float *xyz, unsigned n, unsigned *key, cudaStream_t s);

@@ -133,13 +133,20 @@ static bool g_tuned[2][33];
 
 static int tune_bucket(unsigned nv) { return bits_for(nv); }
 
-GsShape gs_shape(unsigned nv, bool batch) {
+GsShape gs_shape(unsigned nv, bool batch, unsigned biggest) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     const int b = tune_bucket(nv);
     if (g_tuned[batch][b]) return g_tune[batch][b];
-    // untuned: the shapes the tuner picks on balls of 1 000 - 50 000 atoms and on batches
-    // (two vertex updates per worker warp: 14.1 -> 13.0 ms on a served batch of 23 M vertices)
-    return batch ? GsShape{1024, 25000, kGsL1Positions | kGsPair, 0} : GsShape{1024, 4096, kGsL1Positions, 0};
+    // Untuned.  A molecule of V vertices passes through V / target slabs one after another, each
+    // crossing adding a hand-off to the chain of updates, while a slab that is too large queues its
+    // ready vertices for one SM: 6.5 sqrt(V) was within 4 % of the best of seven targets for balls and
+    // shells of 9 500 - 3 500 000 vertices (30 000 vertices: 0.41 ms; 519 per slab 0.46, 4 096 0.48;
+    // 1 670 000: 3.72 ms; 3 875 per slab 4.28, 11 625 3.97).  Far more vertices than fit the SMs at
+    // once are a matter of throughput: two CTAs per SM (14 200 000 vertices: 9.66 ms; one CTA of
+    // 11 904 10.36; a batch of 29 600 000: 6.7 against 8.1).  14 worker warps per CTA are enough, as
+    // each takes a second vertex when more are ready: 1 024 threads 1-9 % slower.
+    const unsigned t = (unsigned)(6.5 * std::sqrt((double)biggest));
+    return GsShape{512, nv > 8000000u ? kGsSlabTwo : std::min(std::max(t, 256u), kGsSlabCap), 0, 0};
 }
 
 void gs_shape_record(unsigned nv, bool batch, GsShape sh) {
@@ -175,25 +182,14 @@ void edt_shape_record(int G, int shape) {
 }
 
 int gs_shape_candidates(GsShape *out, int max) {
-    static const unsigned targets[] = {4096, 8192, 16384, 25000};
-    // the persisting-L2 window (kGsPersistL2) is left to callers that force it: it changes
-    // stream attributes (its segment then runs outside CUDA graphs) and its reset after the
-    // pass costs more than the pass gains
-    static const unsigned flags[] = {0,          kGsL1Positions,          kGsL1Prefetch,          kGsL1Prefetch | kGsL1Positions,
-                                     kGsSmemPos, kGsSmemPos | kGsL1Positions, kGsSmemPos | kGsL1Prefetch,
-                                     kGsSmemPos | kGsL1Prefetch | kGsL1Positions};
-    // two vertices per worker warp with the two policies the one-vertex warps are tuned to:
-    // positions through L1, with or without the slab's own in shared memory (four vertices
-    // per warp, kGsQuad, measured slower than two on single molecules and batches alike)
-    static const unsigned group_flags[] = {kGsPair | kGsL1Positions, kGsPair | kGsSmemPos | kGsL1Positions};
+    // 256 vertices per slab up to what fits; the persisting-L2 window (kGsPersistL2) is left to
+    // callers that force it: it changes stream attributes (its segment then runs outside CUDA
+    // graphs) and its reset after the pass costs more than the pass gains
+    static const unsigned targets[] = {256, 512, 1024, 1536, 2048, 3072, 4096, kGsSlabTwo, 7168, 9216, kGsSlabCap};
     int k = 0;
     for (int t : {512, 1024})
-        for (unsigned tg : targets) {
-            for (unsigned f : flags)
-                if (k < max) out[k++] = GsShape{t, tg, f};
-            for (unsigned f : group_flags)
-                if (k < max) out[k++] = GsShape{t, tg, f};
-        }
+        for (unsigned tg : targets)
+            if (k < max) out[k++] = GsShape{t, tg, 0};
     return k;
 }
 
@@ -255,14 +251,14 @@ static unsigned ceil_div(unsigned long long a, unsigned long long b) { return (u
 
 int gs_plan(int device, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
             GsPlan &pl) {
-    // resident slab CTAs: one molecule's slabs may hold up to the largest slab; a batch's at
-    // most the target, so smaller targets fit more CTAs per SM
-    const bool single = mol_off == nullptr || nm <= 1;
-    const unsigned cap = (sh.flags & kGsSmemPos) ? kGsSmemPosMaxVerts : kGsSlabMaxVerts;
-    const unsigned smax = single && !(sh.flags & kGsSmemPos) ? cap : std::min(std::max(sh.target, 256u), cap);
-    const int pmax = std::min(gs_slab_max_blocks(device, smax, sh.threads, sh.flags), 1024);
+    // every slab's state is in shared memory: at most kGsSlabCap vertices, and smaller targets fit
+    // more CTAs per SM
+    GsShape in = sh;
+    in.flags |= kGsSmemPos;
+    in.cap = kGsSlabCap;
+    const int pmax = std::min(gs_slab_max_blocks(device, std::min(std::max(in.target, 256u), in.cap), in.threads), 1024);
     if (pmax < 1) return QSES_ERR_NO_DEVICE;
-    return gs_plan_for(pmax, sh, nv, mol_off, mol_depth, nm, pl);
+    return gs_plan_for(pmax, in, nv, mol_off, mol_depth, nm, pl);
 }
 
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
@@ -272,7 +268,7 @@ int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_of
     // with the slab's positions in shared memory (kGsSmemPos) slabs hold at most 8192
     // vertices and a molecule may have more slabs than there are resident CTAs
     const bool spos = (sh.flags & kGsSmemPos) != 0;
-    const unsigned Smax = spos ? kGsSmemPosMaxVerts : kGsSlabMaxVerts;
+    const unsigned Smax = sh.cap ? sh.cap : spos ? kGsSmemPosMaxVerts : kGsSlabMaxVerts;
     const unsigned t = std::min(std::max(sh.target, 256u), Smax);
     const bool single = mol_off == nullptr || nm <= 1;
     const unsigned cap = sh.wave ? std::max(sh.wave, 1u) : nv;
@@ -368,19 +364,15 @@ int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_of
     return QSES_OK;
 }
 
-int gs_buffers(qses_context *ctx, const GsPlan &pl, unsigned nv, GsBuffers &out) {
-    const GsLaunch &L = pl.L;
+int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out) {
     const size_t words = pl.table.size();
-    const size_t need = align256(8ull * nv + 8) + align256(4 * words) + align256(4ull * (L.wsize + L.smax + 64)) +
-                        align256(4ull * (L.qcap + 2)) + 4096;
+    const size_t need = align256(4 * words) + 4096;
     const void *old_ws = ctx->gs_ws.base;
     if (ctx->gs_ws.reserve(need) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "smoothing workspace");
     if (ctx->gs_ws.base != old_ws) QSES_SEG_TRACE("smoothing workspace moved (%zu bytes)\n", need);
-    out.home = (uint2 *)ctx->gs_ws.take(8ull * nv + 8);
     out.table = (unsigned *)ctx->gs_ws.take(4 * words);
-    out.inbox = (unsigned *)ctx->gs_ws.take(4ull * (L.wsize + L.smax + 64));
-    out.inbox_tail = (unsigned *)ctx->gs_ws.take(4ull * (L.qcap + 2));  // per slab, then the slab counter
-    if (!out.inbox_tail) return ctx->fail(QSES_ERR_INTERNAL, "smoothing workspace layout");
+    out.next_slab = (unsigned *)ctx->gs_ws.take(256);
+    if (!out.next_slab) return ctx->fail(QSES_ERR_INTERNAL, "smoothing workspace layout");
     if (4 * words > ctx->h_gs_cap) {
         QSES_SEG_TRACE("slab tables: pinned buffer grows to %zu words\n", words);
         ctx->host_gen++;
@@ -400,8 +392,9 @@ int gs_buffers(qses_context *ctx, const GsPlan &pl, unsigned nv, GsBuffers &out)
 }
 
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, float4 *pos4,
-                  unsigned nv, const uint2 *deg, const unsigned *nbr, unsigned short *cnt, int *remote, uint2 *home,
-                  unsigned *table, const unsigned *h_table, unsigned *inbox, unsigned *inbox_tail, int *d_err,
+                  unsigned nv, const unsigned *tri, unsigned *occ, const uint2 *deg, unsigned *nbr, unsigned *word0,
+                  uint4 *pack, unsigned *ext, unsigned *ext0,
+                  unsigned *table, const unsigned *h_table, unsigned *next_slab, int *d_err,
                   unsigned long long *stats, cudaEvent_t before_writeback) {
     cudaStream_t s = ctx->stream;
     launch_to_float4(vq, nv, pos4, s);
@@ -409,19 +402,23 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
     if (sh.flags & kGsPersistL2) gs_l2_window(ctx->device, s, pos4, 16ull * nv);
     if (stats) QCHK(cudaMemsetAsync(stats, 0, 64, s));
     QCHK(cudaMemcpyAsync(table, h_table, 4ull * L.waves * L.table_words, cudaMemcpyHostToDevice, s));
+    for (unsigned w = 0; w < L.waves; w++) {
+        const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
+        launch_gs_lists(tri, occ, deg, nbr, v0, v1, L.smax, table + (size_t)w * L.table_words, word0, pack,
+                        (unsigned char *)(passes > 1 ? ext0 : ext), d_err, s);
+        ctx->launches++;
+    }
+    ctx->mark("smooth_csr");
     for (int pass = 0; pass < passes; pass++) {
+        if (passes > 1) QCHK(cudaMemcpyAsync(ext, ext0, nv, cudaMemcpyDeviceToDevice, s));
         for (unsigned w = 0; w < L.waves; w++) {
             const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
             const unsigned *tb = table + (size_t)w * L.table_words;
-            launch_gs_setup(deg, nbr, v0, v1, tb, cnt, remote, home, s);
-            ctx->launches++;
-            QCHK(cudaMemsetAsync(inbox, 0xff, 4ull * (v1 - v0), s));
-            QCHK(cudaMemsetAsync(inbox_tail, 0, 4ull * (L.qcap + 1), s));
+            QCHK(cudaMemsetAsync(next_slab, 0, 4, s));
             // per-update cycle counters only on profiled calls: their clock reads sit on the
             // dependency chain (1.4 % of the pass on 50 000 atoms)
-            QCHK(launch_gs_slab(pos4, v0, v1, L.smax, tb, L.qcap, inbox_tail + L.qcap, home, L.ctas, sh.threads,
-                                sh.flags, sh.hot, deg, nbr, cnt, remote, inbox, inbox_tail, d_err, 4000000000ll,
-                                ctx->profiling ? stats : nullptr, s));
+            QCHK(launch_gs_slab(pos4, v0, v1, L.smax, tb, L.qcap, next_slab, L.ctas, sh.threads, deg, nbr, word0,
+                                pack, ext, (unsigned)pass + 1u, d_err, 4000000000ll, ctx->profiling ? stats : nullptr, s));
             ctx->launches++;
         }
     }
@@ -545,12 +542,12 @@ struct FinishSeg {
     unsigned *okey, *nbr;  // okey: the corners scattered per vertex
     void *tmpb;
     float4 *pos4;
-    unsigned short *cnt;
-    int *lower;
-    uint2 *home;
+    unsigned *word0;       // per vertex: word and common list of the smoothing pass
+    uint4 *pack;
+    unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
     unsigned *table;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
-    unsigned *inbox, *inbox_tail;
+    unsigned *next_slab;
     unsigned long long *stats;
     unsigned long long n3;
     unsigned nv, nt;
@@ -597,22 +594,16 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
 
     // Gauss-Seidel smoothing on the device
     if (c.passes > 0 && c.nv > 0 && c.nt > 0) {
-        // neighbour lists: count the corners per vertex, scan, scatter them per vertex, then
-        // sort each vertex's few corners back into triangle order (the order
-        // getNeighboorsVertices appends in) and expand them into the lists
+        // neighbour lists: count the corners per vertex, scan, scatter them per vertex
         QCHK(cudaMemsetAsync(c.deg, 0, 8ull * (c.nv + 1), s));
         launch_csr_count(c.tri, c.n3, c.deg, s);
         ctx->launches++;
         QCHK(scan_u2(c.deg, c.deg, c.nv + 1, nullptr, c.tmpb, c.err, s, &ctx->launches));
         launch_csr_scatter(c.tri, c.n3, c.deg, c.okey, s);
         ctx->launches++;
-        launch_csr_sortfill(c.tri, c.okey, c.n3, c.nv, c.deg, c.nbr, s);
-        ctx->launches++;
-        ctx->mark("smooth_csr");
         // the closest-atom pass on the side stream reads the welded positions in vq
-        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.deg, c.nbr, c.cnt, c.lower,
-                                     c.home, c.table, c.h_table, c.inbox, c.inbox_tail, c.err, c.stats,
-                                     c.fork ? ctx->ev_join : nullptr);
+        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.tri, c.okey, c.deg, c.nbr, c.word0, c.pack, c.ext, c.ext0,
+                                     c.table, c.h_table, c.next_slab, c.err, c.stats, c.fork ? ctx->ev_join : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -750,7 +741,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     const size_t nflag = std::max<size_t>((size_t)NE + 1, (size_t)T) + 1;
     size_t needB = 2 * align256(4 * n3) + 2 * align256(8ull * NE) + 2 * align256(4ull * NE) + align256(8ull * nflag) +
                    align256(4ull * NE) + align256(12ull * NE) + 2 * align256(4ull * NE) + align256(4 * n3 + 4) +
-                   align256(8 * n3) + 3 * align256(4ull * NE) + 4096 +
+                   align256(8 * n3) + 3 * align256(4ull * NE) + align256(64ull * NE + 64) + 4096 +
                    align256(16ull * NE + 16) +
                    align256(tmpB) + align256(8ull * T + 16) + align256(scan_u2_tmp_bytes(T + 1)) + 4096;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
@@ -765,7 +756,9 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);
     unsigned *okey = (unsigned *)B.take(4 * n3 + 4);
     unsigned *nbr = (unsigned *)B.take(8 * n3 + 8);
-    int *lower = (int *)B.take(4ull * NE + 4), *cnt = (int *)B.take(4ull * NE + 4);
+    unsigned *ext = (unsigned *)B.take(1ull * NE + 64), *ext0 = (unsigned *)B.take(1ull * NE + 64);
+    unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
+    uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
     float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
     void *tmpb = B.take(tmpB);
     uint2 *tflags = (uint2 *)B.take(8ull * T + 16);      // degenerate filter (side stream)
@@ -847,8 +840,10 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     c.nbr = nbr;
     c.tmpb = tmpb;
     c.pos4 = pos4;
-    c.cnt = (unsigned short *)cnt;
-    c.lower = lower;
+    c.word0 = word0;
+    c.pack = pack;
+    c.ext = ext;
+    c.ext0 = ext0;
     c.stats = (unsigned long long *)((char *)ctx->small + 256);
     c.n3 = n3;
     c.nv = nv;
@@ -858,20 +853,17 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     c.fork = !ctx->profiling && ctx->side != nullptr;
     const bool smoothing = p.smooth_passes > 0 && nv > 0 && T > 0;
     if (smoothing) {
-        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false);
-        c.sh.hot = kGsHotWarpsSingle;
+        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv);
         ctx->gs_used = c.sh;
         GsPlan plan;
         rc = gs_plan(ctx->device, c.sh, nv, nullptr, nullptr, 1, plan);
         if (rc != QSES_OK) return ctx->fail(rc, "smoothing slab plan");
         GsBuffers gb;
-        QCHK_RC(gs_buffers(ctx, plan, nv, gb));
+        QCHK_RC(gs_buffers(ctx, plan, gb));
         c.gl = plan.L;
-        c.home = gb.home;
         c.table = gb.table;
         c.h_table = ctx->h_gs;
-        c.inbox = gb.inbox;
-        c.inbox_tail = gb.inbox_tail;
+        c.next_slab = gb.next_slab;
         ctx->diag[0] = plan.max_slabs;
         ctx->diag[1] = plan.max_len;
     }

@@ -196,12 +196,12 @@ struct BatchFinishSeg {
     unsigned *okey, *nbr;  // okey: the corners scattered per vertex
     void *tmpb;
     float4 *pos4;
-    unsigned short *cnt;
-    int *lower;
-    uint2 *home;
+    unsigned *word0;       // per vertex: word and common list of the smoothing pass
+    uint4 *pack;
+    unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
     unsigned *table;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
-    unsigned *inbox, *inbox_tail;
+    unsigned *next_slab;
     unsigned long long n3;
     unsigned nv, nt;
     int passes, fork;
@@ -252,22 +252,16 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
 
     // Gauss-Seidel over all molecules
     if (c.passes > 0 && c.nv > 0 && c.nt > 0) {
-        // neighbour lists: count the corners per vertex, scan, scatter them per vertex, then
-        // sort each vertex's few corners back into triangle order (the order
-        // getNeighboorsVertices appends in) and expand them into the lists
+        // neighbour lists: count the corners per vertex, scan, scatter them per vertex
         QCHK(cudaMemsetAsync(c.deg, 0, 8ull * (c.nv + 1), s));
         launch_csr_count(c.tri, c.n3, c.deg, s);
         ctx->launches++;
         QCHK(scan_u2(c.deg, c.deg, c.nv + 1, nullptr, c.tmpb, c.err, s, &ctx->launches));
         launch_csr_scatter(c.tri, c.n3, c.deg, c.okey, s);
         ctx->launches++;
-        launch_csr_sortfill(c.tri, c.okey, c.n3, c.nv, c.deg, c.nbr, s);
-        ctx->launches++;
-        ctx->mark("smooth_csr");
         // the closest-atom pass on the side stream reads the welded positions in vq
-        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.deg, c.nbr, c.cnt, c.lower,
-                                     c.home, c.table, c.h_table, c.inbox, c.inbox_tail, c.err, nullptr,
-                                     c.fork ? ctx->ev_join : nullptr);
+        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.tri, c.okey, c.deg, c.nbr, c.word0, c.pack, c.ext, c.ext0,
+                                     c.table, c.h_table, c.next_slab, c.err, nullptr, c.fork ? ctx->ev_join : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -460,7 +454,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     const size_t nflag = std::max<size_t>((size_t)NE + 1, (size_t)T) + 1;
     const size_t needB = 2 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
                          a256(8ull * nflag) + a256(4ull * NE + 4) + a256(12ull * NE + 12) + 3 * a256(4ull * NE + 4) +
-                         a256(4 * n3 + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(16ull * NE + 16) + a256(tmpB) + a256(8ull * T + 16) +
+                         a256(4 * n3 + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) + a256(16ull * NE + 16) + a256(tmpB) + a256(8ull * T + 16) +
                          a256(scan_u2_tmp_bytes(T + 1)) + 8192;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "batch mesh workspace");
     Arena &B = ctx->mesh_ws;
@@ -475,7 +469,9 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);
     unsigned *okey = (unsigned *)B.take(4 * n3 + 4);
     unsigned *nbr = (unsigned *)B.take(8 * n3 + 8);
-    int *lower = (int *)B.take(4ull * NE + 4), *cnt = (int *)B.take(4ull * NE + 4);
+    unsigned *ext = (unsigned *)B.take(1ull * NE + 64), *ext0 = (unsigned *)B.take(1ull * NE + 64);
+    unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
+    uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
     float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
     void *tmpb = B.take(tmpB);
     uint2 *tflags = (uint2 *)B.take(8ull * T + 16);  // degenerate filter (side stream)
@@ -562,8 +558,10 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     c.nbr = nbr;
     c.tmpb = tmpb;
     c.pos4 = pos4;
-    c.cnt = (unsigned short *)cnt;
-    c.lower = lower;
+    c.word0 = word0;
+    c.pack = pack;
+    c.ext = ext;
+    c.ext0 = ext0;
     c.n3 = n3;
     c.nv = nv;
     c.nt = T;
@@ -571,7 +569,9 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     c.fork = !ctx->profiling && ctx->side != nullptr;
     const bool smoothing = passes > 0 && nv > 0 && T > 0;
     if (smoothing) {
-        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(std::min<unsigned>(nv, 152u * kGsSlabMaxVerts), true);
+        unsigned biggest = 0;
+        for (unsigned m = 0; m < nm; m++) biggest = std::max(biggest, vtx_off[m + 1] - vtx_off[m]);
+        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, true, biggest);
         ctx->gs_used = c.sh;
         // molecules are never split between slabs unless larger than one; their grid sizes
         // estimate the dependency depths that order the slabs
@@ -581,13 +581,11 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         const int rp = gs_plan(ctx->device, c.sh, nv, vtx_off.data(), depth.data(), nm, plan);
         if (rp != QSES_OK) return ctx->fail(rp, "smoothing slab plan");
         GsBuffers gb;
-        QCHK_RC(gs_buffers(ctx, plan, nv, gb));
+        QCHK_RC(gs_buffers(ctx, plan, gb));
         c.gl = plan.L;
-        c.home = gb.home;
         c.table = gb.table;
         c.h_table = ctx->h_gs;
-        c.inbox = gb.inbox;
-        c.inbox_tail = gb.inbox_tail;
+        c.next_slab = gb.next_slab;
         ctx->diag[0] = std::max<unsigned long long>(ctx->diag[0], plan.max_slabs);
         ctx->diag[1] = std::max<unsigned long long>(ctx->diag[1], plan.max_len);
     }

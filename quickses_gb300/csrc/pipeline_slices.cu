@@ -220,7 +220,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                                               scan_u2_tmp_bytes(T + 1)});
                 const size_t needB = 3 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
                                      3 * a256(8ull * (NE + 2)) + 2 * a256(4ull * NE + 4) + 2 * a256(12ull * NE + 12) +
-                                     2 * a256(4ull * NE + 4) + a256(8 * n3 + 8) + 2 * a256(4ull * NE + 4) +
+                                     2 * a256(4ull * NE + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) +
                                      a256(16ull * NE + 16) + a256(8ull * T + 16) + a256(tmpB) + 4096;
                 if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
                 Arena &B = ctx->mesh_ws;
@@ -235,7 +235,9 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 float *vq = (float *)B.take(12ull * NE + 12), *vq2 = (float *)B.take(12ull * NE + 12);
                 int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);
                 unsigned *nbr = (unsigned *)B.take(8 * n3 + 8);
-                int *lower = (int *)B.take(4ull * NE + 4), *cnt = (int *)B.take(4ull * NE + 4);
+                unsigned *ext = (unsigned *)B.take(1ull * NE + 64), *ext0 = (unsigned *)B.take(1ull * NE + 64);
+                unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
+                uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
                 float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
                 uint2 *tflags = (uint2 *)B.take(8ull * T + 16);
                 void *tmpb = B.take(tmpB);
@@ -275,20 +277,18 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                     launch_csr_count(tri, n3k, deg, s);
                     SCHK(scan_u2(deg, deg, nv + 1, nullptr, tmpb, d_err, s, &ctx->launches));
                     launch_csr_scatter(tri, n3k, deg, okey, s);
-                    launch_csr_sortfill(tri, okey, n3k, nv, deg, nbr, s);
-                    ctx->launches += 3;
-                    GsShape sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false);
-                    sh.hot = kGsHotWarpsSingle;
+                    ctx->launches += 2;
+                    GsShape sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv);
                     ctx->gs_used = sh;
                     GsPlan plan;
                     const int prc = gs_plan(ctx->device, sh, nv, nullptr, nullptr, 1, plan);
                     if (prc != QSES_OK) return ctx->fail(prc, "smoothing slab plan");
                     GsBuffers gb;
-                    const int brc = gs_buffers(ctx, plan, nv, gb);
+                    const int brc = gs_buffers(ctx, plan, gb);
                     if (brc != QSES_OK) return brc;
-                    const int src = run_smoothing(ctx, sh, plan.L, p.smooth_passes, vq2, pos4, nv, deg, nbr,
-                                                  (unsigned short *)cnt, lower, gb.home, gb.table, ctx->h_gs, gb.inbox,
-                                                  gb.inbox_tail, d_err, stats);
+                    const int src = run_smoothing(ctx, sh, plan.L, p.smooth_passes, vq2, pos4, nv, tri, okey, deg, nbr,
+                                                  word0, pack, ext, ext0, gb.table, ctx->h_gs, gb.next_slab, d_err,
+                                                  stats);
                     if (src != QSES_OK) return src;
                 }
                 const unsigned *tri_out = tri;

@@ -189,14 +189,15 @@ struct SlicedMesh {
 int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_xyz, const float *d_r, unsigned n,
                         SlicedMesh &out);
 // `passes` exact Gauss-Seidel passes over vertices [0, nv): positions vq (3 floats each) in
-// and out, CSR (deg offsets, nbr), shape sh.  The vertices run in sequential waves of at
+// and out, triangle corners occ scattered per vertex (deg offsets), shape sh.  The vertices run in sequential waves of at
 // most the slab kernel's capacity; every dependency points to a lower id, so a wave only
 // depends on earlier, finished waves.
 // `before_writeback` (may be null): event the stream waits for before the smoothed
 // positions overwrite vq (work on another stream that still reads the welded positions).
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, float4 *pos4,
-                  unsigned nv, const uint2 *deg, const unsigned *nbr, unsigned short *cnt, int *remote, uint2 *home,
-                  unsigned *table, const unsigned *h_table, unsigned *inbox, unsigned *inbox_tail, int *d_err,
+                  unsigned nv, const unsigned *tri, unsigned *occ, const uint2 *deg, unsigned *nbr, unsigned *word0,
+                  uint4 *pack, unsigned *ext, unsigned *ext0,
+                  unsigned *table, const unsigned *h_table, unsigned *next_slab, int *d_err,
                   unsigned long long *stats, cudaEvent_t before_writeback = nullptr);
 // Slab plan of a pass over nv vertices.  mol_off (nm + 1 entries, null for one molecule):
 // the molecules' vertex ranges, never split by a slab boundary unless a molecule is larger
@@ -207,13 +208,12 @@ int gs_plan(int device, const GsShape &sh, unsigned nv, const unsigned *mol_off,
 // The same for at most pmax resident slab CTAs (no device query).
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
                 GsPlan &pl);
-// The smoothing workspace of a plan (home records, slab tables, inboxes) in ctx->gs_ws and
-// the plan's tables in ctx->h_gs.  Returns QSES_OK or an error code (ctx->fail called).
+// The smoothing workspace of a plan (slab tables and the slab counter) in ctx->gs_ws and the
+// plan's tables in ctx->h_gs.  Returns QSES_OK or an error code (ctx->fail called).
 struct GsBuffers {
-    uint2 *home;
-    unsigned *table, *inbox, *inbox_tail;
+    unsigned *table, *next_slab;
 };
-int gs_buffers(qses_context *ctx, const GsPlan &pl, unsigned nv, GsBuffers &out);
+int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out);
 // All items share `passes`; the weld keys of every item fit `key_bits` bits and
 // key_bits + bits(count - 1) <= 64.  Results in ctx->batch.
 int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes, int key_bits);
