@@ -178,6 +178,46 @@ __device__ __forceinline__ float add4(float s, float4 q) {
     return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, q.x), q.y), q.z), q.w);
 }
 
+// Waits until slab p and the slabs of all its higher neighbours have had `pass` passes; false if
+// that takes too long.
+__device__ __forceinline__ bool gs_wait_pass(const GsOrder &ord, unsigned p, unsigned pass, long long spin_cycles) {
+    const long long since = clock64();
+    for (unsigned j = p; j <= ord.far[p]; j++)
+        while (ld_acquire_u32(&ord.done[j]) < pass) {
+            if (clock64() - since > spin_cycles) return false;
+            __nanosleep(200);
+        }
+    return true;
+}
+
+// Several passes in one launch: a vertex's pass q needs its lower neighbours' pass q and its higher
+// neighbours' pass q - 1, so pass q can follow pass q - 1 through the slabs a little behind it, and
+// three passes take little longer than one (548 000 vertices: 4.77 ms launched one after another,
+// 2.70 together, one alone 1.6).
+// Item n of the passes of a wave: slabs by their place in the order, pass q of a place `lag` places
+// behind pass q - 1, so that a place's items, and those of the places up to `lag` behind it, come
+// after their previous passes.  items_before(t): the items whose place + lag q is below t.
+struct GsItem {
+    unsigned place, pass;
+};
+__device__ __forceinline__ unsigned long long gs_items_before(unsigned long long t, unsigned Q, unsigned passes,
+                                                              unsigned lag) {
+    const unsigned long long full = t >= Q ? min((unsigned long long)passes, (t - Q) / lag + 1) : 0;
+    const unsigned long long part = t ? min((unsigned long long)passes, (t - 1) / lag + 1) : 0;
+    return full * Q + (part - full) * t - (part > full ? lag * ((part * (part - 1) - full * (full - 1)) / 2) : 0);
+}
+__device__ __forceinline__ GsItem gs_item(unsigned n, unsigned Q, unsigned passes, unsigned lag) {
+    if (passes == 1) return {n, 0u};
+    unsigned long long lo = 0, hi = Q + (unsigned long long)lag * (passes - 1);  // before(lo) <= n < before(hi)
+    while (hi - lo > 1) {
+        const unsigned long long mid = (lo + hi) / 2;
+        if (gs_items_before(mid, Q, passes, lag) <= n) lo = mid; else hi = mid;
+    }
+    const unsigned first = lo >= Q ? (unsigned)((lo - Q) / lag + 1) : 0u;  // passes that have places left at lo
+    const unsigned pass = first + (unsigned)(n - gs_items_before(lo, Q, passes, lag));
+    return {(unsigned)(lo - (unsigned long long)lag * pass), pass};
+}
+
 // Persistent CTAs take the wave's slabs from a counter, in the table's order (a slab only
 // waits for slabs taken before it, by CTAs that were running when they took them, so every
 // wait ends without a co-residency guarantee).  Per slab the first two warps watch the release
@@ -188,11 +228,12 @@ __device__ __forceinline__ float add4(float s, float4 q) {
 __global__ void __launch_bounds__(kGsThreadsMax, 1)
     k_gs_flow(float4 *pos4, unsigned v0, unsigned nv, unsigned smax, const unsigned *__restrict__ table, unsigned qcap,
               unsigned *next_slab, const uint2 *__restrict__ start, const unsigned *__restrict__ nbr,
-              const unsigned *__restrict__ word0, const unsigned *__restrict__ pack, unsigned *ext, unsigned stamp, int *err,
+              const unsigned *__restrict__ word0, const unsigned *__restrict__ pack, unsigned *ext,
+              const unsigned char *__restrict__ ext0, unsigned passes, unsigned stamp0, GsOrder ord, int *err,
               long long spin_cycles, unsigned long long *stats) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ GsQueue s_q;
-    __shared__ unsigned s_slab;
+    __shared__ unsigned s_slab, s_pass;
     // Per worker warp: the neighbours' coordinates, one row per component, summed in list order
     __shared__ __align__(16) float s_row[kGsThreadsMax / 32][3 * kGsRow];
     __shared__ unsigned s_void[32];  // target of touch_l1
@@ -207,7 +248,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
     const unsigned Q = min(__ldg(table), qcap);
     const unsigned *bnd = table + 1, *order = table + 2 + qcap;
     volatile unsigned *v_done = &s_q.done, *v_stop = &s_q.stop;
-    const float fstamp = __uint_as_float(stamp);
+    const unsigned lag = passes > 1 ? *ord.lag : 1u;
     const unsigned v_scratch = (unsigned)__cvta_generic_to_shared(&s_void[lane]);
     unsigned long long polls = 0;
     if (threadIdx.x == 0) {
@@ -218,11 +259,22 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
     for (;;) {
         if (threadIdx.x == 0) {
             const unsigned k = atomicAdd(next_slab, 1u);
-            s_slab = (k < Q && !s_q.stop) ? __ldg(order + k) : 0xffffffffu;
+            s_slab = 0xffffffffu;
+            if (k < Q * passes && !s_q.stop) {
+                const GsItem it = gs_item(k, Q, passes, lag);
+                s_slab = __ldg(order + it.place);
+                s_pass = it.pass;
+                if (it.pass && !gs_wait_pass(ord, s_slab, it.pass, spin_cycles)) {
+                    raise_error(err, QSES_ERR_TIMEOUT);
+                    s_q.stop = 1;
+                    s_slab = 0xffffffffu;
+                }
+            }
             s_q.ticket = 0; s_q.tail = 0; s_q.done = 0;
         }
         __syncthreads();
-        const unsigned p = s_slab;
+        const unsigned p = s_slab, pass = s_pass, stamp = stamp0 + pass;
+        const float fstamp = __uint_as_float(stamp);
         if (p >= Q) break;  // uniform per CTA: no slab left (or an error stopped this CTA)
         const unsigned a = __ldg(bnd + p), b = __ldg(bnd + p + 1), len = b - a;
         if (a < v0 || b > nv || b <= a || len > smax) {  // uniform: a malformed table entry
@@ -524,12 +576,65 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 q.w = fstamp;
                 st_pos(pos4 + a + k, q);
             }
+            if (pass + 1 < passes)
+                for (unsigned v = a + threadIdx.x; v < b; v += T) ((unsigned char *)ext)[v] = ext0[v];
         } else if (stats && threadIdx.x == 0) {
             atomicAdd(stats + 1, 1ull);  // unfinished slabs
         }
         __syncthreads();
+        if (pass + 1 < passes && threadIdx.x == 0 && *v_done >= len) {
+            __threadfence();  // the CTA's stores before the flag
+            st_release_u32(&ord.done[p], pass + 1);
+        }
     }  // next slab
     if (stats && threadIdx.x == 0) atomicMax(stats, polls);
+}
+
+// Where a vertex's lists end up, and the counts that make its word.
+struct GsVertex {
+    unsigned a, b;  // its slab's vertices
+    unsigned v0, v1;
+    unsigned loc, rem, far;  // distinct lower neighbours in the slab and below it; the highest above it
+    // An entry in the pass's form; `again`: an earlier one names the same vertex.
+    __device__ __forceinline__ unsigned take(unsigned v, unsigned u, bool again) {
+        const bool here = u >= a && u < b;
+        if (u < v && u >= v0 && !again) {  // below v0: an earlier wave, already final
+            if (here) loc++; else rem++;
+        }
+        if (u >= b && u < v1) far = max(far, u);
+        return (here ? u - a : u | 0x80000000u) | (u > v ? 0x40000000u : 0u) | (again || u >= v1 ? 0x20000000u : 0u);
+    }
+    __device__ __forceinline__ unsigned slab(const unsigned *__restrict__ table, unsigned v) {
+        const unsigned *bnd = table + 1;
+        unsigned lo = 0, hi = __ldg(table);  // bnd[lo] <= v < bnd[hi]
+        while (hi - lo > 1) {
+            const unsigned mid = (lo + hi) >> 1;
+            if (__ldg(bnd + mid) <= v) lo = mid; else hi = mid;
+        }
+        a = __ldg(bnd + lo);
+        b = __ldg(bnd + lo + 1);
+        return lo;
+    }
+    // w: the word but for its counts.  A vertex is the weld of edges around one grid corner, so its
+    // distinct neighbours lie on the 54 edges of 8 cells: both counts stay below their fields.
+    __device__ __forceinline__ void write(unsigned v, unsigned lo, unsigned w, unsigned *__restrict__ word0,
+                                          unsigned char *__restrict__ ext, unsigned char *__restrict__ ext0,
+                                          const GsOrder &ord, int *err) const {
+        if (rem > 255u || loc > 0x7eu) raise_error(err, QSES_ERR_INTERNAL);
+        word0[v] = w | (loc + (rem ? 1u + kGsPend : 0u));
+        ext[v] = (unsigned char)rem;
+        if (ext0) {  // several passes in one launch
+            ext0[v] = (unsigned char)rem;
+            if (far) atomicMax(&ord.far[lo], far);
+        }
+    }
+};
+
+// The two other corners of corner q's triangle, in triangle order.
+__device__ __forceinline__ uint2 gs_corners(const unsigned *__restrict__ tri, unsigned q) {
+    const unsigned t = q / 3u, c = q - 3u * t;
+    const unsigned x = tri[3ull * t], y = tri[3ull * t + 1], z = tri[3ull * t + 2];
+    return make_uint2(c == 0 ? y : x, c == 2 ? y : z);
 }
 
 // Neighbour lists without a sort of all corners: occ holds each vertex's triangle corners in any
@@ -539,106 +644,164 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
 // form the pass reads, and the count of neighbours in lower slabs.  Vertices [v0, v1) form the
 // slabs of the table (Q, then Q + 1 bounds in id order).  Neighbours below v0 belong to waves that
 // finished before this one (final values); neighbours at or above v1 are read before their update.
-__global__ void __launch_bounds__(128) k_gs_lists(const unsigned *__restrict__ tri, unsigned *__restrict__ occ,
-                                                  const uint2 *__restrict__ start, unsigned *__restrict__ nbr, unsigned v0,
-                                                  unsigned v1, unsigned smax, const unsigned *__restrict__ table,
+// A thread per vertex; vertices of more than 8 corners are left to k_gs_lists_long, as a few of
+// them among a warp's 32 hold up all (3 540 000 vertices, 10 % of them long: the whole list stage
+// 1.19 ms with one kernel, 0.83 with two).
+__global__ void __launch_bounds__(128) k_gs_lists(const unsigned *__restrict__ tri, const unsigned *__restrict__ occ,
+                                                  const uint2 *__restrict__ start, unsigned v0, unsigned v1,
+                                                  unsigned smax, const unsigned *__restrict__ table,
                                                   unsigned *__restrict__ word0, uint4 *__restrict__ pack,
-                                                  unsigned char *__restrict__ ext, int *err) {
+                                                  unsigned char *__restrict__ ext, unsigned char *__restrict__ ext0,
+                                                  GsOrder ord, unsigned *__restrict__ longs, int *err) {
     const unsigned v = v0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= v1) return;
-    const unsigned *bnd = table + 1;
-    unsigned lo = 0, hi = __ldg(table);  // bnd[lo] <= v < bnd[hi]
-    while (hi - lo > 1) {
-        const unsigned mid = (lo + hi) >> 1;
-        if (__ldg(bnd + mid) <= v) lo = mid; else hi = mid;
+    const unsigned o0 = start[v].x, m = start[v + 1].x - o0;  // corners
+    if (m > 8) {
+        longs[atomicAdd(ord.longs, 1u)] = v;
+        return;
     }
-    const unsigned a = __ldg(bnd + lo), b = __ldg(bnd + lo + 1);
-    const unsigned o0 = start[v].x, m = start[v + 1].x - o0;  // occurrences
-    unsigned loc = 0, rem = 0, w;
-    // An entry in the pass's form; `again`: an earlier one names the same vertex.
-    auto take = [&](unsigned u, bool again) {
-        const bool here = u >= a && u < b;
-        if (u < v && u >= v0 && !again) {  // below v0: an earlier wave, already final
-            if (here) loc++; else rem++;
+    GsVertex g{0, 0, v0, v1, 0, 0, 0};
+    const unsigned lo = g.slab(table, v);
+    unsigned r[8];
+#pragma unroll
+    for (unsigned i = 0; i < 8; i++) r[i] = i < m ? occ[o0 + i] : 0xffffffffu;
+#pragma unroll
+    for (unsigned i = 1; i < 8; i++) {
+#pragma unroll
+        for (unsigned j = i; j > 0; j--) {
+            const unsigned x = r[j - 1], y = r[j];
+            r[j - 1] = min(x, y);
+            r[j] = max(x, y);
         }
-        return (here ? u - a : u | 0x80000000u) | (u > v ? 0x40000000u : 0u) | (again || u >= v1 ? 0x20000000u : 0u);
-    };
-    if (m <= 8) {
-        unsigned r[8];
+    }
+    unsigned id[16];
 #pragma unroll
-        for (unsigned i = 0; i < 8; i++) r[i] = i < m ? occ[o0 + i] : 0xffffffffu;
+    for (unsigned i = 0; i < 8; i++) {
+        const uint2 e = i < m ? gs_corners(tri, r[i]) : make_uint2(0xffffffffu, 0xffffffffu);
+        id[2 * i] = e.x;
+        id[2 * i + 1] = e.y;
+    }
+    unsigned code[16];
 #pragma unroll
-        for (unsigned i = 1; i < 8; i++) {
+    for (unsigned i = 0; i < 16; i++) {
+        bool again = false;
 #pragma unroll
-            for (unsigned j = i; j > 0; j--) {
-                const unsigned x = r[j - 1], y = r[j];
-                r[j - 1] = min(x, y);
-                r[j] = max(x, y);
-            }
-        }
-        unsigned id[16];
+        for (unsigned j = 0; j < i; j++) again |= id[j] == id[i];
+        code[i] = i < 2 * m ? g.take(v, id[i], again) : smax;
+    }
 #pragma unroll
-        for (unsigned i = 0; i < 8; i++) {
-            id[2 * i] = id[2 * i + 1] = 0xffffffffu;
-            if (i < m) {
-                const unsigned t = r[i] / 3u, c = r[i] - 3u * t;
-                const unsigned x = tri[3ull * t], y = tri[3ull * t + 1], z = tri[3ull * t + 2];
-                id[2 * i] = c == 0 ? y : x;
-                id[2 * i + 1] = c == 2 ? y : z;
-            }
-        }
-        unsigned code[16];
-#pragma unroll
-        for (unsigned i = 0; i < 16; i++) {
-            bool again = false;
-#pragma unroll
-            for (unsigned j = 0; j < i; j++) again |= id[j] == id[i];
-            code[i] = i < 2 * m ? take(id[i], again) : smax;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            pack[4 * (size_t)v + j] = make_uint4(code[4 * j], code[4 * j + 1], code[4 * j + 2], code[4 * j + 3]);
-        w = m << 9;
-    } else {
-        // insertion sort in place in global memory
-        for (unsigned i = 1; i < m; i++) {
-            const unsigned x = occ[o0 + i];
-            unsigned j = i;
-            while (j > 0 && occ[o0 + j - 1] > x) {
-                occ[o0 + j] = occ[o0 + j - 1];
-                j--;
-            }
-            occ[o0 + j] = x;
-        }
+    for (int j = 0; j < 4; j++)
+        pack[4 * (size_t)v + j] = make_uint4(code[4 * j], code[4 * j + 1], code[4 * j + 2], code[4 * j + 3]);
+    g.write(v, lo, m << 9, word0, ext, ext0, ord, err);
+}
+
+// The vertices of more than 8 corners: a warp each, a corner per lane, sorted by counting the
+// smaller ones; their lists go to the neighbour table at twice the vertex's offset.
+__global__ void __launch_bounds__(256) k_gs_lists_long(const unsigned *__restrict__ tri, unsigned *__restrict__ occ,
+                                                       const uint2 *__restrict__ start, unsigned *__restrict__ nbr,
+                                                       unsigned v0, unsigned v1, const unsigned *__restrict__ table,
+                                                       unsigned *__restrict__ word0, unsigned char *__restrict__ ext,
+                                                       unsigned char *__restrict__ ext0, GsOrder ord,
+                                                       const unsigned *__restrict__ longs, int *err) {
+    __shared__ unsigned s_id[8][64];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, count = *ord.longs;
+    unsigned *row = s_id[warp];
+    for (unsigned x = blockIdx.x * 8 + warp; x < count; x += gridDim.x * 8) {
+        const unsigned v = longs[x], o0 = start[v].x, m = start[v + 1].x - o0;
+        GsVertex g{0, 0, v0, v1, 0, 0, 0};
+        const unsigned lo = g.slab(table, v);
         unsigned *list = nbr + 2 * (size_t)o0;
-        for (unsigned i = 0; i < m; i++) {
-            const unsigned q = occ[o0 + i], t = q / 3u, c = q - 3u * t;
-            const unsigned x = tri[3ull * t], y = tri[3ull * t + 1], z = tri[3ull * t + 2];
-            list[2 * i] = c == 0 ? y : x;
-            list[2 * i + 1] = c == 2 ? y : z;
+        if (m <= 32) {
+            const unsigned q = lane < m ? occ[o0 + lane] : 0xffffffffu;
+            unsigned rank = 0;
+            for (unsigned j = 0; j < m; j++) rank += __shfl_sync(0xffffffffu, q, j) < q;
+            if (lane < m) {
+                const uint2 e = gs_corners(tri, q);
+                row[2 * rank] = e.x;
+                row[2 * rank + 1] = e.y;
+            }
+            __syncwarp();
+            for (unsigned e = lane; e < 2 * m; e += 32) {
+                const unsigned u = row[e];
+                bool again = false;
+                for (unsigned j = 0; j < e; j++) again |= row[j] == u;
+                list[e] = g.take(v, u, again);
+            }
+            __syncwarp();  // the row is rewritten for the next vertex
+            g.loc = __reduce_add_sync(0xffffffffu, g.loc);
+            g.rem = __reduce_add_sync(0xffffffffu, g.rem);
+            g.far = __reduce_max_sync(0xffffffffu, g.far);
+        } else if (lane == 0) {
+            // insertion sort in place
+            for (unsigned i = 1; i < m; i++) {
+                const unsigned q = occ[o0 + i];
+                unsigned j = i;
+                while (j > 0 && occ[o0 + j - 1] > q) {
+                    occ[o0 + j] = occ[o0 + j - 1];
+                    j--;
+                }
+                occ[o0 + j] = q;
+            }
+            for (unsigned i = 0; i < m; i++) {
+                const uint2 e = gs_corners(tri, occ[o0 + i]);
+                list[2 * i] = e.x;
+                list[2 * i + 1] = e.y;
+            }
+            for (unsigned i = 2 * m; i-- > 0;) {  // from the end: the entries before are still ids
+                const unsigned u = list[i];
+                bool again = false;
+                for (unsigned j = 0; j < i; j++) again |= list[j] == u;
+                list[i] = g.take(v, u, again);
+            }
         }
-        for (unsigned i = 2 * m; i-- > 0;) {  // from the end: the entries before are still ids
-            const unsigned u = list[i];
-            bool again = false;
-            for (unsigned j = 0; j < i; j++) again |= list[j] == u;
-            list[i] = take(u, again);
-        }
-        const unsigned o = o0 - start[a].x;
-        w = kGsLong | (o < (1u << 17) && m < kGsLost ? m << 9 | o << 15 : kGsLost << 9);
+        const unsigned o = o0 - start[g.a].x;
+        if (lane == 0)
+            g.write(v, lo, kGsLong | (o < (1u << 17) && m < kGsLost ? m << 9 | o << 15 : kGsLost << 9), word0, ext, ext0, ord,
+                    err);
     }
-    // A vertex is the weld of edges around one grid corner, so its distinct neighbours lie on the
-    // 54 edges of 8 cells: both counts stay below their fields.
-    if (rem > 255u || loc > 0x7eu) raise_error(err, QSES_ERR_INTERNAL);
-    word0[v] = w | (loc + (rem ? 1u + kGsPend : 0u));
-    ext[v] = (unsigned char)rem;
+}
+
+// The slab of each slab's highest neighbour, and how many places of the order a slab's passes have
+// to lie behind one another for all such neighbours to have had the pass before.  One CTA.
+__global__ void __launch_bounds__(1024) k_gs_order(const unsigned *__restrict__ table, unsigned qcap, GsOrder ord) {
+    __shared__ unsigned s_lag;
+    const unsigned Q = min(__ldg(table), qcap);
+    const unsigned *bnd = table + 1, *order = table + 2 + qcap;
+    if (threadIdx.x == 0) s_lag = 0;
+    for (unsigned x = threadIdx.x; x < Q; x += blockDim.x) ord.place[order[x]] = x;
+    __syncthreads();
+    unsigned lag = 0;
+    for (unsigned q = threadIdx.x; q < Q; q += blockDim.x) {
+        unsigned lo = q, hi = Q;  // bnd[lo] <= far < bnd[hi]
+        const unsigned far = ord.far[q];
+        if (far >= bnd[q])
+            while (hi - lo > 1) {
+                const unsigned mid = (lo + hi) >> 1;
+                if (__ldg(bnd + mid) <= far) lo = mid; else hi = mid;
+            }
+        ord.far[q] = lo;
+        const unsigned from = ord.place[q], to = ord.place[lo];
+        if (to > from) lag = max(lag, to - from);
+    }
+    atomicMax(&s_lag, lag);
+    __syncthreads();
+    if (threadIdx.x == 0) *ord.lag = s_lag + 1;
 }
 
 // ------------------------------------------------------------ launchers
 
 void launch_gs_lists(const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
-                     unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext, int *err,
-                     cudaStream_t s) {
-    k_gs_lists<<<(v1 - v0 + 127) / 128, 128, 0, s>>>(tri, occ, start, nbr, v0, v1, smax, table, word0, pack, ext, err);
+                     unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext,
+                     unsigned char *ext0, const GsOrder &ord, unsigned *longs, int *err, cudaStream_t s) {
+    k_gs_lists<<<(v1 - v0 + 127) / 128, 128, 0, s>>>(tri, occ, start, v0, v1, smax, table, word0, pack, ext, ext0, ord, longs,
+                                                     err);
+    // as many CTAs as fit the SMs, or as there can be vertices for
+    const unsigned ctas = (v1 - v0 + 63) / 64;
+    k_gs_lists_long<<<ctas < 1216u ? ctas : 1216u, 256, 0, s>>>(tri, occ, start, nbr, v0, v1, table, word0, ext, ext0, ord,
+                                                                longs, err);
+}
+void launch_gs_order(const unsigned *table, unsigned qcap, const GsOrder &ord, cudaStream_t s) {
+    k_gs_order<<<1, 1024, 0, s>>>(table, qcap, ord);
 }
 
 size_t gs_slab_smem(unsigned S) { return gs_smem(S).bytes; }
@@ -646,13 +809,14 @@ size_t gs_slab_smem(unsigned S) { return gs_smem(S).bytes; }
 cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax, const unsigned *table,
                            unsigned qcap, unsigned *next_slab, int P, int threads,
                            const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
-                           unsigned stamp, int *err, long long spin_cycles, unsigned long long *stats, cudaStream_t s) {
+                           const unsigned char *ext0, unsigned passes, unsigned stamp, const GsOrder &ord, int *err,
+                           long long spin_cycles, unsigned long long *stats, cudaStream_t s) {
     if (smax == 0 || smax > kGsSlabCap) return cudaErrorInvalidValue;
     const size_t smem = gs_slab_smem(smax);
     const void *fn = (const void *)k_gs_flow;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs_slab_smem(kGsSlabCap));
     void *args[] = {&pos, &v0, &nv, &smax, (void *)&table, &qcap, &next_slab, (void *)&start, (void *)&nbr,
-                    (void *)&word0, (void *)&pack, &ext, &stamp, &err, &spin_cycles, &stats};
+                    (void *)&word0, (void *)&pack, &ext, (void *)&ext0, &passes, &stamp, (void *)&ord, &err, &spin_cycles, &stats};
     // A cooperative launch: every CTA resident from the start.  (A plain launch would also be
     // safe - a CTA only waits for slabs taken before its own, by CTAs that were running when
     // they took them - but its CTAs can then take the SMs the side stream's kernels wait for.)

@@ -38,23 +38,32 @@ void launch_csr_scatter(const unsigned *tri, size_t n3, uint2 *start, unsigned *
 // Slab table of one Gauss-Seidel wave (device words): [0] Q slabs, [1, Q + 2) their bounds in
 // id order (qcap + 1 slots), [qcap + 2, qcap + 2 + Q) the slab ids in the order CTAs take them.
 inline size_t gs_table_words(unsigned qcap) { return 2ull * qcap + 2; }
+// Several passes in one launch: done (zeroed) passes of each slab, far (zeroed, then filled by
+// launch_gs_lists with each slab's highest neighbour id and by launch_gs_order with its slab).
+struct GsOrder {
+    unsigned *lag, *longs;         // one value each; longs (zeroed): vertices with long lists
+    unsigned *done, *far, *place;  // one per slab each
+};
 // The pass's lists from the occurrences: word0, pack (64 B) per vertex, lists of more than 16
-// entries in nbr (2 n3) at twice the vertex's offset (k_smooth.cu); ext: one byte per vertex, the
-// neighbours in lower slabs still to come.
+// entries in nbr (2 n3) at twice the vertex's offset (k_smooth.cu); ext, ext0 (may be null): one
+// byte per vertex, the neighbours in lower slabs still to come; longs: scratch, one per vertex.
 void launch_gs_lists(const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
-                     unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext, int *err,
-                     cudaStream_t s);
+                     unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext,
+                     unsigned char *ext0, const GsOrder &ord, unsigned *longs, int *err, cudaStream_t s);
+void launch_gs_order(const unsigned *table, unsigned qcap, const GsOrder &ord, cudaStream_t s);
 size_t gs_slab_smem(unsigned S);
 void launch_to_float4(const float *v3, unsigned nv, float4 *v4, cudaStream_t s);
 void launch_from_float4(const float4 *v4, unsigned nv, float *v3, cudaStream_t s);
-// One Gauss-Seidel pass over vertices [v0, nv) in the table's slabs (each at most smax
-// vertices), taken by P persistent CTAs from *next_slab (zeroed).  stamp: written to w of every
-// position updated (another value than any position holds before the pass).  threads: 512 or
-// 1024 per slab CTA.
+// Gauss-Seidel passes over vertices [v0, nv) in the table's slabs (each at most smax
+// vertices), taken by P persistent CTAs from *next_slab (zeroed).  passes > 1: that many passes,
+// each following the one before through the slabs (ext0: the release counters a pass starts with).
+// stamp: written to w of every position updated, one more for each pass (another value than any
+// position holds before).  threads: 512 or 1024 per slab CTA.
 cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax, const unsigned *table,
                            unsigned qcap, unsigned *next_slab, int P, int threads,
                            const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
-                           unsigned stamp, int *err, long long spin_cycles, unsigned long long *stats, cudaStream_t s);
+                           const unsigned char *ext0, unsigned passes, unsigned stamp, const GsOrder &ord, int *err,
+                           long long spin_cycles, unsigned long long *stats, cudaStream_t s);
 int gs_slab_max_blocks(int device, unsigned S, int threads);
 
 // Gauss-Seidel launch shape: threads per slab CTA and the slab size aimed at (vertices);
@@ -80,7 +89,7 @@ inline bool gs_flags_valid(unsigned f) { return f < 64 && (f & (kGsPair | kGsQua
 void gs_l2_window(int device, cudaStream_t s, const void *p, size_t bytes);
 // Tuned shape for a mesh of nv vertices (batch: many molecules), or the default; biggest: the
 // vertices of the largest molecule.
-GsShape gs_shape(unsigned nv, bool batch, unsigned biggest);
+GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes);
 void gs_shape_record(unsigned nv, bool batch, GsShape s);
 void gs_shape_record_all(bool batch, GsShape s);  // every mesh-size class
 int gs_shape_candidates(GsShape *out, int max);

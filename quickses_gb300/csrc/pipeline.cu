@@ -133,7 +133,7 @@ static bool g_tuned[2][33];
 
 static int tune_bucket(unsigned nv) { return bits_for(nv); }
 
-GsShape gs_shape(unsigned nv, bool batch, unsigned biggest) {
+GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     const int b = tune_bucket(nv);
     if (g_tuned[batch][b]) return g_tune[batch][b];
@@ -145,7 +145,9 @@ GsShape gs_shape(unsigned nv, bool batch, unsigned biggest) {
     // once are a matter of throughput: two CTAs per SM (14 200 000 vertices: 9.66 ms; one CTA of
     // 11 904 10.36; a batch of 29 600 000: 6.7 against 8.1).  14 worker warps per CTA are enough, as
     // each takes a second vertex when more are ready: 1 024 threads 1-9 % slower.
-    const unsigned t = (unsigned)(6.5 * std::sqrt((double)biggest));
+    // Several passes follow one another through the slabs and want shorter ones (548 000 vertices, 3
+    // passes: 4 096 per slab 2.73 ms, 4 811 2.87, 2 048 2.90).
+    const unsigned t = (unsigned)((passes > 1 ? 5.3 : 6.5) * std::sqrt((double)biggest));
     return GsShape{512, nv > 8000000u ? kGsSlabTwo : std::min(std::max(t, 256u), kGsSlabCap), 0, 0};
 }
 
@@ -366,12 +368,19 @@ int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_of
 
 int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out) {
     const size_t words = pl.table.size();
-    const size_t need = align256(4 * words) + 4096;
+    const size_t order_words = 64 + 3ull * pl.L.qcap + 64;
+    const size_t need = align256(4 * words) + align256(4 * order_words) + 4096;
     const void *old_ws = ctx->gs_ws.base;
     if (ctx->gs_ws.reserve(need) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "smoothing workspace");
     if (ctx->gs_ws.base != old_ws) QSES_SEG_TRACE("smoothing workspace moved (%zu bytes)\n", need);
     out.table = (unsigned *)ctx->gs_ws.take(4 * words);
-    out.next_slab = (unsigned *)ctx->gs_ws.take(256);
+    out.next_slab = (unsigned *)ctx->gs_ws.take(4 * order_words);
+    out.ord.lag = out.next_slab + 1;
+    out.ord.longs = out.next_slab + 2;
+    out.ord.done = out.next_slab + 64;
+    out.ord.far = out.ord.done + pl.L.qcap;
+    out.ord.place = out.ord.far + pl.L.qcap;
+    out.zero_words = 64 + 2ull * pl.L.qcap;
     if (!out.next_slab) return ctx->fail(QSES_ERR_INTERNAL, "smoothing workspace layout");
     if (4 * words > ctx->h_gs_cap) {
         QSES_SEG_TRACE("slab tables: pinned buffer grows to %zu words\n", words);
@@ -393,32 +402,38 @@ int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out) {
 
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, float4 *pos4,
                   unsigned nv, const unsigned *tri, unsigned *occ, const uint2 *deg, unsigned *nbr, unsigned *word0,
-                  uint4 *pack, unsigned *ext, unsigned *ext0,
-                  unsigned *table, const unsigned *h_table, unsigned *next_slab, int *d_err,
-                  unsigned long long *stats, cudaEvent_t before_writeback) {
+                  uint4 *pack, unsigned *ext, unsigned *ext0, unsigned *scratch, const GsBuffers &gb,
+                  const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback) {
     cudaStream_t s = ctx->stream;
     launch_to_float4(vq, nv, pos4, s);
     ctx->launches++;
     if (sh.flags & kGsPersistL2) gs_l2_window(ctx->device, s, pos4, 16ull * nv);
     if (stats) QCHK(cudaMemsetAsync(stats, 0, 64, s));
-    QCHK(cudaMemcpyAsync(table, h_table, 4ull * L.waves * L.table_words, cudaMemcpyHostToDevice, s));
+    QCHK(cudaMemcpyAsync(gb.table, h_table, 4ull * L.waves * L.table_words, cudaMemcpyHostToDevice, s));
+    // several passes over one wave run in one launch, each following the one before through the slabs
+    const bool together = L.waves == 1;
+    QCHK(cudaMemsetAsync(gb.next_slab, 0, 4 * gb.zero_words, s));
     for (unsigned w = 0; w < L.waves; w++) {
         const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
-        launch_gs_lists(tri, occ, deg, nbr, v0, v1, L.smax, table + (size_t)w * L.table_words, word0, pack,
-                        (unsigned char *)(passes > 1 ? ext0 : ext), d_err, s);
+        if (w) QCHK(cudaMemsetAsync(gb.ord.longs, 0, 4, s));
+        launch_gs_lists(tri, occ, deg, nbr, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, word0, pack,
+                        (unsigned char *)ext, passes > 1 ? (unsigned char *)ext0 : nullptr, gb.ord, scratch, d_err, s);
+        ctx->launches += 2;
+    }
+    if (together && passes > 1) {
+        launch_gs_order(gb.table, L.qcap, gb.ord, s);
         ctx->launches++;
     }
     ctx->mark("smooth_csr");
-    for (int pass = 0; pass < passes; pass++) {
-        if (passes > 1) QCHK(cudaMemcpyAsync(ext, ext0, nv, cudaMemcpyDeviceToDevice, s));
+    for (int pass = 0; pass < (together ? 1 : passes); pass++) {
+        if (pass) QCHK(cudaMemcpyAsync(ext, ext0, nv, cudaMemcpyDeviceToDevice, s));
         for (unsigned w = 0; w < L.waves; w++) {
             const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
-            const unsigned *tb = table + (size_t)w * L.table_words;
-            QCHK(cudaMemsetAsync(next_slab, 0, 4, s));
-            // per-update cycle counters only on profiled calls: their clock reads sit on the
-            // dependency chain (1.4 % of the pass on 50 000 atoms)
-            QCHK(launch_gs_slab(pos4, v0, v1, L.smax, tb, L.qcap, next_slab, L.ctas, sh.threads, deg, nbr, word0,
-                                pack, ext, (unsigned)pass + 1u, d_err, 4000000000ll, ctx->profiling ? stats : nullptr, s));
+            if (pass || w) QCHK(cudaMemsetAsync(gb.next_slab, 0, 4, s));
+            QCHK(launch_gs_slab(pos4, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, L.qcap, gb.next_slab, L.ctas,
+                                sh.threads, deg, nbr, word0, pack, ext, (const unsigned char *)ext0,
+                                together ? (unsigned)passes : 1u, (unsigned)pass + 1u, gb.ord, d_err, 4000000000ll,
+                                ctx->profiling ? stats : nullptr, s));
             ctx->launches++;
         }
     }
@@ -544,10 +559,10 @@ struct FinishSeg {
     float4 *pos4;
     unsigned *word0;       // per vertex: word and common list of the smoothing pass
     uint4 *pack;
+    unsigned *scratch;     // one word per vertex
     unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
-    unsigned *table;
+    GsBuffers gb;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
-    unsigned *next_slab;
     unsigned long long *stats;
     unsigned long long n3;
     unsigned nv, nt;
@@ -603,7 +618,7 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
         ctx->launches++;
         // the closest-atom pass on the side stream reads the welded positions in vq
         const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.tri, c.okey, c.deg, c.nbr, c.word0, c.pack, c.ext, c.ext0,
-                                     c.table, c.h_table, c.next_slab, c.err, c.stats, c.fork ? ctx->ev_join : nullptr);
+                                     c.scratch, c.gb, c.h_table, c.err, c.stats, c.fork ? ctx->ev_join : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -844,6 +859,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     c.pack = pack;
     c.ext = ext;
     c.ext0 = ext0;
+    c.scratch = vmap;  // free after the weld
     c.stats = (unsigned long long *)((char *)ctx->small + 256);
     c.n3 = n3;
     c.nv = nv;
@@ -853,7 +869,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     c.fork = !ctx->profiling && ctx->side != nullptr;
     const bool smoothing = p.smooth_passes > 0 && nv > 0 && T > 0;
     if (smoothing) {
-        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv);
+        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv, p.smooth_passes);
         ctx->gs_used = c.sh;
         GsPlan plan;
         rc = gs_plan(ctx->device, c.sh, nv, nullptr, nullptr, 1, plan);
@@ -861,9 +877,8 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
         GsBuffers gb;
         QCHK_RC(gs_buffers(ctx, plan, gb));
         c.gl = plan.L;
-        c.table = gb.table;
+        c.gb = gb;
         c.h_table = ctx->h_gs;
-        c.next_slab = gb.next_slab;
         ctx->diag[0] = plan.max_slabs;
         ctx->diag[1] = plan.max_len;
     }

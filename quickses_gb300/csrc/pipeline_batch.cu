@@ -198,10 +198,10 @@ struct BatchFinishSeg {
     float4 *pos4;
     unsigned *word0;       // per vertex: word and common list of the smoothing pass
     uint4 *pack;
+    unsigned *scratch;     // one word per vertex
     unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
-    unsigned *table;
+    GsBuffers gb;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
-    unsigned *next_slab;
     unsigned long long n3;
     unsigned nv, nt;
     int passes, fork;
@@ -261,7 +261,7 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
         ctx->launches++;
         // the closest-atom pass on the side stream reads the welded positions in vq
         const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.tri, c.okey, c.deg, c.nbr, c.word0, c.pack, c.ext, c.ext0,
-                                     c.table, c.h_table, c.next_slab, c.err, nullptr, c.fork ? ctx->ev_join : nullptr);
+                                     c.scratch, c.gb, c.h_table, c.err, nullptr, c.fork ? ctx->ev_join : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -562,6 +562,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     c.pack = pack;
     c.ext = ext;
     c.ext0 = ext0;
+    c.scratch = vmap;  // free after the weld
     c.n3 = n3;
     c.nv = nv;
     c.nt = T;
@@ -571,7 +572,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     if (smoothing) {
         unsigned biggest = 0;
         for (unsigned m = 0; m < nm; m++) biggest = std::max(biggest, vtx_off[m + 1] - vtx_off[m]);
-        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, true, biggest);
+        c.sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, true, biggest, passes);
         ctx->gs_used = c.sh;
         // molecules are never split between slabs unless larger than one; their grid sizes
         // estimate the dependency depths that order the slabs
@@ -583,9 +584,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         GsBuffers gb;
         QCHK_RC(gs_buffers(ctx, plan, gb));
         c.gl = plan.L;
-        c.table = gb.table;
+        c.gb = gb;
         c.h_table = ctx->h_gs;
-        c.next_slab = gb.next_slab;
         ctx->diag[0] = std::max<unsigned long long>(ctx->diag[0], plan.max_slabs);
         ctx->diag[1] = std::max<unsigned long long>(ctx->diag[1], plan.max_len);
     }

@@ -278,7 +278,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                     SCHK(scan_u2(deg, deg, nv + 1, nullptr, tmpb, d_err, s, &ctx->launches));
                     launch_csr_scatter(tri, n3k, deg, okey, s);
                     ctx->launches += 2;
-                    GsShape sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv);
+                    GsShape sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv, p.smooth_passes);
                     ctx->gs_used = sh;
                     GsPlan plan;
                     const int prc = gs_plan(ctx->device, sh, nv, nullptr, nullptr, 1, plan);
@@ -287,7 +287,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                     const int brc = gs_buffers(ctx, plan, gb);
                     if (brc != QSES_OK) return brc;
                     const int src = run_smoothing(ctx, sh, plan.L, p.smooth_passes, vq2, pos4, nv, tri, okey, deg, nbr,
-                                                  word0, pack, ext, ext0, gb.table, ctx->h_gs, gb.next_slab, d_err,
+                                                  word0, pack, ext, ext0, vmap, gb, ctx->h_gs, d_err,
                                                   stats);
                     if (src != QSES_OK) return src;
                 }

@@ -188,17 +188,26 @@ struct SlicedMesh {
 };
 int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_xyz, const float *d_r, unsigned n,
                         SlicedMesh &out);
+// The smoothing workspace of a plan (slab tables, the slab counter, the passes' order) in
+// ctx->gs_ws and the plan's tables in ctx->h_gs.  Returns QSES_OK or an error code (ctx->fail called).
+struct GsBuffers {
+    unsigned *table, *next_slab;
+    GsOrder ord;
+    unsigned long long zero_words;  // from next_slab on: the counter, ord.done and ord.far
+};
+int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out);
 // `passes` exact Gauss-Seidel passes over vertices [0, nv): positions vq (3 floats each) in
-// and out, triangle corners occ scattered per vertex (deg offsets), shape sh.  The vertices run in sequential waves of at
-// most the slab kernel's capacity; every dependency points to a lower id, so a wave only
-// depends on earlier, finished waves.
+// and out, triangle corners occ scattered per vertex (deg offsets), shape sh; scratch: one word
+// per vertex.  Vertices in one
+// wave: one launch for all passes.  Otherwise waves and passes follow one another; every
+// dependency points to a lower id, so a wave only depends on earlier, finished waves.
 // `before_writeback` (may be null): event the stream waits for before the smoothed
 // positions overwrite vq (work on another stream that still reads the welded positions).
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, float4 *pos4,
                   unsigned nv, const unsigned *tri, unsigned *occ, const uint2 *deg, unsigned *nbr, unsigned *word0,
-                  uint4 *pack, unsigned *ext, unsigned *ext0,
-                  unsigned *table, const unsigned *h_table, unsigned *next_slab, int *d_err,
-                  unsigned long long *stats, cudaEvent_t before_writeback = nullptr);
+                  uint4 *pack, unsigned *ext, unsigned *ext0, unsigned *scratch, const GsBuffers &gb,
+                  const unsigned *h_table, int *d_err, unsigned long long *stats,
+                  cudaEvent_t before_writeback = nullptr);
 // Slab plan of a pass over nv vertices.  mol_off (nm + 1 entries, null for one molecule):
 // the molecules' vertex ranges, never split by a slab boundary unless a molecule is larger
 // than the slab size; mol_depth: a per-molecule estimate of the dependency depth (grid size),
@@ -208,12 +217,6 @@ int gs_plan(int device, const GsShape &sh, unsigned nv, const unsigned *mol_off,
 // The same for at most pmax resident slab CTAs (no device query).
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
                 GsPlan &pl);
-// The smoothing workspace of a plan (slab tables and the slab counter) in ctx->gs_ws and the
-// plan's tables in ctx->h_gs.  Returns QSES_OK or an error code (ctx->fail called).
-struct GsBuffers {
-    unsigned *table, *next_slab;
-};
-int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out);
 // All items share `passes`; the weld keys of every item fit `key_bits` bits and
 // key_bits + bits(count - 1) <= 64.  Results in ctx->batch.
 int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes, int key_bits);
