@@ -537,7 +537,8 @@ QSES_API int qses_compute_batch(qses_context *ctx, const qses_request *reqs, uns
         const std::vector<unsigned> &ids = grp.second;
         size_t at = 0;
         while (at < ids.size()) {
-            // Largest prefix whose molecule-tagged weld keys fit 64 bits.
+            // One pass takes at most as many molecules as their grids' positions and a molecule
+            // number fit 64 bits: it bounds the pass by the size of the grids in it.
             size_t end = at;
             int kb = 0;
             while (end < ids.size()) {
@@ -560,7 +561,7 @@ QSES_API int qses_compute_batch(qses_context *ctx, const qses_request *reqs, uns
             }
             ctx->dl = qses::HostDownload();
             ctx->dl.want = true;
-            int rc = qses::run_batch(ctx, items.data(), (unsigned)items.size(), grp.first, kb);
+            int rc = qses::run_batch(ctx, items.data(), (unsigned)items.size(), grp.first);
             if (rc != QSES_OK && ctx->dl.block) {  // copies into it may still be queued
                 cudaStreamSynchronize(ctx->stream);
                 cudaStreamSynchronize(ctx->side);

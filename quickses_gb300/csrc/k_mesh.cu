@@ -6,7 +6,7 @@
 //                 one quantised key per active edge (generateTriangleVerticesSMEM +
 //                 groupVertices, MarchingCubes.cu:736-862).  One warp per row; the sign of
 //                 32 voxels is one word, so cube indices and edge activity are bit ops.
-//  k_weld_*       unique quantised positions in lexicographic order (CudaSurf.cu:444-457)
+//  k_weld         unique quantised positions in lexicographic order (CudaSurf.cu:444-457)
 //  k_closest      closest atom per welded vertex (closestAtomPerVertex, Kernels.cu:547-604)
 //  k_tri_*        drop triangles with a repeated index (CudaSurf.cu:820-829)
 //  k_csr_*        neighbour lists in triangle order (getNeighboorsVertices,
@@ -64,9 +64,7 @@ __device__ unsigned long long edge_key(const QGrid &g, const unsigned char *__re
     long long mx = (long long)roundf(__fdiv_rn(p[0], QSES_WELD_TOL));
     long long my = (long long)roundf(__fdiv_rn(p[1], QSES_WELD_TOL));
     long long mz = (long long)roundf(__fdiv_rn(p[2], QSES_WELD_TOL));
-    return ((unsigned long long)(mx - g.bx) * (unsigned long long)g.Rq + (unsigned long long)(my - g.by)) *
-               (unsigned long long)g.Rq +
-           (unsigned long long)(mz - g.bz);
+    return ((unsigned long long)(mx - g.bx) << 42) | ((unsigned long long)(my - g.by) << 21) | (unsigned long long)(mz - g.bz);
 }
 
 __device__ __forceinline__ unsigned sel4(int o, unsigned a, unsigned b, unsigned c, unsigned d) {
@@ -98,8 +96,6 @@ __device__ __forceinline__ unsigned grp_incl_scan(unsigned v, int sub, int Lg) {
 
 // One owner row (i, j) of a molecule's grid per group of Lg lanes; every lane of the warp
 // calls this (groups whose row is past the end pass valid = false and write nothing).
-// Edge keys get `keyhi` added (the molecule's slot above the local key bits in a batch, 0
-// for a single molecule).
 // Bits [a, b) of a 32-bit word, the bounds clamped to [0, 32].
 __device__ __forceinline__ unsigned bits_in(int a, int b) {
     a = max(a, 0);
@@ -119,7 +115,7 @@ __device__ __forceinline__ void mc_row(const QGrid &g, long long row, bool valid
                                        const float *lut, const unsigned long long *s_tab,
                                        uint2 *__restrict__ rowCount, const uint2 *__restrict__ rowBase,
                                        unsigned *__restrict__ tri, unsigned long long *__restrict__ vkey,
-                                       unsigned long long keyhi, unsigned *s_rec) {
+                                       unsigned *s_rec) {
     // FULL: one row per warp (Lg = 32, every group valid), known at compile time.
     if (FULL) {
         Lg = 32;
@@ -248,7 +244,7 @@ __device__ __forceinline__ void mc_row(const QGrid &g, long long row, bool valid
                     }
                     if (ax == 2 && ((Yo >> b) & 1u) && qa == 0) ax = 1;
                     const int k = (w0 + lo) * 32 + b;
-                    vkey[eb0 + ec0 + e] = keyhi + edge_key(g, codes, lut, i, j, k, ax);
+                    vkey[eb0 + ec0 + e] = edge_key(g, codes, lut, i, j, k, ax);
                 }
             }
         }
@@ -342,7 +338,7 @@ __global__ void __launch_bounds__(256, 4) k_mc(QGrid g, const unsigned *__restri
     const long long first = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 / Lg), nrow = (long long)E * E;
     if (first >= nrow) return;  // the whole warp
     const long long row = first + (threadIdx.x & 31) / Lg;
-    mc_row<EMIT, FULL>(g, row, row < nrow, Lg, sign, codes, s_lut, s_tab, rowCount, rowBase, tri, vkey, 0ull,
+    mc_row<EMIT, FULL>(g, row, row < nrow, Lg, sign, codes, s_lut, s_tab, rowCount, rowBase, tri, vkey,
                        s_rec + (EMIT ? (threadIdx.x >> 5) * 32 * kRecW : 0));
 }
 
@@ -372,62 +368,196 @@ __global__ void __launch_bounds__(256, 4) k_mc_batch(QBatch b, const unsigned *_
     const unsigned row = (unit - __ldg(b.mc_unit_off + m)) * (32u / Lg) + (threadIdx.x & 31) / Lg;
     if (Lg == 32)  // warp-uniform
         mc_row<EMIT, true>(g, (long long)row, true, 32, sign + mol.mask_off, codes + mol.code_off,
-                           b.lut + 256ull * m, s_tab, rowCount + r0, rowBase + r0, tri, vkey,
-                           (unsigned long long)m << b.key_bits, rec);
+                           b.lut + 256ull * m, s_tab, rowCount + r0, rowBase + r0, tri, vkey, rec);
     else
         mc_row<EMIT, false>(g, (long long)row, row < nrow, Lg, sign + mol.mask_off, codes + mol.code_off,
-                            b.lut + 256ull * m, s_tab, rowCount + r0, rowBase + r0, tri, vkey,
-                            (unsigned long long)m << b.key_bits, rec);
+                            b.lut + 256ull * m, s_tab, rowCount + r0, rowBase + r0, tri, vkey, rec);
 }
 
 // ------------------------------------------------------------------ weld
 
-__global__ void k_weld_flags(const unsigned long long *__restrict__ skey, unsigned n, uint2 *__restrict__ flags) {
-    unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    flags[p] = make_uint2((p == 0 || skey[p] != skey[p - 1]) ? 1u : 0u, 0u);
+// The weld: unique quantised positions in lexicographic order, in one kernel, a CTA per grid plane
+// (x layer).  The edges of owner rows i come in contiguous slots and their keys lie between the
+// planes i and i + 1: a layer's vertices are those on plane i (every y and z edge, and x edges of
+// either side quantised onto it) and the x edges between it and the next.  The CTA counts its
+// layer's keys into bins that follow the key order - y ranges for the plane, x ranges and within
+// them y ranges for the rest - scatters them, ranks each key among its bin's few, and with the
+// number of vertices of the layers before (decoupled look-back) numbers them.  A grid has at most
+// 4096 layers and a layer of a small molecule is a few hundred keys: then latency bounds it, the
+// phases' dozen barriers and the launch; a layer of a large one is bound by the comparisons within
+// the bins and their loads.
+//
+// A radix sort of all keys (7 or 8 passes over 24 B, flags, scan, scatter) took the weld with its
+// corner remap 0.14 ms at 30 000 edges, 0.83 at 3 700 000, 24.1 at 138 000 000 (0.03, 0.24 and 8.5 so,
+// 3.2 of the last the remap).  A warp sorting each bin of 8 to 32 in registers instead of the
+// comparisons: 0.57 and 18.4.
+constexpr int kWeldT = 1024;
+constexpr unsigned kWeldCap = 4096;  // bins at most, of either sort
+constexpr unsigned long long kWeldFirst = 1ull << 63;  // the first of equal keys: the vertex
+constexpr unsigned kWeldX = 4096;       // x ranges of a layer at most: quanta, for voxels up to 4 A
+// Quantised x of grid plane i, as edge_key has it for the edges in the plane.
+__device__ __forceinline__ unsigned plane_quantum(const QGrid &g, int i) {
+    float p = vox(i, g.dx, g.ox);
+    if (g.off[0] | g.off[1] | g.off[2]) p = __fadd_rn(p, __fmul_rn((float)g.off[0], g.dx));
+    return (unsigned)((long long)roundf(__fdiv_rn(p, QSES_WELD_TOL)) - g.bx);
 }
-
-__global__ void k_weld_scatter(QGrid g, const unsigned long long *__restrict__ skey,
-                               const unsigned *__restrict__ sval, const uint2 *__restrict__ excl, unsigned n,
-                               unsigned *__restrict__ vmap, float *__restrict__ vq) {
-    unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const bool first = (p == 0 || skey[p] != skey[p - 1]);
-    const unsigned rank = excl[p].x + (first ? 1u : 0u) - 1u;
-    vmap[sval[p]] = rank;
-    if (first) {
-        const unsigned long long key = skey[p], R = (unsigned long long)g.Rq;
-        const long long mz = (long long)(key % R) + g.bz;
-        const long long my = (long long)((key / R) % R) + g.by;
-        const long long mx = (long long)(key / (R * R)) + g.bx;
-        vq[3ull * rank] = __fmul_rn((float)mx, QSES_WELD_TOL);
-        vq[3ull * rank + 1] = __fmul_rn((float)my, QSES_WELD_TOL);
-        vq[3ull * rank + 2] = __fmul_rn((float)mz, QSES_WELD_TOL);
+// In place: exclusive sums of x[0, n), by the whole block; the total is returned.
+template <int NT>
+__device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, unsigned *s_tmp) {
+    const unsigned per = (n + NT - 1) / NT, lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
+    unsigned sum = 0, total;
+    for (unsigned k = lo; k < hi; k++) sum += x[k];
+    unsigned run = block_excl_scan<NT>(sum, total, s_tmp);
+    for (unsigned k = lo; k < hi; k++) {
+        const unsigned c = x[k];
+        x[k] = run;
+        run += c;
     }
+    __syncthreads();
+    return total;
 }
 
-// Batch form: the key's high bits name the molecule whose grid decodes the low bits.
-__global__ void k_weld_scatter_batch(QBatch b, const unsigned long long *__restrict__ skey,
-                                     const unsigned *__restrict__ sval, const uint2 *__restrict__ excl, unsigned n,
-                                     unsigned *__restrict__ vmap, float *__restrict__ vq, unsigned *__restrict__ vmol) {
-    unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const bool first = (p == 0 || skey[p] != skey[p - 1]);
-    const unsigned rank = excl[p].x + (first ? 1u : 0u) - 1u;
-    vmap[sval[p]] = rank;
-    if (first) {
-        const unsigned m = (unsigned)(skey[p] >> b.key_bits);
-        const unsigned long long key = skey[p] & ((1ull << b.key_bits) - 1ull);
-        const QGrid &g = b.mols[m].g;
-        const unsigned long long R = (unsigned long long)g.Rq;
-        const long long mz = (long long)(key % R) + g.bz;
-        const long long my = (long long)((key / R) % R) + g.by;
-        const long long mx = (long long)(key / (R * R)) + g.bx;
-        vq[3ull * rank] = __fmul_rn((float)mx, QSES_WELD_TOL);
-        vq[3ull * rank + 1] = __fmul_rn((float)my, QSES_WELD_TOL);
-        vq[3ull * rank + 2] = __fmul_rn((float)mz, QSES_WELD_TOL);
-        vmol[rank] = m;
+template <bool BATCH>
+__global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned cap,
+                                                    const unsigned long long *__restrict__ vkey,
+                                                    const uint2 *__restrict__ rowBase, unsigned ne, unsigned layers,
+                                                    const unsigned *__restrict__ edge_off, unsigned long long *skey,
+                                                    unsigned *sslot, unsigned *__restrict__ vmap,
+                                                    float *__restrict__ vq, unsigned *__restrict__ vmol,
+                                                    unsigned *__restrict__ vtx_off, uint2 *__restrict__ total,
+                                                    unsigned long long *status, unsigned *ticket, int *err) {
+    extern __shared__ unsigned s_bin[];  // 2 x (2 cap + 2) and kWeldX / 2
+    __shared__ unsigned s_tmp[kWeldT / 32], s_tile, s_pushed, s_before;
+    if (threadIdx.x == 0) {
+        s_tile = atomicAdd(ticket, 1u);  // layers in the order CTAs start, so that every wait ends
+        s_pushed = 0;
+    }
+    __syncthreads();
+    const unsigned tile = s_tile, m = BATCH ? qses_find(b.layer_off, b.n_mol, tile) : 0u;
+    const QGrid &g = BATCH ? b.mols[m].g : g1;
+    const unsigned i = BATCH ? tile - __ldg(b.layer_off + m) : tile, E = (unsigned)g.Gc + 1;
+    const uint2 *rows = rowBase + (BATCH ? b.mols[m].row_off : 0u);
+    const unsigned s1 = rows[(size_t)i * E].y, s0 = i ? rows[(size_t)(i - 1) * E].y : s1;
+    const unsigned s2 = i + 1 < E ? rows[(size_t)(i + 1) * E].y : BATCH ? __ldg(edge_off + m + 1) : ne;
+    const unsigned X0 = plane_quantum(g, (int)i), X1 = plane_quantum(g, (int)i + 1);
+    const unsigned Rq = (unsigned)g.Rq;
+    unsigned *cur = s_bin, *uniq = s_bin + 2 * cap + 2;
+    unsigned short *x_at = (unsigned short *)(uniq + 2 * cap + 2);
+    // y ranges of the plane
+    unsigned sy = 0, sx = 0, sq = 0;
+    while ((Rq >> sy) + 1 > cap) sy++;
+    const unsigned np = (Rq >> sy) + 1;
+    // x ranges above it
+    while (((X1 - X0) >> sx) + 1 > kWeldX) sx++;
+    const unsigned nx = ((X1 - X0) >> sx) + 1;
+    // Field values are few, so x takes a tenth of its quanta.  Each that some 4096 of the layer's
+    // keys fall on gets bins for y ranges; what lies between two of them is one bin.  Even ranges
+    // would put 90 keys into a bin of the largest grids: 22.0 ms instead of 8.6 (0.26 and 0.24).
+    for (unsigned k = threadIdx.x; k < nx; k += kWeldT) s_bin[k] = 0;
+    __syncthreads();
+    const unsigned step = (s2 - s1) / 4096 + 1;
+    for (unsigned long long s = s1 + threadIdx.x * step; s < s2; s += kWeldT * step) {
+        const unsigned X = (unsigned)(__ldg(vkey + s) >> 42);
+        if (X > X0) s_bin[min((X - X0) >> sx, nx - 1)] = 1;
+    }
+    __syncthreads();
+    for (unsigned k = threadIdx.x; k < nx; k += kWeldT) x_at[k] = (unsigned short)s_bin[k];
+    const unsigned used = block_excl_sums<kWeldT>(s_bin, nx, s_tmp);
+    const bool split = sx == 0 && 4 * used <= cap;  // else a bin for each used x and the ones up to it
+    while (split && (Rq >> sq) + 1 > cap / (used + 1) - 1) sq++;
+    const unsigned nq = split ? (Rq >> sq) + 1 : 0, nbin = np + min((used + 1) * (nq + 1), cap + 1);
+    for (unsigned k = threadIdx.x; k < nx; k += kWeldT) x_at[k] = (unsigned short)(2 * s_bin[k] + x_at[k]);
+    __syncthreads();
+    // a key's bin: any map that follows the key order serves
+    auto bin_of = [&](unsigned long long key) {
+        const unsigned X = (unsigned)(key >> 42), Y = (unsigned)(key >> 21) & 0x1fffffu;
+        if (X <= X0) return min(Y >> sy, np - 1);
+        const unsigned x = x_at[min((X - X0) >> sx, nx - 1)];
+        return min(np + (x >> 1) * (nq + 1) + (split && (x & 1) ? 1 + min(Y >> sq, nq - 1) : 0), nbin - 1);
+    };
+    // The keys of owner rows i lie in [X0, X1] (planes are 0.15 A and more apart, and rounding
+    // moves a position by a few quanta at most): those at X1 and above are the next layer's.
+    auto mine = [&](unsigned slot, unsigned long long key) {
+        const unsigned X = (unsigned)(key >> 42);
+        return slot < s1 ? X >= X0 : X < X1 || i + 1 == E;
+    };
+    for (unsigned k = threadIdx.x; k <= nbin; k += kWeldT) cur[k] = uniq[k] = 0;
+    __syncthreads();
+    // count
+    unsigned below = 0;
+    for (unsigned s = s0 + threadIdx.x; s < s2; s += kWeldT) {
+        const unsigned long long key = __ldg(vkey + s);
+        if (!mine(s, key)) continue;
+        atomicAdd(&cur[bin_of(key)], 1u);
+        below += s < s1;
+    }
+    if (below) atomicAdd(&s_pushed, below);
+    __syncthreads();
+    const unsigned n = block_excl_sums<kWeldT>(cur, nbin, s_tmp);
+    // scatter: the layer's keys to [base, base + n) (the ones before it are the slots before s1 less
+    // those pushed up into this layer), bin after bin; cur[k] becomes the end of bin k
+    const unsigned base = s1 - s_pushed;
+    for (unsigned s = s0 + threadIdx.x; s < s2; s += kWeldT) {
+        const unsigned long long key = __ldg(vkey + s);
+        if (!mine(s, key)) continue;
+        const unsigned q = base + atomicAdd(&cur[bin_of(key)], 1u);
+        if (q < ne) {
+            skey[q] = key;
+            sslot[q] = s;
+        }
+    }
+    __syncthreads();
+    // the first of equal keys is the vertex; distinct keys per bin
+    for (unsigned q = threadIdx.x; q < n; q += kWeldT) {
+        const unsigned long long key = skey[base + q];
+        const unsigned k = bin_of(key), lo = k ? cur[k - 1] : 0u;
+        bool first = true;
+#pragma unroll 4
+        for (unsigned p = lo; p < q; p++) first &= (skey[base + p] & ~kWeldFirst) != key;
+        if (first) {
+            skey[base + q] = key | kWeldFirst;
+            atomicAdd(&uniq[k], 1u);
+        }
+    }
+    __syncthreads();
+    const unsigned distinct = block_excl_sums<kWeldT>(uniq, nbin, s_tmp);
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        unsigned before = 0;
+        if (lane == 0 && tile) st_release(&status[tile], kFlagAgg | distinct);
+        for (int j = (int)tile - 1; j >= 0; j -= 32) {  // a small grid's layers are all in flight: 32 at a time
+            const unsigned long long st = j >= lane ? wait_status(&status[j - lane], err) : kFlagPre;
+            const unsigned pre = __ballot_sync(0xffffffffu, (st >> 62) != 1);  // an inclusive prefix (or timed out)
+            before += __reduce_add_sync(0xffffffffu, lane <= (pre ? __ffs(pre) - 1 : 31) ? (unsigned)st : 0u);
+            if (pre) break;
+        }
+        if (lane == 0) {
+            st_release(&status[tile], kFlagPre | (unsigned long long)(before + distinct));
+            s_before = before;
+            if (BATCH && i == 0) vtx_off[m] = before;
+            if (tile == layers - 1) {
+                *total = make_uint2(before + distinct, 0u);
+                if (BATCH) vtx_off[b.n_mol] = before + distinct;
+            }
+        }
+    }
+    __syncthreads();
+    const unsigned before = s_before;
+    for (unsigned q = threadIdx.x; q < n; q += kWeldT) {
+        const unsigned long long own = skey[base + q], key = own & ~kWeldFirst;
+        const unsigned k = bin_of(key), lo = k ? cur[k - 1] : 0u, hi = cur[k];
+        unsigned rank = before + uniq[k];
+#pragma unroll 4
+        for (unsigned p = lo; p < hi; p++) rank += (skey[base + p] ^ kWeldFirst) < key;
+        vmap[sslot[base + q]] = rank;
+        if (own != key && rank < ne) {
+            const long long mx = (long long)(key >> 42) + g.bx, my = (long long)((key >> 21) & 0x1fffffu) + g.by,
+                            mz = (long long)(key & 0x1fffffu) + g.bz;
+            vq[3ull * rank] = __fmul_rn((float)mx, QSES_WELD_TOL);
+            vq[3ull * rank + 1] = __fmul_rn((float)my, QSES_WELD_TOL);
+            vq[3ull * rank + 2] = __fmul_rn((float)mz, QSES_WELD_TOL);
+            if (BATCH) vmol[rank] = m;
+        }
     }
 }
 
@@ -642,10 +772,37 @@ void launch_mc_emit_batch(const QBatch &b, unsigned units, const unsigned *sign,
                           const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s) {
     k_mc_batch<true><<<nblk(units, 8), 256, 0, s>>>(b, sign, codes, nullptr, rowBase, tri, vkey);
 }
-void launch_weld_scatter_batch(const QBatch &b, const unsigned long long *skey, const unsigned *sval,
-                               const uint2 *excl, unsigned n, unsigned *vmap, float *vq, unsigned *vmol,
-                               cudaStream_t s) {
-    k_weld_scatter_batch<<<nblk(n, 256), 256, 0, s>>>(b, skey, sval, excl, n, vmap, vq, vmol);
+size_t weld_tmp_bytes(unsigned layers) { return 256 + 8ull * layers; }
+template <bool BATCH>
+static cudaError_t weld_with(const QGrid &g, const QBatch &b, const unsigned long long *vkey, const uint2 *rowBase,
+                             unsigned ne, unsigned layers, const unsigned *edge_off, unsigned long long *skey,
+                             unsigned *sslot, unsigned *vmap, float *vq, unsigned *vmol, unsigned *vtx_off, uint2 *total,
+                             void *tmp, int *err, cudaStream_t s) {
+    // A bin of either sort for each key of an average layer: a key is compared with its whole bin.
+    // Half or twice as many bins take the same time, 8192 at most (one CTA per SM) 9.3 ms for 8.6.
+    const unsigned per = ne / layers, cap = per < 1024 ? 1024 : per > kWeldCap ? kWeldCap : per;
+    static_assert(4 * 1024 + 4 >= kWeldX, "the x marks lie where the bins will");
+    const size_t smem = 8ull * (2 * cap + 2) + 2 * kWeldX;
+    cudaError_t e = cudaFuncSetAttribute((const void *)k_weld<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         8 * (2 * kWeldCap + 2) + 2 * kWeldX);
+    if (e == cudaSuccess) e = cudaMemsetAsync(tmp, 0, weld_tmp_bytes(layers), s);
+    if (e != cudaSuccess) return e;
+    k_weld<BATCH><<<layers, kWeldT, smem, s>>>(g, b, cap, vkey, rowBase, ne, layers, edge_off, skey, sslot, vmap, vq, vmol,
+                                               vtx_off, total, (unsigned long long *)((char *)tmp + 256), (unsigned *)tmp, err);
+    return cudaGetLastError();
+}
+cudaError_t launch_weld(const QGrid &g, const unsigned long long *vkey, const uint2 *rowBase, unsigned ne,
+                        unsigned long long *skey, unsigned *sslot, unsigned *vmap, float *vq, uint2 *total, void *tmp,
+                        int *err, cudaStream_t s) {
+    return weld_with<false>(g, QBatch{}, vkey, rowBase, ne, (unsigned)g.Gc + 1, nullptr, skey, sslot, vmap, vq, nullptr,
+                            nullptr, total, tmp, err, s);
+}
+cudaError_t launch_weld_batch(const QBatch &b, unsigned layers, const unsigned long long *vkey, const uint2 *rowBase,
+                              unsigned ne, const unsigned *edge_off, unsigned long long *skey, unsigned *sslot,
+                              unsigned *vmap, float *vq, unsigned *vmol, unsigned *vtx_off, uint2 *total, void *tmp, int *err,
+                              cudaStream_t s) {
+    return weld_with<true>(QGrid{}, b, vkey, rowBase, ne, layers, edge_off, skey, sslot, vmap, vq, vmol, vtx_off, total, tmp,
+                           err, s);
 }
 void launch_gather_offsets(const uint2 *excl, const unsigned *at, unsigned n_mol, unsigned n, const uint2 *total,
                            unsigned *outx, unsigned *outy, cudaStream_t s) {
@@ -662,13 +819,6 @@ void launch_tri_flags_batch(const QBatch &b, const unsigned *tri, unsigned nt, u
 void launch_tri_compact_batch(const QBatch &b, const unsigned *tri, unsigned nt, const uint2 *excl, unsigned *out,
                               cudaStream_t s) {
     k_tri_compact_batch<<<nblk(nt, 256), 256, 0, s>>>(b, tri, nt, excl, out);
-}
-void launch_weld_flags(const unsigned long long *skey, unsigned n, uint2 *flags, cudaStream_t s) {
-    k_weld_flags<<<nblk(n, 256), 256, 0, s>>>(skey, n, flags);
-}
-void launch_weld_scatter(const QGrid &g, const unsigned long long *skey, const unsigned *sval, const uint2 *excl,
-                         unsigned n, unsigned *vmap, float *vq, cudaStream_t s) {
-    k_weld_scatter<<<nblk(n, 256), 256, 0, s>>>(g, skey, sval, excl, n, vmap, vq);
 }
 void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s) {
     k_remap<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, vmap);

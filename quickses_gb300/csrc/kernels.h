@@ -23,9 +23,12 @@ void launch_edt(const QGrid &g, const unsigned *inMask, const unsigned *outMask,
 void launch_mc_count(const QGrid &g, const unsigned *sign, uint2 *rowCount, cudaStream_t s);
 void launch_mc_emit(const QGrid &g, const unsigned *sign, const unsigned char *codes, const float *lut,
                     const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s);
-void launch_weld_flags(const unsigned long long *skey, unsigned n, uint2 *flags, cudaStream_t s);
-void launch_weld_scatter(const QGrid &g, const unsigned long long *skey, const unsigned *sval, const uint2 *excl,
-                         unsigned n, unsigned *vmap, float *vq, cudaStream_t s);
+// Vertex ids (vmap, per edge slot), welded positions and their count from the edge keys in owner
+// row order (rowBase: the scanned row counts).  skey, sslot: scratch, one entry per edge.
+size_t weld_tmp_bytes(unsigned layers);
+cudaError_t launch_weld(const QGrid &g, const unsigned long long *vkey, const uint2 *rowBase, unsigned ne,
+                        unsigned long long *skey, unsigned *sslot, unsigned *vmap, float *vq, uint2 *total, void *tmp,
+                        int *err, cudaStream_t s);
 void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s);
 void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *atoms, const uint2 *cells,
                     const unsigned *sorted_to_input, int *asorted, int *ainput, cudaStream_t s);
@@ -114,9 +117,11 @@ int mc_rows_per_warp(int Gc);
 void launch_mc_count_batch(const QBatch &b, unsigned units, const unsigned *sign, uint2 *rowCount, cudaStream_t s);
 void launch_mc_emit_batch(const QBatch &b, unsigned units, const unsigned *sign, const unsigned char *codes,
                           const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s);
-void launch_weld_scatter_batch(const QBatch &b, const unsigned long long *skey, const unsigned *sval,
-                               const uint2 *excl, unsigned n, unsigned *vmap, float *vq, unsigned *vmol,
-                               cudaStream_t s);
+// layers: owner planes (Gc + 1) of all molecules; vtx_off receives each molecule's first vertex.
+cudaError_t launch_weld_batch(const QBatch &b, unsigned layers, const unsigned long long *vkey, const uint2 *rowBase,
+                              unsigned ne, const unsigned *edge_off, unsigned long long *skey, unsigned *sslot,
+                              unsigned *vmap, float *vq, unsigned *vmol, unsigned *vtx_off, uint2 *total, void *tmp, int *err,
+                              cudaStream_t s);
 void launch_gather_offsets(const uint2 *excl, const unsigned *at, unsigned n_mol, unsigned n, const uint2 *total,
                            unsigned *outx, unsigned *outy, cudaStream_t s);
 void launch_closest_batch(const QBatch &b, const float *vq, const unsigned *vmol, unsigned nv, const float4 *atoms,

@@ -154,7 +154,7 @@ extern "C" QSES_API int qses_field_codes_noalloc(const float *d_xyz, const float
 
     launch_atom_hash(g, d_xyz, n, key, s);
     int alt = 0;
-    if (radix_sort<unsigned>(key, key2, idx, idx2, n, atom_bits, true, tmp, d_err, s, nullptr, &alt) != cudaSuccess)
+    if (radix_sort(key, key2, idx, idx2, n, atom_bits, true, tmp, d_err, s, nullptr, &alt) != cudaSuccess)
         return fail(QSES_ERR_CUDA);
     const unsigned *skey = alt ? key2 : key, *sidx = alt ? idx2 : idx;
     if (cudaMemsetAsync(cells, 0, 8 * ncell, s) != cudaSuccess) return fail(QSES_ERR_CUDA);

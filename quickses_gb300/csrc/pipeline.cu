@@ -92,7 +92,7 @@ int grid_from_bounds(const float mn_in[3], const float mx_in[3], float maxR_in, 
             break;
         }
     }
-    // Weld key: quantised position relative to the quantised origin, mixed radix Rq.
+    // Weld key: quantised position relative to the quantised origin, 21 bits per axis.
     const double extent = (double)g.G * (double)dx;
     if (std::fabs((double)g.ox) + extent > 16000.0 || std::fabs((double)g.oy) + extent > 16000.0 ||
         std::fabs((double)g.oz) + extent > 16000.0) {
@@ -470,7 +470,7 @@ static int enqueue_field(qses_context *ctx, const FieldSeg &a, SegOut &o) {
     QCHK(cudaMemcpyAsync(a.lut, a.h_lut, 1024, cudaMemcpyHostToDevice, s));
     launch_atom_hash(a.g, a.xyz, a.n, a.key, s);
     ctx->launches++;
-    QCHK(radix_sort<unsigned>(a.key, a.key2, a.idx, a.idx2, a.n, a.atom_bits, true, a.tmp, a.err, s, &ctx->launches,
+    QCHK(radix_sort(a.key, a.key2, a.idx, a.idx2, a.n, a.atom_bits, true, a.tmp, a.err, s, &ctx->launches,
                               &o.alt));
     const unsigned *skey = o.alt ? a.key2 : a.key, *sidx = o.alt ? a.idx2 : a.idx;
     QCHK(cudaMemsetAsync(a.cells, 0, 8 * a.ncell, s));
@@ -501,8 +501,8 @@ struct MeshSeg {
     const uint2 *rows;
     unsigned *tri;
     unsigned long long *vk, *vk2;
-    unsigned *vv, *vv2;
-    uint2 *flags, *tot;
+    unsigned *vv;
+    uint2 *tot;
     unsigned *vmap;
     float *vq;
     void *tmp;
@@ -510,7 +510,7 @@ struct MeshSeg {
     unsigned char *h_out;  // pinned: [0, 8) vertex total
     unsigned long long n3;
     unsigned ne;
-    int key_bits;
+    int pad_;
     QGrid g;
 };
 
@@ -520,14 +520,7 @@ static int enqueue_mesh(qses_context *ctx, const MeshSeg &b, SegOut &o) {
     ctx->launches++;
     ctx->mark("mc_emit");
     if (b.ne > 0) {
-        QCHK(radix_sort<unsigned long long>(b.vk, b.vk2, b.vv, b.vv2, b.ne, b.key_bits, true, b.tmp, b.err, s,
-                                            &ctx->launches, &o.alt));
-        const unsigned long long *sk = o.alt ? b.vk2 : b.vk;
-        const unsigned *sv = o.alt ? b.vv2 : b.vv;
-        launch_weld_flags(sk, b.ne, b.flags, s);
-        ctx->launches++;
-        QCHK(scan_u2(b.flags, b.flags, b.ne, b.tot, b.tmp, b.err, s, &ctx->launches));
-        launch_weld_scatter(b.g, sk, sv, b.flags, b.ne, b.vmap, b.vq, s);
+        QCHK(launch_weld(b.g, b.vk, b.rows, b.ne, b.vk2, b.vv, b.vmap, b.vq, b.tot, b.tmp, b.err, s));
         ctx->launches++;
         launch_remap(b.tri, b.n3, b.vmap, s);
         ctx->launches++;
@@ -749,10 +742,8 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    const int key_bits = bits_for((unsigned long long)g.Rq * g.Rq * g.Rq - 1);
-    const int vbits = bits_for(NE ? NE - 1 : 0);
-    size_t tmpB = std::max({radix_sort_tmp_bytes(NE, key_bits), radix_sort_tmp_bytes((unsigned)n3, vbits),
-                            scan_u2_tmp_bytes(NE), scan_u2_tmp_bytes(T), scan_u2_tmp_bytes(NE + 1)});
+    size_t tmpB = std::max({weld_tmp_bytes((unsigned)E), scan_u2_tmp_bytes(NE), scan_u2_tmp_bytes(T),
+                            scan_u2_tmp_bytes(NE + 1)});
     const size_t nflag = std::max<size_t>((size_t)NE + 1, (size_t)T) + 1;
     size_t needB = 2 * align256(4 * n3) + 2 * align256(8ull * NE) + 2 * align256(4ull * NE) + align256(8ull * nflag) +
                    align256(4ull * NE) + align256(12ull * NE) + 2 * align256(4ull * NE) + align256(4 * n3 + 4) +
@@ -764,7 +755,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
     unsigned *tri_kept = (unsigned *)B.take(4 * n3 + 4);
     unsigned long long *vk = (unsigned long long *)B.take(8ull * NE + 8), *vk2 = (unsigned long long *)B.take(8ull * NE + 8);
-    unsigned *vv = (unsigned *)B.take(4ull * NE + 4), *vv2 = (unsigned *)B.take(4ull * NE + 4);
+    unsigned *vv = (unsigned *)B.take(4ull * NE + 4);
     uint2 *flags = (uint2 *)B.take(8ull * nflag);
     unsigned *vmap = (unsigned *)B.take(4ull * NE + 4);
     float *vq = (float *)B.take(12ull * NE + 12);
@@ -792,8 +783,6 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     b.vk = vk;
     b.vk2 = vk2;
     b.vv = vv;
-    b.vv2 = vv2;
-    b.flags = flags;
     b.tot = a.tot;
     b.vmap = vmap;
     b.vq = vq;
@@ -802,7 +791,6 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     b.h_out = ctx->h_small;
     b.n3 = n3;
     b.ne = NE;
-    b.key_bits = key_bits;
     b.g = g;
     SegOut ob;
     ctx->tick(2);

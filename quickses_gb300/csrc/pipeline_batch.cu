@@ -11,8 +11,8 @@
 //     work counter;
 //   * marching-cubes rows are numbered molecule after molecule, so one scan gives each
 //     molecule a contiguous range of triangles and edge slots;
-//   * weld keys carry the molecule above the local key bits, so one sort + unique welds
-//     every molecule separately and numbers its vertices contiguously in its own order;
+//   * the weld takes a grid plane per CTA, molecule after molecule, and numbers each
+//     molecule's vertices contiguously in its own order;
 //   * Gauss-Seidel runs as one dataflow over all molecules (no dependency crosses a
 //     molecule, so each molecule is smoothed exactly as alone, and the critical path is the
 //     deepest molecule, not the sum), in waves of at most 152 x 25 000 vertices.
@@ -94,7 +94,7 @@ static int enqueue_batch_field(qses_context *ctx, const BatchFieldSeg &a, SegOut
     // atoms
     launch_atom_hash_batch(a.b, a.d_x, a.n, a.key, s);
     ctx->launches++;
-    QCHK(radix_sort<unsigned>(a.key, a.key2, a.idx, a.idx2, a.n, a.cell_bits, true, a.tmp, a.err, s, &ctx->launches,
+    QCHK(radix_sort(a.key, a.key2, a.idx, a.idx2, a.n, a.cell_bits, true, a.tmp, a.err, s, &ctx->launches,
                               &o.alt));
     const unsigned *skey = o.alt ? a.key2 : a.key, *sidx = o.alt ? a.idx2 : a.idx;
     QCHK(cudaMemsetAsync(a.cells, 0, 8 * a.cell_tot, s));
@@ -119,7 +119,7 @@ static int enqueue_batch_field(qses_context *ctx, const BatchFieldSeg &a, SegOut
     return QSES_OK;
 }
 
-// ---- segment 2: triangles and molecule-tagged weld keys, one weld for all molecules
+// ---- segment 2: triangles and weld keys, one weld for all molecules
 struct BatchMeshSeg {
     unsigned long long mem;  // free counters of the buffers it uses
     const unsigned *sign_mask;
@@ -127,8 +127,8 @@ struct BatchMeshSeg {
     const uint2 *rows;
     unsigned *tri;
     unsigned long long *vk, *vk2;
-    unsigned *vv, *vv2;
-    uint2 *flags, *tot;
+    unsigned *vv;
+    uint2 *tot;
     unsigned *vmap;
     float *vq;
     unsigned *vmol;
@@ -139,7 +139,7 @@ struct BatchMeshSeg {
     void *h_vtx;           // pinned: per-molecule first vertex
     unsigned long long n3;
     unsigned units, ne;
-    int tot_bits, pad_;
+    unsigned layers, pad_;
     QBatch b;
 };
 
@@ -150,18 +150,8 @@ static int enqueue_batch_mesh(qses_context *ctx, const BatchMeshSeg &m, SegOut &
     ctx->launches++;
     ctx->mark("mc_emit");
     if (m.ne > 0) {
-        QCHK(radix_sort<unsigned long long>(m.vk, m.vk2, m.vv, m.vv2, m.ne, m.tot_bits, true, m.tmp, m.err, s,
-                                            &ctx->launches, &o.alt));
-        const unsigned long long *sk = o.alt ? m.vk2 : m.vk;
-        const unsigned *sv = o.alt ? m.vv2 : m.vv;
-        launch_weld_flags(sk, m.ne, m.flags, s);
-        ctx->launches++;
-        QCHK(scan_u2(m.flags, m.flags, m.ne, m.tot, m.tmp, m.err, s, &ctx->launches));
-        launch_weld_scatter_batch(m.b, sk, sv, m.flags, m.ne, m.vmap, m.vq, m.vmol, s);
-        ctx->launches++;
-        // molecule k's edges occupy sorted positions [edge_off[k], edge_off[k+1]) (its keys
-        // sort between the other molecules'), so its first vertex is the rank there
-        launch_gather_offsets(m.flags, m.edge_off, nm, m.ne, m.tot, m.vtx_off, nullptr, s);
+        QCHK(launch_weld_batch(m.b, m.layers, m.vk, m.rows, m.ne, m.edge_off, m.vk2, m.vv, m.vmap, m.vq, m.vmol, m.vtx_off,
+                               m.tot, m.tmp, m.err, s));
         ctx->launches++;
         launch_remap(m.tri, m.n3, m.vmap, s);
         ctx->launches++;
@@ -272,7 +262,7 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
     return QSES_OK;
 }
 
-int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes, int key_bits) {
+int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes) {
     cudaStream_t s = ctx->stream;
     QSES_SEG_TRACE("batch: %u molecules, %d passes\n", count, passes);
     memset(ctx->timeline, 0, sizeof(ctx->timeline));
@@ -292,8 +282,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     // ---- per-molecule layout on the host
     const unsigned nm = count;
     std::vector<QMol> mols(nm);
-    std::vector<unsigned> tile_off(nm + 1), atom_off(nm + 1), row_off(nm + 1), unit_off(nm + 1), word_off(nm + 1);
-    unsigned long long mask_tot = 0, code_tot = 0, cell_tot = 0, tiles = 0, rows = 0, atoms_tot = 0, units = 0;
+    std::vector<unsigned> tile_off(nm + 1), atom_off(nm + 1), row_off(nm + 1), unit_off(nm + 1), word_off(nm + 1), layer_off(nm + 1);
+    unsigned long long mask_tot = 0, code_tot = 0, cell_tot = 0, tiles = 0, rows = 0, atoms_tot = 0, units = 0, layers = 0;
     for (unsigned m = 0; m < nm; m++) {
         const QGrid &g = items[m].g;
         QMol &q = mols[m];
@@ -310,6 +300,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         row_off[m] = (unsigned)rows;
         unit_off[m] = (unsigned)units;
         word_off[m] = (unsigned)mask_tot;
+        layer_off[m] = (unsigned)layers;
+        layers += (unsigned long long)g.Gc + 1;
         mask_tot += (unsigned long long)g.G * g.G * g.W;
         code_tot += (unsigned long long)g.G * g.G * g.Gp;
         cell_tot += (unsigned long long)g.gnb * g.gnb * g.gnb;
@@ -325,13 +317,14 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     row_off[nm] = (unsigned)rows;
     unit_off[nm] = (unsigned)units;
     word_off[nm] = (unsigned)mask_tot;
+    layer_off[nm] = (unsigned)layers;
     if (tiles >= (1ull << 31) || rows >= (1ull << 31) || cell_tot >= (1ull << 31) || atoms_tot >= (1ull << 30) ||
         mask_tot >= (1ull << 32))
         return ctx->fail(QSES_ERR_UNSUPPORTED, "batch too large for 32-bit item indices; split it");
     const unsigned N = (unsigned)atoms_tot;
 
     // ---- pinned staging: descriptor block then atoms, one copy each
-    const size_t desc_bytes = a256(sizeof(QMol) * nm) + 9 * a256(4ull * (nm + 1)) + a256(1024ull * nm);
+    const size_t desc_bytes = a256(sizeof(QMol) * nm) + 10 * a256(4ull * (nm + 1)) + a256(1024ull * nm);
     const size_t atom_bytes = 16ull * N;
     if (stage_reserve(ctx, desc_bytes + atom_bytes + 256) != QSES_OK)
         return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "pinned batch staging");
@@ -348,6 +341,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     hput(row_off.data(), 4ull * (nm + 1));
     hput(unit_off.data(), 4ull * (nm + 1));
     hput(word_off.data(), 4ull * (nm + 1));
+    hput(layer_off.data(), 4ull * (nm + 1));
     hput(nullptr, 4ull * (nm + 1));  // tri_off   (device-filled)
     hput(nullptr, 4ull * (nm + 1));  // edge_off  (device-filled)
     hput(nullptr, 4ull * (nm + 1));  // vtx_off   (device-filled)
@@ -396,13 +390,13 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         b.row_off = (const unsigned *)at(ob);
         b.mc_unit_off = (const unsigned *)at(ob);
         b.word_off = (const unsigned *)at(ob);
+        b.layer_off = (const unsigned *)at(ob);
         b.tri_off = (const unsigned *)at(ob);
         d_edge_off = (unsigned *)at(ob);
         b.vtx_off = (const unsigned *)at(ob);
         d_kept_off = (unsigned *)at(ob);
         b.lut = (const float *)at(1024ull * nm);
         b.n_mol = nm;
-        b.key_bits = key_bits;
     }
     unsigned *d_tri_off = (unsigned *)b.tri_off, *d_vtx_off = (unsigned *)b.vtx_off;
     a.key = (unsigned *)A.take(4ull * N);
@@ -445,12 +439,9 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     const unsigned T = hsm[0], NE = hsm[1];
 
     // ---- mesh workspace
-    const int mol_bits = bits_for(nm - 1);
-    const int tot_bits = key_bits + mol_bits;
     const size_t n3 = 3ull * T;
-    const int vbits = bits_for(NE ? NE - 1 : 0);
-    const size_t tmpB = std::max({radix_sort_tmp_bytes(NE, tot_bits), radix_sort_tmp_bytes((unsigned)n3, vbits),
-                                  scan_u2_tmp_bytes(NE), scan_u2_tmp_bytes(T), scan_u2_tmp_bytes(NE + 1)});
+    const size_t tmpB = std::max({weld_tmp_bytes(layer_off[nm]), scan_u2_tmp_bytes(NE), scan_u2_tmp_bytes(T),
+                                  scan_u2_tmp_bytes(NE + 1)});
     const size_t nflag = std::max<size_t>((size_t)NE + 1, (size_t)T) + 1;
     const size_t needB = 2 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
                          a256(8ull * nflag) + a256(4ull * NE + 4) + a256(12ull * NE + 12) + 3 * a256(4ull * NE + 4) +
@@ -461,7 +452,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
     unsigned *tri_kept = (unsigned *)B.take(4 * n3 + 4);
     unsigned long long *vk = (unsigned long long *)B.take(8ull * NE + 8), *vk2 = (unsigned long long *)B.take(8ull * NE + 8);
-    unsigned *vv = (unsigned *)B.take(4ull * NE + 4), *vv2 = (unsigned *)B.take(4ull * NE + 4);
+    unsigned *vv = (unsigned *)B.take(4ull * NE + 4);
     uint2 *flags = (uint2 *)B.take(8ull * nflag);
     unsigned *vmap = (unsigned *)B.take(4ull * NE + 4);
     float *vq = (float *)B.take(12ull * NE + 12);
@@ -478,7 +469,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     void *tmp2 = B.take(scan_u2_tmp_bytes(T + 1));   // its scan's scratch
     if (!tmpb || !tflags || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "batch mesh workspace layout");
 
-    // ---- triangles + molecule-tagged weld keys, then one weld for all molecules
+    // ---- triangles + weld keys, then one weld for all molecules
     BatchMeshSeg mb;
     memset(&mb, 0, sizeof(mb));
     mb.mem = ctx->field.gen + ctx->mesh_ws.gen + ctx->host_gen;
@@ -489,8 +480,6 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     mb.vk = vk;
     mb.vk2 = vk2;
     mb.vv = vv;
-    mb.vv2 = vv2;
-    mb.flags = flags;
     mb.tot = a.tot;
     mb.vmap = vmap;
     mb.vq = vq;
@@ -504,7 +493,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     mb.n3 = n3;
     mb.units = (unsigned)units;
     mb.ne = NE;
-    mb.tot_bits = tot_bits;
+    mb.layers = layer_off[nm];
     mb.b = b;
     SegOut ob;
     ctx->tick(2);

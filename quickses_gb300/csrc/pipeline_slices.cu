@@ -143,7 +143,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
     launch_atom_hash(g, d_xyz, n, key, s);
     ctx->launches++;
     int alt = 0;
-    SCHK(radix_sort<unsigned>(key, key2, idx, idx2, n, atom_bits, true, tmp, d_err, s, &ctx->launches, &alt));
+    SCHK(radix_sort(key, key2, idx, idx2, n, atom_bits, true, tmp, d_err, s, &ctx->launches, &alt));
     const unsigned *skey = alt ? key2 : key, *sidx = alt ? idx2 : idx;
     SCHK(cudaMemsetAsync(cells, 0, 8 * ncell, s));
     launch_atom_gather(d_xyz, d_r, skey, sidx, n, atoms, cells, s);
@@ -215,8 +215,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
 
                 // ---- mesh workspace of this slice
                 const size_t n3 = 3ull * T, n3k = 3ull * T1;
-                const int key_bits = bits_for((unsigned long long)b.Rq * b.Rq * b.Rq - 1);
-                const size_t tmpB = std::max({radix_sort_tmp_bytes(NE, key_bits), scan_u2_tmp_bytes(NE + 1),
+                const size_t tmpB = std::max({weld_tmp_bytes((unsigned)b.Gc + 1), scan_u2_tmp_bytes(NE + 1),
                                               scan_u2_tmp_bytes(T + 1)});
                 const size_t needB = 3 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
                                      3 * a256(8ull * (NE + 2)) + 2 * a256(4ull * NE + 4) + 2 * a256(12ull * NE + 12) +
@@ -228,7 +227,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 unsigned *okey = (unsigned *)B.take(4 * n3 + 4);
                 unsigned long long *vk = (unsigned long long *)B.take(8ull * NE + 8);
                 unsigned long long *vk2 = (unsigned long long *)B.take(8ull * NE + 8);
-                unsigned *vv = (unsigned *)B.take(4ull * NE + 4), *vv2 = (unsigned *)B.take(4ull * NE + 4);
+                unsigned *vv = (unsigned *)B.take(4ull * NE + 4);
                 uint2 *flags = (uint2 *)B.take(8ull * (NE + 2)), *used = (uint2 *)B.take(8ull * (NE + 2));
                 uint2 *excl = (uint2 *)B.take(8ull * (NE + 2));
                 unsigned *vmap = (unsigned *)B.take(4ull * NE + 4), *vmap2 = (unsigned *)B.take(4ull * NE + 4);
@@ -245,16 +244,9 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
 
                 // ---- triangles and edge keys; weld; the last triangle's own vertices out
                 launch_mc_emit(b, sign_mask, codes, lut, rows, tri, vk, s);
-                int walt = 0;
-                SCHK(radix_sort<unsigned long long>(vk, vk2, vv, vv2, NE, key_bits, true, tmpb, d_err, s,
-                                                    &ctx->launches, &walt));
-                const unsigned long long *sk = walt ? vk2 : vk;
-                const unsigned *sv = walt ? vv2 : vv;
-                launch_weld_flags(sk, NE, flags, s);
-                SCHK(scan_u2(flags, flags, NE, tot, tmpb, d_err, s, &ctx->launches));
-                launch_weld_scatter(b, sk, sv, flags, NE, vmap, vq, s);
+                SCHK(launch_weld(b, vk, rows, NE, vk2, vv, vmap, vq, tot, tmpb, d_err, s));
                 launch_remap(tri, n3k, vmap, s);
-                ctx->launches += 4;
+                ctx->launches += 3;
                 SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
                 SCHK(cudaStreamSynchronize(s));
                 const unsigned V = h_tot->x;

@@ -217,7 +217,6 @@ int gs_plan(int device, const GsShape &sh, unsigned nv, const unsigned *mol_off,
 // The same for at most pmax resident slab CTAs (no device query).
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
                 GsPlan &pl);
-// All items share `passes`; the weld keys of every item fit `key_bits` bits and
-// key_bits + bits(count - 1) <= 64.  Results in ctx->batch.
-int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes, int key_bits);
+// All items share `passes`.  Results in ctx->batch.
+int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes);
 }

@@ -32,7 +32,7 @@ struct QGrid {
     int negmin;        // smallest code n with value(n) < 0
     unsigned N;        // atoms
     long long bx, by, bz;  // weld key base (quantised origin - margin)
-    long long Rq;          // weld key radix per axis
+    long long Rq;          // quanta per axis (below 2^21: a weld key holds 21 bits of each)
     // A box of the reference's slicing (else the whole grid: offsets 0, limits G - 1, cell
     // ranges [0, Gc)).  Voxel (i, j, k) of the box is voxel (i + off[0], j + off[1],
     // k + off[2]) of the molecule's grid: SAS positions use the grid index, vertex positions
@@ -66,8 +66,9 @@ struct QBatch {
     const unsigned *tri_off;   // pre-filter triangles (valid after the row scan)
     const unsigned *vtx_off;   // welded vertices (valid after the weld)
     const float *lut;          // 256 field values per molecule
+    const unsigned *layer_off; // owner planes (Gc + 1) per molecule
     unsigned n_mol;
-    int key_bits;              // bits of a molecule-local weld key; the molecule sits above
+    int pad_;
 };
 
 // Largest m with off[m] <= x, for off[0] = 0 <= x < off[n].
