@@ -8,7 +8,7 @@
 //                 32 voxels is one word, so cube indices and edge activity are bit ops.
 //  k_weld         unique quantised positions in lexicographic order (CudaSurf.cu:444-457)
 //  k_closest      closest atom per welded vertex (closestAtomPerVertex, Kernels.cu:547-604)
-//  k_tri_*        drop triangles with a repeated index (CudaSurf.cu:820-829)
+//  k_tri_filter   drop triangles with a repeated index (CudaSurf.cu:820-829)
 //  k_csr_*        neighbour lists in triangle order (getNeighboorsVertices,
 //                 SmoothMesh.cpp:45-123) for the Gauss-Seidel dataflow (k_smooth.cu)
 #include <cfloat>
@@ -388,8 +388,8 @@ __global__ void __launch_bounds__(256, 4) k_mc_batch(QBatch b, const unsigned *_
 // the bins and their loads.
 //
 // A radix sort of all keys (7 or 8 passes over 24 B, flags, scan, scatter) took the weld with its
-// corner remap 0.14 ms at 30 000 edges, 0.83 at 3 700 000, 24.1 at 138 000 000 (0.03, 0.24 and 8.5 so,
-// 3.2 of the last the remap).  A warp sorting each bin of 8 to 32 in registers instead of the
+// corner remap 0.14 ms at 30 000 edges, 0.83 at 3 700 000, 24.1 at 138 000 000 (0.03, 0.20 and 6.6 so,
+// 1.1 of the last the remap).  A warp sorting each bin of 8 to 32 in registers instead of the
 // comparisons: 0.57 and 18.4.
 constexpr int kWeldT = 1024;
 constexpr unsigned kWeldCap = 4096;  // bins at most, of either sort
@@ -522,17 +522,8 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
     __syncthreads();
     const unsigned distinct = block_excl_sums<kWeldT>(uniq, nbin, s_tmp);
     if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        unsigned before = 0;
-        if (lane == 0 && tile) st_release(&status[tile], kFlagAgg | distinct);
-        for (int j = (int)tile - 1; j >= 0; j -= 32) {  // a small grid's layers are all in flight: 32 at a time
-            const unsigned long long st = j >= lane ? wait_status(&status[j - lane], err) : kFlagPre;
-            const unsigned pre = __ballot_sync(0xffffffffu, (st >> 62) != 1);  // an inclusive prefix (or timed out)
-            before += __reduce_add_sync(0xffffffffu, lane <= (pre ? __ffs(pre) - 1 : 31) ? (unsigned)st : 0u);
-            if (pre) break;
-        }
-        if (lane == 0) {
-            st_release(&status[tile], kFlagPre | (unsigned long long)(before + distinct));
+        const unsigned before = (unsigned)look_back(status, tile, distinct, err);
+        if (threadIdx.x == 0) {
             s_before = before;
             if (BATCH && i == 0) vtx_off[m] = before;
             if (tile == layers - 1) {
@@ -574,9 +565,17 @@ __global__ void k_gather_offsets(const uint2 *__restrict__ excl, const unsigned 
     if (outy) outy[m] = v.y;
 }
 
+// Corners from edge slots to vertices.  Bound by the gathers, so each thread has four under way:
+// 832 000 000 corners in 1.1 ms, one to a thread took 3.2.
 __global__ void k_remap(unsigned *__restrict__ tri, size_t n3, const unsigned *__restrict__ vmap) {
-    size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n3) tri[q] = vmap[tri[q]];
+    const size_t q = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (q + 4 <= n3) {
+        uint4 t = *(const uint4 *)(tri + q);
+        t.x = __ldg(vmap + t.x), t.y = __ldg(vmap + t.y), t.z = __ldg(vmap + t.z), t.w = __ldg(vmap + t.w);
+        *(uint4 *)(tri + q) = t;
+    } else {
+        for (size_t e = q; e < n3; e++) tri[e] = vmap[tri[e]];
+    }
 }
 
 // ------------------------------------------------------------ closest atom
@@ -656,47 +655,76 @@ __global__ void k_closest_batch(QBatch b, const float *__restrict__ vq, const un
 
 // ------------------------------------------------------ degenerate filter
 
-__global__ void k_tri_flags(const unsigned *__restrict__ tri, unsigned nt, uint2 *__restrict__ flags) {
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
-    const unsigned a = tri[3ull * t], b = tri[3ull * t + 1], c = tri[3ull * t + 2];
-    flags[t] = make_uint2((a != b && b != c && a != c) ? 1u : 0u, 0u);
-}
-
-__global__ void k_tri_compact(const unsigned *__restrict__ tri, unsigned nt, const uint2 *__restrict__ excl,
-                              unsigned *__restrict__ out) {
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
-    const unsigned a = tri[3ull * t], b = tri[3ull * t + 1], c = tri[3ull * t + 2];
-    if (a != b && b != c && a != c) {
-        const size_t o = 3ull * excl[t].x;
-        out[o] = a; out[o + 1] = b; out[o + 2] = c;
+// Drops the triangles with a repeated corner in one pass: a block's 4096 triangles stay in
+// registers, the kept ones go to shared memory in order and from there, behind those of the blocks
+// before (look-back), to whole lines of `out`.  Batch: molecules flagged QSES_FLAG_KEEP_DEGENERATE
+// keep every triangle, corners become molecule-local vertex ids and kept_off receives each
+// molecule's first kept triangle.  Bound by memory, 24 B a triangle, and by the look-back that
+// orders the blocks: 1024 triangles each took 2.7 ms for 277 000 000, 2048 2.1, 4096 1.9; a flag per
+// triangle, a scan of the flags and a copy 5.2.  7 400 000: 0.19 -> 0.07 ms.
+constexpr int kFiltT = 512, kFiltN = 8, kFiltTile = kFiltN * kFiltT;
+template <bool BATCH>
+__global__ void __launch_bounds__(kFiltT) k_tri_filter(QBatch b, const unsigned *__restrict__ tri, unsigned nt,
+                                                       unsigned *__restrict__ out, unsigned *__restrict__ kept_off,
+                                                       uint2 *__restrict__ total, unsigned long long *status,
+                                                       unsigned *ticket, int *err) {
+    __shared__ unsigned s_out[3 * kFiltTile];
+    __shared__ unsigned s_tmp[kFiltT / 32], s_tile, s_before;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const unsigned tile = s_tile, t0 = tile * kFiltTile + kFiltN * threadIdx.x;
+    unsigned c[3 * kFiltN], m[kFiltN], keep = 0;
+    if (t0 + kFiltN <= nt) {
+        const uint4 *q = (const uint4 *)(tri + 3ull * t0);
+#pragma unroll
+        for (int r = 0; r < 3 * kFiltN / 4; r++) {
+            const uint4 v = q[r];
+            c[4 * r] = v.x, c[4 * r + 1] = v.y, c[4 * r + 2] = v.z, c[4 * r + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 3 * kFiltN; r++) c[r] = t0 + r / 3 < nt ? tri[3ull * t0 + r] : 0u;
     }
-}
-
-// Batch form: molecules flagged QSES_FLAG_KEEP_DEGENERATE keep every triangle; corners are
-// rewritten as molecule-local vertex ids.
-__global__ void k_tri_flags_batch(QBatch b, const unsigned *__restrict__ tri, unsigned nt, uint2 *__restrict__ flags) {
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
-    const unsigned m = qses_find(b.tri_off, b.n_mol, t);
-    const unsigned a = tri[3ull * t], c1 = tri[3ull * t + 1], c2 = tri[3ull * t + 2];
-    const bool keep = (b.mols[m].flags & QSES_FLAG_KEEP_DEGENERATE) || (a != c1 && c1 != c2 && a != c2);
-    flags[t] = make_uint2(keep ? 1u : 0u, 0u);
-}
-
-__global__ void k_tri_compact_batch(QBatch b, const unsigned *__restrict__ tri, unsigned nt,
-                                    const uint2 *__restrict__ excl, unsigned *__restrict__ out) {
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
-    const unsigned m = qses_find(b.tri_off, b.n_mol, t);
-    const unsigned a = tri[3ull * t], c1 = tri[3ull * t + 1], c2 = tri[3ull * t + 2];
-    const bool keep = (b.mols[m].flags & QSES_FLAG_KEEP_DEGENERATE) || (a != c1 && c1 != c2 && a != c2);
-    if (keep) {
-        const unsigned v0 = __ldg(b.vtx_off + m);
-        const size_t o = 3ull * excl[t].x;
-        out[o] = a - v0; out[o + 1] = c1 - v0; out[o + 2] = c2 - v0;
+    unsigned at = BATCH && t0 < nt ? qses_find(b.tri_off, b.n_mol, t0) : 0u;
+#pragma unroll
+    for (int r = 0; r < kFiltN; r++) {
+        if (t0 + r >= nt) continue;
+        if (BATCH)
+            while (__ldg(b.tri_off + at + 1) <= t0 + r) at++;
+        m[r] = at;
+        const unsigned x = c[3 * r], y = c[3 * r + 1], z = c[3 * r + 2];
+        keep |= ((x != y && y != z && x != z) || (BATCH && (b.mols[at].flags & QSES_FLAG_KEEP_DEGENERATE))) << r;
     }
+    unsigned n;
+    const unsigned lo = block_excl_scan<kFiltT>(__popc(keep), n, s_tmp);
+    if (threadIdx.x < 32) {
+        const unsigned before = (unsigned)look_back(status, tile, n, err);
+        if (threadIdx.x == 0) {
+            s_before = before;
+            if (tile == gridDim.x - 1) *total = make_uint2(before + n, 0u);
+        }
+    }
+    unsigned k = lo;
+#pragma unroll
+    for (int r = 0; r < kFiltN; r++)
+        if (keep >> r & 1) {
+            const unsigned v0 = BATCH ? __ldg(b.vtx_off + m[r]) : 0u;
+            s_out[3 * k] = c[3 * r] - v0, s_out[3 * k + 1] = c[3 * r + 1] - v0, s_out[3 * k + 2] = c[3 * r + 2] - v0;
+            k++;
+        }
+    __syncthreads();
+    const unsigned before = s_before;
+    if (BATCH) {  // molecules that start at one of the thread's triangles, or behind the last
+#pragma unroll
+        for (int r = 0; r < kFiltN; r++)
+            if (t0 + r < nt)
+                for (int q = (int)m[r]; q >= 0 && __ldg(b.tri_off + q) == t0 + r; q--)
+                    kept_off[q] = before + lo + __popc(keep & ((1u << r) - 1u));
+        if (tile == gridDim.x - 1 && threadIdx.x == 0)
+            for (int q = (int)b.n_mol; q >= 0 && __ldg(b.tri_off + q) == nt; q--) kept_off[q] = before + n;
+    }
+    if (before <= nt - min(n, nt))
+        for (unsigned q = threadIdx.x; q < 3 * n; q += kFiltT) out[3ull * before + q] = s_out[q];
 }
 
 // --------------------------------------------------------------- smoothing
@@ -813,25 +841,30 @@ void launch_closest_batch(const QBatch &b, const float *vq, const unsigned *vmol
                           cudaStream_t s) {
     k_closest_batch<<<nblk(nv, 128), 128, 0, s>>>(b, vq, vmol, nv, atoms, cells, sorted_to_input, asorted, ainput);
 }
-void launch_tri_flags_batch(const QBatch &b, const unsigned *tri, unsigned nt, uint2 *flags, cudaStream_t s) {
-    k_tri_flags_batch<<<nblk(nt, 256), 256, 0, s>>>(b, tri, nt, flags);
-}
-void launch_tri_compact_batch(const QBatch &b, const unsigned *tri, unsigned nt, const uint2 *excl, unsigned *out,
-                              cudaStream_t s) {
-    k_tri_compact_batch<<<nblk(nt, 256), 256, 0, s>>>(b, tri, nt, excl, out);
-}
 void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s) {
-    k_remap<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, vmap);
+    k_remap<<<nblk((n3 + 3) / 4, 256), 256, 0, s>>>(tri, n3, vmap);
 }
 void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *atoms, const uint2 *cells,
                     const unsigned *sorted_to_input, int *asorted, int *ainput, cudaStream_t s) {
     k_closest<<<nblk(nv, 128), 128, 0, s>>>(g, vq, nv, atoms, cells, sorted_to_input, asorted, ainput);
 }
-void launch_tri_flags(const unsigned *tri, unsigned nt, uint2 *flags, cudaStream_t s) {
-    k_tri_flags<<<nblk(nt, 256), 256, 0, s>>>(tri, nt, flags);
+size_t tri_filter_tmp_bytes(unsigned nt) { return 256 + 8 * (((size_t)nt + kFiltTile - 1) / kFiltTile); }
+template <bool BATCH>
+static cudaError_t filter_with(const QBatch &b, const unsigned *tri, unsigned nt, unsigned *out, unsigned *kept_off,
+                               uint2 *total, void *tmp, int *err, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(tmp, 0, tri_filter_tmp_bytes(nt), s);
+    if (e != cudaSuccess) return e;
+    k_tri_filter<BATCH><<<nblk(nt, kFiltTile), kFiltT, 0, s>>>(b, tri, nt, out, kept_off, total,
+                                                                (unsigned long long *)((char *)tmp + 256), (unsigned *)tmp, err);
+    return cudaGetLastError();
 }
-void launch_tri_compact(const unsigned *tri, unsigned nt, const uint2 *excl, unsigned *out, cudaStream_t s) {
-    k_tri_compact<<<nblk(nt, 256), 256, 0, s>>>(tri, nt, excl, out);
+cudaError_t launch_tri_filter(const unsigned *tri, unsigned nt, unsigned *out, uint2 *total, void *tmp, int *err,
+                              cudaStream_t s) {
+    return filter_with<false>(QBatch{}, tri, nt, out, nullptr, total, tmp, err, s);
+}
+cudaError_t launch_tri_filter_batch(const QBatch &b, const unsigned *tri, unsigned nt, unsigned *out, unsigned *kept_off,
+                                    uint2 *total, void *tmp, int *err, cudaStream_t s) {
+    return filter_with<true>(b, tri, nt, out, kept_off, total, tmp, err, s);
 }
 void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, cudaStream_t s) {
     k_csr_count<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, start);

@@ -32,8 +32,10 @@ cudaError_t launch_weld(const QGrid &g, const unsigned long long *vkey, const ui
 void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s);
 void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *atoms, const uint2 *cells,
                     const unsigned *sorted_to_input, int *asorted, int *ainput, cudaStream_t s);
-void launch_tri_flags(const unsigned *tri, unsigned nt, uint2 *flags, cudaStream_t s);
-void launch_tri_compact(const unsigned *tri, unsigned nt, const uint2 *excl, unsigned *out, cudaStream_t s);
+// Triangles without a repeated corner, in order, to out; their number to *total.
+size_t tri_filter_tmp_bytes(unsigned nt);
+cudaError_t launch_tri_filter(const unsigned *tri, unsigned nt, unsigned *out, uint2 *total, void *tmp, int *err,
+                              cudaStream_t s);
 // Neighbour lists by counting: start (nv + 1 entries, zeroed) -> counts -> (scan) -> corner
 // occurrences scattered per vertex into occ (n3), in any order.
 void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, cudaStream_t s);
@@ -127,8 +129,7 @@ void launch_gather_offsets(const uint2 *excl, const unsigned *at, unsigned n_mol
 void launch_closest_batch(const QBatch &b, const float *vq, const unsigned *vmol, unsigned nv, const float4 *atoms,
                           const uint2 *cells, const unsigned *sorted_to_input, int *asorted, int *ainput,
                           cudaStream_t s);
-void launch_tri_flags_batch(const QBatch &b, const unsigned *tri, unsigned nt, uint2 *flags, cudaStream_t s);
-void launch_tri_compact_batch(const QBatch &b, const unsigned *tri, unsigned nt, const uint2 *excl, unsigned *out,
-                              cudaStream_t s);  // 8 B of shared memory per vertex, 16-bit slab offsets
+cudaError_t launch_tri_filter_batch(const QBatch &b, const unsigned *tri, unsigned nt, unsigned *out, unsigned *kept_off,
+                                    uint2 *total, void *tmp, int *err, cudaStream_t s);  // 8 B of shared memory per vertex, 16-bit slab offsets
 
 }  // namespace qses

@@ -539,7 +539,6 @@ struct FinishSeg {
     int *asorted, *ainput;
     float *vq;
     unsigned *tri, *tri_kept;
-    uint2 *tflags;
     void *tmp2;
     uint2 *tot;
     int *err;
@@ -579,10 +578,7 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
     ctx->mark("closest_atom");
     // drop degenerate triangles (API_computeSES filter)
     if (!c.keep_all && c.nt > 0) {
-        launch_tri_flags(c.tri, c.nt, c.tflags, sd);
-        ctx->launches++;
-        QCHK(scan_u2(c.tflags, c.tflags, c.nt, c.tot, c.tmp2, c.err, sd, &ctx->launches));
-        launch_tri_compact(c.tri, c.nt, c.tflags, c.tri_kept, sd);
+        QCHK(launch_tri_filter(c.tri, c.nt, c.tri_kept, c.tot, c.tmp2, c.err, sd));
         ctx->launches++;
         QCHK(cudaMemcpyAsync(c.h_out, c.tot, sizeof(uint2), cudaMemcpyDeviceToHost, sd));
     }
@@ -742,14 +738,13 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    size_t tmpB = std::max({weld_tmp_bytes((unsigned)E), scan_u2_tmp_bytes(NE), scan_u2_tmp_bytes(T),
-                            scan_u2_tmp_bytes(NE + 1)});
-    const size_t nflag = std::max<size_t>((size_t)NE + 1, (size_t)T) + 1;
+    size_t tmpB = std::max(weld_tmp_bytes((unsigned)E), scan_u2_tmp_bytes(NE + 1));
+    const size_t nflag = (size_t)NE + 2;
     size_t needB = 2 * align256(4 * n3) + 2 * align256(8ull * NE) + 2 * align256(4ull * NE) + align256(8ull * nflag) +
                    align256(4ull * NE) + align256(12ull * NE) + 2 * align256(4ull * NE) + align256(4 * n3 + 4) +
                    align256(8 * n3) + 3 * align256(4ull * NE) + align256(64ull * NE + 64) + 4096 +
                    align256(16ull * NE + 16) +
-                   align256(tmpB) + align256(8ull * T + 16) + align256(scan_u2_tmp_bytes(T + 1)) + 4096;
+                   align256(tmpB) + align256(tri_filter_tmp_bytes(T)) + 4096;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
@@ -767,9 +762,8 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
     float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
     void *tmpb = B.take(tmpB);
-    uint2 *tflags = (uint2 *)B.take(8ull * T + 16);      // degenerate filter (side stream)
-    void *tmp2 = B.take(scan_u2_tmp_bytes(T + 1));       // its scan's scratch
-    if (!tmpb || !tflags || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
+    void *tmp2 = B.take(tri_filter_tmp_bytes(T));  // degenerate filter (side stream)
+    if (!tmpb || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
 
     // ---- triangles + pre-weld vertex keys; weld
     MeshSeg b;
@@ -827,7 +821,6 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     c.vq = vq;
     c.tri = tri;
     c.tri_kept = tri_kept;
-    c.tflags = tflags;
     c.tmp2 = tmp2;
     c.tot = a.tot;
     c.err = d_err;

@@ -173,11 +173,10 @@ struct BatchFinishSeg {
     int *asorted, *ainput;
     float *vq;
     unsigned *tri, *tri_kept;
-    uint2 *tflags;
     void *tmp2;
     uint2 *tot;
     int *err;
-    unsigned *tri_off, *kept_off;
+    unsigned *kept_off;
     unsigned char *h_out;  // pinned: [0, 8) kept triangles, [8, 12) error word
     void *h_kept;          // pinned: per-molecule first kept triangle
     char *h_dl;            // pinned host mesh block, or null
@@ -214,12 +213,7 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
     ctx->mark("closest_atom");
     // per-molecule filter and molecule-local corner ids
     if (c.nt > 0) {
-        launch_tri_flags_batch(c.b, c.tri, c.nt, c.tflags, sd);
-        ctx->launches++;
-        QCHK(scan_u2(c.tflags, c.tflags, c.nt, c.tot, c.tmp2, c.err, sd, &ctx->launches));
-        launch_tri_compact_batch(c.b, c.tri, c.nt, c.tflags, c.tri_kept, sd);
-        ctx->launches++;
-        launch_gather_offsets(c.tflags, c.tri_off, nm, c.nt, c.tot, c.kept_off, nullptr, sd);
+        QCHK(launch_tri_filter_batch(c.b, c.tri, c.nt, c.tri_kept, c.kept_off, c.tot, c.tmp2, c.err, sd));
         ctx->launches++;
     } else {
         QCHK(cudaMemsetAsync(c.kept_off, 0, 4ull * (nm + 1), sd));
@@ -440,13 +434,12 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    const size_t tmpB = std::max({weld_tmp_bytes(layer_off[nm]), scan_u2_tmp_bytes(NE), scan_u2_tmp_bytes(T),
-                                  scan_u2_tmp_bytes(NE + 1)});
-    const size_t nflag = std::max<size_t>((size_t)NE + 1, (size_t)T) + 1;
+    const size_t tmpB = std::max(weld_tmp_bytes(layer_off[nm]), scan_u2_tmp_bytes(NE + 1));
+    const size_t nflag = (size_t)NE + 2;
     const size_t needB = 2 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
                          a256(8ull * nflag) + a256(4ull * NE + 4) + a256(12ull * NE + 12) + 3 * a256(4ull * NE + 4) +
-                         a256(4 * n3 + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) + a256(16ull * NE + 16) + a256(tmpB) + a256(8ull * T + 16) +
-                         a256(scan_u2_tmp_bytes(T + 1)) + 8192;
+                         a256(4 * n3 + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) + a256(16ull * NE + 16) + a256(tmpB) +
+                         a256(tri_filter_tmp_bytes(T)) + 8192;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "batch mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
@@ -465,9 +458,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
     float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
     void *tmpb = B.take(tmpB);
-    uint2 *tflags = (uint2 *)B.take(8ull * T + 16);  // degenerate filter (side stream)
-    void *tmp2 = B.take(scan_u2_tmp_bytes(T + 1));   // its scan's scratch
-    if (!tmpb || !tflags || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "batch mesh workspace layout");
+    void *tmp2 = B.take(tri_filter_tmp_bytes(T));  // degenerate filter (side stream)
+    if (!tmpb || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "batch mesh workspace layout");
 
     // ---- triangles + weld keys, then one weld for all molecules
     BatchMeshSeg mb;
@@ -528,11 +520,9 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     c.vq = vq;
     c.tri = tri;
     c.tri_kept = tri_kept;
-    c.tflags = tflags;
     c.tmp2 = tmp2;
     c.tot = a.tot;
     c.err = d_err;
-    c.tri_off = d_tri_off;
     c.kept_off = d_kept_off;
     c.h_out = ctx->h_small;
     c.h_kept = ctx->h_stage;

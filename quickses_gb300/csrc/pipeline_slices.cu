@@ -216,11 +216,11 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 // ---- mesh workspace of this slice
                 const size_t n3 = 3ull * T, n3k = 3ull * T1;
                 const size_t tmpB = std::max({weld_tmp_bytes((unsigned)b.Gc + 1), scan_u2_tmp_bytes(NE + 1),
-                                              scan_u2_tmp_bytes(T + 1)});
+                                              tri_filter_tmp_bytes(T)});
                 const size_t needB = 3 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
                                      3 * a256(8ull * (NE + 2)) + 2 * a256(4ull * NE + 4) + 2 * a256(12ull * NE + 12) +
                                      2 * a256(4ull * NE + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) +
-                                     a256(16ull * NE + 16) + a256(8ull * T + 16) + a256(tmpB) + 4096;
+                                     a256(16ull * NE + 16) + a256(tmpB) + 4096;
                 if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
                 Arena &B = ctx->mesh_ws;
                 unsigned *tri = (unsigned *)B.take(4 * n3 + 4), *tri_kept = (unsigned *)B.take(4 * n3 + 4);
@@ -238,7 +238,6 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
                 uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
                 float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
-                uint2 *tflags = (uint2 *)B.take(8ull * T + 16);
                 void *tmpb = B.take(tmpB);
                 if (!tmpb) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
 
@@ -286,10 +285,8 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 const unsigned *tri_out = tri;
                 unsigned nt = T1;
                 if (!keep_all) {
-                    launch_tri_flags(tri, T1, tflags, s);
-                    SCHK(scan_u2(tflags, tflags, T1, tot, tmpb, d_err, s, &ctx->launches));
-                    launch_tri_compact(tri, T1, tflags, tri_kept, s);
-                    ctx->launches += 2;
+                    SCHK(launch_tri_filter(tri, T1, tri_kept, tot, tmpb, d_err, s));
+                    ctx->launches++;
                     SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
                     SCHK(cudaStreamSynchronize(s));
                     nt = h_tot->x;
