@@ -400,11 +400,60 @@ int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out) {
     return QSES_OK;
 }
 
-int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, float4 *pos4,
-                  unsigned nv, const unsigned *tri, unsigned *occ, const uint2 *deg, unsigned *nbr, unsigned *word0,
-                  uint4 *pack, unsigned *ext, unsigned *ext0, unsigned *scratch, const GsBuffers &gb,
+// The two sets in the same memory: nothing of the weld is read after it.
+static bool take_weld(Arena &a, unsigned ne, unsigned layers, WeldBuffers &w) {
+    w.vk = (unsigned long long *)a.take(8ull * ne + 8);
+    w.vk2 = (unsigned long long *)a.take(8ull * ne + 8);
+    w.vv = (unsigned *)a.take(4ull * ne + 4);
+    return (w.tmp = a.take(weld_tmp_bytes(layers))) != nullptr;
+}
+static bool take_smooth(Arena &a, unsigned ne, size_t n3, SmoothBuffers &sb) {
+    sb.deg = (uint2 *)a.take(8ull * (ne + 2));
+    sb.occ = (unsigned *)a.take(4 * n3 + 4);
+    sb.nbr = (unsigned *)a.take(8 * n3 + 8);
+    sb.word0 = (unsigned *)a.take(4ull * ne + 4);
+    sb.pack = (uint4 *)a.take(64ull * ne + 64);
+    sb.ext = (unsigned *)a.take(1ull * ne + 64);
+    sb.ext0 = (unsigned *)a.take(1ull * ne + 64);
+    sb.pos4 = (float4 *)a.take(16ull * ne + 16);
+    return (sb.tmp = a.take(scan_u2_tmp_bytes(ne + 1))) != nullptr;
+}
+size_t weld_or_smooth_bytes(unsigned ne, unsigned layers, size_t n3, bool smooth) {
+    WeldBuffers w;
+    SmoothBuffers sb;
+    Arena m;  // measures: no memory behind it, every take fits
+    m.cap = ~(size_t)0 / 2;
+    take_weld(m, ne, layers, w);
+    size_t bytes = m.off;
+    if (smooth) {
+        m.off = 0;
+        take_smooth(m, ne, n3, sb);
+        bytes = std::max(bytes, m.off);
+    }
+    return bytes + 256;
+}
+bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool smooth, WeldBuffers &w, SmoothBuffers &sb) {
+    Arena part;
+    part.cap = weld_or_smooth_bytes(ne, layers, n3, smooth);
+    part.base = a.take(part.cap);
+    if (!part.base || !take_weld(part, ne, layers, w)) return false;
+    part.off = 0;
+    memset(&sb, 0, sizeof(sb));
+    return !smooth || take_smooth(part, ne, n3, sb);
+}
+
+int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
+                  const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
                   const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback) {
     cudaStream_t s = ctx->stream;
+    float4 *pos4 = sb.pos4;
+    // neighbour lists: count the corners per vertex, scan, scatter them per vertex
+    QCHK(cudaMemsetAsync(sb.deg, 0, 8ull * (nv + 1), s));
+    launch_csr_count(tri, n3, sb.deg, s);
+    ctx->launches++;
+    QCHK(scan_u2(sb.deg, sb.deg, nv + 1, nullptr, sb.tmp, d_err, s, &ctx->launches));
+    launch_csr_scatter(tri, n3, sb.deg, sb.occ, s);
+    ctx->launches++;
     launch_to_float4(vq, nv, pos4, s);
     ctx->launches++;
     if (sh.flags & kGsPersistL2) gs_l2_window(ctx->device, s, pos4, 16ull * nv);
@@ -416,8 +465,9 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
     for (unsigned w = 0; w < L.waves; w++) {
         const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
         if (w) QCHK(cudaMemsetAsync(gb.ord.longs, 0, 4, s));
-        launch_gs_lists(tri, occ, deg, nbr, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, word0, pack,
-                        (unsigned char *)ext, passes > 1 ? (unsigned char *)ext0 : nullptr, gb.ord, scratch, d_err, s);
+        launch_gs_lists(tri, sb.occ, sb.deg, sb.nbr, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, sb.word0,
+                        sb.pack, (unsigned char *)sb.ext, passes > 1 ? (unsigned char *)sb.ext0 : nullptr, gb.ord, scratch,
+                        d_err, s);
         ctx->launches += 2;
     }
     if (together && passes > 1) {
@@ -426,12 +476,12 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
     }
     ctx->mark("smooth_csr");
     for (int pass = 0; pass < (together ? 1 : passes); pass++) {
-        if (pass) QCHK(cudaMemcpyAsync(ext, ext0, nv, cudaMemcpyDeviceToDevice, s));
+        if (pass) QCHK(cudaMemcpyAsync(sb.ext, sb.ext0, nv, cudaMemcpyDeviceToDevice, s));
         for (unsigned w = 0; w < L.waves; w++) {
             const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
             if (pass || w) QCHK(cudaMemsetAsync(gb.next_slab, 0, 4, s));
             QCHK(launch_gs_slab(pos4, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, L.qcap, gb.next_slab, L.ctas,
-                                sh.threads, deg, nbr, word0, pack, ext, (const unsigned char *)ext0,
+                                sh.threads, sb.deg, sb.nbr, sb.word0, sb.pack, sb.ext, (const unsigned char *)sb.ext0,
                                 together ? (unsigned)passes : 1u, (unsigned)pass + 1u, gb.ord, d_err, 4000000000ll,
                                 ctx->profiling ? stats : nullptr, s));
             ctx->launches++;
@@ -545,14 +595,8 @@ struct FinishSeg {
     unsigned char *h_out;  // pinned: [0, 8) kept triangles, [8, 12) error word, [2048, 2112) stats
     char *h_dl;            // pinned host mesh block, or null
     unsigned long long dl_vb, dl_tb, dl_ab;
-    uint2 *deg;
-    unsigned *okey, *nbr;  // okey: the corners scattered per vertex
-    void *tmpb;
-    float4 *pos4;
-    unsigned *word0;       // per vertex: word and common list of the smoothing pass
-    uint4 *pack;
+    SmoothBuffers sb;
     unsigned *scratch;     // one word per vertex
-    unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
     GsBuffers gb;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
     unsigned long long *stats;
@@ -598,16 +642,8 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
 
     // Gauss-Seidel smoothing on the device
     if (c.passes > 0 && c.nv > 0 && c.nt > 0) {
-        // neighbour lists: count the corners per vertex, scan, scatter them per vertex
-        QCHK(cudaMemsetAsync(c.deg, 0, 8ull * (c.nv + 1), s));
-        launch_csr_count(c.tri, c.n3, c.deg, s);
-        ctx->launches++;
-        QCHK(scan_u2(c.deg, c.deg, c.nv + 1, nullptr, c.tmpb, c.err, s, &ctx->launches));
-        launch_csr_scatter(c.tri, c.n3, c.deg, c.okey, s);
-        ctx->launches++;
         // the closest-atom pass on the side stream reads the welded positions in vq
-        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.tri, c.okey, c.deg, c.nbr, c.word0, c.pack, c.ext, c.ext0,
-                                     c.scratch, c.gb, c.h_table, c.err, c.stats, c.fork ? ctx->ev_join : nullptr);
+        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table, c.err, c.stats, c.fork ? ctx->ev_join : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -738,32 +774,22 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    size_t tmpB = std::max(weld_tmp_bytes((unsigned)E), scan_u2_tmp_bytes(NE + 1));
-    const size_t nflag = (size_t)NE + 2;
-    size_t needB = 2 * align256(4 * n3) + 2 * align256(8ull * NE) + 2 * align256(4ull * NE) + align256(8ull * nflag) +
-                   align256(4ull * NE) + align256(12ull * NE) + 2 * align256(4ull * NE) + align256(4 * n3 + 4) +
-                   align256(8 * n3) + 3 * align256(4ull * NE) + align256(64ull * NE + 64) + 4096 +
-                   align256(16ull * NE + 16) +
-                   align256(tmpB) + align256(tri_filter_tmp_bytes(T)) + 4096;
+    const bool may_smooth = p.smooth_passes > 0;
+    const size_t needB = 2 * align256(4 * n3 + 4) + 3 * align256(4ull * NE + 4) + align256(12ull * NE + 12) +
+                         align256(weld_or_smooth_bytes(NE, (unsigned)E, n3, may_smooth)) +
+                         align256(tri_filter_tmp_bytes(T)) + 4096;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
     unsigned *tri_kept = (unsigned *)B.take(4 * n3 + 4);
-    unsigned long long *vk = (unsigned long long *)B.take(8ull * NE + 8), *vk2 = (unsigned long long *)B.take(8ull * NE + 8);
-    unsigned *vv = (unsigned *)B.take(4ull * NE + 4);
-    uint2 *flags = (uint2 *)B.take(8ull * nflag);
     unsigned *vmap = (unsigned *)B.take(4ull * NE + 4);
     float *vq = (float *)B.take(12ull * NE + 12);
     int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);
-    unsigned *okey = (unsigned *)B.take(4 * n3 + 4);
-    unsigned *nbr = (unsigned *)B.take(8 * n3 + 8);
-    unsigned *ext = (unsigned *)B.take(1ull * NE + 64), *ext0 = (unsigned *)B.take(1ull * NE + 64);
-    unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
-    uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
-    float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
-    void *tmpb = B.take(tmpB);
     void *tmp2 = B.take(tri_filter_tmp_bytes(T));  // degenerate filter (side stream)
-    if (!tmpb || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
+    WeldBuffers wb;
+    SmoothBuffers sb;
+    const bool fits = take_weld_or_smooth(B, NE, (unsigned)E, n3, may_smooth, wb, sb);
+    if (!tmp2 || !fits) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
 
     // ---- triangles + pre-weld vertex keys; weld
     MeshSeg b;
@@ -774,13 +800,13 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     b.lut = a.lut;
     b.rows = a.rows;
     b.tri = tri;
-    b.vk = vk;
-    b.vk2 = vk2;
-    b.vv = vv;
+    b.vk = wb.vk;
+    b.vk2 = wb.vk2;
+    b.vv = wb.vv;
     b.tot = a.tot;
     b.vmap = vmap;
     b.vq = vq;
-    b.tmp = tmpb;
+    b.tmp = wb.tmp;
     b.err = d_err;
     b.h_out = ctx->h_small;
     b.n3 = n3;
@@ -831,15 +857,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
         c.dl_tb = dl.tb;
         c.dl_ab = dl.ab;
     }
-    c.deg = flags;  // reuse: nv + 1 <= NE + 1 entries
-    c.okey = okey;
-    c.nbr = nbr;
-    c.tmpb = tmpb;
-    c.pos4 = pos4;
-    c.word0 = word0;
-    c.pack = pack;
-    c.ext = ext;
-    c.ext0 = ext0;
+    c.sb = sb;
     c.scratch = vmap;  // free after the weld
     c.stats = (unsigned long long *)((char *)ctx->small + 256);
     c.n3 = n3;

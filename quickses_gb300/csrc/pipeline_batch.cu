@@ -181,14 +181,8 @@ struct BatchFinishSeg {
     void *h_kept;          // pinned: per-molecule first kept triangle
     char *h_dl;            // pinned host mesh block, or null
     unsigned long long dl_vb, dl_tb, dl_ab;
-    uint2 *deg;
-    unsigned *okey, *nbr;  // okey: the corners scattered per vertex
-    void *tmpb;
-    float4 *pos4;
-    unsigned *word0;       // per vertex: word and common list of the smoothing pass
-    uint4 *pack;
+    SmoothBuffers sb;
     unsigned *scratch;     // one word per vertex
-    unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
     GsBuffers gb;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
     unsigned long long n3;
@@ -236,16 +230,8 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
 
     // Gauss-Seidel over all molecules
     if (c.passes > 0 && c.nv > 0 && c.nt > 0) {
-        // neighbour lists: count the corners per vertex, scan, scatter them per vertex
-        QCHK(cudaMemsetAsync(c.deg, 0, 8ull * (c.nv + 1), s));
-        launch_csr_count(c.tri, c.n3, c.deg, s);
-        ctx->launches++;
-        QCHK(scan_u2(c.deg, c.deg, c.nv + 1, nullptr, c.tmpb, c.err, s, &ctx->launches));
-        launch_csr_scatter(c.tri, c.n3, c.deg, c.okey, s);
-        ctx->launches++;
         // the closest-atom pass on the side stream reads the welded positions in vq
-        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.pos4, c.nv, c.tri, c.okey, c.deg, c.nbr, c.word0, c.pack, c.ext, c.ext0,
-                                     c.scratch, c.gb, c.h_table, c.err, nullptr, c.fork ? ctx->ev_join : nullptr);
+        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table, c.err, nullptr, c.fork ? ctx->ev_join : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -434,32 +420,21 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    const size_t tmpB = std::max(weld_tmp_bytes(layer_off[nm]), scan_u2_tmp_bytes(NE + 1));
-    const size_t nflag = (size_t)NE + 2;
-    const size_t needB = 2 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
-                         a256(8ull * nflag) + a256(4ull * NE + 4) + a256(12ull * NE + 12) + 3 * a256(4ull * NE + 4) +
-                         a256(4 * n3 + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) + a256(16ull * NE + 16) + a256(tmpB) +
-                         a256(tri_filter_tmp_bytes(T)) + 8192;
+    const size_t needB = 2 * a256(4 * n3 + 4) + 4 * a256(4ull * NE + 4) + a256(12ull * NE + 12) +
+                         a256(weld_or_smooth_bytes(NE, layer_off[nm], n3, passes > 0)) + a256(tri_filter_tmp_bytes(T)) + 4096;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "batch mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
     unsigned *tri_kept = (unsigned *)B.take(4 * n3 + 4);
-    unsigned long long *vk = (unsigned long long *)B.take(8ull * NE + 8), *vk2 = (unsigned long long *)B.take(8ull * NE + 8);
-    unsigned *vv = (unsigned *)B.take(4ull * NE + 4);
-    uint2 *flags = (uint2 *)B.take(8ull * nflag);
     unsigned *vmap = (unsigned *)B.take(4ull * NE + 4);
     float *vq = (float *)B.take(12ull * NE + 12);
     unsigned *vmol = (unsigned *)B.take(4ull * NE + 4);
     int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);
-    unsigned *okey = (unsigned *)B.take(4 * n3 + 4);
-    unsigned *nbr = (unsigned *)B.take(8 * n3 + 8);
-    unsigned *ext = (unsigned *)B.take(1ull * NE + 64), *ext0 = (unsigned *)B.take(1ull * NE + 64);
-    unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
-    uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
-    float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
-    void *tmpb = B.take(tmpB);
     void *tmp2 = B.take(tri_filter_tmp_bytes(T));  // degenerate filter (side stream)
-    if (!tmpb || !tmp2) return ctx->fail(QSES_ERR_INTERNAL, "batch mesh workspace layout");
+    WeldBuffers wb;
+    SmoothBuffers sb;
+    const bool fits = take_weld_or_smooth(B, NE, layer_off[nm], n3, passes > 0, wb, sb);
+    if (!tmp2 || !fits) return ctx->fail(QSES_ERR_INTERNAL, "batch mesh workspace layout");
 
     // ---- triangles + weld keys, then one weld for all molecules
     BatchMeshSeg mb;
@@ -469,14 +444,14 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     mb.codes = a.codes;
     mb.rows = a.rows;
     mb.tri = tri;
-    mb.vk = vk;
-    mb.vk2 = vk2;
-    mb.vv = vv;
+    mb.vk = wb.vk;
+    mb.vk2 = wb.vk2;
+    mb.vv = wb.vv;
     mb.tot = a.tot;
     mb.vmap = vmap;
     mb.vq = vq;
     mb.vmol = vmol;
-    mb.tmp = tmpb;
+    mb.tmp = wb.tmp;
     mb.err = d_err;
     mb.edge_off = d_edge_off;
     mb.vtx_off = d_vtx_off;
@@ -532,15 +507,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         c.dl_tb = dl.tb;
         c.dl_ab = dl.ab;
     }
-    c.deg = flags;
-    c.okey = okey;
-    c.nbr = nbr;
-    c.tmpb = tmpb;
-    c.pos4 = pos4;
-    c.word0 = word0;
-    c.pack = pack;
-    c.ext = ext;
-    c.ext0 = ext0;
+    c.sb = sb;
     c.scratch = vmap;  // free after the weld
     c.n3 = n3;
     c.nv = nv;

@@ -215,35 +215,27 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
 
                 // ---- mesh workspace of this slice
                 const size_t n3 = 3ull * T, n3k = 3ull * T1;
-                const size_t tmpB = std::max({weld_tmp_bytes((unsigned)b.Gc + 1), scan_u2_tmp_bytes(NE + 1),
-                                              tri_filter_tmp_bytes(T)});
-                const size_t needB = 3 * a256(4 * n3 + 4) + 2 * a256(8ull * NE + 8) + 2 * a256(4ull * NE + 4) +
-                                     3 * a256(8ull * (NE + 2)) + 2 * a256(4ull * NE + 4) + 2 * a256(12ull * NE + 12) +
-                                     2 * a256(4ull * NE + 4) + a256(8 * n3 + 8) + 3 * a256(4ull * NE + 4) + a256(64ull * NE + 64) +
-                                     a256(16ull * NE + 16) + a256(tmpB) + 4096;
+                const bool may_smooth = p.smooth_passes > 0;
+                const size_t tmpB = std::max(scan_u2_tmp_bytes(NE + 1), tri_filter_tmp_bytes(T));
+                const size_t needB = 2 * a256(4 * n3 + 4) + 2 * a256(8ull * (NE + 2)) + 4 * a256(4ull * NE + 4) +
+                                     2 * a256(12ull * NE + 12) + a256(tmpB) +
+                                     a256(weld_or_smooth_bytes(NE, (unsigned)b.Gc + 1, n3, may_smooth)) + 4096;
                 if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
                 Arena &B = ctx->mesh_ws;
                 unsigned *tri = (unsigned *)B.take(4 * n3 + 4), *tri_kept = (unsigned *)B.take(4 * n3 + 4);
-                unsigned *okey = (unsigned *)B.take(4 * n3 + 4);
-                unsigned long long *vk = (unsigned long long *)B.take(8ull * NE + 8);
-                unsigned long long *vk2 = (unsigned long long *)B.take(8ull * NE + 8);
-                unsigned *vv = (unsigned *)B.take(4ull * NE + 4);
-                uint2 *flags = (uint2 *)B.take(8ull * (NE + 2)), *used = (uint2 *)B.take(8ull * (NE + 2));
-                uint2 *excl = (uint2 *)B.take(8ull * (NE + 2));
+                uint2 *used = (uint2 *)B.take(8ull * (NE + 2)), *excl = (uint2 *)B.take(8ull * (NE + 2));
                 unsigned *vmap = (unsigned *)B.take(4ull * NE + 4), *vmap2 = (unsigned *)B.take(4ull * NE + 4);
                 float *vq = (float *)B.take(12ull * NE + 12), *vq2 = (float *)B.take(12ull * NE + 12);
                 int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);
-                unsigned *nbr = (unsigned *)B.take(8 * n3 + 8);
-                unsigned *ext = (unsigned *)B.take(1ull * NE + 64), *ext0 = (unsigned *)B.take(1ull * NE + 64);
-                unsigned *word0 = (unsigned *)B.take(4ull * NE + 4);
-                uint4 *pack = (uint4 *)B.take(64ull * NE + 64);
-                float4 *pos4 = (float4 *)B.take(16ull * NE + 16);
                 void *tmpb = B.take(tmpB);
-                if (!tmpb) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
+                WeldBuffers wb;
+                SmoothBuffers sb;
+                const bool fits = take_weld_or_smooth(B, NE, (unsigned)b.Gc + 1, n3, may_smooth, wb, sb);
+                if (!tmpb || !fits) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
 
                 // ---- triangles and edge keys; weld; the last triangle's own vertices out
-                launch_mc_emit(b, sign_mask, codes, lut, rows, tri, vk, s);
-                SCHK(launch_weld(b, vk, rows, NE, vk2, vv, vmap, vq, tot, tmpb, d_err, s));
+                launch_mc_emit(b, sign_mask, codes, lut, rows, tri, wb.vk, s);
+                SCHK(launch_weld(b, wb.vk, rows, NE, wb.vk2, wb.vv, vmap, vq, tot, wb.tmp, d_err, s));
                 launch_remap(tri, n3k, vmap, s);
                 ctx->launches += 3;
                 SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
@@ -263,12 +255,6 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 launch_closest(g, vq2, nv, atoms, cells, sidx, asorted, ainput, s);
                 ctx->launches++;
                 if (p.smooth_passes > 0 && nv > 0) {
-                    uint2 *deg = flags;  // nv + 1 <= NE + 1 entries
-                    SCHK(cudaMemsetAsync(deg, 0, 8ull * (nv + 1), s));
-                    launch_csr_count(tri, n3k, deg, s);
-                    SCHK(scan_u2(deg, deg, nv + 1, nullptr, tmpb, d_err, s, &ctx->launches));
-                    launch_csr_scatter(tri, n3k, deg, okey, s);
-                    ctx->launches += 2;
                     GsShape sh = ctx->gs_force.threads ? ctx->gs_force : gs_shape(nv, false, nv, p.smooth_passes);
                     ctx->gs_used = sh;
                     GsPlan plan;
@@ -277,9 +263,8 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                     GsBuffers gb;
                     const int brc = gs_buffers(ctx, plan, gb);
                     if (brc != QSES_OK) return brc;
-                    const int src = run_smoothing(ctx, sh, plan.L, p.smooth_passes, vq2, pos4, nv, tri, okey, deg, nbr,
-                                                  word0, pack, ext, ext0, vmap, gb, ctx->h_gs, d_err,
-                                                  stats);
+                    const int src = run_smoothing(ctx, sh, plan.L, p.smooth_passes, vq2, nv, tri, n3k, sb, vmap, gb,
+                                                  ctx->h_gs, d_err, stats);
                     if (src != QSES_OK) return src;
                 }
                 const unsigned *tri_out = tri;

@@ -196,16 +196,32 @@ struct GsBuffers {
     unsigned long long zero_words;  // from next_slab on: the counter, ord.done and ord.far
 };
 int gs_buffers(qses_context *ctx, const GsPlan &pl, GsBuffers &out);
+// What the smoothing works in, for up to ne vertices and n3 triangle corners.
+struct SmoothBuffers {
+    uint2 *deg;            // neighbour-list offsets
+    unsigned *occ, *nbr;   // occ: the corners scattered per vertex
+    unsigned *word0;       // per vertex: word and common list of a pass
+    uint4 *pack;
+    unsigned *ext, *ext0;  // release counters, one byte per vertex, and what a pass starts with
+    float4 *pos4;
+    void *tmp;
+};
+// A mesh workspace's part that the weld needs first and the smoothing, if there is any, afterwards.
+struct WeldBuffers {
+    unsigned long long *vk, *vk2;
+    unsigned *vv;
+    void *tmp;
+};
+size_t weld_or_smooth_bytes(unsigned ne, unsigned layers, size_t n3, bool smooth);
+bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool smooth, WeldBuffers &w, SmoothBuffers &sb);
 // `passes` exact Gauss-Seidel passes over vertices [0, nv): positions vq (3 floats each) in
-// and out, triangle corners occ scattered per vertex (deg offsets), shape sh; scratch: one word
-// per vertex.  Vertices in one
+// and out, triangles tri (n3 corners), shape sh; scratch: one word per vertex.  Vertices in one
 // wave: one launch for all passes.  Otherwise waves and passes follow one another; every
 // dependency points to a lower id, so a wave only depends on earlier, finished waves.
 // `before_writeback` (may be null): event the stream waits for before the smoothed
 // positions overwrite vq (work on another stream that still reads the welded positions).
-int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, float4 *pos4,
-                  unsigned nv, const unsigned *tri, unsigned *occ, const uint2 *deg, unsigned *nbr, unsigned *word0,
-                  uint4 *pack, unsigned *ext, unsigned *ext0, unsigned *scratch, const GsBuffers &gb,
+int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
+                  const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
                   const unsigned *h_table, int *d_err, unsigned long long *stats,
                   cudaEvent_t before_writeback = nullptr);
 // Slab plan of a pass over nv vertices.  mol_off (nm + 1 entries, null for one molecule):
