@@ -1,11 +1,12 @@
 // Marching cubes, vertex weld, closest atom, degenerate filter and Laplacian smoothing.
 //
-//  k_mc<false>    per (x, y) row of cells: triangle count and active-edge count
-//                 (countVertexPerCell, MarchingCubes.cu:571-658, single-slice cell range)
-//  k_mc<true>     the same rows again: triangles in cell linear order x*G^2 + y*G + z and
-//                 one quantised key per active edge (generateTriangleVerticesSMEM +
-//                 groupVertices, MarchingCubes.cu:736-862).  One warp per row; the sign of
-//                 32 voxels is one word, so cube indices and edge activity are bit ops.
+//  k_mc_count     per (x, y) row of cells: triangle count and active-edge count
+//                 (countVertexPerCell, MarchingCubes.cu:571-658, single-slice cell range),
+//                 and for each word of a row what the words before it have
+//  k_mc_emit      triangles in cell linear order x*G^2 + y*G + z and one quantised key per
+//                 active edge (generateTriangleVerticesSMEM + groupVertices,
+//                 MarchingCubes.cu:736-862).  The sign of 32 voxels is one word, so cube
+//                 indices and edge activity are bit ops.
 //  k_weld         unique quantised positions in lexicographic order (CudaSurf.cu:444-457)
 //  k_closest      closest atom per welded vertex (closestAtomPerVertex, Kernels.cu:547-604)
 //  k_tri_filter   drop triangles with a repeated index (CudaSurf.cu:820-829)
@@ -24,12 +25,6 @@ namespace qses {
 
 __constant__ unsigned long long c_mc[256] = QSES_MC_TABLE_INIT;
 
-// Owner of each cube edge relative to the cell: bit0 di, bit1 dj, bit2 dk, bits3-4 axis.
-// Edges follow MarchingCubes.cu:814-825 with corners as in :625-632.
-constexpr unsigned long long kEdgeOwner =
-    (0ull << 0) | (9ull << 5) | (2ull << 10) | (8ull << 15) | (4ull << 20) | (13ull << 25) | (6ull << 30) |
-    (12ull << 35) | (16ull << 40) | (17ull << 45) | (19ull << 50) | (18ull << 55);
-
 __device__ __forceinline__ unsigned ld_sign(const unsigned *__restrict__ sign, const QGrid &g, int i, int j, int w) {
     if (i >= g.G || j >= g.G || w >= g.W) return 0u;
     return __ldg(&sign[((size_t)i * g.G + j) * g.W + w]);
@@ -43,32 +38,35 @@ __device__ __forceinline__ unsigned cube_index(unsigned b, unsigned c0, unsigned
 
 __device__ __forceinline__ unsigned warp_sum(unsigned v) { return __reduce_add_sync(0xffffffffu, v); }
 
+// round(p / 0.001) (groupVertices, MarchingCubes.cu:859).  Division by a constant with one
+// multiplication and one correction (Markstein, IBM J. Res. Dev. 34, 1990): the rounded quotient is
+// that of p / 0.001f for every |p| up to 16384, the coordinates a grid may have (all floats tried).
+__device__ __forceinline__ int quantum(float p) {
+    constexpr float r = 1.0f / QSES_WELD_TOL;
+    const float q = __fmul_rn(p, r);
+    return (int)roundf(__fmaf_rn(__fmaf_rn(-q, QSES_WELD_TOL, p), r, q));
+}
 // Quantised key of the vertex on edge (i, j, k) -> (i, j, k) + e_axis.
-__device__ unsigned long long edge_key(const QGrid &g, const unsigned char *__restrict__ codes, const float *lut,
-                                       int i, int j, int k, int ax) {
+__device__ __forceinline__ unsigned long long edge_key(const QGrid &g, const unsigned char *__restrict__ codes,
+                                                       const float *__restrict__ lut, int i, int j, int k, int ax) {
     const size_t base = ((size_t)i * g.G + j) * g.Gp + k;
     const size_t step = ax == 0 ? (size_t)g.G * g.Gp : (ax == 1 ? (size_t)g.Gp : (size_t)1);
-    const float fa = lut[__ldg(codes + base)], fb = lut[__ldg(codes + base + step)];
+    const float fa = __ldg(lut + __ldg(codes + base)), fb = __ldg(lut + __ldg(codes + base + step));
     const float t = __fdiv_rn(-fa, __fsub_rn(fb, fa));  // vertexInterp (MarchingCubes.cu:731-734)
     float p[3] = {vox(i, g.dx, g.ox), vox(j, g.dx, g.oy), vox(k, g.dx, g.oz)};
-    const float o[3] = {g.ox, g.oy, g.oz};
-    const int idx[3] = {i, j, k};
+    const float from = ax == 0 ? p[0] : (ax == 1 ? p[1] : p[2]);
+    const float to = vox((ax == 0 ? i : (ax == 1 ? j : k)) + 1, g.dx, ax == 0 ? g.ox : (ax == 1 ? g.oy : g.oz));
+    const float at = __fmaf_rn(t, __fsub_rn(to, from), from);
 #pragma unroll
     for (int c = 0; c < 3; c++)
-        if (c == ax) p[c] = __fmaf_rn(t, __fsub_rn(vox(idx[c] + 1, g.dx, o[c]), p[c]), p[c]);
+        if (c == ax) p[c] = at;
     if (g.off[0] | g.off[1] | g.off[2]) {  // a slice box: + offset * dx (MarchingCubes.cu:841-848)
 #pragma unroll
         for (int c = 0; c < 3; c++) p[c] = __fadd_rn(p[c], __fmul_rn((float)g.off[c], g.dx));
     }
-    // groupVertices: round(v / 0.001) (MarchingCubes.cu:859)
-    long long mx = (long long)roundf(__fdiv_rn(p[0], QSES_WELD_TOL));
-    long long my = (long long)roundf(__fdiv_rn(p[1], QSES_WELD_TOL));
-    long long mz = (long long)roundf(__fdiv_rn(p[2], QSES_WELD_TOL));
-    return ((unsigned long long)(mx - g.bx) << 42) | ((unsigned long long)(my - g.by) << 21) | (unsigned long long)(mz - g.bz);
-}
-
-__device__ __forceinline__ unsigned sel4(int o, unsigned a, unsigned b, unsigned c, unsigned d) {
-    return o == 0 ? a : (o == 1 ? b : (o == 2 ? c : d));
+    const unsigned x = (unsigned)(quantum(p[0]) - (int)g.bx), y = (unsigned)(quantum(p[1]) - (int)g.by),
+                   z = (unsigned)(quantum(p[2]) - (int)g.bz);
+    return ((unsigned long long)x << 42) | ((unsigned long long)y << 21) | z;
 }
 
 // Lanes per owner row: the row's words (voxels 0..Gc) rounded up to a power of two, at
@@ -80,12 +78,7 @@ __host__ __device__ __forceinline__ int mc_lanes(int Gc) {
     return L;
 }
 
-// Sum / inclusive scan over aligned groups of Lg lanes (Lg a power of two, warp-uniform).
-__device__ __forceinline__ unsigned grp_sum(unsigned v, int Lg) {
-    if (Lg == 32) return __reduce_add_sync(0xffffffffu, v);
-    for (int o = Lg >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, Lg);
-    return v;
-}
+// Inclusive scan over aligned groups of Lg lanes (Lg a power of two, warp-uniform).
 __device__ __forceinline__ unsigned grp_incl_scan(unsigned v, int sub, int Lg) {
     for (int o = 1; o < Lg; o <<= 1) {
         const unsigned a = __shfl_up_sync(0xffffffffu, v, o, Lg);
@@ -105,17 +98,29 @@ __device__ __forceinline__ unsigned bits_in(int a, int b) {
     return below_b & ~((1u << a) - 1u);
 }
 
-// Words per lane record of the triangle pass (34 used; an odd stride spreads the lanes'
-// writes over the shared-memory banks).
-constexpr int kRecW = 35;
+// Which edges and cells of row (i, j) and word w are in the emitted range [clo, chi) per axis (the
+// whole grid: [0, Gc)).  A row's +x edges are used when a cell of the range has them (x in
+// [clo, chi), y in [clo, chi]), likewise +y; its +z edges when x and y are in [clo, chi].
+struct McRange {
+    int lox, hix, loy, hiy, loz, hiz;
+    __device__ __forceinline__ explicit McRange(const QGrid &g)
+        : lox(g.clo[0]), hix(g.chi[0]), loy(g.clo[1]), hiy(g.chi[1]), loz(g.clo[2]), hiz(g.chi[2]) {}
+    __device__ __forceinline__ bool xr(int a, int b) const { return a >= lox && a < hix && b >= loy && b <= hiy; }
+    __device__ __forceinline__ bool yr(int a, int b) const { return a >= lox && a <= hix && b >= loy && b < hiy; }
+    __device__ __forceinline__ bool zr(int a, int b) const { return a >= lox && a <= hix && b >= loy && b <= hiy; }
+    __device__ __forceinline__ bool cells(int a, int b) const { return a >= lox && a < hix && b >= loy && b < hiy; }
+    __device__ __forceinline__ unsigned kv(int kb) const { return bits_in(loz - kb, hiz - kb + 1); }  // voxels in [loz, hiz]
+    __device__ __forceinline__ unsigned kc(int kb) const { return bits_in(loz - kb, hiz - kb); }  // cells, z edges in [loz, hiz)
+};
 
-template <bool EMIT, bool FULL>
-__device__ __forceinline__ void mc_row(const QGrid &g, long long row, bool valid, int Lg,
-                                       const unsigned *__restrict__ sign, const unsigned char *__restrict__ codes,
-                                       const float *lut, const unsigned long long *s_tab,
-                                       uint2 *__restrict__ rowCount, const uint2 *__restrict__ rowBase,
-                                       unsigned *__restrict__ tri, unsigned long long *__restrict__ vkey,
-                                       unsigned *s_rec) {
+// One owner row (i, j) of a molecule's grid per group of Lg lanes; every lane of the warp
+// calls this (groups whose row is past the end pass valid = false and write nothing).
+// words[row * Wc + w]: what the row's words before w have, edges in bits 0-15 (3 a voxel at most)
+// and triangles in bits 16-30 (5 a cell), and bit 31 if word w has any itself.
+template <bool FULL>
+__device__ __forceinline__ void mc_count_row(const QGrid &g, long long row, bool valid, int Lg,
+                                             const unsigned *__restrict__ sign, const unsigned long long *s_tab,
+                                             uint2 *__restrict__ rowCount, unsigned *__restrict__ words) {
     // FULL: one row per warp (Lg = 32, every group valid), known at compile time.
     if (FULL) {
         Lg = 32;
@@ -125,253 +130,283 @@ __device__ __forceinline__ void mc_row(const QGrid &g, long long row, bool valid
     const int Gc = g.Gc, E = Gc + 1;
     if (!valid) row = 0;
     const int i = (int)(row / E), j = (int)(row % E);
-    // Emitted cells: [clo, chi) per axis (the whole grid: [0, Gc)).  A row's +x edges are
-    // used when a cell of the range has them (x in [clo, chi), y in [clo, chi]), likewise +y;
-    // its +z edges when x and y are in [clo, chi].
-    const int lox = g.clo[0], hix = g.chi[0], loy = g.clo[1], hiy = g.chi[1], loz = g.clo[2], hiz = g.chi[2];
-    auto xr = [&](int a, int b) { return a >= lox && a < hix && b >= loy && b <= hiy; };
-    auto yr = [&](int a, int b) { return a >= lox && a <= hix && b >= loy && b < hiy; };
-    auto zr = [&](int a, int b) { return a >= lox && a <= hix && b >= loy && b <= hiy; };
-    const bool cellsRow = valid && i >= lox && i < hix && j >= loy && j < hiy;
+    const McRange in(g);
     const int Wc = (Gc + 32) / 32;  // words holding voxels 0..Gc
-
-    unsigned triBase = 0, eb0 = 0, eb1 = 0, eb2 = 0, eb3 = 0;  // owners (0,0) (0,1) (1,0) (1,1)
-    if (EMIT && valid) {
-        triBase = rowBase[row].x;
-        eb0 = rowBase[row].y;
-        if (j + 1 <= Gc) eb1 = rowBase[(size_t)i * E + j + 1].y;
-        if (i + 1 <= Gc) eb2 = rowBase[(size_t)(i + 1) * E + j].y;
-        if (i + 1 <= Gc && j + 1 <= Gc) eb3 = rowBase[(size_t)(i + 1) * E + j + 1].y;
-    }
-    unsigned triCarry = 0, ec0 = 0, ec1 = 0, ec2 = 0, ec3 = 0;
+    unsigned carry = 0;
     for (int w0 = 0; w0 < Wc; w0 += Lg) {
         const int w = w0 + sub;
         const bool act = valid && w < Wc;
         const int kb = w * 32;
-        unsigned kv = 0u, kc = 0u;
-        if (act) {
-            kv = bits_in(loz - kb, hiz - kb + 1);  // voxels in [loz, hiz]
-            kc = bits_in(loz - kb, hiz - kb);      // cells / z-edges in [loz, hiz)
-        }
-        const bool nxt = act && (kb + 32 <= hiz) && (kb + 32 >= loz);
+        const unsigned kv = act ? in.kv(kb) : 0u, kc = act ? in.kc(kb) : 0u;
         auto L = [&](int a, int b, int ww) { return act ? ld_sign(sign, g, i + a, j + b, ww) : 0u; };
         const unsigned S00 = L(0, 0, w), S10 = L(1, 0, w), S01 = L(0, 1, w), S11 = L(1, 1, w);
         const unsigned N00 = L(0, 0, w + 1), N10 = L(1, 0, w + 1), N01 = L(0, 1, w + 1), N11 = L(1, 1, w + 1);
         const unsigned P00 = (S00 >> 1) | (N00 << 31), P10 = (S10 >> 1) | (N10 << 31);
         const unsigned P01 = (S01 >> 1) | (N01 << 31), P11 = (S11 >> 1) | (N11 << 31);
-        const unsigned X00 = xr(i, j) ? (S00 ^ S10) & kv : 0u;
-        const unsigned Y00 = yr(i, j) ? (S00 ^ S01) & kv : 0u;
-        const unsigned Z00 = zr(i, j) ? (S00 ^ P00) & kc : 0u;
-        const unsigned c00 = __popc(X00) + __popc(Y00) + __popc(Z00);
-        unsigned cellm = 0u, ntri = 0u, nt0 = 0u, nt1 = 0u, nt2 = 0u;  // nt bit k of each active cell
-        if (cellsRow) {
-            cellm = ((S00 ^ S10) | (S00 ^ S11) | (S00 ^ S01) | (S00 ^ P00) | (S00 ^ P10) | (S00 ^ P11) |
-                     (S00 ^ P01)) & kc;
+        const unsigned X00 = in.xr(i, j) ? (S00 ^ S10) & kv : 0u;
+        const unsigned Y00 = in.yr(i, j) ? (S00 ^ S01) & kv : 0u;
+        const unsigned Z00 = in.zr(i, j) ? (S00 ^ P00) & kc : 0u;
+        unsigned n = __popc(X00) + __popc(Y00) + __popc(Z00);
+        if (in.cells(i, j)) {
+            const unsigned cellm = ((S00 ^ S10) | (S00 ^ S11) | (S00 ^ S01) | (S00 ^ P00) | (S00 ^ P10) | (S00 ^ P11) |
+                                    (S00 ^ P01)) & kc;
             for (unsigned m = cellm; m; m &= m - 1u) {
-                unsigned b = __ffs(m) - 1;
-                const unsigned nt = (unsigned)(s_tab[cube_index(b, S00, S10, S11, S01, P00, P10, P11, P01)] >> 60);
-                ntri += nt;
-                if (EMIT) {
-                    nt0 |= (nt & 1u) << b;
-                    nt1 |= ((nt >> 1) & 1u) << b;
-                    nt2 |= ((nt >> 2) & 1u) << b;
-                }
+                const unsigned b = __ffs(m) - 1;
+                n += (unsigned)(s_tab[cube_index(b, S00, S10, S11, S01, P00, P10, P11, P01)] >> 60) << 16;
             }
         }
-        if (!EMIT) {
-            triCarry += grp_sum(ntri, Lg);
-            ec0 += grp_sum(c00, Lg);
-            continue;
-        }
-        // Edges owned by the three neighbouring rows, for triangle corners.
-        const unsigned S20 = L(2, 0, w), S21 = L(2, 1, w), S02 = L(0, 2, w), S12 = L(1, 2, w);
-        const unsigned N20 = L(2, 0, w + 1), N21 = L(2, 1, w + 1), N02 = L(0, 2, w + 1), N12 = L(1, 2, w + 1);
-        const unsigned X01 = xr(i, j + 1) ? (S01 ^ S11) & kv : 0u;
-        const unsigned Y01 = yr(i, j + 1) ? (S01 ^ S02) & kv : 0u;
-        const unsigned Z01 = zr(i, j + 1) ? (S01 ^ P01) & kc : 0u;
-        const unsigned X10 = xr(i + 1, j) ? (S10 ^ S20) & kv : 0u;
-        const unsigned Y10 = yr(i + 1, j) ? (S10 ^ S11) & kv : 0u;
-        const unsigned Z10 = zr(i + 1, j) ? (S10 ^ P10) & kc : 0u;
-        const unsigned X11 = xr(i + 1, j + 1) ? (S11 ^ S21) & kv : 0u;
-        const unsigned Y11 = yr(i + 1, j + 1) ? (S11 ^ S12) & kv : 0u;
-        const unsigned Z11 = zr(i + 1, j + 1) ? (S11 ^ P11) & kc : 0u;
-        const unsigned c01 = __popc(X01) + __popc(Y01) + __popc(Z01);
-        const unsigned c10 = __popc(X10) + __popc(Y10) + __popc(Z10);
-        const unsigned c11 = __popc(X11) + __popc(Y11) + __popc(Z11);
-        // Activity of the x/y edges of voxel kb+32 (bit 0 of the next word).
-        const unsigned xn0 = (nxt && xr(i, j)) ? ((N00 ^ N10) & 1u) : 0u, yn0 = (nxt && yr(i, j)) ? ((N00 ^ N01) & 1u) : 0u;
-        const unsigned xn1 = (nxt && xr(i, j + 1)) ? ((N01 ^ N11) & 1u) : 0u, yn1 = (nxt && yr(i, j + 1)) ? ((N01 ^ N02) & 1u) : 0u;
-        const unsigned xn2 = (nxt && xr(i + 1, j)) ? ((N10 ^ N20) & 1u) : 0u, yn2 = (nxt && yr(i + 1, j)) ? ((N10 ^ N11) & 1u) : 0u;
-        const unsigned xn3 = (nxt && xr(i + 1, j + 1)) ? ((N11 ^ N21) & 1u) : 0u, yn3 = (nxt && yr(i + 1, j + 1)) ? ((N11 ^ N12) & 1u) : 0u;
-
-        const unsigned p0 = grp_incl_scan(c00, sub, Lg) - c00, p1 = grp_incl_scan(c01, sub, Lg) - c01;
-        const unsigned p2 = grp_incl_scan(c10, sub, Lg) - c10, p3 = grp_incl_scan(c11, sub, Lg) - c11;
-        const unsigned tp = grp_incl_scan(ntri, sub, Lg) - ntri;
-
-        // Vertices owned by this row, in voxel order, x then y then z within a voxel: edge e of
-        // the group's words goes to slot eb0 + ec0 + e.  The few words a surface crosses hold
-        // all of a row's edges, so the edges are dealt out over the group's lanes: lane `sub`
-        // takes e = sub, sub + Lg, ..., finds the owning lane (largest L with p0[L] <= e) and
-        // the voxel and axis of the edge inside that lane's word.
-        {
-            const unsigned etot = grp_sum(c00, Lg);
-            const unsigned emax = FULL ? etot : __reduce_max_sync(0xffffffffu, etot);  // warp-uniform
-            const int gbase = (int)(threadIdx.x & 31) & ~(Lg - 1);
-            for (unsigned eb = 0; eb < emax; eb += (unsigned)Lg) {
-                const unsigned e = eb + (unsigned)sub;
-                int lo = 0;
-                for (int step = Lg >> 1; step > 0; step >>= 1) {
-                    const unsigned pl = __shfl_sync(0xffffffffu, p0, gbase + lo + step);
-                    if (pl <= e) lo += step;
-                }
-                const unsigned Xo = __shfl_sync(0xffffffffu, X00, gbase + lo);
-                const unsigned Yo = __shfl_sync(0xffffffffu, Y00, gbase + lo);
-                const unsigned Zo = __shfl_sync(0xffffffffu, Z00, gbase + lo);
-                const unsigned po = __shfl_sync(0xffffffffu, p0, gbase + lo);
-                if (e < etot) {
-                    const unsigned r = e - po;  // rank of the edge inside the owner's word
-                    int b = 0;                  // its voxel: the largest b with fewer than r+1 edges below
-                    for (int step = 16; step > 0; step >>= 1) {
-                        const unsigned lt = (1u << (b + step)) - 1u;
-                        if ((unsigned)(__popc(Xo & lt) + __popc(Yo & lt) + __popc(Zo & lt)) <= r) b += step;
-                    }
-                    const unsigned lt = (1u << b) - 1u;
-                    unsigned qa = r - (unsigned)(__popc(Xo & lt) + __popc(Yo & lt) + __popc(Zo & lt));
-                    int ax = 2;
-                    if ((Xo >> b) & 1u) {
-                        if (qa == 0) ax = 0;
-                        else qa--;
-                    }
-                    if (ax == 2 && ((Yo >> b) & 1u) && qa == 0) ax = 1;
-                    const int k = (w0 + lo) * 32 + b;
-                    vkey[eb0 + ec0 + e] = edge_key(g, codes, lut, i, j, k, ax);
-                }
-            }
-        }
-        // Triangles in cell order, corners as pre-weld vertex slots.  The few words a surface
-        // crosses hold all of a row's cells, so the row's active cells are dealt out over the
-        // group's lanes: every lane publishes its word's sign words, edge masks, slot bases and
-        // per-cell triangle counts, and lane `sub` takes the row's active cells sub, sub + Lg,
-        // ...; a cell's first triangle is its word's first plus the counts of the cells below.
-        {
-            unsigned *my = s_rec + (threadIdx.x & 31) * kRecW;
-            my[0] = S00; my[1] = S10; my[2] = S11; my[3] = S01;
-            my[4] = P00; my[5] = P10; my[6] = P11; my[7] = P01;
-            my[8] = X00; my[9] = Y00; my[10] = Z00; my[11] = X01; my[12] = Y01; my[13] = Z01;
-            my[14] = X10; my[15] = Y10; my[16] = Z10; my[17] = X11; my[18] = Y11; my[19] = Z11;
-            my[20] = eb0 + ec0 + p0; my[21] = eb1 + ec1 + p1; my[22] = eb2 + ec2 + p2; my[23] = eb3 + ec3 + p3;
-            my[24] = c00; my[25] = c01; my[26] = c10; my[27] = c11;
-            my[28] = xn0 | (yn0 << 1) | (xn1 << 2) | (yn1 << 3) | (xn2 << 4) | (yn2 << 5) | (xn3 << 6) | (yn3 << 7);
-            my[29] = nt0; my[30] = nt1; my[31] = nt2; my[32] = cellm; my[33] = triBase + triCarry + tp;
-            __syncwarp();
-            const unsigned nc = __popc(cellm);
-            const unsigned cp = grp_incl_scan(nc, sub, Lg) - nc;
-            const unsigned ctot = grp_sum(nc, Lg);
-            const unsigned cmax = FULL ? ctot : __reduce_max_sync(0xffffffffu, ctot);  // warp-uniform
-            const int gbase = (int)(threadIdx.x & 31) & ~(Lg - 1);
-            for (unsigned cb = 0; cb < cmax; cb += (unsigned)Lg) {
-                const unsigned ci = cb + (unsigned)sub;
-                int lo = 0;
-                for (int step = Lg >> 1; step > 0; step >>= 1) {
-                    const unsigned pl = __shfl_sync(0xffffffffu, cp, gbase + lo + step);
-                    if (pl <= ci) lo += step;
-                }
-                const unsigned po = __shfl_sync(0xffffffffu, cp, gbase + lo);
-                if (ci < ctot) {
-                    const unsigned *R = s_rec + (gbase + lo) * kRecW;
-                    const unsigned cm = R[32], r = ci - po;
-                    int b = 0;  // the r-th active cell of the owner's word: the largest b with r cells below
-                    for (int step = 16; step > 0; step >>= 1)
-                        if ((unsigned)__popc(cm & ((1u << (b + step)) - 1u)) <= r) b += step;
-                    const unsigned lt = (1u << b) - 1u;
-                    const unsigned ts = R[33] + __popc(R[29] & lt) + 2u * __popc(R[30] & lt) + 4u * __popc(R[31] & lt);
-                    const unsigned long long e = s_tab[cube_index(b, R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7])];
-                    const unsigned nt = (unsigned)(e >> 60);
-                    for (unsigned q = 0; q < 3 * nt; q++) {
-                        const unsigned edge = (unsigned)(e >> (4 * q)) & 15u;
-                        const unsigned own = (unsigned)(kEdgeOwner >> (5 * edge)) & 31u;
-                        const int o = (int)((own & 1u) * 2 + ((own >> 1) & 1u));  // (di, dj) -> owner index
-                        const unsigned dk = (own >> 2) & 1u, ax = own >> 3;
-                        const unsigned Xo = R[8 + 3 * o], Yo = R[9 + 3 * o], Zo = R[10 + 3 * o];
-                        unsigned slot = R[20 + o];
-                        const unsigned vb = (unsigned)b + dk;
-                        if (vb < 32) {
-                            const unsigned lt2 = (1u << vb) - 1u;
-                            slot += __popc(Xo & lt2) + __popc(Yo & lt2) + __popc(Zo & lt2);
-                            if (ax >= 1) slot += (Xo >> vb) & 1u;
-                            if (ax >= 2) slot += (Yo >> vb) & 1u;
-                        } else {
-                            slot += R[24 + o];
-                            if (ax >= 1) slot += (R[28] >> (2 * o)) & 1u;
-                            if (ax >= 2) slot += (R[28] >> (2 * o + 1)) & 1u;
-                        }
-                        tri[3ull * ts + q] = slot;
-                    }
-                }
-            }
-            __syncwarp();  // the records are read before the next words' are written
-        }
-        triCarry += grp_sum(ntri, Lg);
-        ec0 += grp_sum(c00, Lg);
-        ec1 += grp_sum(c01, Lg);
-        ec2 += grp_sum(c10, Lg);
-        ec3 += grp_sum(c11, Lg);
+        const unsigned incl = grp_incl_scan(n, sub, Lg);
+        if (act) words[(size_t)row * Wc + w] = (carry + incl - n) | (n ? 0x80000000u : 0u);
+        carry += __shfl_sync(0xffffffffu, incl, Lg - 1, Lg);
     }
-    if (!EMIT && valid && sub == 0) rowCount[row] = make_uint2(triCarry, ec0);
+    if (valid && sub == 0) rowCount[row] = make_uint2(carry >> 16, carry & 0xffffu);
 }
 
-// Resident CTAs per SM: the emit is latency-bound, so four CTAs (64 registers, a few spilled)
-// beat three: whole-warp rows 0.89 -> 0.82 ms on a 664^3 grid, 4-lane rows 0.780 -> 0.750 ms.
-template <bool EMIT, bool FULL>
-__global__ void __launch_bounds__(256, 4) k_mc(QGrid g, const unsigned *__restrict__ sign,
-                                            const unsigned char *__restrict__ codes, const float *__restrict__ lut,
-                                            uint2 *__restrict__ rowCount, const uint2 *__restrict__ rowBase,
-                                            unsigned *__restrict__ tri, unsigned long long *__restrict__ vkey,
-                                            int lanes) {
+template <bool FULL>
+__global__ void __launch_bounds__(256, 4) k_mc_count(QGrid g, const unsigned *__restrict__ sign,
+                                                     uint2 *__restrict__ rowCount, unsigned *__restrict__ words, int lanes) {
     __shared__ unsigned long long s_tab[256];
-    __shared__ float s_lut[256];
-    __shared__ unsigned s_rec[EMIT ? 8 * 32 * kRecW : 1];  // per warp: one record per lane
     s_tab[threadIdx.x] = c_mc[threadIdx.x];
-    if (EMIT) s_lut[threadIdx.x] = lut[threadIdx.x];
     __syncthreads();
     const int E = g.Gc + 1, Lg = FULL ? 32 : lanes;
     const long long first = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 / Lg), nrow = (long long)E * E;
     if (first >= nrow) return;  // the whole warp
     const long long row = first + (threadIdx.x & 31) / Lg;
-    mc_row<EMIT, FULL>(g, row, row < nrow, Lg, sign, codes, s_lut, s_tab, rowCount, rowBase, tri, vkey,
-                       s_rec + (EMIT ? (threadIdx.x >> 5) * 32 * kRecW : 0));
+    mc_count_row<FULL>(g, row, row < nrow, Lg, sign, s_tab, rowCount, words);
 }
 
 // Batch form: rows are numbered molecule after molecule, so one scan over all rows gives
 // every molecule's triangles and edge slots contiguous ranges in molecule order.  Each warp
 // takes one unit of 32 / Lg rows of one molecule (units numbered by mc_unit_off).
-// Four resident CTAs per SM (7.17 -> 5.68 ms for the emit of 256 molecules against two).
-template <bool EMIT>
-__global__ void __launch_bounds__(256, 4) k_mc_batch(QBatch b, const unsigned *__restrict__ sign,
-                                                  const unsigned char *__restrict__ codes, uint2 *__restrict__ rowCount,
-                                                  const uint2 *__restrict__ rowBase, unsigned *__restrict__ tri,
-                                                  unsigned long long *__restrict__ vkey) {
+__global__ void __launch_bounds__(256, 4) k_mc_count_batch(QBatch b, const unsigned *__restrict__ sign,
+                                                           uint2 *__restrict__ rowCount, unsigned *__restrict__ words) {
     __shared__ unsigned long long s_tab[256];
-    __shared__ unsigned s_rec[EMIT ? 8 * 32 * kRecW : 1];  // per warp: one record per lane
     s_tab[threadIdx.x] = c_mc[threadIdx.x];
     __syncthreads();
-    unsigned *rec = s_rec + (EMIT ? (threadIdx.x >> 5) * 32 * kRecW : 0);
     const unsigned unit = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (unit >= __ldg(b.mc_unit_off + b.n_mol)) return;  // the whole warp
     const unsigned m = qses_find(b.mc_unit_off, b.n_mol, unit);
     const QMol &mol = b.mols[m];
     const QGrid g = mol.g;
-    // the batch keeps the words-per-row width (narrow groups, as the single-molecule
-    // launches use, measured slower here: emit 5.68 -> 6.12 ms on a 256-molecule batch)
     const int Lg = mc_lanes(g.Gc);
     const unsigned r0 = mol.row_off, nrow = (unsigned)(g.Gc + 1) * (unsigned)(g.Gc + 1);
     const unsigned row = (unit - __ldg(b.mc_unit_off + m)) * (32u / Lg) + (threadIdx.x & 31) / Lg;
     if (Lg == 32)  // warp-uniform
-        mc_row<EMIT, true>(g, (long long)row, true, 32, sign + mol.mask_off, codes + mol.code_off,
-                           b.lut + 256ull * m, s_tab, rowCount + r0, rowBase + r0, tri, vkey, rec);
+        mc_count_row<true>(g, (long long)row, true, 32, sign + mol.mask_off, s_tab, rowCount + r0, words + mol.mask_off);
     else
-        mc_row<EMIT, false>(g, (long long)row, row < nrow, Lg, sign + mol.mask_off, codes + mol.code_off,
-                            b.lut + 256ull * m, s_tab, rowCount + r0, rowBase + r0, tri, vkey, rec);
+        mc_count_row<false>(g, (long long)row, row < nrow, Lg, sign + mol.mask_off, s_tab, rowCount + r0,
+                            words + mol.mask_off);
+}
+
+// The emission.  A warp takes `chunk` consecutive words of the grid, collects the ones that have
+// edges or triangles and works on 32 of them at a time: a lane per word for its masks and slots,
+// then a lane per edge and a lane per cell of all of them together, whichever rows they are in.
+// What consecutive words emit is contiguous, so keys and corners go out in whole lines, the corners
+// by way of shared memory.
+//
+// Bound by instruction issue: 664^3 (3 700 000 edges, 7 400 000 triangles) takes 126 M warp
+// instructions at 1.9 a cycle, 16 warps an SM.  Rows dealt to 4 or 32 lanes, each corner's slot from
+// the words' masks and stored by itself: 0.74 ms there (568 M instructions), 0.24 so; 1738^3
+// (138 000 000 edges) 13.0 and 4.6; 85^3 0.025 and 0.020.  Blocks of 8 warps wait for their slowest
+// (0.26, 4.9); of 1 or 2 they load the table more often than that gains.
+constexpr int kEmitRec = 9;    // uint4 a lane's record takes (8 used; odd, for the banks)
+constexpr int kEmitQueue = 160;  // words waiting: 31 and 4 x 32 more
+constexpr int kEmitWarps = 4;
+struct EmitSmem {
+    uint4 rec[32 * kEmitRec];
+    unsigned slot[12 * 32];  // a cell's 12 edges, per lane
+    unsigned out[32 * 15];   // corners of up to 32 cells
+    unsigned short queue[kEmitQueue];
+};
+
+// The edge or cell of rank r: the largest b with at most r below it.
+template <typename F> __device__ __forceinline__ unsigned bit_of_rank(F below, unsigned r) {
+    unsigned b = 0;
+#pragma unroll
+    for (unsigned step = 16; step > 0; step >>= 1)
+        if (below((1u << (b + step)) - 1u) <= r) b += step;
+    return b;
+}
+// The lane whose items include item e: the largest with first <= e.
+__device__ __forceinline__ unsigned lane_of_item(unsigned first, unsigned e) {
+    unsigned lo = 0;
+#pragma unroll
+    for (unsigned step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, first, lo + step) <= e) lo += step;
+    return lo;
+}
+
+// Up to 32 words (has: this lane's is one), in ascending order by lane: `at` words from row row0's start.
+__device__ __forceinline__ void emit_words(const QGrid &g, const unsigned *__restrict__ sign,
+                                           const unsigned char *__restrict__ codes, const float *__restrict__ lut,
+                                           const unsigned *__restrict__ words, const uint2 *__restrict__ rowBase,
+                                           unsigned *__restrict__ tri, unsigned long long *__restrict__ vkey,
+                                           const unsigned long long *s_tab, EmitSmem &sm, bool has, unsigned row0, unsigned at) {
+    const unsigned lane = threadIdx.x & 31;
+    const int E = g.Gc + 1, Wc = (g.Gc + 32) / 32;
+    unsigned nedge = 0, ncell = 0;
+    if (has) {
+        const unsigned row = row0 + at / (unsigned)Wc;
+        const int w = (int)(at % (unsigned)Wc), i = (int)(row / (unsigned)E), j = (int)(row % (unsigned)E);
+        const McRange in(g);
+        const unsigned kv = in.kv(32 * w), kc = in.kc(32 * w);
+        auto L = [&](int a, int b, int ww) { return ld_sign(sign, g, i + a, j + b, ww); };
+        const unsigned S00 = L(0, 0, w), S10 = L(1, 0, w), S01 = L(0, 1, w), S11 = L(1, 1, w);
+        const unsigned N00 = L(0, 0, w + 1), N10 = L(1, 0, w + 1), N01 = L(0, 1, w + 1), N11 = L(1, 1, w + 1);
+        const unsigned S20 = L(2, 0, w), S21 = L(2, 1, w), S02 = L(0, 2, w), S12 = L(1, 2, w), N20 = L(2, 0, w + 1);
+        const unsigned P00 = (S00 >> 1) | (N00 << 31), P10 = (S10 >> 1) | (N10 << 31);
+        const unsigned P01 = (S01 >> 1) | (N01 << 31), P11 = (S11 >> 1) | (N11 << 31);
+        // edges owned by the row and by the rows (i, j + 1), (i + 1, j) and (i + 1, j + 1)
+        const unsigned X00 = in.xr(i, j) ? (S00 ^ S10) & kv : 0u, Y00 = in.yr(i, j) ? (S00 ^ S01) & kv : 0u;
+        const unsigned Z00 = in.zr(i, j) ? (S00 ^ P00) & kc : 0u;
+        const unsigned X01 = in.xr(i, j + 1) ? (S01 ^ S11) & kv : 0u, Y01 = in.yr(i, j + 1) ? (S01 ^ S02) & kv : 0u;
+        const unsigned Z01 = in.zr(i, j + 1) ? (S01 ^ P01) & kc : 0u;
+        const unsigned X10 = in.xr(i + 1, j) ? (S10 ^ S20) & kv : 0u, Y10 = in.yr(i + 1, j) ? (S10 ^ S11) & kv : 0u;
+        const unsigned Z10 = in.zr(i + 1, j) ? (S10 ^ P10) & kc : 0u;
+        const unsigned X11 = in.xr(i + 1, j + 1) ? (S11 ^ S21) & kv : 0u, Y11 = in.yr(i + 1, j + 1) ? (S11 ^ S12) & kv : 0u;
+        const unsigned Z11 = in.zr(i + 1, j + 1) ? (S11 ^ P11) & kc : 0u;
+        // the +x edge of voxel 32 w + 32 of row (i + 1, j)
+        const unsigned xn = in.xr(i + 1, j) && 32 * w + 32 <= in.hiz && 32 * w + 32 >= in.loz ? (N10 ^ N20) & 1u : 0u;
+        const bool nj = j + 1 < E, ni = i + 1 < E;
+        auto first = [&](unsigned r) { return __ldg(&rowBase[r].y) + (__ldg(words + (size_t)r * Wc + w) & 0xffffu); };
+        const uint2 own = __ldg(rowBase + row);
+        const unsigned pre = __ldg(words + (size_t)row * Wc + w);
+        const unsigned e0 = own.y + (pre & 0xffffu), e1 = nj ? first(row + 1) : 0u, e2 = ni ? first(row + E) : 0u,
+                       e3 = ni && nj ? first(row + E + 1) : 0u;
+        const unsigned cellm = !in.cells(i, j) ? 0u
+                               : ((S00 ^ S10) | (S00 ^ S11) | (S00 ^ S01) | (S00 ^ P00) | (S00 ^ P10) | (S00 ^ P11) | (S00 ^ P01)) & kc;
+        uint4 *my = sm.rec + lane * kEmitRec;
+        my[0] = make_uint4(S00, S10, S11, S01);
+        my[1] = make_uint4(P00, P10, P11, P01);
+        my[2] = make_uint4(X00, Y00, Z00, e0);
+        my[3] = make_uint4(X01, Y01, Z01, e1);
+        my[4] = make_uint4(X10, Y10, Z10, e2);
+        my[5] = make_uint4(X11, Y11, Z11, e3);
+        my[6] = make_uint4(cellm, xn | ((unsigned)w << 1), (unsigned)i, (unsigned)j);
+        if (lane == 0) my[7].x = own.x + ((pre >> 16) & 0x7fffu);
+        nedge = __popc(X00) + __popc(Y00) + __popc(Z00);
+        ncell = __popc(cellm);
+    }
+    __syncwarp();
+    // the words' own edges, in voxel order, x then y then z within a voxel
+    {
+        const unsigned incl = warp_incl_scan(nedge), total = __shfl_sync(0xffffffffu, incl, 31), from = incl - nedge;
+        const unsigned base = sm.rec[2].w;
+        for (unsigned e0 = 0; e0 < total; e0 += 32) {
+            const unsigned e = e0 + lane, lo = lane_of_item(from, e);
+            const unsigned r = e - __shfl_sync(0xffffffffu, from, lo);
+            if (e >= total) continue;
+            const uint4 o = sm.rec[lo * kEmitRec + 2], id = sm.rec[lo * kEmitRec + 6];
+            auto below = [&](unsigned lt) { return (unsigned)(__popc(o.x & lt) + __popc(o.y & lt) + __popc(o.z & lt)); };
+            const unsigned b = bit_of_rank(below, r);
+            const unsigned q = r - below((1u << b) - 1u), x = (o.x >> b) & 1u, y = (o.y >> b) & 1u;
+            const int ax = q < x ? 0 : (q < x + y ? 1 : 2);
+            vkey[(size_t)base + e] = edge_key(g, codes, lut, (int)id.z, (int)id.w, (int)(32 * (id.y >> 1) + b), ax);
+        }
+    }
+    // the words' cells in order, corners as edge slots
+    {
+        const unsigned incl = warp_incl_scan(ncell), total = __shfl_sync(0xffffffffu, incl, 31), from = incl - ncell;
+        unsigned *out = tri + 3ull * sm.rec[7].x;
+        for (unsigned c0 = 0; c0 < total; c0 += 32) {
+            const unsigned c = c0 + lane, lo = lane_of_item(from, c);
+            const unsigned r = c - __shfl_sync(0xffffffffu, from, lo);
+            unsigned long long corners = 0;
+            if (c < total) {
+                const uint4 *R = sm.rec + lo * kEmitRec;
+                const uint4 s = R[0], p = R[1], id = R[6];
+                const unsigned b = bit_of_rank([&](unsigned lt) { return (unsigned)__popc(id.x & lt); }, r), lt = (1u << b) - 1u;
+                corners = s_tab[cube_index(b, s.x, s.y, s.z, s.w, p.x, p.y, p.z, p.w)];
+                // the rows' edges before voxel b; the next voxel's follow behind this one's
+                auto before = [&](const uint4 &o) { return o.w + __popc(o.x & lt) + __popc(o.y & lt) + __popc(o.z & lt); };
+                auto bit = [&](unsigned v) { return (v >> b) & 1u; };
+                const uint4 o0 = R[2], o1 = R[3], o2 = R[4], o3 = R[5];
+                const unsigned a0 = before(o0), a1 = before(o1), a2 = before(o2), a3 = before(o3);
+                const unsigned z0 = a0 + bit(o0.x) + bit(o0.y), z1 = a1 + bit(o1.x) + bit(o1.y),
+                               z2 = a2 + bit(o2.x) + bit(o2.y), z3 = a3 + bit(o3.x) + bit(o3.y);
+                const unsigned n0 = z0 + bit(o0.z), n1 = z1 + bit(o1.z), n2 = z2 + bit(o2.z);
+                unsigned *S = sm.slot + lane;  // by the table's edge number (MarchingCubes.cu:814-825)
+                S[0] = a0;
+                S[32] = a2 + bit(o2.x);
+                S[64] = a1;
+                S[96] = a0 + bit(o0.x);
+                S[128] = n0;
+                S[160] = n2 + (b < 31 ? (o2.x >> (b + 1)) & 1u : id.y & 1u);
+                S[192] = n1;
+                S[224] = n0 + bit(p.x ^ p.y);
+                S[256] = z0;
+                S[288] = z2;
+                S[320] = z3;
+                S[352] = z1;
+            }
+            const unsigned nt = (unsigned)(corners >> 60), ti = warp_incl_scan(nt);
+            const unsigned n3 = 3 * __shfl_sync(0xffffffffu, ti, 31);
+            unsigned *o = sm.out + 3 * (ti - nt);
+            for (unsigned t = 0; t < nt; t++, corners >>= 12, o += 3)
+#pragma unroll
+                for (unsigned v = 0; v < 3; v++) o[v] = sm.slot[(((unsigned)corners >> (4 * v)) & 15u) * 32 + lane];
+            __syncwarp();
+            for (unsigned q = lane; q < n3; q += 32) out[q] = sm.out[q];
+            out += n3;
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(32 * kEmitWarps, 6) k_mc_emit(QGrid g1, QBatch b, const unsigned *__restrict__ sign,
+                                                                const unsigned char *__restrict__ codes,
+                                                                const float *__restrict__ lut,
+                                                                const unsigned *__restrict__ words,
+                                                                const uint2 *__restrict__ rowBase,
+                                                                unsigned *__restrict__ tri,
+                                                                unsigned long long *__restrict__ vkey, unsigned chunk,
+                                                                unsigned units) {
+    extern __shared__ uint4 s_emit[];
+    __shared__ unsigned long long s_tab[256];
+    for (unsigned k = threadIdx.x; k < 256; k += 32 * kEmitWarps) s_tab[k] = c_mc[k];
+    __syncthreads();
+    EmitSmem &sm = ((EmitSmem *)s_emit)[threadIdx.x >> 5];
+    const unsigned unit = blockIdx.x * kEmitWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (unit >= units) return;  // the whole warp
+    const unsigned m = BATCH ? qses_find(b.emit_off, b.n_mol, unit) : 0u;
+    const QGrid &g = BATCH ? b.mols[m].g : g1;
+    if (BATCH) {
+        const QMol &mol = b.mols[m];
+        sign += mol.mask_off, codes += mol.code_off, words += mol.mask_off, rowBase += mol.row_off, lut = b.lut + 256ull * m;
+    }
+    const unsigned long long all = (unsigned long long)(g.Gc + 1) * (g.Gc + 1) * ((g.Gc + 32) / 32);
+    const unsigned long long w0 = (unsigned long long)(BATCH ? unit - __ldg(b.emit_off + m) : unit) * chunk;
+    const unsigned n = (unsigned)min((unsigned long long)chunk, all - w0);
+    const unsigned Wc = (unsigned)(g.Gc + 32) / 32, row0 = (unsigned)(w0 / Wc), off = (unsigned)(w0 - (unsigned long long)row0 * Wc);
+    unsigned have = 0;  // words in the queue
+    for (unsigned k = 0; k < n; k += 128) {
+        unsigned v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = k + 32 * q + lane < n ? __ldg(words + w0 + k + 32 * q + lane) : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const unsigned some = __ballot_sync(0xffffffffu, v[q] >> 31);
+            if (v[q] >> 31) sm.queue[have + __popc(some & ((1u << lane) - 1u))] = (unsigned short)(k + 32 * q + lane);
+            have += __popc(some);
+        }
+        __syncwarp();
+        const bool flush = k + 128 >= n;  // the last: whatever is there
+        unsigned at = 0;
+        while (have - at >= 32 || (flush && at < have)) {
+            const bool has = at + lane < have;
+            emit_words(g, sign, codes, lut, words, rowBase, tri, vkey, s_tab, sm, has, row0,
+                       off + (has ? sm.queue[at + lane] : 0));
+            at = min(at + 32, have);
+        }
+        const unsigned left = have - at;  // below 32
+        const unsigned short keep = lane < left ? sm.queue[at + lane] : 0;
+        __syncwarp();
+        if (lane < left) sm.queue[lane] = keep;
+        have = left;
+        __syncwarp();
+    }
 }
 
 // ------------------------------------------------------------------ weld
@@ -399,7 +434,7 @@ constexpr unsigned kWeldX = 4096;       // x ranges of a layer at most: quanta, 
 __device__ __forceinline__ unsigned plane_quantum(const QGrid &g, int i) {
     float p = vox(i, g.dx, g.ox);
     if (g.off[0] | g.off[1] | g.off[2]) p = __fadd_rn(p, __fmul_rn((float)g.off[0], g.dx));
-    return (unsigned)((long long)roundf(__fdiv_rn(p, QSES_WELD_TOL)) - g.bx);
+    return (unsigned)(quantum(p) - (int)g.bx);
 }
 // In place: exclusive sums of x[0, n), by the whole block; the total is returned.
 template <int NT>
@@ -764,41 +799,50 @@ __global__ void k_from_float4(const float4 *__restrict__ v4, unsigned nv, float 
 static inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
 int mc_rows_per_warp(int Gc) { return 32 / mc_lanes(Gc); }
-// Lanes per row of the single-molecule count and emit (the per-row totals do not depend on
-// it, so the two may differ).  Narrow groups put more rows in flight per warp; measured on
-// GB300 (count / emit ms): 664^3 grid 0.248 / 0.821 with whole-warp rows, 0.127 / 0.780
-// with 2 / 4 lanes; 502^3 0.105 / 0.404 -> 0.074 / 0.370; 85^3 emit 0.029 -> 0.023 with 8.
-static int mc_lanes_for(int Gc, bool emit) {
-    const int Wc = (Gc + 32) / 32;
-    if (Wc >= 8) return emit ? 4 : 2;
-    return emit ? 8 : mc_lanes(Gc);
-}
-void launch_mc_count(const QGrid &g, const unsigned *sign, uint2 *rowCount, cudaStream_t s) {
-    size_t rows = (size_t)(g.Gc + 1) * (g.Gc + 1);
-    const int L = mc_lanes_for(g.Gc, false);
+void launch_mc_count(const QGrid &g, const unsigned *sign, uint2 *rowCount, unsigned *words, cudaStream_t s) {
+    const size_t rows = (size_t)(g.Gc + 1) * (g.Gc + 1);
+    // Narrow groups put more rows in flight per warp: 664^3 grid 0.248 ms with whole-warp rows, 0.127
+    // with 2 lanes; 502^3 0.105 and 0.074.
+    const int L = (g.Gc + 32) / 32 >= 8 ? 2 : mc_lanes(g.Gc);
     if (L == 32)
-        k_mc<false, true><<<nblk(rows, 8), 256, 0, s>>>(g, sign, nullptr, nullptr, rowCount, nullptr, nullptr,
-                                                         nullptr, 32);
+        k_mc_count<true><<<nblk(rows, 8), 256, 0, s>>>(g, sign, rowCount, words, 32);
     else
-        k_mc<false, false><<<nblk(rows, 8 * (32 / L)), 256, 0, s>>>(g, sign, nullptr, nullptr,
-                                                                    rowCount, nullptr, nullptr, nullptr, L);
+        k_mc_count<false><<<nblk(rows, 8 * (32 / L)), 256, 0, s>>>(g, sign, rowCount, words, L);
 }
-void launch_mc_emit(const QGrid &g, const unsigned *sign, const unsigned char *codes, const float *lut,
-                    const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s) {
-    size_t rows = (size_t)(g.Gc + 1) * (g.Gc + 1);
-    const int L = mc_lanes_for(g.Gc, true);
-    if (L == 32)
-        k_mc<true, true><<<nblk(rows, 8), 256, 0, s>>>(g, sign, codes, lut, nullptr, rowBase, tri, vkey, 32);
-    else
-        k_mc<true, false><<<nblk(rows, 8 * (32 / L)), 256, 0, s>>>(g, sign, codes, lut, nullptr,
-                                                                   rowBase, tri, vkey, L);
+void launch_mc_count_batch(const QBatch &b, unsigned units, const unsigned *sign, uint2 *rowCount, unsigned *words,
+                           cudaStream_t s) {
+    k_mc_count_batch<<<nblk(units, 8), 256, 0, s>>>(b, sign, rowCount, words);
 }
-void launch_mc_count_batch(const QBatch &b, unsigned units, const unsigned *sign, uint2 *rowCount, cudaStream_t s) {
-    k_mc_batch<false><<<nblk(units, 8), 256, 0, s>>>(b, sign, nullptr, rowCount, nullptr, nullptr, nullptr);
+unsigned long long mc_words(int Gc) { return (unsigned long long)(Gc + 1) * (Gc + 1) * ((Gc + 32) / 32); }
+// Words a warp of the emission takes: enough that it seldom works on fewer than 32 at a time, but
+// no more than leave every SM a few blocks.
+unsigned mc_emit_chunk(unsigned long long words) {
+    const unsigned long long c = (words / 8192 + 31) / 32 * 32;
+    return (unsigned)(c < 32 ? 32 : c > 512 ? 512 : c);
 }
-void launch_mc_emit_batch(const QBatch &b, unsigned units, const unsigned *sign, const unsigned char *codes,
-                          const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s) {
-    k_mc_batch<true><<<nblk(units, 8), 256, 0, s>>>(b, sign, codes, nullptr, rowBase, tri, vkey);
+template <bool BATCH>
+static cudaError_t emit_with(const QGrid &g, const QBatch &b, const unsigned *sign, const unsigned char *codes,
+                             const float *lut, const unsigned *words, const uint2 *rowBase, unsigned *tri,
+                             unsigned long long *vkey, unsigned chunk, unsigned units, cudaStream_t s) {
+    const cudaError_t e = cudaFuncSetAttribute((const void *)k_mc_emit<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(kEmitWarps * sizeof(EmitSmem)));
+    if (e != cudaSuccess) return e;
+    k_mc_emit<BATCH><<<nblk(units, kEmitWarps), 32 * kEmitWarps, kEmitWarps * sizeof(EmitSmem), s>>>(
+        g, b, sign, codes, lut, words, rowBase, tri, vkey, chunk, units);
+    return cudaGetLastError();
+}
+cudaError_t launch_mc_emit(const QGrid &g, const unsigned *sign, const unsigned char *codes, const float *lut,
+                           const unsigned *words, const uint2 *rowBase, unsigned *tri, unsigned long long *vkey,
+                           cudaStream_t s) {
+    const unsigned long long all = mc_words(g.Gc);
+    const unsigned chunk = mc_emit_chunk(all);
+    return emit_with<false>(g, QBatch{}, sign, codes, lut, words, rowBase, tri, vkey, chunk,
+                            (unsigned)((all + chunk - 1) / chunk), s);
+}
+cudaError_t launch_mc_emit_batch(const QBatch &b, unsigned chunk, unsigned units, const unsigned *sign,
+                                 const unsigned char *codes, const unsigned *words, const uint2 *rowBase, unsigned *tri,
+                                 unsigned long long *vkey, cudaStream_t s) {
+    return emit_with<true>(QGrid{}, b, sign, codes, nullptr, words, rowBase, tri, vkey, chunk, units, s);
 }
 size_t weld_tmp_bytes(unsigned layers) { return 256 + 8ull * layers; }
 template <bool BATCH>

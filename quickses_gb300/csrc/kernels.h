@@ -20,9 +20,11 @@ void launch_sas(const QGrid &g, const float4 *atoms, const uint2 *cells, unsigne
 void launch_edt(const QGrid &g, const unsigned *inMask, const unsigned *outMask, unsigned char *codes,
                 unsigned *signMask, cudaStream_t s, int shape = 0, unsigned char *zd = nullptr);
 
-void launch_mc_count(const QGrid &g, const unsigned *sign, uint2 *rowCount, cudaStream_t s);
-void launch_mc_emit(const QGrid &g, const unsigned *sign, const unsigned char *codes, const float *lut,
-                    const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s);
+// words: one per 32 voxels of an owner row, what its row's words before it have (k_mesh.cu).
+void launch_mc_count(const QGrid &g, const unsigned *sign, uint2 *rowCount, unsigned *words, cudaStream_t s);
+cudaError_t launch_mc_emit(const QGrid &g, const unsigned *sign, const unsigned char *codes, const float *lut,
+                           const unsigned *words, const uint2 *rowBase, unsigned *tri, unsigned long long *vkey,
+                           cudaStream_t s);
 // Vertex ids (vmap, per edge slot), welded positions and their count from the edge keys in owner
 // row order (rowBase: the scanned row counts).  skey, sslot: scratch, one entry per edge.
 size_t weld_tmp_bytes(unsigned layers);
@@ -116,9 +118,15 @@ void launch_edt_batch(const QBatch &b, unsigned tiles, const unsigned *inMask, c
                       unsigned char *zd = nullptr);
 // Owner rows a marching-cubes warp covers for a grid with Gc emitted cells per axis.
 int mc_rows_per_warp(int Gc);
-void launch_mc_count_batch(const QBatch &b, unsigned units, const unsigned *sign, uint2 *rowCount, cudaStream_t s);
-void launch_mc_emit_batch(const QBatch &b, unsigned units, const unsigned *sign, const unsigned char *codes,
-                          const uint2 *rowBase, unsigned *tri, unsigned long long *vkey, cudaStream_t s);
+void launch_mc_count_batch(const QBatch &b, unsigned units, const unsigned *sign, uint2 *rowCount, unsigned *words,
+                           cudaStream_t s);
+// Words of a molecule's rows, and how many of them a warp of the emission takes (a batch: of the
+// words of all; emit_off counts each molecule's in such chunks).
+unsigned long long mc_words(int Gc);
+unsigned mc_emit_chunk(unsigned long long words);
+cudaError_t launch_mc_emit_batch(const QBatch &b, unsigned chunk, unsigned units, const unsigned *sign,
+                                 const unsigned char *codes, const unsigned *words, const uint2 *rowBase, unsigned *tri,
+                                 unsigned long long *vkey, cudaStream_t s);
 // layers: owner planes (Gc + 1) of all molecules; vtx_off receives each molecule's first vertex.
 cudaError_t launch_weld_batch(const QBatch &b, unsigned layers, const unsigned long long *vkey, const uint2 *rowBase,
                               unsigned ne, const unsigned *edge_off, unsigned long long *skey, unsigned *sslot,

@@ -534,7 +534,7 @@ static int enqueue_field(qses_context *ctx, const FieldSeg &a, SegOut &o) {
     ctx->launches++;
     ctx->launches++;
     ctx->mark("refine");
-    launch_mc_count(a.g, a.sign_mask, a.rows, s);
+    launch_mc_count(a.g, a.sign_mask, a.rows, a.in_mask, s);  // the atoms' masks are done with
     ctx->launches++;
     QCHK(scan_u2(a.rows, a.rows, (unsigned)a.nrow, a.tot, a.tmp, a.err, s, &ctx->launches));
     QCHK(cudaMemcpyAsync(a.h_out, a.tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
@@ -548,6 +548,7 @@ struct MeshSeg {
     const unsigned *sign_mask;
     const unsigned char *codes;
     const float *lut;
+    const unsigned *words;  // of the rows
     const uint2 *rows;
     unsigned *tri;
     unsigned long long *vk, *vk2;
@@ -566,7 +567,7 @@ struct MeshSeg {
 
 static int enqueue_mesh(qses_context *ctx, const MeshSeg &b, SegOut &o) {
     cudaStream_t s = ctx->stream;
-    launch_mc_emit(b.g, b.sign_mask, b.codes, b.lut, b.rows, b.tri, b.vk, s);
+    QCHK(launch_mc_emit(b.g, b.sign_mask, b.codes, b.lut, b.words, b.rows, b.tri, b.vk, s));
     ctx->launches++;
     ctx->mark("mc_emit");
     if (b.ne > 0) {
@@ -796,6 +797,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     memset(&b, 0, sizeof(b));
     b.mem = ctx->field.gen + ctx->mesh_ws.gen;
     b.sign_mask = a.sign_mask;
+    b.words = a.in_mask;
     b.codes = a.codes;
     b.lut = a.lut;
     b.rows = a.rows;

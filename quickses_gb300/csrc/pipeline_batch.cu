@@ -109,7 +109,7 @@ static int enqueue_batch_field(qses_context *ctx, const BatchFieldSeg &a, SegOut
     ctx->launches += 2;
     ctx->mark("refine");
     // marching-cubes counts, one scan over all rows, per-molecule offsets
-    launch_mc_count_batch(a.b, a.units, a.sign_mask, a.rows, s);
+    launch_mc_count_batch(a.b, a.units, a.sign_mask, a.rows, a.in_mask, s);  // the atoms' masks are done with
     ctx->launches++;
     QCHK(scan_u2(a.rows, a.rows, (unsigned)a.n_rows, a.tot, a.tmp, a.err, s, &ctx->launches));
     launch_gather_offsets(a.rows, a.b.row_off, a.b.n_mol, (unsigned)a.n_rows, a.tot, a.tri_off, a.edge_off, s);
@@ -124,6 +124,7 @@ struct BatchMeshSeg {
     unsigned long long mem;  // free counters of the buffers it uses
     const unsigned *sign_mask;
     const unsigned char *codes;
+    const unsigned *words;  // of the rows
     const uint2 *rows;
     unsigned *tri;
     unsigned long long *vk, *vk2;
@@ -139,14 +140,14 @@ struct BatchMeshSeg {
     void *h_vtx;           // pinned: per-molecule first vertex
     unsigned long long n3;
     unsigned units, ne;
-    unsigned layers, pad_;
+    unsigned layers, chunk;
     QBatch b;
 };
 
 static int enqueue_batch_mesh(qses_context *ctx, const BatchMeshSeg &m, SegOut &o) {
     cudaStream_t s = ctx->stream;
     const unsigned nm = m.b.n_mol;
-    launch_mc_emit_batch(m.b, m.units, m.sign_mask, m.codes, m.rows, m.tri, m.vk, s);
+    QCHK(launch_mc_emit_batch(m.b, m.chunk, m.units, m.sign_mask, m.codes, m.words, m.rows, m.tri, m.vk, s));
     ctx->launches++;
     ctx->mark("mc_emit");
     if (m.ne > 0) {
@@ -262,8 +263,10 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     // ---- per-molecule layout on the host
     const unsigned nm = count;
     std::vector<QMol> mols(nm);
-    std::vector<unsigned> tile_off(nm + 1), atom_off(nm + 1), row_off(nm + 1), unit_off(nm + 1), word_off(nm + 1), layer_off(nm + 1);
-    unsigned long long mask_tot = 0, code_tot = 0, cell_tot = 0, tiles = 0, rows = 0, atoms_tot = 0, units = 0, layers = 0;
+    std::vector<unsigned> tile_off(nm + 1), atom_off(nm + 1), row_off(nm + 1), unit_off(nm + 1), word_off(nm + 1), layer_off(nm + 1), emit_off(nm + 1);
+    unsigned long long mask_tot = 0, code_tot = 0, cell_tot = 0, tiles = 0, rows = 0, atoms_tot = 0, units = 0, layers = 0, emits = 0, mc_tot = 0;
+    for (unsigned m = 0; m < nm; m++) mc_tot += mc_words(items[m].g.Gc);
+    const unsigned chunk = mc_emit_chunk(mc_tot);
     for (unsigned m = 0; m < nm; m++) {
         const QGrid &g = items[m].g;
         QMol &q = mols[m];
@@ -282,6 +285,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         word_off[m] = (unsigned)mask_tot;
         layer_off[m] = (unsigned)layers;
         layers += (unsigned long long)g.Gc + 1;
+        emit_off[m] = (unsigned)emits;
+        emits += (mc_words(g.Gc) + chunk - 1) / chunk;
         mask_tot += (unsigned long long)g.G * g.G * g.W;
         code_tot += (unsigned long long)g.G * g.G * g.Gp;
         cell_tot += (unsigned long long)g.gnb * g.gnb * g.gnb;
@@ -298,13 +303,14 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     unit_off[nm] = (unsigned)units;
     word_off[nm] = (unsigned)mask_tot;
     layer_off[nm] = (unsigned)layers;
+    emit_off[nm] = (unsigned)emits;
     if (tiles >= (1ull << 31) || rows >= (1ull << 31) || cell_tot >= (1ull << 31) || atoms_tot >= (1ull << 30) ||
         mask_tot >= (1ull << 32))
         return ctx->fail(QSES_ERR_UNSUPPORTED, "batch too large for 32-bit item indices; split it");
     const unsigned N = (unsigned)atoms_tot;
 
     // ---- pinned staging: descriptor block then atoms, one copy each
-    const size_t desc_bytes = a256(sizeof(QMol) * nm) + 10 * a256(4ull * (nm + 1)) + a256(1024ull * nm);
+    const size_t desc_bytes = a256(sizeof(QMol) * nm) + 11 * a256(4ull * (nm + 1)) + a256(1024ull * nm);
     const size_t atom_bytes = 16ull * N;
     if (stage_reserve(ctx, desc_bytes + atom_bytes + 256) != QSES_OK)
         return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "pinned batch staging");
@@ -322,6 +328,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     hput(unit_off.data(), 4ull * (nm + 1));
     hput(word_off.data(), 4ull * (nm + 1));
     hput(layer_off.data(), 4ull * (nm + 1));
+    hput(emit_off.data(), 4ull * (nm + 1));
     hput(nullptr, 4ull * (nm + 1));  // tri_off   (device-filled)
     hput(nullptr, 4ull * (nm + 1));  // edge_off  (device-filled)
     hput(nullptr, 4ull * (nm + 1));  // vtx_off   (device-filled)
@@ -371,6 +378,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         b.mc_unit_off = (const unsigned *)at(ob);
         b.word_off = (const unsigned *)at(ob);
         b.layer_off = (const unsigned *)at(ob);
+        b.emit_off = (const unsigned *)at(ob);
         b.tri_off = (const unsigned *)at(ob);
         d_edge_off = (unsigned *)at(ob);
         b.vtx_off = (const unsigned *)at(ob);
@@ -441,6 +449,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     memset(&mb, 0, sizeof(mb));
     mb.mem = ctx->field.gen + ctx->mesh_ws.gen + ctx->host_gen;
     mb.sign_mask = a.sign_mask;
+    mb.words = a.in_mask;
+    mb.chunk = chunk;
     mb.codes = a.codes;
     mb.rows = a.rows;
     mb.tri = tri;
@@ -458,7 +468,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     mb.h_out = ctx->h_small;
     mb.h_vtx = ctx->h_stage;
     mb.n3 = n3;
-    mb.units = (unsigned)units;
+    mb.units = (unsigned)emits;
     mb.ne = NE;
     mb.layers = layer_off[nm];
     mb.b = b;

@@ -189,7 +189,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 uint2 *h_tot = (uint2 *)ctx->h_small;
                 if (cells_any) {
                     const size_t E = (size_t)b.Gc + 1;
-                    launch_mc_count(b, sign_mask, rows, s);
+                    launch_mc_count(b, sign_mask, rows, in_mask, s);  // the atoms' masks are done with
                     ctx->launches++;
                     SCHK(scan_u2(rows, rows, (unsigned)(E * E), tot, tmp, d_err, s, &ctx->launches));
                     SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
@@ -234,7 +234,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 if (!tmpb || !fits) return ctx->fail(QSES_ERR_INTERNAL, "mesh workspace layout");
 
                 // ---- triangles and edge keys; weld; the last triangle's own vertices out
-                launch_mc_emit(b, sign_mask, codes, lut, rows, tri, wb.vk, s);
+                SCHK(launch_mc_emit(b, sign_mask, codes, lut, in_mask, rows, tri, wb.vk, s));
                 SCHK(launch_weld(b, wb.vk, rows, NE, wb.vk2, wb.vv, vmap, vq, tot, wb.tmp, d_err, s));
                 launch_remap(tri, n3k, vmap, s);
                 ctx->launches += 3;

@@ -67,6 +67,7 @@ struct QBatch {
     const unsigned *vtx_off;   // welded vertices (valid after the weld)
     const float *lut;          // 256 field values per molecule
     const unsigned *layer_off; // owner planes (Gc + 1) per molecule
+    const unsigned *emit_off;  // marching-cubes emission chunks of words per molecule
     unsigned n_mol;
     int pad_;
 };
