@@ -68,17 +68,21 @@ __global__ void k_atom_gather(const float *__restrict__ xyz, const float *__rest
 
 // ------------------------------------------------------------------ SAS
 
-constexpr int kSasTX = 8, kSasTY = 8, kSasNT = kSasTX * kSasTY, kSasCap = 768;
+// The SAS pass is bound by instruction issue (3 a cycle): the candidates of a tile and, per row and
+// atom, the interval's ends.  664^3, 50 000 atoms: 0.56 ms with a cell per thread in the search and
+// every interval verified, 0.46 without the intervals a row has already, 0.40 with half a column of
+// cells per thread; 1738^3 5.1, 5.2 and 3.8; 85^3 0.040 and 0.031.  512 candidates (12 KB) let as many
+// blocks run as the registers do; 768 take 0.50.
+constexpr int kSasTX = 8, kSasTY = 8, kSasNT = kSasTX * kSasTY, kSasCap = 512;
 
 // Exact per-voxel test along a z row: fma(ez, ez, sxy) < t with ez = z(k) - az.
-__device__ __forceinline__ bool zpred(int k, float az, float sxy, float t, float dx, float oz) {
-    float ez = __fsub_rn(vox(k, dx, oz), az);
+__device__ __forceinline__ bool zpred(float k, float az, float sxy, float t, float dx, float oz) {
+    const float ez = __fsub_rn(__fmaf_rn(k, dx, oz), az);
     return __fmaf_rn(ez, ez, sxy) < t;
 }
 
 __device__ __forceinline__ unsigned span_bits(int a, int b) {  // bits a..b inclusive, 0 <= a <= b <= 31
-    unsigned m = (b - a == 31) ? 0xffffffffu : ((1u << (b - a + 1)) - 1u);
-    return m << a;
+    return (0xffffffffu >> (31 - (b - a))) << a;
 }
 
 __device__ __forceinline__ float sqrt_approx(float x) {
@@ -87,43 +91,53 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     return r;
 }
 
-// Voxels k in [k0, klim] of one z row whose squared distance to the atom is below t.
-// The set is an interval (the predicate is monotone in |k - k_atom|); its ends are
-// estimated in closed form and verified with the exact predicate, with a brute-force
-// fallback if the estimate does not verify (so the estimate's square root need not be
-// correctly rounded: one approximate instruction).
-__device__ __forceinline__ unsigned zmask(float az, float sxy, float t, int k0, int klim, float dx, float oz,
-                                          float inv_dx) {
-    float kcf = fminf(fmaxf((az - oz) * inv_dx, -1.0e6f), 1.0e6f);
-    float h = sqrt_approx(fmaxf(t - sxy, 0.0f)) * inv_dx;
-    int lo = max(k0, (int)ceilf(kcf - h));
-    int hi = min(klim, (int)floorf(kcf + h));
-    if (lo <= hi) {
-        if (zpred(lo, az, sxy, t, dx, oz) && zpred(hi, az, sxy, t, dx, oz) &&
-            (lo == k0 || !zpred(lo - 1, az, sxy, t, dx, oz)) && (hi == klim || !zpred(hi + 1, az, sxy, t, dx, oz)))
-            return span_bits(lo - k0, hi - k0);
-    } else {
-        int c = min(max(__float2int_rn(kcf), k0), klim);
-        if (!zpred(c, az, sxy, t, dx, oz) && (c == k0 || !zpred(c - 1, az, sxy, t, dx, oz)) &&
-            (c == klim || !zpred(c + 1, az, sxy, t, dx, oz)))
-            return 0u;
+// A z row's voxels, bit k of a word each: grid indices k0 .. klim.
+struct ZRow {
+    int k0, klim;
+    float dx, oz, inv_dx;
+};
+// Adds to `word` the voxels of a z row whose squared distance to the atom (kc: its z as a voxel
+// index) is below t.  They are an interval (the predicate is monotone in |k - kc|); its ends are
+// estimated in closed form, and if `word` has it already with a voxel more at either end, that is
+// all.  Else the ends are verified with the exact predicate, with a brute-force fallback if the
+// estimate does not verify (so the estimate's square root need not be correctly rounded: one
+// approximate instruction).  The estimate is good to a voxel while the rounding of t is small beside
+// a voxel's square: below 100 A, by far.
+__device__ __forceinline__ void add_zmask(unsigned &word, float az, float kc, float sxy, float t, const ZRow &z) {
+    const float h = sqrt_approx(fmaxf(t - sxy, 0.0f)) * z.inv_dx;
+    const float k0 = (float)z.k0, klim = (float)z.klim;
+    const float lo = fmaxf(ceilf(kc - h), k0), hi = fminf(floorf(kc + h), klim);
+    const int a = (int)lo - z.k0, b = (int)hi - z.k0;
+    const int wa = max(a - 1, 0), wb = min(b + 1, z.klim - z.k0);
+    if (t < 10000.0f) {
+        if (wa > wb) return;
+        const unsigned wide = span_bits(wa, wb);
+        if ((word & wide) == wide) return;
     }
-    unsigned m = 0;
-    for (int k = k0; k <= klim; k++)
-        if (zpred(k, az, sxy, t, dx, oz)) m |= 1u << (k - k0);
-    return m;
+    auto at = [&](float k) { return zpred(k, az, sxy, t, z.dx, z.oz); };
+    if (lo <= hi) {
+        if (at(lo) & at(hi) & (lo == k0 || !at(lo - 1.0f)) & (hi == klim || !at(hi + 1.0f))) {
+            word |= span_bits(a, b);
+            return;
+        }
+    } else {
+        const float c = fminf(fmaxf(rintf(kc), k0), klim);
+        if (!at(c) & (c == k0 || !at(c - 1.0f)) & (c == klim || !at(c + 1.0f))) return;
+    }
+    for (int k = z.k0; k <= z.klim; k++)
+        if (at((float)k)) word |= 1u << (k - z.k0);
 }
 
-// Row-interval classification of one z row against one atom.
-__device__ __forceinline__ void sas_row_atom(float px, float py, float ax, float ay, float az, float tin, float tsas,
-                                             int k0, int klim, const QGrid &g, float inv_dx, unsigned &sasw,
-                                             unsigned &inw) {
-    float ex = __fsub_rn(px, ax), ey = __fsub_rn(py, ay);
-    float sxy = __fmaf_rn(ey, ey, __fmul_rn(ex, ex));
-    if (sxy < tsas) {
-        sasw |= zmask(az, sxy, tsas, k0, klim, g.dx, g.oz, inv_dx);
-        if (sxy < tin) inw |= zmask(az, sxy, tin, k0, klim, g.dx, g.oz, inv_dx);
-    }
+// Row-interval classification of one z row against one atom (kc: its z as a voxel index).
+__device__ __forceinline__ void sas_row_atom(float px, float py, const float4 &a, float tin, float kc, const ZRow &z,
+                                             unsigned full, unsigned &sasw, unsigned &inw) {  // a.w: tsas
+    const float ex = __fsub_rn(px, a.x), ey = __fsub_rn(py, a.y);
+    const float sxy = __fmaf_rn(ey, ey, __fmul_rn(ex, ex));
+    if (sxy < a.w && sasw != full) add_zmask(sasw, a.z, kc, sxy, a.w, z);
+    if (sxy < tin && inw != full) add_zmask(inw, a.z, kc, sxy, tin, z);
+}
+__device__ __forceinline__ float voxel_index(float z, float oz, float inv_dx) {
+    return fminf(fmaxf((z - oz) * inv_dx, -1.0e6f), 1.0e6f);
 }
 
 __device__ __forceinline__ void atom_thresholds(float r, const QGrid &g, float &tin, float &tsas) {
@@ -137,8 +151,9 @@ __device__ __forceinline__ void atom_thresholds(float r, const QGrid &g, float &
 __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, const float4 *__restrict__ atoms,
                                          const uint2 *__restrict__ cells, unsigned *__restrict__ inMask,
                                          unsigned *__restrict__ outMask) {
-    __shared__ float s_x[kSasCap], s_y[kSasCap], s_z[kSasCap], s_tin[kSasCap], s_ts[kSasCap];
-    __shared__ int s_n, s_over;
+    __shared__ float4 s_a[kSasCap];  // x, y, z, threshold of probe + r
+    __shared__ float2 s_t[kSasCap];  // threshold of r - dx, z as a voxel index
+    __shared__ int s_n;
     const int j0 = jb * kSasTY, i0 = ib * kSasTX;
     const int t = threadIdx.x, i = i0 + t / kSasTY, j = j0 + t % kSasTY, k0 = w * 32;
     // Voxels with an index >= lim on an axis are never computed and stay outside: the last
@@ -167,53 +182,72 @@ __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, 
         crange(bx0, bx1, g.ox, cx0, cx1);
         crange(by0, by1, g.oy, cy0, cy1);
         crange(bz0, bz1, g.oz, cz0, cz1);
-        const int ncy = cy1 - cy0 + 1, ncz = cz1 - cz0 + 1, ncell = (cx1 - cx0 + 1) * ncy * ncz;
-        if (t == 0) { s_n = 0; s_over = 0; }
-        __syncthreads();
-        // Stage every atom whose probe-inflated sphere can reach the tile (conservative box test).
-        for (int c = t; c < ncell; c += kSasNT) {
-            int cz = c % ncz, cy = (c / ncz) % ncy, cx = c / (ncz * ncy);
-            uint2 rg = cells[((size_t)(cx0 + cx) * g.gnb + (cy0 + cy)) * g.gnb + (cz0 + cz)];
-            for (unsigned s = rg.x; s < rg.y; s++) {
-                float4 a = atoms[s];
-                float ddx = fmaxf(fmaxf(bx0 - a.x, a.x - bx1), 0.0f);
-                float ddy = fmaxf(fmaxf(by0 - a.y, a.y - by1), 0.0f);
-                float ddz = fmaxf(fmaxf(bz0 - a.z, a.z - bz1), 0.0f);
-                float rs = g.probe + a.w;
-                if (ddx * ddx + ddy * ddy + ddz * ddz <= rs * rs * 1.001f + 1e-3f) {
-                    int q = atomicAdd(&s_n, 1);
-                    if (q < kSasCap) {
-                        float tin, tsas;
-                        atom_thresholds(a.w, g, tin, tsas);
-                        s_x[q] = a.x; s_y[q] = a.y; s_z[q] = a.z; s_tin[q] = tin; s_ts[q] = tsas;
-                    } else {
-                        s_over = 1;
-                    }
-                }
+        const int ncy = cy1 - cy0 + 1, ncz = cz1 - cz0 + 1, ncol = (cx1 - cx0 + 1) * ncy;
+        // Stage every atom whose probe-inflated sphere can reach the tile (conservative box test).  A
+        // thread takes half a column of cells, whose atoms are one run (an empty cell is (0, 0)).
+        auto run = [&](int c) {
+            const int cx = (c >> 1) / ncy, cy = (c >> 1) - cx * ncy;
+            const int z0 = cz0 + (c & 1 ? ncz / 2 : 0), z1 = c & 1 ? cz1 + 1 : cz0 + ncz / 2;
+            const uint2 *col = cells + ((size_t)(cx0 + cx) * g.gnb + (cy0 + cy)) * g.gnb;
+            uint2 r = make_uint2(0xffffffffu, 0u);
+            for (int z = z0; z < z1; z++) {
+                const uint2 rg = __ldg(col + z);
+                if (rg.y) r.x = min(r.x, rg.x);
+                r.y = max(r.y, rg.y);
             }
+            return r;
+        };
+        auto stage = [&](unsigned s) {
+            const float4 a = __ldg(atoms + s);
+            const float ddx = fmaxf(fmaxf(bx0 - a.x, a.x - bx1), 0.0f);
+            const float ddy = fmaxf(fmaxf(by0 - a.y, a.y - by1), 0.0f);
+            const float ddz = fmaxf(fmaxf(bz0 - a.z, a.z - bz1), 0.0f);
+            const float rs = g.probe + a.w;
+            if (!(ddx * ddx + ddy * ddy + ddz * ddz <= rs * rs * 1.001f + 1e-3f)) return;
+            const int q = atomicAdd(&s_n, 1);
+            if (q >= kSasCap) return;
+            float tin, tsas;
+            atom_thresholds(a.w, g, tin, tsas);
+            s_a[q] = make_float4(a.x, a.y, a.z, tsas);
+            s_t[q] = make_float2(tin, voxel_index(a.z, g.oz, inv_dx));
+        };
+        const float px = vox(i + oi, g.dx, g.ox), py = vox(j + oj, g.dx, g.oy);
+        const ZRow z{k0 + ok, klim + ok, g.dx, g.oz, inv_dx};  // z range as grid indices
+        const unsigned full = span_bits(0, klim - k0);
+        auto classify = [&](int na) {
+            if (i > lastx || j > lasty) return;
+            for (int q = 0; q < na; q++) {
+                const float2 u = s_t[q];
+                sas_row_atom(px, py, s_a[q], u.x, u.y, z, full, sasw, inw);
+            }
+        };
+        if (t == 0) s_n = 0;
+        __syncthreads();
+        for (int c = t; c < 2 * ncol; c += kSasNT) {
+            const uint2 r = run(c);
+            for (unsigned s = r.x; s < r.y; s++) stage(s);
         }
         __syncthreads();
-        if (i <= lastx && j <= lasty) {
-            const float px = vox(i + oi, g.dx, g.ox), py = vox(j + oj, g.dx, g.oy);
-            const int kg0 = k0 + ok, kglim = klim + ok;  // z range as grid indices (bits from kg0)
-            if (!s_over) {
-                const int na = s_n;
-                for (int q = 0; q < na; q++)
-                    sas_row_atom(px, py, s_x[q], s_y[q], s_z[q], s_tin[q], s_ts[q], kg0, kglim, g, inv_dx, sasw,
-                                 inw);
-            } else {
-                // Too many candidates for shared memory: walk the cells directly.
-                for (int c = 0; c < ncell; c++) {
-                    int cz = c % ncz, cy = (c / ncz) % ncy, cx = c / (ncz * ncy);
-                    uint2 rg = cells[((size_t)(cx0 + cx) * g.gnb + (cy0 + cy)) * g.gnb + (cz0 + cz)];
-                    for (unsigned s = rg.x; s < rg.y; s++) {
-                        float4 a = atoms[s];
-                        float tin, tsas;
-                        atom_thresholds(a.w, g, tin, tsas);
-                        sas_row_atom(px, py, a.x, a.y, a.z, tin, tsas, kg0, kglim, g, inv_dx, sasw, inw);
-                    }
+        if (s_n <= kSasCap) {
+            classify(s_n);
+        } else {
+            // More than fit (crowded atoms, coarse voxels): all threads run through the columns
+            // together and classify whenever there may be no room for another 64.
+            for (int c = 0; c < 2 * ncol; c++) {
+                const uint2 r = run(c);
+                for (unsigned s = r.x; s < r.y; s += kSasNT) {
+                    __syncthreads();
+                    const int n = s_n > kSasCap ? 0 : s_n;  // the first round starts over
+                    const bool flush = n > kSasCap - kSasNT;
+                    if (flush) classify(n);
+                    __syncthreads();
+                    if (t == 0) s_n = flush ? 0 : n;
+                    __syncthreads();
+                    if (s + t < r.y) stage(s + t);
                 }
             }
+            __syncthreads();
+            classify(s_n);
         }
     }
     if (i < G && j < G) {
