@@ -277,27 +277,109 @@ constexpr int kEdtNT = 256;
 
 // One refine tile: z-word w of the TX x TY rows starting at (TX ib, TY jb), with an R halo.
 // Larger tiles re-read less halo per row (the z pass runs on (TX+2R)(TY+2R) rows for TX TY
-// output rows) at the cost of shared memory (dynamic, edt_smem_bytes); the shape is chosen
+// output rows) at the cost of shared memory (dynamic, edt_layout); the shape is chosen
 // by the autotuner.
+//
+// Bound by instruction issue where there is a border, by the codes' bytes elsewhere.  664^3 (R = 6)
+// 0.61 ms, 1738^3 (R = 3, most tiles without a border) 4.6.  With the z distances of all voxels in
+// memory, written and read back with the halo, 0.67 and 7.6; with byte rows spread at each tap, taps
+// one by one and codes voxel by voxel 0.83 and 7.6.
 
-// Min-plus on four byte distances of a word (255 = none) without the byte-SIMD add and
-// min, which this GPU runs as several instructions each: the bytes are spread over two
-// words of 16-bit halves (one byte permute each), where adding a square <= 81 cannot carry
-// (255 + 81 < 2^16) and the 16-bit min is one instruction; packing back clamps at 255.
+// Min-plus without the byte-SIMD add and min, which this GPU runs as several instructions each:
+// four byte distances (255 = none) are spread over two words of 16-bit halves (one byte permute
+// each), where the 16-bit add and min are one instruction, and stay so through the y and x passes.
 // Real distances stay below 255 (y <= 2 R^2 = 162, x <= 3 R^2 = 243) and "none" at or above
-// it, so the results equal the saturating byte arithmetic's.
+// it; the taps at distance 0 bring it back to 255.
 __device__ __forceinline__ unsigned spread_lo(unsigned w) { return __byte_perm(w, 0u, 0x4140); }  // bytes 0, 1
 __device__ __forceinline__ unsigned spread_hi(unsigned w) { return __byte_perm(w, 0u, 0x4342); }  // bytes 2, 3
-__device__ __forceinline__ unsigned pack_bytes(unsigned lo, unsigned hi) {
-    return __byte_perm(__vminu2(lo, 0x00ff00ffu), __vminu2(hi, 0x00ff00ffu), 0x6420);
+// The y pass of a tile: squared distances in the (y, z) plane, 8 voxels of a halo row's output at a
+// time, from the z distances of its 2R + 1 neighbours, two at the same distance together.
+__device__ __forceinline__ uint4 y_taps(const uint2 *g, int stride, int R) {  // g: of the row itself
+    const uint2 c = g[0];
+    uint4 v = make_uint4(spread_lo(c.x), spread_hi(c.x), spread_lo(c.y), spread_hi(c.y));
+    unsigned d2 = 0x00010001u;
+    for (int d = 1; d <= R; d++) {
+        const uint2 m = g[-d * stride], p = g[d * stride];
+        v.x = __vminu2(v.x, __vminu2(spread_lo(m.x), spread_lo(p.x)) + d2);
+        v.y = __vminu2(v.y, __vminu2(spread_hi(m.x), spread_hi(p.x)) + d2);
+        v.z = __vminu2(v.z, __vminu2(spread_lo(m.y), spread_lo(p.y)) + d2);
+        v.w = __vminu2(v.w, __vminu2(spread_hi(m.y), spread_hi(p.y)) + d2);
+        d2 += (unsigned)(2 * d + 1) * 0x00010001u;
+    }
+    return v;
+}
+// The x pass, the same over the y pass's rows.
+__device__ __forceinline__ uint4 x_taps(const uint4 *h, int stride, int R) {
+    uint4 v = h[0];
+    unsigned d2 = 0x00010001u;
+    for (int d = 1; d <= R; d++) {
+        const uint4 m = h[-d * stride], p = h[d * stride];
+        v.x = __vminu2(v.x, __vminu2(m.x, p.x) + d2);
+        v.y = __vminu2(v.y, __vminu2(m.y, p.y) + d2);
+        v.z = __vminu2(v.z, __vminu2(m.z, p.z) + d2);
+        v.w = __vminu2(v.w, __vminu2(m.w, p.w) + d2);
+        d2 += (unsigned)(2 * d + 1) * 0x00010001u;
+    }
+    return v;
+}
+// Voxels (4 bits) of two words of halves that are at or above a threshold (below: 0x8000 less it).
+__device__ __forceinline__ unsigned at_least(unsigned lo, unsigned hi, unsigned below) {
+    const unsigned a = (lo + below) & 0x80008000u, b = (hi + below) & 0x80008000u;
+    return (a >> 15 & 1u) | (a >> 30) | (b >> 13 & 4u) | (b >> 28);
 }
 
+__device__ __forceinline__ unsigned nibble_bytes(unsigned nib) {  // 4 bits -> 0xff in each set bit's byte
+    return ((nib * 0x00204081u) & 0x01010101u) * 0xffu;           // copies at bits 0, 7, 14, 21: no carries
+}
 // Squared z distances of one 32-voxel word c (bit = outside voxel) with its neighbouring
 // words a (below) and d (above), one byte per voxel (<= R^2, 255 = none), four per output
 // word.  Bit-parallel: the outside set grows by one voxel per step (two funnel shifts over
-// the neighbouring words), and the voxels first covered at step k are at distance k.
-__device__ __forceinline__ unsigned nibble_bytes(unsigned nib) {  // 4 bits -> 0xff in each set bit's byte
-    return ((nib * 0x00204081u) & 0x01010101u) * 0xffu;           // copies at bits 0, 7, 14, 21: no carries
+// the neighbouring words), and the voxels first covered at step k are at distance k.  The distances
+// are collected as bit planes; four voxels' planes make a selector, and one byte permute looks up
+// their squares (FAR: two, for distances above 6): some 100 instructions a word; writing the squares
+// into the bytes step by step took 350.
+template <bool FAR>
+__device__ __forceinline__ void z_planes(unsigned a, unsigned c, unsigned d, int R, unsigned out[8]) {
+    unsigned cov = c, p[4] = {0u, 0u, 0u, 0u};  // voxels with an outside voxel within k; bits of k
+#pragma unroll
+    for (int k = 1; k <= (FAR ? QSES_RMAX : 6); k++) {
+        if (k > R) break;
+        // bit b of the right funnel shift is voxel b + k, of the left one voxel b - k
+        const unsigned nc = cov | __funnelshift_r(c, d, k) | __funnelshift_l(a, c, k);
+        const unsigned nw = nc & ~cov;  // nearest outside voxel at distance k
+        cov = nc;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (k >> q & 1) p[q] |= nw;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) p[q] |= ~cov;  // none: 15, or 7 of the three planes
+    // per four voxels the planes' nibbles side by side, even and odd groups; a 4 x 4 bit transpose
+    // (two delta swaps, two groups at a time) turns them into the voxels' selectors
+    const unsigned n = 0x0f0f0f0fu;
+    const unsigned e01 = (p[0] & n) | ((p[1] & n) << 4), o01 = ((p[0] >> 4) & n) | (p[1] & ~n);
+    const unsigned e23 = (p[2] & n) | (FAR ? (p[3] & n) << 4 : 0u), o23 = ((p[2] >> 4) & n) | (FAR ? p[3] & ~n : 0u);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {  // voxels 8 j .. 8 j + 7
+        const unsigned pick = (unsigned)j | (unsigned)(4 + j) << 4;
+        unsigned x = __byte_perm(e01, e23, pick) & 0xffffu;
+        x |= __byte_perm(o01, o23, pick) << 16;
+        unsigned t = (x ^ (x >> 3)) & 0x0a0a0a0au;
+        x ^= t ^ (t << 3);
+        t = (x ^ (x >> 6)) & 0x00cc00ccu;
+        x ^= t ^ (t << 6);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const unsigned sel = (h ? x >> 16 : x) & (FAR ? 0x7777u : 0xffffu);
+            if (FAR) {
+                const unsigned m = nibble_bytes((p[3] >> (8 * j + 4 * h)) & 0xfu);
+                out[2 * j + h] = (__byte_perm(0x09040100u, 0x31241910u, sel) & ~m) |
+                                 (__byte_perm(0x00005140u, 0xff000000u, sel) & m);
+            } else {
+                out[2 * j + h] = __byte_perm(0x09040100u, 0xff241910u, sel);
+            }
+        }
+    }
 }
 __device__ __forceinline__ void z_word(unsigned a, unsigned c, unsigned d, int R, unsigned out[8]) {
     if ((a | c | d) == 0u || c == 0xffffffffu) {  // no outside voxel within 32, or all outside
@@ -305,22 +387,10 @@ __device__ __forceinline__ void z_word(unsigned a, unsigned c, unsigned d, int R
         for (int k = 0; k < 8; k++) out[k] = c ? 0u : 0xffffffffu;
         return;
     }
-#pragma unroll
-    for (int j = 0; j < 8; j++) out[j] = ~nibble_bytes((c >> (4 * j)) & 0xfu);  // outside: 0, else none
-    unsigned cov = c;  // voxels with an outside voxel within k
-    for (int k = 1; k <= R; k++) {
-        // bit b of the right funnel shift is voxel b + k, of the left one voxel b - k
-        const unsigned nc = cov | __funnelshift_r(c, d, k) | __funnelshift_l(a, c, k);
-        const unsigned nw = nc & ~cov;  // nearest outside voxel at distance k
-        cov = nc;
-        if (nw == 0u) continue;
-        const unsigned v = (unsigned)(k * k) * 0x01010101u;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const unsigned m = nibble_bytes((nw >> (4 * j)) & 0xfu);
-            out[j] = (out[j] & ~m) | (v & m);
-        }
-    }
+    if (R <= 6)
+        z_planes<false>(a, c, d, R, out);
+    else
+        z_planes<true>(a, c, d, R, out);
 }
 
 // Shared-memory layout of one refine tile for a window of R voxels: the halo rows' outside
@@ -328,14 +398,13 @@ __device__ __forceinline__ void z_word(unsigned a, unsigned c, unsigned d, int R
 // tile's in/out words.  Sized per launch, so a smaller window (a larger voxel) fits more CTAs
 // per SM; the largest layout (R = QSES_RMAX, no z distances) bounds every other.
 struct EdtLayout {
-    size_t g_off, h_off, in_off, ot_off, bytes;
+    size_t h_off, in_off, ot_off, bytes;
 };
-__host__ __device__ __forceinline__ EdtLayout edt_layout(int TX, int TY, int R, bool have_zd) {
+__host__ __device__ __forceinline__ EdtLayout edt_layout(int TX, int TY, int R) {
     const size_t HX = (size_t)TX + 2 * R, HY = (size_t)TY + 2 * R;
     EdtLayout L;
-    L.g_off = have_zd ? 0 : ((12 * HX * HY + 15) & ~(size_t)15);  // [HX HY][3] outside words first
-    L.h_off = L.g_off + 32 * HX * HY;                                 // [HX HY][32] z distances
-    L.in_off = L.h_off + 32 * HX * (size_t)TY;                         // [HX][TY][32] y-pass rows
+    L.h_off = 32 * HX * HY;                     // [HX HY][32] z distances first
+    L.in_off = L.h_off + 64 * HX * (size_t)TY;  // [HX][TY][32] y-pass rows, 16 bits
     L.ot_off = L.in_off + 4 * (size_t)TX * TY;
     L.bytes = L.ot_off + 4 * (size_t)TX * TY;
     return L;
@@ -344,15 +413,12 @@ __host__ __device__ __forceinline__ EdtLayout edt_layout(int TX, int TY, int R, 
 template <int TX, int TY>
 __device__ __forceinline__ void edt_tile(const QGrid &g, int w, int jb, int ib, const unsigned *__restrict__ inMask,
                                          const unsigned *__restrict__ outMask, unsigned char *__restrict__ codes,
-                                         unsigned *__restrict__ signMask,
-                                         const unsigned char *__restrict__ zd = nullptr) {
-    const EdtLayout L = edt_layout(TX, TY, g.R, zd != nullptr);
+                                         unsigned *__restrict__ signMask) {
+    const EdtLayout L = edt_layout(TX, TY, g.R);
     extern __shared__ __align__(16) unsigned char edt_smem[];
-    unsigned (*s_out)[3] = reinterpret_cast<unsigned (*)[3]>(edt_smem);  // without zd only
-    // Squared distances, one byte per voxel (255 = none); the y and x passes work on four
-    // voxels per 32-bit word with saturating byte adds, so 255 stays "none".
-    unsigned char (*s_g)[32] = reinterpret_cast<unsigned char (*)[32]>(edt_smem + L.g_off);
-    unsigned char (*s_h)[TY][32] = reinterpret_cast<unsigned char (*)[TY][32]>(edt_smem + L.h_off);
+    // squared z distances, one byte per voxel (255 = none)
+    unsigned char (*s_g)[32] = reinterpret_cast<unsigned char (*)[32]>(edt_smem);
+    uint4 *s_h = reinterpret_cast<uint4 *>(edt_smem + L.h_off);  // [HX][TY][4]
     unsigned *s_in = reinterpret_cast<unsigned *>(edt_smem + L.in_off);
     unsigned *s_ot = reinterpret_cast<unsigned *>(edt_smem + L.ot_off);
     const int j0 = jb * TY, i0 = ib * TX;
@@ -375,72 +441,31 @@ __device__ __forceinline__ void edt_tile(const QGrid &g, int w, int jb, int ib, 
     }
     const int has_border = __syncthreads_or(anyb);
     int has_out = 0;
-    if (has_border && zd) {
-        // z distances computed once per voxel by k_edt_z: load the halo rows' bytes
-        int any = 0;
-        for (int q = t; q < HX * HY * 2; q += kEdtNT) {
-            const int row = q >> 1, half = q & 1;
-            const int i = i0 - R + row / HY, j = j0 - R + row % HY;
-            uint4 v = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-            if (i >= 0 && i < G && j >= 0 && j < G)
-                v = __ldg(reinterpret_cast<const uint4 *>(zd + ((size_t)i * G + j) * g.Gp + (size_t)k0) + half);
-            reinterpret_cast<uint4 *>(s_g[row])[half] = v;
-            any |= (v.x & v.y & v.z & v.w) != 0xffffffffu;
-        }
-        has_out = __syncthreads_or(any);
-        if (has_out) {
-            // y: min over dj of dj^2 + g^2 (<= 2 R^2 = 162 < 255), four voxels per word.
-            for (int q = t; q < HX * TY * 8; q += kEdtNT) {
-                const int w4 = q & 7, y = (q >> 3) % TY, hx = (q >> 3) / TY;
-                unsigned lo = 0xffffffffu, hi = 0xffffffffu;
-                for (int dj = -R; dj <= R; dj++) {
-                    const unsigned gw = reinterpret_cast<const unsigned *>(s_g[hx * HY + y + R + dj])[w4];
-                    const unsigned d2 = (unsigned)(dj * dj) * 0x00010001u;
-                    lo = __vminu2(lo, spread_lo(gw) + d2);
-                    hi = __vminu2(hi, spread_hi(gw) + d2);
-                }
-                reinterpret_cast<unsigned *>(s_h[hx][y])[w4] = pack_bytes(lo, hi);
-            }
-            __syncthreads();
-        }
-    } else if (has_border) {
+    if (has_border) {
+        // z: squared distance (in voxels, <= R^2) to the nearest outside voxel along the row, a halo
+        // row's 32 voxels per thread
         int any = 0;
         for (int q = t; q < HX * HY; q += kEdtNT) {
-            int i = i0 - R + q / HY, j = j0 - R + q % HY;
-            unsigned a = 0u, b = 0u, c = 0u;
+            const int i = i0 - R + q / HY, j = j0 - R + q % HY;
+            unsigned a = 0u, c = 0u, d = 0u, out[8];
             if (i >= 0 && i < G && j >= 0 && j < G) {
-                size_t base = ((size_t)i * G + j) * W;
-                if (w > 0) a = outMask[base + w - 1];
-                b = outMask[base + w];
-                if (w + 1 < W) c = outMask[base + w + 1];
+                const unsigned *m = outMask + ((size_t)i * G + j) * W + w;
+                if (w > 0) a = __ldg(m - 1);
+                c = __ldg(m);
+                if (w + 1 < W) d = __ldg(m + 1);
             }
-            s_out[q][0] = a; s_out[q][1] = b; s_out[q][2] = c;
-            any |= (a | b | c) != 0u;
-        }
-        has_out = __syncthreads_or(any);
-    }
-    if (has_border && has_out && !zd) {
-        // z: squared distance (in voxels, <= R^2) to the nearest outside voxel along the row,
-        // one row of 32 voxels per thread
-        for (int q = t; q < HX * HY; q += kEdtNT) {
-            unsigned out[8];
-            z_word(s_out[q][0], s_out[q][1], s_out[q][2], R, out);
+            any |= (a | c | d) != 0u;
+            z_word(a, c, d, R, out);
             uint4 *dst = reinterpret_cast<uint4 *>(s_g[q]);
             dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
             dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
         }
-        __syncthreads();
-        // y: min over dj of dj^2 + g^2 (<= 2 R^2 = 162 < 255), four voxels per word.
-        for (int q = t; q < HX * TY * 8; q += kEdtNT) {
-            const int w4 = q & 7, y = (q >> 3) % TY, hx = (q >> 3) / TY;
-            unsigned lo = 0xffffffffu, hi = 0xffffffffu;
-            for (int dj = -R; dj <= R; dj++) {
-                const unsigned gw = reinterpret_cast<const unsigned *>(s_g[hx * HY + y + R + dj])[w4];
-                const unsigned d2 = (unsigned)(dj * dj) * 0x00010001u;
-                lo = __vminu2(lo, spread_lo(gw) + d2);
-                hi = __vminu2(hi, spread_hi(gw) + d2);
-            }
-            reinterpret_cast<unsigned *>(s_h[hx][y])[w4] = pack_bytes(lo, hi);
+        has_out = __syncthreads_or(any);
+    }
+    if (has_border && has_out) {
+        for (int q = t; q < HX * TY * 4; q += kEdtNT) {
+            const int w8 = q & 3, y = (q >> 2) % TY, hx = (q >> 2) / TY;
+            s_h[(hx * TY + y) * 4 + w8] = y_taps(reinterpret_cast<const uint2 *>(s_g[hx * HY + y + R]) + w8, 4, R);
         }
         __syncthreads();
     }
@@ -451,38 +476,20 @@ __device__ __forceinline__ void edt_tile(const QGrid &g, int w, int jb, int ib, 
     unsigned sgn = 0u;
     if (i < G && j < G) {
         const unsigned iw = s_in[row], ow = s_ot[row];
-        // min over di of di^2 + h (<= 3 R^2 = 243 < 255) for this thread's 8 voxels
-        unsigned bw0 = 0xffffffffu, bw1 = 0xffffffffu;
-        if (has_out) {
-            unsigned l0 = 0xffffffffu, h0 = 0xffffffffu, l1 = 0xffffffffu, h1 = 0xffffffffu;
-            for (int di = -R; di <= R; di++) {
-                const uint2 hw = reinterpret_cast<const uint2 *>(s_h[x + R + di][y])[part];
-                const unsigned d2 = (unsigned)(di * di) * 0x00010001u;
-                l0 = __vminu2(l0, spread_lo(hw.x) + d2);
-                h0 = __vminu2(h0, spread_hi(hw.x) + d2);
-                l1 = __vminu2(l1, spread_lo(hw.y) + d2);
-                h1 = __vminu2(h1, spread_hi(hw.y) + d2);
-            }
-            bw0 = pack_bytes(l0, h0);
-            bw1 = pack_bytes(l1, h1);
-        }
-        unsigned long long packed = 0ull;
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const int b = part * 8 + e;
-            const unsigned bit = 1u << b;
-            unsigned code;
-            if (!(valid & bit)) code = QSES_CODE_OUT;  // row padding, never read
-            else if (ow & bit) code = QSES_CODE_OUT;
-            else if (iw & bit) code = QSES_CODE_IN;
-            else {
-                const unsigned best = ((e < 4 ? bw0 : bw1) >> (8 * (e & 3))) & 0xffu;
-                code = best != 255u ? best : QSES_CODE_NONE;
-            }
-            packed |= (unsigned long long)code << (8 * e);
-            if ((valid & bit) && code != QSES_CODE_OUT && (int)code >= g.negmin) sgn |= bit;
-        }
-        *(unsigned long long *)(codes + ((size_t)i * G + j) * g.Gp + k0 + part * 8) = packed;
+        // this thread's 8 voxels: squared distances where they are neither inside nor outside
+        const unsigned o8 = ((ow | ~valid) >> (8 * part)) & 0xffu, i8 = (iw >> (8 * part)) & 0xffu & ~o8;
+        uint4 v = make_uint4(0x00ff00ffu, 0x00ff00ffu, 0x00ff00ffu, 0x00ff00ffu);
+        if (has_out) v = x_taps(s_h + ((x + R) * TY + y) * 4 + part, 4 * TY, R);
+        const unsigned none = (unsigned)QSES_CODE_NONE * 0x00010001u;  // above every distance, below 255
+        v.x = __vminu2(v.x, none), v.y = __vminu2(v.y, none), v.z = __vminu2(v.z, none), v.w = __vminu2(v.w, none);
+        const unsigned below = (0x8000u - (unsigned)g.negmin) * 0x00010001u;
+        sgn = ((at_least(v.x, v.y, below) | at_least(v.z, v.w, below) << 4 | i8) & ~o8) << (8 * part);
+        auto codes4 = [&](unsigned lo, unsigned hi, unsigned o, unsigned in) {
+            const unsigned om = nibble_bytes(o), im = nibble_bytes(in);  // IN = 254, OUT = 255
+            return (__byte_perm(lo, hi, 0x6420) | om | im) & ~(im & 0x01010101u);
+        };
+        *(uint2 *)(codes + ((size_t)i * G + j) * g.Gp + k0 + part * 8) =
+            make_uint2(codes4(v.x, v.y, o8 & 15u, i8 & 15u), codes4(v.z, v.w, o8 >> 4, i8 >> 4));
     }
     sgn |= __shfl_xor_sync(0xffffffffu, sgn, 1);
     sgn |= __shfl_xor_sync(0xffffffffu, sgn, 2);
@@ -490,45 +497,13 @@ __device__ __forceinline__ void edt_tile(const QGrid &g, int w, int jb, int ib, 
     }
 }
 
-// z pass of the refine, once per voxel: squared distance (in voxels, <= R^2, 255 = none) to
-// the nearest outside voxel along the z row within the R window, one thread per 32-voxel
-// word.  zd has the codes' layout.
-__device__ __forceinline__ void edt_z_word(const QGrid &g, size_t q, const unsigned *__restrict__ outMask,
-                                           unsigned char *__restrict__ zd) {
-    const size_t row = q / g.W;
-    const int w = (int)(q - row * g.W), W = g.W;
-    const size_t base = row * W;
-    const unsigned a = w > 0 ? __ldg(outMask + base + w - 1) : 0u, c = __ldg(outMask + base + w),
-                   d = w + 1 < W ? __ldg(outMask + base + w + 1) : 0u;
-    unsigned out[8];
-    z_word(a, c, d, g.R, out);
-    uint4 *dst = reinterpret_cast<uint4 *>(zd + row * g.Gp + (size_t)w * 32);
-    dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
-    dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
-}
-
-__global__ void __launch_bounds__(256) k_edt_z(QGrid g, const unsigned *__restrict__ outMask,
-                                               unsigned char *__restrict__ zd) {
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < (size_t)g.G * g.G * g.W) edt_z_word(g, q, outMask, zd);
-}
-
-// Batch form: one thread per mask word of every molecule.
-__global__ void __launch_bounds__(256) k_edt_z_batch(QBatch b, unsigned words, const unsigned *__restrict__ outMask,
-                                                     unsigned char *__restrict__ zd) {
-    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= words) return;
-    const unsigned m = qses_find(b.word_off, b.n_mol, q);
-    const QMol &mol = b.mols[m];
-    edt_z_word(mol.g, q - __ldg(b.word_off + m), outMask + mol.mask_off, zd + mol.code_off);
-}
-
+// Four blocks an SM: with five (48 registers, as many as fit) 1738^3 takes 6.1 ms for 4.6, for more
+// of them write their rows of codes at once.
 template <int TX, int TY>
-__global__ void __launch_bounds__(kEdtNT) k_edt(QGrid g, const unsigned *__restrict__ inMask,
+__global__ void __launch_bounds__(kEdtNT, 4) k_edt(QGrid g, const unsigned *__restrict__ inMask,
                                                 const unsigned *__restrict__ outMask,
-                                                unsigned char *__restrict__ codes, unsigned *__restrict__ signMask,
-                                                const unsigned char *__restrict__ zd) {
-    edt_tile<TX, TY>(g, blockIdx.x, blockIdx.y, blockIdx.z, inMask, outMask, codes, signMask, zd);
+                                                unsigned char *__restrict__ codes, unsigned *__restrict__ signMask) {
+    edt_tile<TX, TY>(g, blockIdx.x, blockIdx.y, blockIdx.z, inMask, outMask, codes, signMask);
 }
 
 // ------------------------------------------------------------ batched field
@@ -568,14 +543,13 @@ __global__ void __launch_bounds__(kSasNT) k_sas_batch(QBatch b, const float4 *__
 __global__ void __launch_bounds__(kEdtNT) k_edt_batch(QBatch b, const unsigned *__restrict__ inMask,
                                                       const unsigned *__restrict__ outMask,
                                                       unsigned char *__restrict__ codes,
-                                                      unsigned *__restrict__ signMask, unsigned *counter,
-                                                      const unsigned char *__restrict__ zd) {
+                                                      unsigned *__restrict__ signMask, unsigned *counter) {
     unsigned m;
     int w, jb, ib;
     while (next_tile(b, counter, m, w, jb, ib)) {
         const QMol mol = b.mols[m];
         edt_tile<8, 8>(mol.g, w, jb, ib, inMask + mol.mask_off, outMask + mol.mask_off, codes + mol.code_off,
-                       signMask + mol.mask_off, zd ? zd + mol.code_off : nullptr);
+                       signMask + mol.mask_off);
     }
 }
 
@@ -598,34 +572,26 @@ void launch_sas(const QGrid &g, const float4 *atoms, const uint2 *cells, unsigne
 }
 template <int TX, int TY>
 static void launch_edt_shape(const QGrid &g, const unsigned *inMask, const unsigned *outMask, unsigned char *codes,
-                             unsigned *signMask, cudaStream_t s, const unsigned char *zd) {
+                             unsigned *signMask, cudaStream_t s) {
     static const bool attr = [] {
         return cudaFuncSetAttribute((const void *)k_edt<TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)edt_layout(TX, TY, QSES_RMAX, false).bytes) == cudaSuccess;
+                                    (int)edt_layout(TX, TY, QSES_RMAX).bytes) == cudaSuccess;
     }();
     (void)attr;
-    const size_t smem = edt_layout(TX, TY, g.R, zd != nullptr).bytes;
+    const size_t smem = edt_layout(TX, TY, g.R).bytes;
     dim3 grid(g.W, (g.G + TY - 1) / TY, (g.G + TX - 1) / TX);
-    k_edt<TX, TY><<<grid, kEdtNT, smem, s>>>(g, inMask, outMask, codes, signMask, zd);
+    k_edt<TX, TY><<<grid, kEdtNT, smem, s>>>(g, inMask, outMask, codes, signMask);
 }
 
 void launch_edt(const QGrid &g, const unsigned *inMask, const unsigned *outMask, unsigned char *codes,
-                unsigned *signMask, cudaStream_t s, int shape, unsigned char *zd) {
-    // zd (G G Gp bytes, optional): the z pass once per voxel, then tiles load it.  Without
-    // it each tile computes its halo rows' z distances itself (the allocation-free entry
-    // point); with the bit-parallel z pass that measured the same or slower (0.846 against
-    // 0.836 ms on the 664^3 grid), so the pipeline keeps the separate pass.
-    if (zd) {
-        const size_t words = (size_t)g.G * g.G * g.W;
-        k_edt_z<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(g, outMask, zd);
-    }
-    // shape 0: 8 x 8 rows, 1: 16 x 8, 2: 16 x 16, 3: 32 x 16 (shared memory per CTA at R = 7
-    // with z distances: 21, 29, 45 and 70 KB)
+                unsigned *signMask, cudaStream_t s, int shape) {
+    // shape 0: 8 x 8 rows, 1: 16 x 8, 2: 16 x 16, 3: 32 x 16 (shared memory per CTA at R = 7: 27, 38,
+    // 62 and 95 KB)
     switch (shape) {
-        case 3: launch_edt_shape<32, 16>(g, inMask, outMask, codes, signMask, s, zd); break;
-        case 2: launch_edt_shape<16, 16>(g, inMask, outMask, codes, signMask, s, zd); break;
-        case 1: launch_edt_shape<16, 8>(g, inMask, outMask, codes, signMask, s, zd); break;
-        default: launch_edt_shape<8, 8>(g, inMask, outMask, codes, signMask, s, zd); break;
+        case 3: launch_edt_shape<32, 16>(g, inMask, outMask, codes, signMask, s); break;
+        case 2: launch_edt_shape<16, 16>(g, inMask, outMask, codes, signMask, s); break;
+        case 1: launch_edt_shape<16, 8>(g, inMask, outMask, codes, signMask, s); break;
+        default: launch_edt_shape<8, 8>(g, inMask, outMask, codes, signMask, s); break;
     }
 }
 static unsigned persistent_blocks(const void *fn, int threads, unsigned items, size_t smem = 0) {
@@ -642,12 +608,10 @@ void launch_sas_batch(const QBatch &b, unsigned tiles, const float4 *atoms, cons
         b, atoms, cells, inMask, outMask, counter);
 }
 void launch_edt_batch(const QBatch &b, unsigned tiles, const unsigned *inMask, const unsigned *outMask,
-                      unsigned char *codes, unsigned *signMask, unsigned *counter, cudaStream_t s, unsigned words,
-                      unsigned char *zd) {
-    if (zd) k_edt_z_batch<<<(words + 255) / 256, 256, 0, s>>>(b, words, outMask, zd);
-    const size_t smem = edt_layout(8, 8, QSES_RMAX, false).bytes;  // molecules of any window
+                      unsigned char *codes, unsigned *signMask, unsigned *counter, cudaStream_t s) {
+    const size_t smem = edt_layout(8, 8, QSES_RMAX).bytes;  // molecules of any window
     k_edt_batch<<<persistent_blocks((const void *)k_edt_batch, kEdtNT, tiles, smem), kEdtNT, smem, s>>>(
-        b, inMask, outMask, codes, signMask, counter, zd);
+        b, inMask, outMask, codes, signMask, counter);
 }
 
 }  // namespace qses

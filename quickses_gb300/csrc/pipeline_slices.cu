@@ -123,7 +123,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
     const int atom_bits = bits_for(ncell ? ncell - 1 : 0);
     const size_t tmpA = std::max(radix_sort_tmp_bytes(n, atom_bits), scan_u2_tmp_bytes((unsigned)nrow));
     const size_t needA = a256(4ull * n) * 4 + a256(16ull * n) + a256(8 * ncell) + 3 * a256(4 * nmask) +
-                         2 * a256(ncode) + a256(1024) + a256(8 * nrow) + a256(64) + a256(tmpA) + 4096;
+                         a256(ncode) + a256(1024) + a256(8 * nrow) + a256(64) + a256(tmpA) + 4096;
     if (ctx->field.reserve(needA) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "field workspace");
     Arena &A = ctx->field;
     unsigned *key = (unsigned *)A.take(4ull * n), *key2 = (unsigned *)A.take(4ull * n);
@@ -132,7 +132,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
     uint2 *cells = (uint2 *)A.take(8 * ncell);
     unsigned *in_mask = (unsigned *)A.take(4 * nmask), *out_mask = (unsigned *)A.take(4 * nmask);
     unsigned *sign_mask = (unsigned *)A.take(4 * nmask);
-    unsigned char *codes = (unsigned char *)A.take(ncode), *zd = (unsigned char *)A.take(ncode);
+    unsigned char *codes = (unsigned char *)A.take(ncode);
     float *lut = (float *)A.take(1024);
     uint2 *rows = (uint2 *)A.take(8 * nrow);
     uint2 *tot = (uint2 *)A.take(64);
@@ -184,7 +184,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 SCHK(cudaMemsetAsync(d_border, 0, 8, s));
                 launch_sas(b, atoms, cells, in_mask, out_mask, s);
                 k_border_count<<<blocks(nmask, 256 * 8), 256, 0, s>>>(in_mask, out_mask, nmask, W, D, d_border);
-                launch_edt(b, in_mask, out_mask, codes, sign_mask, s, edt, zd);
+                launch_edt(b, in_mask, out_mask, codes, sign_mask, s, edt);
                 ctx->launches += 4;
                 uint2 *h_tot = (uint2 *)ctx->h_small;
                 if (cells_any) {
