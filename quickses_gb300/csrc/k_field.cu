@@ -280,7 +280,7 @@ constexpr int kEdtNT = 256;
 // output rows) at the cost of shared memory (dynamic, edt_layout); the shape is chosen
 // by the autotuner.
 //
-// Bound by instruction issue where there is a border, by the codes' bytes elsewhere.  664^3 (R = 6)
+// Bound by instruction issue where there is a border, by the codes' bytes elsewhere.  664^3 (R = 7)
 // 0.61 ms, 1738^3 (R = 3, most tiles without a border) 4.6.  With the z distances of all voxels in
 // memory, written and read back with the halo, 0.67 and 7.6; with byte rows spread at each tap, taps
 // one by one and codes voxel by voxel 0.83 and 7.6.

@@ -696,38 +696,61 @@ __global__ void __launch_bounds__(128) k_gs_lists(const unsigned *__restrict__ t
 }
 
 // The vertices of more than 8 corners: a warp each, a corner per lane, sorted by counting the
-// smaller ones; their lists go to the neighbour table at twice the vertex's offset.
+// smaller ones; a hash table finds the entries that name a vertex again; their lists go to the
+// neighbour table at twice the vertex's offset.  At 0.2 A, where the surface runs through grid
+// points, a tenth of the vertices have 9 to 27 corners: 370 000 of 3 700 000 in 0.225 ms (each entry
+// compared with all before it: 0.286).
 __global__ void __launch_bounds__(256) k_gs_lists_long(const unsigned *__restrict__ tri, unsigned *__restrict__ occ,
                                                        const uint2 *__restrict__ start, unsigned *__restrict__ nbr,
                                                        unsigned v0, unsigned v1, const unsigned *__restrict__ table,
                                                        unsigned *__restrict__ word0, unsigned char *__restrict__ ext,
                                                        unsigned char *__restrict__ ext0, GsOrder ord,
                                                        const unsigned *__restrict__ longs, int *err) {
-    __shared__ unsigned s_id[8][64];
+    __shared__ unsigned s_q[8][32], s_id[8][64];
+    __shared__ uint2 s_seen[8][128];  // hash table: an id, the first entry that has it
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, count = *ord.longs;
-    unsigned *row = s_id[warp];
+    unsigned *row = s_id[warp], *sq = s_q[warp];
+    uint2 *seen = s_seen[warp];
     for (unsigned x = blockIdx.x * 8 + warp; x < count; x += gridDim.x * 8) {
         const unsigned v = longs[x], o0 = start[v].x, m = start[v + 1].x - o0;
         GsVertex g{0, 0, v0, v1, 0, 0, 0};
         const unsigned lo = g.slab(table, v);
         unsigned *list = nbr + 2 * (size_t)o0;
         if (m <= 32) {
+#pragma unroll
+            for (unsigned k = 0; k < 4; k++) seen[lane + 32 * k] = make_uint2(0xffffffffu, 0xffffffffu);
             const unsigned q = lane < m ? occ[o0 + lane] : 0xffffffffu;
+            sq[lane] = q;
+            __syncwarp();
             unsigned rank = 0;
-            for (unsigned j = 0; j < m; j++) rank += __shfl_sync(0xffffffffu, q, j) < q;
+            for (unsigned j = 0; j < m; j++) rank += sq[j] < q;
             if (lane < m) {
                 const uint2 e = gs_corners(tri, q);
                 row[2 * rank] = e.x;
                 row[2 * rank + 1] = e.y;
             }
             __syncwarp();
-            for (unsigned e = lane; e < 2 * m; e += 32) {
-                const unsigned u = row[e];
-                bool again = false;
-                for (unsigned j = 0; j < e; j++) again |= row[j] == u;
-                list[e] = g.take(v, u, again);
+            unsigned u[2], at[2];
+#pragma unroll
+            for (unsigned k = 0; k < 2; k++) {
+                const unsigned e = lane + 32 * k;
+                u[k] = e < 2 * m ? row[e] : 0u;
+                at[k] = (u[k] * 2654435761u) >> 25;
+                if (e >= 2 * m) continue;
+                for (;;) {  // at most 64 ids: there is a free slot
+                    const unsigned was = atomicCAS(&seen[at[k]].x, 0xffffffffu, u[k]);
+                    if (was == 0xffffffffu || was == u[k]) break;
+                    at[k] = (at[k] + 1u) & 127u;
+                }
+                atomicMin(&seen[at[k]].y, e);
             }
-            __syncwarp();  // the row is rewritten for the next vertex
+            __syncwarp();
+#pragma unroll
+            for (unsigned k = 0; k < 2; k++) {
+                const unsigned e = lane + 32 * k;
+                if (e < 2 * m) list[e] = g.take(v, u[k], seen[at[k]].y < e);
+            }
+            __syncwarp();  // the rows are rewritten for the next vertex
             g.loc = __reduce_add_sync(0xffffffffu, g.loc);
             g.rem = __reduce_add_sync(0xffffffffu, g.rem);
             g.far = __reduce_max_sync(0xffffffffu, g.far);
