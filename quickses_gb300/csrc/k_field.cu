@@ -14,6 +14,7 @@
 // with no outside voxel in its window (-dx), 254 = inside (-dx), 255 = outside (probe).
 #include "device_common.cuh"
 #include "kernels.h"
+#include "prims.h"
 
 namespace qses {
 
@@ -64,6 +65,27 @@ __global__ void k_atom_gather(const float *__restrict__ xyz, const float *__rest
     unsigned k = skey[s];
     if (s == 0 || skey[s - 1] != k) cells[k].x = s;
     if (s == n - 1 || skey[s + 1] != k) cells[k].y = s + 1;
+}
+
+cudaError_t order_atoms(const QGrid &g, const float *xyz, const float *r, unsigned n, unsigned *key, unsigned *key2,
+                        unsigned *idx, unsigned *idx2, int bits, float4 *atoms, uint2 *cells, size_t ncell, void *tmp,
+                        int *err, cudaStream_t s, int *launches, int *alt) {
+    *alt = 0;
+    cudaError_t e = cudaMemsetAsync(cells, 0, 8 * ncell, s);
+    if (e != cudaSuccess) return e;
+    // in one launch while its n^2 comparisons are cheaper than the launches it saves, and a key and an
+    // atom's number fit 32 bits
+    if (n <= kFewAtoms && ncell < 0xffffffffull / kFewAtoms) {
+        launch_atoms_few(g, xyz, r, n, key, idx, atoms, cells, s);
+        if (launches) (*launches)++;
+        return cudaGetLastError();
+    }
+    launch_atom_hash(g, xyz, n, key, s);
+    e = radix_sort(key, key2, idx, idx2, n, bits, true, tmp, err, s, launches, alt);
+    if (e != cudaSuccess) return e;
+    launch_atom_gather(xyz, r, *alt ? key2 : key, *alt ? idx2 : idx, n, atoms, cells, s);
+    if (launches) *launches += 2;
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ SAS

@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kRsT) k_rs_pass(const unsigned *__restrict__ k
 size_t radix_sort_tmp_bytes(unsigned n, int bits) {
     int npass = (bits + 7) / 8;
     size_t tiles = (n + kRsT * kRsI - 1) / (kRsT * kRsI);
-    return 256 + (size_t)npass * 256 * sizeof(unsigned) + tiles * 256 * sizeof(unsigned long long);
+    return 256 + (size_t)(npass > 0 ? npass : 1) * 256 * (sizeof(unsigned) + tiles * sizeof(unsigned long long));
 }
 
 cudaError_t radix_sort(unsigned *keys, unsigned *keys_alt, unsigned *vals, unsigned *vals_alt, unsigned n, int bits,
@@ -231,7 +231,7 @@ cudaError_t radix_sort(unsigned *keys, unsigned *keys_alt, unsigned *vals, unsig
     unsigned *ticket = (unsigned *)tmp;
     unsigned *hist = (unsigned *)((char *)tmp + 256);
     unsigned long long *status = (unsigned long long *)((char *)hist + (size_t)npass * 256 * sizeof(unsigned));
-    cudaError_t e = cudaMemsetAsync(hist, 0, (size_t)npass * 256 * sizeof(unsigned), s);
+    cudaError_t e = cudaMemsetAsync(tmp, 0, radix_sort_tmp_bytes(n, bits), s);  // every pass's at once
     if (e != cudaSuccess) return e;
     unsigned hblocks = (n + 255) / 256;
     if (hblocks > 1216) hblocks = 1216;
@@ -242,10 +242,8 @@ cudaError_t radix_sort(unsigned *keys, unsigned *keys_alt, unsigned *vals, unsig
     unsigned *dst = keys_alt, *other = keys;  // passes after the first ping-pong between keys_alt and keys
     unsigned *vsrc = identity ? nullptr : vals, *vdst = vals_alt;
     for (int p = 0; p < npass; p++) {
-        e = cudaMemsetAsync(ticket, 0, 256, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, (size_t)tiles * 256 * sizeof(unsigned long long), s);
-        if (e != cudaSuccess) return e;
-        k_rs_pass<<<tiles, kRsT, 0, s>>>(src, dst, vsrc, vdst, n, 8 * p, hist + p * 256, status, ticket, d_err);
+        k_rs_pass<<<tiles, kRsT, 0, s>>>(src, dst, vsrc, vdst, n, 8 * p, hist + p * 256,
+                                         status + (size_t)p * tiles * 256, ticket + p, d_err);
         if (launches) (*launches)++;
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

@@ -8,6 +8,14 @@
 namespace qses {
 
 void launch_atom_minmax(const float *xyz, const float *r, unsigned n, unsigned *mm, cudaStream_t s);
+constexpr unsigned kFewAtoms = 8192;  // that are ordered in one launch
+void launch_atoms_few(const QGrid &g, const float *xyz, const float *r, unsigned n, unsigned *skey, unsigned *sidx,
+                      float4 *atoms, uint2 *cells, cudaStream_t s);
+// Atoms and their input numbers in cell order (stable) and the cells' ranges; the sorted keys and
+// numbers end up in (key, idx) or, with *alt, in (key2, idx2).
+cudaError_t order_atoms(const QGrid &g, const float *xyz, const float *r, unsigned n, unsigned *key, unsigned *key2,
+                        unsigned *idx, unsigned *idx2, int bits, float4 *atoms, uint2 *cells, size_t ncell, void *tmp,
+                        int *err, cudaStream_t s, int *launches, int *alt);
 void launch_atom_hash(const QGrid &g, const float *xyz, unsigned n, unsigned *key, cudaStream_t s);
 void launch_atom_gather(const float *xyz, const float *r, const unsigned *skey, const unsigned *sidx, unsigned n,
                         float4 *atoms, uint2 *cells, cudaStream_t s);

@@ -152,13 +152,10 @@ extern "C" QSES_API int qses_field_codes_noalloc(const float *d_xyz, const float
     const int atom_bits = bits_for(ncell - 1);
     if (radix_sort_tmp_bytes(n, atom_bits) > kTmpBytes) return QSES_ERR_INTERNAL;
 
-    launch_atom_hash(g, d_xyz, n, key, s);
     int alt = 0;
-    if (radix_sort(key, key2, idx, idx2, n, atom_bits, true, tmp, d_err, s, nullptr, &alt) != cudaSuccess)
+    if (order_atoms(g, d_xyz, d_radii, n, key, key2, idx, idx2, atom_bits, atoms, cells, ncell, tmp, d_err, s, nullptr,
+                    &alt) != cudaSuccess)
         return fail(QSES_ERR_CUDA);
-    const unsigned *skey = alt ? key2 : key, *sidx = alt ? idx2 : idx;
-    if (cudaMemsetAsync(cells, 0, 8 * ncell, s) != cudaSuccess) return fail(QSES_ERR_CUDA);
-    launch_atom_gather(d_xyz, d_radii, skey, sidx, n, atoms, cells, s);
     launch_sas(g, atoms, cells, inMask, outMask, s);
     launch_edt(g, inMask, outMask, codes, signMask, s);
     // Padded rows (32-voxel words) in the scratch -> tight G*G*G rows for the caller.

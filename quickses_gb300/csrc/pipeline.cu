@@ -518,20 +518,13 @@ struct FieldSeg {
 static int enqueue_field(qses_context *ctx, const FieldSeg &a, SegOut &o) {
     cudaStream_t s = ctx->stream;
     QCHK(cudaMemcpyAsync(a.lut, a.h_lut, 1024, cudaMemcpyHostToDevice, s));
-    launch_atom_hash(a.g, a.xyz, a.n, a.key, s);
-    ctx->launches++;
-    QCHK(radix_sort(a.key, a.key2, a.idx, a.idx2, a.n, a.atom_bits, true, a.tmp, a.err, s, &ctx->launches,
-                              &o.alt));
-    const unsigned *skey = o.alt ? a.key2 : a.key, *sidx = o.alt ? a.idx2 : a.idx;
-    QCHK(cudaMemsetAsync(a.cells, 0, 8 * a.ncell, s));
-    launch_atom_gather(a.xyz, a.r, skey, sidx, a.n, a.atoms, a.cells, s);
-    ctx->launches++;
+    QCHK(order_atoms(a.g, a.xyz, a.r, a.n, a.key, a.key2, a.idx, a.idx2, a.atom_bits, a.atoms, a.cells, a.ncell, a.tmp,
+                     a.err, s, &ctx->launches, &o.alt));
     ctx->mark("atoms");
     launch_sas(a.g, a.atoms, a.cells, a.in_mask, a.out_mask, s);
     ctx->launches++;
     ctx->mark("sas");
     launch_edt(a.g, a.in_mask, a.out_mask, a.codes, a.sign_mask, s, a.edt);
-    ctx->launches++;
     ctx->launches++;
     ctx->mark("refine");
     launch_mc_count(a.g, a.sign_mask, a.rows, a.in_mask, s);  // the atoms' masks are done with

@@ -106,7 +106,7 @@ static int enqueue_batch_field(qses_context *ctx, const BatchFieldSeg &a, SegOut
     ctx->launches++;
     ctx->mark("sas");
     launch_edt_batch(a.b, a.tiles, a.in_mask, a.out_mask, a.codes, a.sign_mask, a.counters + 1, s);
-    ctx->launches += 2;
+    ctx->launches++;
     ctx->mark("refine");
     // marching-cubes counts, one scan over all rows, per-molecule offsets
     launch_mc_count_batch(a.b, a.units, a.sign_mask, a.rows, a.in_mask, s);  // the atoms' masks are done with

@@ -140,14 +140,10 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
     if (!tmp) return ctx->fail(QSES_ERR_INTERNAL, "field workspace layout");
 
     // ---- atoms into the molecule's neighbour cells, once for every slice
-    launch_atom_hash(g, d_xyz, n, key, s);
-    ctx->launches++;
     int alt = 0;
-    SCHK(radix_sort(key, key2, idx, idx2, n, atom_bits, true, tmp, d_err, s, &ctx->launches, &alt));
-    const unsigned *skey = alt ? key2 : key, *sidx = alt ? idx2 : idx;
-    SCHK(cudaMemsetAsync(cells, 0, 8 * ncell, s));
-    launch_atom_gather(d_xyz, d_r, skey, sidx, n, atoms, cells, s);
-    ctx->launches++;
+    SCHK(order_atoms(g, d_xyz, d_r, n, key, key2, idx, idx2, atom_bits, atoms, cells, ncell, tmp, d_err, s, &ctx->launches,
+                     &alt));
+    const unsigned *sidx = alt ? idx2 : idx;
     fill_lut(g, (float *)(ctx->h_small + 64));
     SCHK(cudaMemcpyAsync(lut, ctx->h_small + 64, 1024, cudaMemcpyHostToDevice, s));
     SCHK(cudaStreamSynchronize(s));  // the pinned table is rewritten below
@@ -185,7 +181,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 launch_sas(b, atoms, cells, in_mask, out_mask, s);
                 k_border_count<<<blocks(nmask, 256 * 8), 256, 0, s>>>(in_mask, out_mask, nmask, W, D, d_border);
                 launch_edt(b, in_mask, out_mask, codes, sign_mask, s, edt);
-                ctx->launches += 4;
+                ctx->launches += 3;
                 uint2 *h_tot = (uint2 *)ctx->h_small;
                 if (cells_any) {
                     const size_t E = (size_t)b.Gc + 1;
