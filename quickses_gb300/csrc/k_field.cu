@@ -26,7 +26,7 @@ __device__ __forceinline__ unsigned enc_f(float f) {
 }
 
 __global__ void k_atom_minmax(const float *__restrict__ xyz, const float *__restrict__ r, unsigned n,
-                              unsigned *mm /* 7: min xyz, max xyz, max r (order-preserving encodings) */) {
+                              unsigned *mm /* 7, zeroed: complements of min xyz; max xyz, max r (order-preserving encodings) */) {
     unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[4] = {0u, 0u, 0u, 0u};
     for (size_t a = (size_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (size_t)gridDim.x * blockDim.x) {
 #pragma unroll
@@ -48,7 +48,7 @@ __global__ void k_atom_minmax(const float *__restrict__ xyz, const float *__rest
     }
     if ((threadIdx.x & 31) == 0) {
         for (int c = 0; c < 3; c++) {
-            atomicMin(&mm[c], lo[c]);
+            atomicMax(&mm[c], ~lo[c]);
             atomicMax(&mm[3 + c], hi[c]);
         }
         atomicMax(&mm[6], hi[3]);

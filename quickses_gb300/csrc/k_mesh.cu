@@ -767,9 +767,12 @@ __global__ void __launch_bounds__(kFiltT) k_tri_filter(QBatch b, const unsigned 
 // corners (start[v].x, later scanned); scatter: each corner q is written into its vertex's
 // range at a position taken with an atomic (start[v].y, zero after the scan), so the order
 // within a range is arbitrary (k_gs_lists sorts it).
-__global__ void k_csr_count(const unsigned *__restrict__ tri, size_t n3, uint2 *__restrict__ start) {
+// The count also clears the smoothing's counters, for the kernels after it.
+__global__ void k_csr_count(const unsigned *__restrict__ tri, size_t n3, uint2 *__restrict__ start,
+                            unsigned *__restrict__ zero, unsigned nzero) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n3) atomicAdd(&start[tri[q]].x, 1u);
+    for (size_t z = q; z < nzero; z += (size_t)gridDim.x * blockDim.x) zero[z] = 0u;
 }
 
 __global__ void k_csr_scatter(const unsigned *__restrict__ tri, size_t n3, uint2 *__restrict__ start,
@@ -782,10 +785,6 @@ __global__ void k_csr_scatter(const unsigned *__restrict__ tri, size_t n3, uint2
     occ[(unsigned)old + (unsigned)(old >> 32)] = (unsigned)q;
 }
 
-__global__ void k_to_float4(const float *__restrict__ v3, unsigned nv, float4 *__restrict__ v4) {
-    unsigned v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < nv) v4[v] = make_float4(v3[3ull * v], v3[3ull * v + 1], v3[3ull * v + 2], 0.0f);
-}
 __global__ void k_from_float4(const float4 *__restrict__ v4, unsigned nv, float *__restrict__ v3) {
     unsigned v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < nv) {
@@ -910,14 +909,11 @@ cudaError_t launch_tri_filter_batch(const QBatch &b, const unsigned *tri, unsign
                                     uint2 *total, void *tmp, int *err, cudaStream_t s) {
     return filter_with<true>(b, tri, nt, out, kept_off, total, tmp, err, s);
 }
-void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, cudaStream_t s) {
-    k_csr_count<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, start);
+void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, unsigned *zero, unsigned nzero, cudaStream_t s) {
+    k_csr_count<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, start, zero, nzero);
 }
 void launch_csr_scatter(const unsigned *tri, size_t n3, uint2 *start, unsigned *occ, cudaStream_t s) {
     k_csr_scatter<<<nblk(n3, 256), 256, 0, s>>>(tri, n3, start, occ);
-}
-void launch_to_float4(const float *v3, unsigned nv, float4 *v4, cudaStream_t s) {
-    k_to_float4<<<nblk(nv, 256), 256, 0, s>>>(v3, nv, v4);
 }
 void launch_from_float4(const float4 *v4, unsigned nv, float *v3, cudaStream_t s) {
     k_from_float4<<<nblk(nv, 256), 256, 0, s>>>(v4, nv, v3);

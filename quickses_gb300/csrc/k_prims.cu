@@ -81,7 +81,7 @@ size_t scan_u2_tmp_bytes(unsigned n) {
 }
 
 cudaError_t scan_u2(const uint2 *in, uint2 *out, unsigned n, uint2 *d_total, void *tmp, int *d_err,
-                    cudaStream_t s, int *launches) {
+                    cudaStream_t s, int *launches, bool cleared) {
     unsigned tiles = (n + kScanTile - 1) / kScanTile;
     if (tiles == 0) {
         if (d_total) return cudaMemsetAsync(d_total, 0, sizeof(uint2), s);
@@ -89,8 +89,10 @@ cudaError_t scan_u2(const uint2 *in, uint2 *out, unsigned n, uint2 *d_total, voi
     }
     unsigned *ticket = (unsigned *)tmp;
     unsigned long long *status = (unsigned long long *)((char *)tmp + 256);
-    cudaError_t e = cudaMemsetAsync(tmp, 0, scan_u2_tmp_bytes(n), s);
-    if (e != cudaSuccess) return e;
+    if (!cleared) {
+        const cudaError_t e = cudaMemsetAsync(tmp, 0, scan_u2_tmp_bytes(n), s);
+        if (e != cudaSuccess) return e;
+    }
     k_scan_u2<<<tiles, kScanT, 0, s>>>(in, out, n, status, ticket, d_total, d_err);
     if (launches) (*launches)++;
     return cudaGetLastError();

@@ -647,7 +647,8 @@ __device__ __forceinline__ uint2 gs_corners(const unsigned *__restrict__ tri, un
 // A thread per vertex; vertices of more than 8 corners are left to k_gs_lists_long, as a few of
 // them among a warp's 32 hold up all (3 540 000 vertices, 10 % of them long: the whole list stage
 // 1.19 ms with one kernel, 0.83 with two).
-__global__ void __launch_bounds__(128) k_gs_lists(const unsigned *__restrict__ tri, const unsigned *__restrict__ occ,
+__global__ void __launch_bounds__(128) k_gs_lists(const float *__restrict__ vq, float4 *__restrict__ pos,
+                                                  const unsigned *__restrict__ tri, const unsigned *__restrict__ occ,
                                                   const uint2 *__restrict__ start, unsigned v0, unsigned v1,
                                                   unsigned smax, const unsigned *__restrict__ table,
                                                   unsigned *__restrict__ word0, uint4 *__restrict__ pack,
@@ -656,6 +657,7 @@ __global__ void __launch_bounds__(128) k_gs_lists(const unsigned *__restrict__ t
     const unsigned v = v0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= v1) return;
     const unsigned o0 = start[v].x, m = start[v + 1].x - o0;  // corners
+    pos[v] = make_float4(vq[3ull * v], vq[3ull * v + 1], vq[3ull * v + 2], 0.0f);
     if (m > 8) {
         longs[atomicAdd(ord.longs, 1u)] = v;
         return;
@@ -813,10 +815,10 @@ __global__ void __launch_bounds__(1024) k_gs_order(const unsigned *__restrict__ 
 
 // ------------------------------------------------------------ launchers
 
-void launch_gs_lists(const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
+void launch_gs_lists(const float *vq, float4 *pos, const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
                      unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext,
                      unsigned char *ext0, const GsOrder &ord, unsigned *longs, int *err, cudaStream_t s) {
-    k_gs_lists<<<(v1 - v0 + 127) / 128, 128, 0, s>>>(tri, occ, start, v0, v1, smax, table, word0, pack, ext, ext0, ord, longs,
+    k_gs_lists<<<(v1 - v0 + 127) / 128, 128, 0, s>>>(vq, pos, tri, occ, start, v0, v1, smax, table, word0, pack, ext, ext0, ord, longs,
                                                      err);
     // as many CTAs as fit the SMs, or as there can be vertices for
     const unsigned ctas = (v1 - v0 + 63) / 64;

@@ -46,7 +46,7 @@ cudaError_t launch_tri_filter(const unsigned *tri, unsigned nt, unsigned *out, u
                               cudaStream_t s);
 // Neighbour lists by counting: start (nv + 1 entries, zeroed) -> counts -> (scan) -> corner
 // occurrences scattered per vertex into occ (n3), in any order.
-void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, cudaStream_t s);
+void launch_csr_count(const unsigned *tri, size_t n3, uint2 *start, unsigned *zero, unsigned nzero, cudaStream_t s);
 void launch_csr_scatter(const unsigned *tri, size_t n3, uint2 *start, unsigned *occ, cudaStream_t s);
 // Slab table of one Gauss-Seidel wave (device words): [0] Q slabs, [1, Q + 2) their bounds in
 // id order (qcap + 1 slots), [qcap + 2, qcap + 2 + Q) the slab ids in the order CTAs take them.
@@ -60,12 +60,11 @@ struct GsOrder {
 // The pass's lists from the occurrences: word0, pack (64 B) per vertex, lists of more than 16
 // entries in nbr (2 n3) at twice the vertex's offset (k_smooth.cu); ext, ext0 (may be null): one
 // byte per vertex, the neighbours in lower slabs still to come; longs: scratch, one per vertex.
-void launch_gs_lists(const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
+void launch_gs_lists(const float *vq, float4 *pos, const unsigned *tri, unsigned *occ, const uint2 *start, unsigned *nbr, unsigned v0, unsigned v1,
                      unsigned smax, const unsigned *table, unsigned *word0, uint4 *pack, unsigned char *ext,
                      unsigned char *ext0, const GsOrder &ord, unsigned *longs, int *err, cudaStream_t s);
 void launch_gs_order(const unsigned *table, unsigned qcap, const GsOrder &ord, cudaStream_t s);
 size_t gs_slab_smem(unsigned S);
-void launch_to_float4(const float *v3, unsigned nv, float4 *v4, cudaStream_t s);
 void launch_from_float4(const float4 *v4, unsigned nv, float *v3, cudaStream_t s);
 // Gauss-Seidel passes over vertices [v0, nv) in the table's slabs (each at most smax
 // vertices), taken by P persistent CTAs from *next_slab (zeroed).  passes > 1: that many passes,

@@ -115,9 +115,7 @@ extern "C" QSES_API int qses_field_codes_noalloc(const float *d_xyz, const float
     // Bounds and grid sizing, exactly as the allocating path computes them.
     unsigned *d_mm = (unsigned *)base;
     int *d_err = (int *)(base + kOffErr);
-    if (cudaMemsetAsync(d_mm, 0xff, 3 * sizeof(unsigned), s) != cudaSuccess ||
-        cudaMemsetAsync(d_mm + 3, 0, 5 * sizeof(unsigned), s) != cudaSuccess ||
-        cudaMemsetAsync(d_err, 0, sizeof(int), s) != cudaSuccess)
+    if (cudaMemsetAsync(base, 0, kOffErr + sizeof(int), s) != cudaSuccess)
         return fail(QSES_ERR_CUDA);
     launch_atom_minmax(d_xyz, d_radii, n, d_mm, s);
     if (cudaMemcpyAsync(g_na_bounds, d_mm, sizeof(g_na_bounds), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -130,7 +128,7 @@ extern "C" QSES_API int qses_field_codes_noalloc(const float *d_xyz, const float
         memcpy(&f, &b, 4);
         return f;
     };
-    const float mn[3] = {dec(g_na_bounds[0]), dec(g_na_bounds[1]), dec(g_na_bounds[2])};
+    const float mn[3] = {dec(~g_na_bounds[0]), dec(~g_na_bounds[1]), dec(~g_na_bounds[2])};
     const float mx[3] = {dec(g_na_bounds[3]), dec(g_na_bounds[4]), dec(g_na_bounds[5])};
     QGrid g;
     int rc = grid_from_bounds(mn, mx, dec(g_na_bounds[6]), n, voxel, g, nullptr, nullptr);

@@ -408,6 +408,7 @@ static bool take_weld(Arena &a, unsigned ne, unsigned layers, WeldBuffers &w) {
     return (w.tmp = a.take(weld_tmp_bytes(layers))) != nullptr;
 }
 static bool take_smooth(Arena &a, unsigned ne, size_t n3, SmoothBuffers &sb) {
+    sb.tmp = a.take(scan_u2_tmp_bytes(ne + 1));  // cleared together with deg, which follows
     sb.deg = (uint2 *)a.take(8ull * (ne + 2));
     sb.occ = (unsigned *)a.take(4 * n3 + 4);
     sb.nbr = (unsigned *)a.take(8 * n3 + 8);
@@ -415,8 +416,7 @@ static bool take_smooth(Arena &a, unsigned ne, size_t n3, SmoothBuffers &sb) {
     sb.pack = (uint4 *)a.take(64ull * ne + 64);
     sb.ext = (unsigned *)a.take(1ull * ne + 64);
     sb.ext0 = (unsigned *)a.take(1ull * ne + 64);
-    sb.pos4 = (float4 *)a.take(16ull * ne + 16);
-    return (sb.tmp = a.take(scan_u2_tmp_bytes(ne + 1))) != nullptr;
+    return (sb.pos4 = (float4 *)a.take(16ull * ne + 16)) != nullptr;
 }
 size_t weld_or_smooth_bytes(unsigned ne, unsigned layers, size_t n3, bool smooth) {
     WeldBuffers w;
@@ -448,24 +448,21 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
     cudaStream_t s = ctx->stream;
     float4 *pos4 = sb.pos4;
     // neighbour lists: count the corners per vertex, scan, scatter them per vertex
-    QCHK(cudaMemsetAsync(sb.deg, 0, 8ull * (nv + 1), s));
-    launch_csr_count(tri, n3, sb.deg, s);
+    QCHK(cudaMemsetAsync(sb.tmp, 0, (size_t)((char *)(sb.deg + nv + 1) - (char *)sb.tmp), s));
+    launch_csr_count(tri, n3, sb.deg, gb.next_slab, (unsigned)gb.zero_words, s);
     ctx->launches++;
-    QCHK(scan_u2(sb.deg, sb.deg, nv + 1, nullptr, sb.tmp, d_err, s, &ctx->launches));
+    QCHK(scan_u2(sb.deg, sb.deg, nv + 1, nullptr, sb.tmp, d_err, s, &ctx->launches, true));
     launch_csr_scatter(tri, n3, sb.deg, sb.occ, s);
     ctx->launches++;
-    launch_to_float4(vq, nv, pos4, s);
-    ctx->launches++;
     if (sh.flags & kGsPersistL2) gs_l2_window(ctx->device, s, pos4, 16ull * nv);
-    if (stats) QCHK(cudaMemsetAsync(stats, 0, 64, s));
+    if (stats && ctx->profiling) QCHK(cudaMemsetAsync(stats, 0, 64, s));
     QCHK(cudaMemcpyAsync(gb.table, h_table, 4ull * L.waves * L.table_words, cudaMemcpyHostToDevice, s));
     // several passes over one wave run in one launch, each following the one before through the slabs
     const bool together = L.waves == 1;
-    QCHK(cudaMemsetAsync(gb.next_slab, 0, 4 * gb.zero_words, s));
     for (unsigned w = 0; w < L.waves; w++) {
         const unsigned v0 = w * L.wsize, v1 = std::min(nv, v0 + L.wsize);
         if (w) QCHK(cudaMemsetAsync(gb.ord.longs, 0, 4, s));
-        launch_gs_lists(tri, sb.occ, sb.deg, sb.nbr, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, sb.word0,
+        launch_gs_lists(vq, pos4, tri, sb.occ, sb.deg, sb.nbr, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, sb.word0,
                         sb.pack, (unsigned char *)sb.ext, passes > 1 ? (unsigned char *)sb.ext0 : nullptr, gb.ord, scratch,
                         d_err, s);
         ctx->launches += 2;
@@ -654,10 +651,7 @@ int molecule_grid(qses_context *ctx, const qses_params &p, const float *d_xyz, c
     cudaStream_t s = ctx->stream;
     ctx->oversize = false;
     unsigned *d_mm = (unsigned *)ctx->small;
-    int *d_err = (int *)((char *)ctx->small + 64);
-    QCHK(cudaMemsetAsync(d_mm, 0xff, 3 * sizeof(unsigned), s));  // min encodings start high
-    QCHK(cudaMemsetAsync(d_mm + 3, 0, 5 * sizeof(unsigned), s));  // max encodings start low
-    QCHK(cudaMemsetAsync(d_err, 0, sizeof(int), s));
+    QCHK(cudaMemsetAsync(ctx->small, 0, 320, s));  // the bounds, the error word (at 64) and the smoothing's statistics (256)
     launch_atom_minmax(d_xyz, d_r, n, d_mm, s);
     ctx->launches++;
     QCHK(cudaGetLastError());
@@ -670,7 +664,7 @@ int molecule_grid(qses_context *ctx, const qses_params &p, const float *d_xyz, c
         memcpy(&f, &b, 4);
         return f;
     };
-    float mn[3] = {dec(h_mm[0]), dec(h_mm[1]), dec(h_mm[2])}, mx[3] = {dec(h_mm[3]), dec(h_mm[4]), dec(h_mm[5])};
+    float mn[3] = {dec(~h_mm[0]), dec(~h_mm[1]), dec(~h_mm[2])}, mx[3] = {dec(h_mm[3]), dec(h_mm[4]), dec(h_mm[5])};
     float maxR = dec(h_mm[6]);
     std::string why;
     int rc = grid_from_bounds(mn, mx, maxR, n, p.voxel, g, &ctx->info, &why, sliced);
@@ -698,7 +692,6 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     ctx->slice_nv.clear();
     ctx->slice_nt.clear();
     memset(ctx->diag, 0, sizeof(ctx->diag));
-    QCHK(cudaMemsetAsync((char *)ctx->small + 256, 0, 64, ctx->stream));
     ctx->mark("start");
 
     // ---- bounds (one read-back) and sizing on the host

@@ -107,7 +107,6 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
     ctx->slice_nv.clear();
     ctx->slice_nt.clear();
     if (p.slice < 1) return ctx->fail(QSES_ERR_INVALID_ARG, "slice must be >= 1");
-    SCHK(cudaMemsetAsync((char *)ctx->small + 256, 0, 64, s));
     QGrid g;
     const int grc = molecule_grid(ctx, p, d_xyz, d_r, n, g, true);
     if (grc != QSES_OK) return grc;

@@ -7,9 +7,10 @@
 namespace qses {
 
 // Exclusive scan of n uint2 values (in place allowed).  *d_total (device) receives the sum.
+// cleared: tmp is zero already.
 size_t scan_u2_tmp_bytes(unsigned n);
 cudaError_t scan_u2(const uint2 *in, uint2 *out, unsigned n, uint2 *d_total, void *tmp, int *d_err,
-                    cudaStream_t s, int *launches);
+                    cudaStream_t s, int *launches, bool cleared = false);
 
 // Stable LSD radix sort of (32-bit key, value) pairs on the low `bits` bits of the keys.
 // Ping-pongs between (keys, vals) and (keys_alt, vals_alt); *in_alt tells which pair holds
