@@ -827,7 +827,7 @@ QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int
     if (e == cudaSuccess) e = cudaMemcpyAsync(pos, pos_h, sizeof(pos_h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = qses::launch_gs_slab(pos, 0, 4, 2, table, 2, next_slab, 2, 512, start, nbr, word0, pack, ext, nullptr, 1u, 1u,
-                                 qses::GsOrder{}, err, spin_cycles, nullptr, s);
+                                 qses::GsOrder{}, err, nullptr, spin_cycles, nullptr, s);
     int h_err = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

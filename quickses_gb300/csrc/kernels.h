@@ -75,7 +75,7 @@ cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax,
                            unsigned qcap, unsigned *next_slab, int P, int threads,
                            const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
                            const unsigned char *ext0, unsigned passes, unsigned stamp, const GsOrder &ord, int *err,
-                           long long spin_cycles, unsigned long long *stats, cudaStream_t s);
+                           float *out, long long spin_cycles, unsigned long long *stats, cudaStream_t s);
 int gs_slab_max_blocks(int device, unsigned S, int threads);
 
 // Gauss-Seidel launch shape: threads per slab CTA and the slab size aimed at (vertices);

@@ -444,7 +444,7 @@ bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool
 
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
                   const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
-                  const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback) {
+                  const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback, float *h_out) {
     cudaStream_t s = ctx->stream;
     float4 *pos4 = sb.pos4;
     // neighbour lists: count the corners per vertex, scan, scatter them per vertex
@@ -479,7 +479,8 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
             if (pass || w) QCHK(cudaMemsetAsync(gb.next_slab, 0, 4, s));
             QCHK(launch_gs_slab(pos4, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, L.qcap, gb.next_slab, L.ctas,
                                 sh.threads, sb.deg, sb.nbr, sb.word0, sb.pack, sb.ext, (const unsigned char *)sb.ext0,
-                                together ? (unsigned)passes : 1u, (unsigned)pass + 1u, gb.ord, d_err, 4000000000ll,
+                                together ? (unsigned)passes : 1u, (unsigned)pass + 1u, gb.ord, d_err,
+                                together || pass == passes - 1 ? h_out : nullptr, 4000000000ll,
                                 ctx->profiling ? stats : nullptr, s));
             ctx->launches++;
         }
@@ -632,13 +633,16 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
     if (c.fork) QCHK(cudaEventRecord(ctx->ev_join, sd));
 
     // Gauss-Seidel smoothing on the device
-    if (c.passes > 0 && c.nv > 0 && c.nt > 0) {
+    const bool smooth = c.passes > 0 && c.nv > 0 && c.nt > 0;
+    char *h_vertices = smooth && c.dl_vb ? c.h_dl : nullptr;  // the smoothing writes the host's vertices itself
+    if (smooth) {
         // the closest-atom pass on the side stream reads the welded positions in vq
-        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table, c.err, c.stats, c.fork ? ctx->ev_join : nullptr);
+        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table,
+                                     c.err, c.stats, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices);
         if (rc) return rc;
     }
     ctx->mark("smooth");
-    if (c.h_dl && c.dl_vb) QCHK(cudaMemcpyAsync(c.h_dl, c.vq, c.dl_vb, cudaMemcpyDeviceToHost, s));
+    if (c.h_dl && c.dl_vb && !h_vertices) QCHK(cudaMemcpyAsync(c.h_dl, c.vq, c.dl_vb, cudaMemcpyDeviceToHost, s));
     if (c.h_dl && !c.fork) QCHK_RC(download_rest(s));
     if (c.fork) QCHK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
     QCHK(cudaMemcpyAsync(c.h_out + 8, c.err, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -230,13 +230,16 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
     if (c.fork) QCHK(cudaEventRecord(ctx->ev_join, sd));
 
     // Gauss-Seidel over all molecules
-    if (c.passes > 0 && c.nv > 0 && c.nt > 0) {
+    const bool smooth = c.passes > 0 && c.nv > 0 && c.nt > 0;
+    char *h_vertices = smooth && c.dl_vb ? c.h_dl : nullptr;  // the smoothing writes the host's vertices itself
+    if (smooth) {
         // the closest-atom pass on the side stream reads the welded positions in vq
-        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table, c.err, nullptr, c.fork ? ctx->ev_join : nullptr);
+        const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table,
+                                     c.err, nullptr, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices);
         if (rc) return rc;
     }
     ctx->mark("smooth");
-    if (c.h_dl && c.dl_vb) QCHK(cudaMemcpyAsync(c.h_dl, c.vq, c.dl_vb, cudaMemcpyDeviceToHost, s));
+    if (c.h_dl && c.dl_vb && !h_vertices) QCHK(cudaMemcpyAsync(c.h_dl, c.vq, c.dl_vb, cudaMemcpyDeviceToHost, s));
     if (c.h_dl && !c.fork) QCHK_RC(download_rest(s));
     if (c.fork) QCHK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
     QCHK(cudaMemcpyAsync(c.h_out + 8, c.err, sizeof(int), cudaMemcpyDeviceToHost, s));
