@@ -851,7 +851,15 @@ cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax,
     // A cooperative launch: every CTA resident from the start.  (A plain launch would also be
     // safe - a CTA only waits for slabs taken before its own, by CTAs that were running when
     // they took them - but its CTAs can then take the SMs the side stream's kernels wait for.)
-    return cudaLaunchCooperativeKernel(fn, dim3(P), dim3(threads >= 1024 ? 1024 : 512), args, smem, s);
+    // With one CTA to an SM anyway, and slabs enough to keep most SMs busy, 18 worker warps instead of
+    // 14: 3 700 000 vertices 5.43 -> 5.35 ms, 3 900 000 at 0.3 A 5.80 -> 5.64, three passes over 650 000
+    // 2.70 -> 2.61 (22 warps 5.38, 5.69 and 2.61).  Two CTAs fit an SM with 512 threads only: 16 frames
+    // 1.25 ms, with 640 1.35.
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int block = threads >= 1024 ? 1024 : P <= sms && 2 * P > sms ? 640 : 512;
+    return cudaLaunchCooperativeKernel(fn, dim3(P), dim3(block), args, smem, s);
 }
 void gs_l2_window(int device, cudaStream_t s, const void *p, size_t bytes) {
     int max_persist = 0, max_window = 0;

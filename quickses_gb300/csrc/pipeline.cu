@@ -143,8 +143,8 @@ GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes) {
     // shells of 9 500 - 3 500 000 vertices (30 000 vertices: 0.41 ms; 519 per slab 0.46, 4 096 0.48;
     // 1 670 000: 3.72 ms; 3 875 per slab 4.28, 11 625 3.97).  Far more vertices than fit the SMs at
     // once are a matter of throughput: two CTAs per SM (14 200 000 vertices: 9.66 ms; one CTA of
-    // 11 904 10.36; a batch of 29 600 000: 6.7 against 8.1).  14 worker warps per CTA are enough, as
-    // each takes a second vertex when more are ready: 1 024 threads 1-9 % slower.
+    // 11 904 10.36; a batch of 29 600 000: 6.7 against 8.1).  14 to 18 worker warps per CTA are enough
+    // (launch_gs_slab), as each takes a second vertex when more are ready: 1 024 threads 1-9 % slower.
     // Several passes follow one another through the slabs and want shorter ones (548 000 vertices, 3
     // passes: 4 096 per slab 2.73 ms, 4 811 2.87, 2 048 2.90).
     const unsigned t = (unsigned)((passes > 1 ? 5.3 : 6.5) * std::sqrt((double)biggest));
