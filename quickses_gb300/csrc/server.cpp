@@ -44,7 +44,7 @@ struct Job {
 // workspace), from its grid alone; used only for admission.
 unsigned long long estimate_bytes(const QGrid &g, unsigned n) {
     const double G = g.G;
-    // codes and the refine's z distances (one byte each per padded voxel), three masks, cells
+    // codes (one byte per padded voxel, and as much again in reserve), three masks, cells
     const double field = 2.0 * G * G * (double)g.Gp + 3.0 * G * G * g.W * 4.0 + 8.0 * (double)g.gnb * g.gnb * g.gnb +
                          48.0 * n + 8.0 * (g.Gc + 1.0) * (g.Gc + 1.0);
     const double edges = 12.0 * G * G;  // active edges of a globular surface, generous
