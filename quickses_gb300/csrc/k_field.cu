@@ -175,7 +175,9 @@ __device__ __forceinline__ void atom_thresholds(float r, const QGrid &g, float &
     tsas = __fmul_rn(rs, rs);
 }
 
-// One SAS tile: z-word w of the 8 x 8 rows starting at (i0, j0) = (8 ib, 8 jb).
+// One SAS tile: z-word w of the 8 x 8 rows starting at (i0, j0) = (8 ib, 8 jb), SPLIT threads to a row
+// that share its candidates out.
+template <int SPLIT>
 __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, const float4 *__restrict__ atoms,
                                          const uint2 *__restrict__ cells, unsigned *__restrict__ inMask,
                                          unsigned *__restrict__ outMask) {
@@ -183,7 +185,8 @@ __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, 
     __shared__ float2 s_t[kSasCap];  // threshold of r - dx, z as a voxel index
     __shared__ int s_n;
     const int j0 = jb * kSasTY, i0 = ib * kSasTX;
-    const int t = threadIdx.x, i = i0 + t / kSasTY, j = j0 + t % kSasTY, k0 = w * 32;
+    constexpr int NT = kSasNT * SPLIT;
+    const int t = threadIdx.x, row = t / SPLIT, i = i0 + row / kSasTY, j = j0 + row % kSasTY, k0 = w * 32;
     // Voxels with an index >= lim on an axis are never computed and stay outside: the last
     // layer G-1 (Kernels.cu:436-441) and, for a slice box, its own last layer and whatever
     // lies at or past the molecule grid's last layer.  Positions use the grid index
@@ -244,14 +247,14 @@ __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, 
         const unsigned full = span_bits(0, klim - k0);
         auto classify = [&](int na) {
             if (i > lastx || j > lasty) return;
-            for (int q = 0; q < na; q++) {
+            for (int q = t % SPLIT; q < na; q += SPLIT) {
                 const float2 u = s_t[q];
                 sas_row_atom(px, py, s_a[q], u.x, u.y, z, full, sasw, inw);
             }
         };
         if (t == 0) s_n = 0;
         __syncthreads();
-        for (int c = t; c < 2 * ncol; c += kSasNT) {
+        for (int c = t; c < 2 * ncol; c += NT) {
             const uint2 r = run(c);
             for (unsigned s = r.x; s < r.y; s++) stage(s);
         }
@@ -260,13 +263,13 @@ __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, 
             classify(s_n);
         } else {
             // More than fit (crowded atoms, coarse voxels): all threads run through the columns
-            // together and classify whenever there may be no room for another 64.
+            // together and classify whenever there may be no room for another round.
             for (int c = 0; c < 2 * ncol; c++) {
                 const uint2 r = run(c);
-                for (unsigned s = r.x; s < r.y; s += kSasNT) {
+                for (unsigned s = r.x; s < r.y; s += NT) {
                     __syncthreads();
                     const int n = s_n > kSasCap ? 0 : s_n;  // the first round starts over
-                    const bool flush = n > kSasCap - kSasNT;
+                    const bool flush = n > kSasCap - NT;
                     if (flush) classify(n);
                     __syncthreads();
                     if (t == 0) s_n = flush ? 0 : n;
@@ -278,7 +281,12 @@ __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, 
             classify(s_n);
         }
     }
-    if (i < G && j < G) {
+#pragma unroll
+    for (int o = 1; o < SPLIT; o <<= 1) {
+        sasw |= __shfl_xor_sync(0xffffffffu, sasw, o);
+        inw |= __shfl_xor_sync(0xffffffffu, inw, o);
+    }
+    if (i < G && j < G && t % SPLIT == 0) {
         unsigned outw, inw2;
         if (i > lastx || j > lasty) {
             outw = valid;
@@ -293,10 +301,11 @@ __device__ __forceinline__ void sas_tile(const QGrid &g, int w, int jb, int ib, 
     }
 }
 
-__global__ void __launch_bounds__(kSasNT) k_sas(QGrid g, const float4 *__restrict__ atoms,
+template <int SPLIT>
+__global__ void __launch_bounds__(kSasNT * SPLIT) k_sas(QGrid g, const float4 *__restrict__ atoms,
                                                 const uint2 *__restrict__ cells, unsigned *__restrict__ inMask,
                                                 unsigned *__restrict__ outMask) {
-    sas_tile(g, blockIdx.x, blockIdx.y, blockIdx.z, atoms, cells, inMask, outMask);
+    sas_tile<SPLIT>(g, blockIdx.x, blockIdx.y, blockIdx.z, atoms, cells, inMask, outMask);
 }
 
 // ------------------------------------------------------------------ refine
@@ -564,7 +573,7 @@ __global__ void __launch_bounds__(kSasNT) k_sas_batch(QBatch b, const float4 *__
     int w, jb, ib;
     while (next_tile(b, counter, m, w, jb, ib)) {
         const QMol mol = b.mols[m];
-        sas_tile(mol.g, w, jb, ib, atoms, cells + mol.cell_off, inMask + mol.mask_off, outMask + mol.mask_off);
+        sas_tile<1>(mol.g, w, jb, ib, atoms, cells + mol.cell_off, inMask + mol.mask_off, outMask + mol.mask_off);
     }
 }
 
@@ -595,8 +604,15 @@ void launch_atom_gather(const float *xyz, const float *r, const unsigned *skey, 
 }
 void launch_sas(const QGrid &g, const float4 *atoms, const uint2 *cells, unsigned *inMask, unsigned *outMask,
                 cudaStream_t s) {
-    dim3 grid(g.W, (g.G + kSasTY - 1) / kSasTY, (g.G + kSasTX - 1) / kSasTX);
-    k_sas<<<grid, kSasNT, 0, s>>>(g, atoms, cells, inMask, outMask);
+    const dim3 grid(g.W, (g.G + kSasTY - 1) / kSasTY, (g.G + kSasTX - 1) / kSasTX);
+    // Small grids have a few blocks to an SM, and the time is a row's walk through its candidates:
+    // 85^3 (363 tiles) 31 us with a thread to a row, 25, 19 and 16 with 2, 4 and 8.  From some thousand
+    // tiles on all SMs are busy, and the shared rows verify more intervals: 171^3 (2 904 tiles) 28 us
+    // with 1, 34 with 4; 301^3 57 and 102.
+    if ((unsigned long long)grid.x * grid.y * grid.z <= 1000u)
+        k_sas<8><<<grid, 8 * kSasNT, 0, s>>>(g, atoms, cells, inMask, outMask);
+    else
+        k_sas<1><<<grid, kSasNT, 0, s>>>(g, atoms, cells, inMask, outMask);
 }
 template <int TX, int TY>
 static void launch_edt_shape(const QGrid &g, const unsigned *inMask, const unsigned *outMask, unsigned char *codes,
