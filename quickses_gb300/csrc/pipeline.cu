@@ -444,7 +444,8 @@ bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool
 
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
                   const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
-                  const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback, float *h_out) {
+                  const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback, float *h_out,
+                  const std::function<int()> &beside) {
     cudaStream_t s = ctx->stream;
     float4 *pos4 = sb.pos4;
     // neighbour lists: count the corners per vertex, scan, scatter them per vertex
@@ -472,6 +473,7 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
         ctx->launches++;
     }
     ctx->mark("smooth_csr");
+    if (beside) QCHK_RC(beside());
     for (int pass = 0; pass < (together ? 1 : passes); pass++) {
         if (pass) QCHK(cudaMemcpyAsync(sb.ext, sb.ext0, nv, cudaMemcpyDeviceToDevice, s));
         for (unsigned w = 0; w < L.waves; w++) {
@@ -594,31 +596,27 @@ struct FinishSeg {
     unsigned long long *stats;
     unsigned long long n3;
     unsigned nv, nt;
-    int passes, keep_all, fork, pad_;
+    int passes, keep_all, fork, late;  // late: the side stream starts behind the neighbour lists
     GsShape sh;
     GsLaunch gl;
     QGrid g;
 };
 
+// The side stream's kernels start with the smoothing instead of with its neighbour lists while the
+// smoothing leaves them room: one CTA to an SM, or CTAs that run out of slabs before the last chain
+// ends.  50 000 atoms 7.95 -> 7.79 ms, 200 000 8.67 -> 8.42, an uneven batch (580 slabs for 304 CTAs)
+// 3.74 -> 3.60, 200 atoms 0.464 -> 0.454.  Where two CTAs fill every SM to the end they would wait for
+// it, and the downloads with them: 16 frames (982 slabs) 3.20 -> 3.48, 10 to 12 frames (612, 736) 2.48
+// -> 2.50 and 2.71 -> 2.82.
+bool side_work_late(int device, int ctas, unsigned slabs) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return ctas <= sms || slabs <= 2u * (unsigned)ctas;
+}
+
 static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
     cudaStream_t s = ctx->stream, sd = c.fork ? ctx->side : s;
-    if (c.fork) {
-        QCHK(cudaEventRecord(ctx->ev_fork, s));
-        QCHK(cudaStreamWaitEvent(sd, ctx->ev_fork, 0));
-    }
-    // closest atom per welded vertex (before smoothing, as in the reference)
-    if (c.nv > 0) {
-        launch_closest(c.g, c.vq, c.nv, c.atoms, c.cells, c.sidx, c.asorted, c.ainput, sd);
-        ctx->launches++;
-    }
-    ctx->mark("closest_atom");
-    // drop degenerate triangles (API_computeSES filter)
-    if (!c.keep_all && c.nt > 0) {
-        QCHK(launch_tri_filter(c.tri, c.nt, c.tri_kept, c.tot, c.tmp2, c.err, sd));
-        ctx->launches++;
-        QCHK(cudaMemcpyAsync(c.h_out, c.tot, sizeof(uint2), cudaMemcpyDeviceToHost, sd));
-    }
-    ctx->mark("filter");
+    const bool smooth = c.passes > 0 && c.nv > 0 && c.nt > 0;
     const unsigned *tri_out = c.keep_all ? c.tri : c.tri_kept;
     // triangles and atom ids to the host: beside the smoothing when forked, else (stage
     // timing) in the download stage
@@ -629,16 +627,40 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
             QCHK(cudaMemcpyAsync(c.h_dl + c.dl_vb + c.dl_tb + c.dl_ab, c.ainput, c.dl_ab, cudaMemcpyDeviceToHost, q));
         return QSES_OK;
     };
-    if (c.h_dl && c.fork) QCHK_RC(download_rest(sd));
-    if (c.fork) QCHK(cudaEventRecord(ctx->ev_join, sd));
+    // Closest atoms, filter and the downloads that do not wait for the smoothing: beside the neighbour
+    // lists they only take from them what they do themselves, beside the smoothing, which leaves
+    // half of each SM idle, they cost little (side_work_late).
+    auto beside = [&]() -> int {
+        if (c.fork) {
+            QCHK(cudaEventRecord(ctx->ev_fork, s));
+            QCHK(cudaStreamWaitEvent(sd, ctx->ev_fork, 0));
+        }
+        // closest atom per welded vertex (before smoothing, as in the reference)
+        if (c.nv > 0) {
+            launch_closest(c.g, c.vq, c.nv, c.atoms, c.cells, c.sidx, c.asorted, c.ainput, sd);
+            ctx->launches++;
+        }
+        ctx->mark("closest_atom");
+        // drop degenerate triangles (API_computeSES filter)
+        if (!c.keep_all && c.nt > 0) {
+            QCHK(launch_tri_filter(c.tri, c.nt, c.tri_kept, c.tot, c.tmp2, c.err, sd));
+            ctx->launches++;
+            QCHK(cudaMemcpyAsync(c.h_out, c.tot, sizeof(uint2), cudaMemcpyDeviceToHost, sd));
+        }
+        ctx->mark("filter");
+        if (c.h_dl && c.fork) QCHK_RC(download_rest(sd));
+        if (c.fork) QCHK(cudaEventRecord(ctx->ev_join, sd));
+        return QSES_OK;
+    };
+    if (!c.late) QCHK_RC(beside());
 
     // Gauss-Seidel smoothing on the device
-    const bool smooth = c.passes > 0 && c.nv > 0 && c.nt > 0;
     char *h_vertices = smooth && c.dl_vb ? c.h_dl : nullptr;  // the smoothing writes the host's vertices itself
     if (smooth) {
         // the closest-atom pass on the side stream reads the welded positions in vq
         const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table,
-                                     c.err, c.stats, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices);
+                                     c.err, c.stats, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices,
+                                     c.late ? std::function<int()>(beside) : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -869,6 +891,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
         c.gl = plan.L;
         c.gb = gb;
         c.h_table = ctx->h_gs;
+        c.late = c.fork && side_work_late(ctx->device, plan.L.ctas, (unsigned)plan.max_slabs);
         ctx->diag[0] = plan.max_slabs;
         ctx->diag[1] = plan.max_len;
     }

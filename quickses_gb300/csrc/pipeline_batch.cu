@@ -188,7 +188,7 @@ struct BatchFinishSeg {
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
     unsigned long long n3;
     unsigned nv, nt;
-    int passes, fork;
+    int passes, fork, late, pad_;  // late: the side stream starts behind the neighbour lists
     GsShape sh;
     GsLaunch gl;
     QBatch b;
@@ -197,26 +197,7 @@ struct BatchFinishSeg {
 static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegOut &o) {
     cudaStream_t s = ctx->stream, sd = c.fork ? ctx->side : s;
     const unsigned nm = c.b.n_mol;
-    if (c.fork) {
-        QCHK(cudaEventRecord(ctx->ev_fork, s));
-        QCHK(cudaStreamWaitEvent(sd, ctx->ev_fork, 0));
-    }
-    if (c.nv > 0) {
-        launch_closest_batch(c.b, c.vq, c.vmol, c.nv, c.atoms, c.cells, c.sidx, c.asorted, c.ainput, sd);
-        ctx->launches++;
-    }
-    ctx->mark("closest_atom");
-    // per-molecule filter and molecule-local corner ids
-    if (c.nt > 0) {
-        QCHK(launch_tri_filter_batch(c.b, c.tri, c.nt, c.tri_kept, c.kept_off, c.tot, c.tmp2, c.err, sd));
-        ctx->launches++;
-    } else {
-        QCHK(cudaMemsetAsync(c.kept_off, 0, 4ull * (nm + 1), sd));
-        QCHK(cudaMemsetAsync(c.tot, 0, sizeof(uint2), sd));
-    }
-    QCHK(cudaMemcpyAsync(c.h_out, c.tot, sizeof(uint2), cudaMemcpyDeviceToHost, sd));
-    QCHK(cudaMemcpyAsync(c.h_kept, c.kept_off, 4ull * (nm + 1), cudaMemcpyDeviceToHost, sd));
-    ctx->mark("filter");
+    const bool smooth = c.passes > 0 && c.nv > 0 && c.nt > 0;
     // triangles and atom ids to the host: beside the smoothing when forked, else (stage
     // timing) in the download stage
     auto download_rest = [&](cudaStream_t q) -> int {
@@ -226,16 +207,43 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
             QCHK(cudaMemcpyAsync(c.h_dl + c.dl_vb + c.dl_tb + c.dl_ab, c.ainput, c.dl_ab, cudaMemcpyDeviceToHost, q));
         return QSES_OK;
     };
-    if (c.h_dl && c.fork) QCHK_RC(download_rest(sd));
-    if (c.fork) QCHK(cudaEventRecord(ctx->ev_join, sd));
+    // Closest atoms, filter and the downloads that do not wait for the smoothing: beside the neighbour
+    // lists they only take from them what they do themselves, beside the smoothing, which leaves
+    // half of each SM idle, they cost little (side_work_late).
+    auto beside = [&]() -> int {
+        if (c.fork) {
+            QCHK(cudaEventRecord(ctx->ev_fork, s));
+            QCHK(cudaStreamWaitEvent(sd, ctx->ev_fork, 0));
+        }
+        if (c.nv > 0) {
+            launch_closest_batch(c.b, c.vq, c.vmol, c.nv, c.atoms, c.cells, c.sidx, c.asorted, c.ainput, sd);
+            ctx->launches++;
+        }
+        ctx->mark("closest_atom");
+        // per-molecule filter and molecule-local corner ids
+        if (c.nt > 0) {
+            QCHK(launch_tri_filter_batch(c.b, c.tri, c.nt, c.tri_kept, c.kept_off, c.tot, c.tmp2, c.err, sd));
+            ctx->launches++;
+        } else {
+            QCHK(cudaMemsetAsync(c.kept_off, 0, 4ull * (nm + 1), sd));
+            QCHK(cudaMemsetAsync(c.tot, 0, sizeof(uint2), sd));
+        }
+        QCHK(cudaMemcpyAsync(c.h_out, c.tot, sizeof(uint2), cudaMemcpyDeviceToHost, sd));
+        QCHK(cudaMemcpyAsync(c.h_kept, c.kept_off, 4ull * (nm + 1), cudaMemcpyDeviceToHost, sd));
+        ctx->mark("filter");
+        if (c.h_dl && c.fork) QCHK_RC(download_rest(sd));
+        if (c.fork) QCHK(cudaEventRecord(ctx->ev_join, sd));
+        return QSES_OK;
+    };
+    if (!c.late) QCHK_RC(beside());
 
     // Gauss-Seidel over all molecules
-    const bool smooth = c.passes > 0 && c.nv > 0 && c.nt > 0;
     char *h_vertices = smooth && c.dl_vb ? c.h_dl : nullptr;  // the smoothing writes the host's vertices itself
     if (smooth) {
         // the closest-atom pass on the side stream reads the welded positions in vq
         const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table,
-                                     c.err, nullptr, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices);
+                                     c.err, nullptr, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices,
+                                     c.late ? std::function<int()>(beside) : nullptr);
         if (rc) return rc;
     }
     ctx->mark("smooth");
@@ -537,6 +545,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
         GsBuffers gb;
         QCHK_RC(gs_buffers(ctx, plan, gb));
         c.gl = plan.L;
+        c.late = c.fork && side_work_late(ctx->device, plan.L.ctas, (unsigned)plan.max_slabs);
         c.gb = gb;
         c.h_table = ctx->h_gs;
         ctx->diag[0] = std::max<unsigned long long>(ctx->diag[0], plan.max_slabs);

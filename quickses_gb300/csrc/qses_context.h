@@ -6,6 +6,7 @@
 #include <chrono>
 #include <string>
 #include <utility>
+#include <functional>
 #include <vector>
 
 #include "kernels.h"
@@ -221,10 +222,13 @@ bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool
 // `before_writeback` (may be null): event the stream waits for before the smoothed
 // positions overwrite vq (work on another stream that still reads the welded positions).
 // h_out (may be null): pinned host memory that receives the smoothed positions too.
+// beside (may be null): enqueues other streams' work, once the lists are done.
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
                   const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
                   const unsigned *h_table, int *d_err, unsigned long long *stats,
-                  cudaEvent_t before_writeback = nullptr, float *h_out = nullptr);
+                  cudaEvent_t before_writeback = nullptr, float *h_out = nullptr,
+                  const std::function<int()> &beside = nullptr);
+bool side_work_late(int device, int ctas, unsigned slabs);
 // Slab plan of a pass over nv vertices.  mol_off (nm + 1 entries, null for one molecule):
 // the molecules' vertex ranges, never split by a slab boundary unless a molecule is larger
 // than the slab size; mol_depth: a per-molecule estimate of the dependency depth (grid size),
