@@ -693,13 +693,15 @@ __global__ void k_closest_batch(QBatch b, const float *__restrict__ vq, const un
 // registers, the kept ones go to shared memory in order and from there, behind those of the blocks
 // before (look-back), to whole lines of `out`.  Batch: molecules flagged QSES_FLAG_KEEP_DEGENERATE
 // keep every triangle, corners become molecule-local vertex ids and kept_off receives each
-// molecule's first kept triangle.  Bound by memory, 24 B a triangle, and by the look-back that
+// molecule's first kept triangle.  `out` may be `tri`: a block writes behind the kept triangles of the
+// blocks before it, which have read theirs when they publish their counts, and never past its own.
+// Bound by memory, 24 B a triangle, and by the look-back that
 // orders the blocks: 1024 triangles each took 2.7 ms for 277 000 000, 2048 2.1, 4096 1.9; a flag per
 // triangle, a scan of the flags and a copy 5.2.  7 400 000: 0.19 -> 0.07 ms.
 constexpr int kFiltT = 512, kFiltN = 8, kFiltTile = kFiltN * kFiltT;
 template <bool BATCH>
-__global__ void __launch_bounds__(kFiltT) k_tri_filter(QBatch b, const unsigned *__restrict__ tri, unsigned nt,
-                                                       unsigned *__restrict__ out, unsigned *__restrict__ kept_off,
+__global__ void __launch_bounds__(kFiltT) k_tri_filter(QBatch b, const unsigned *tri, unsigned nt,
+                                                       unsigned *out, unsigned *__restrict__ kept_off,
                                                        uint2 *__restrict__ total, unsigned long long *status,
                                                        unsigned *ticket, int *err) {
     __shared__ unsigned s_out[3 * kFiltTile];

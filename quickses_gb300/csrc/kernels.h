@@ -40,7 +40,7 @@ cudaError_t launch_weld(const QGrid &g, const unsigned long long *vkey, const ui
 void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s);
 void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *atoms, const uint2 *cells,
                     const unsigned *sorted_to_input, int *asorted, int *ainput, cudaStream_t s);
-// Triangles without a repeated corner, in order, to out; their number to *total.
+// Triangles without a repeated corner, in order, to out (which may be tri); their number to *total.
 size_t tri_filter_tmp_bytes(unsigned nt);
 cudaError_t launch_tri_filter(const unsigned *tri, unsigned nt, unsigned *out, uint2 *total, void *tmp, int *err,
                               cudaStream_t s);

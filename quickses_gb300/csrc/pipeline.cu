@@ -787,13 +787,15 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
     const bool may_smooth = p.smooth_passes > 0;
-    const size_t needB = 2 * align256(4 * n3 + 4) + 3 * align256(4ull * NE + 4) + align256(12ull * NE + 12) +
+    // the filter works in place unless the smoothing reads the triangles beside it
+    const bool own_kept = may_smooth && !(p.flags & QSES_FLAG_KEEP_DEGENERATE);
+    const size_t needB = (own_kept ? 2 : 1) * align256(4 * n3 + 4) + 3 * align256(4ull * NE + 4) + align256(12ull * NE + 12) +
                          align256(weld_or_smooth_bytes(NE, (unsigned)E, n3, may_smooth)) +
                          align256(tri_filter_tmp_bytes(T)) + 4096;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
-    unsigned *tri_kept = (unsigned *)B.take(4 * n3 + 4);
+    unsigned *tri_kept = own_kept ? (unsigned *)B.take(4 * n3 + 4) : tri;
     unsigned *vmap = (unsigned *)B.take(4ull * NE + 4);
     float *vq = (float *)B.take(12ull * NE + 12);
     int *asorted = (int *)B.take(4ull * NE + 4), *ainput = (int *)B.take(4ull * NE + 4);

@@ -433,12 +433,13 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    const size_t needB = 2 * a256(4 * n3 + 4) + 4 * a256(4ull * NE + 4) + a256(12ull * NE + 12) +
+    // the filter works in place unless the smoothing reads the triangles beside it
+    const size_t needB = (passes > 0 ? 2 : 1) * a256(4 * n3 + 4) + 4 * a256(4ull * NE + 4) + a256(12ull * NE + 12) +
                          a256(weld_or_smooth_bytes(NE, layer_off[nm], n3, passes > 0)) + a256(tri_filter_tmp_bytes(T)) + 4096;
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "batch mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
-    unsigned *tri_kept = (unsigned *)B.take(4 * n3 + 4);
+    unsigned *tri_kept = passes > 0 ? (unsigned *)B.take(4 * n3 + 4) : tri;
     unsigned *vmap = (unsigned *)B.take(4ull * NE + 4);
     float *vq = (float *)B.take(12ull * NE + 12);
     unsigned *vmol = (unsigned *)B.take(4ull * NE + 4);

@@ -212,12 +212,12 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 const size_t n3 = 3ull * T, n3k = 3ull * T1;
                 const bool may_smooth = p.smooth_passes > 0;
                 const size_t tmpB = std::max(scan_u2_tmp_bytes(NE + 1), tri_filter_tmp_bytes(T));
-                const size_t needB = 2 * a256(4 * n3 + 4) + 2 * a256(8ull * (NE + 2)) + 4 * a256(4ull * NE + 4) +
+                const size_t needB = a256(4 * n3 + 4) + 2 * a256(8ull * (NE + 2)) + 4 * a256(4ull * NE + 4) +
                                      2 * a256(12ull * NE + 12) + a256(tmpB) +
                                      a256(weld_or_smooth_bytes(NE, (unsigned)b.Gc + 1, n3, may_smooth)) + 4096;
                 if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "mesh workspace");
                 Arena &B = ctx->mesh_ws;
-                unsigned *tri = (unsigned *)B.take(4 * n3 + 4), *tri_kept = (unsigned *)B.take(4 * n3 + 4);
+                unsigned *tri = (unsigned *)B.take(4 * n3 + 4);
                 uint2 *used = (uint2 *)B.take(8ull * (NE + 2)), *excl = (uint2 *)B.take(8ull * (NE + 2));
                 unsigned *vmap = (unsigned *)B.take(4ull * NE + 4), *vmap2 = (unsigned *)B.take(4ull * NE + 4);
                 float *vq = (float *)B.take(12ull * NE + 12), *vq2 = (float *)B.take(12ull * NE + 12);
@@ -262,15 +262,13 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                                                   ctx->h_gs, d_err, stats);
                     if (src != QSES_OK) return src;
                 }
-                const unsigned *tri_out = tri;
                 unsigned nt = T1;
                 if (!keep_all) {
-                    SCHK(launch_tri_filter(tri, T1, tri_kept, tot, tmpb, d_err, s));
+                    SCHK(launch_tri_filter(tri, T1, tri, tot, tmpb, d_err, s));  // the smoothing is done with them
                     ctx->launches++;
                     SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
                     SCHK(cudaStreamSynchronize(s));
                     nt = h_tot->x;
-                    tri_out = tri_kept;
                 }
 
                 // ---- download, appended to the concatenated mesh
@@ -285,7 +283,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                     SCHK(cudaMemcpyAsync(out.atom_input.data() + v0, ainput, 4ull * nv, cudaMemcpyDeviceToHost, s));
                 }
                 if (nt)
-                    SCHK(cudaMemcpyAsync(out.triangles.data() + t0, tri_out, 12ull * nt, cudaMemcpyDeviceToHost, s));
+                    SCHK(cudaMemcpyAsync(out.triangles.data() + t0, tri, 12ull * nt, cudaMemcpyDeviceToHost, s));
                 SCHK(cudaMemcpyAsync(ctx->h_small + 24, d_err, 4, cudaMemcpyDeviceToHost, s));
                 SCHK(cudaStreamSynchronize(s));
                 memcpy(&herr, ctx->h_small + 24, 4);
