@@ -200,7 +200,8 @@ QSES_API int qses_autotune(qses_context *ctx, const qses_params *p, const qses_f
  * 3 = 32 x 16 (less halo per row, more shared memory); -1 returns to the tuned/default
  * shape.  Same codes for all. */
 QSES_API int qses_set_field_shape(qses_context *ctx, int shape);
-/* Fixes the smoothing launch shape of ctx: threads 512 or 1024 per slab CTA, slab size
+/* Fixes the smoothing launch shape of ctx: threads 512 (640 where one CTA fits an
+ * SM anyway) or 1024 per slab CTA, slab size
  * aimed at (>= 256 vertices; slabs hold at most 11 904), cache_flags bit 2 = keep the
  * positions in persisting L2 lines during the pass (a window on the context's stream, cleared
  * after it); bits 0, 1, 3, 4 and 5 (not 4 and 5 together) are accepted and without effect: a
