@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256, 4) k_mc_count_batch(QBatch b, const unsig
 // What consecutive words emit is contiguous, so keys and corners go out in whole lines, the corners
 // by way of shared memory.
 //
-// Bound by instruction issue: 664^3 (3 700 000 edges, 7 400 000 triangles) takes 126 M warp
+// Bound by instruction issue: 664^3 (4 160 000 edges, 8 310 000 triangles) takes 126 M warp
 // instructions at 1.9 a cycle, 16 warps an SM.  Rows dealt to 4 or 32 lanes, each corner's slot from
 // the words' masks and stored by itself: 0.74 ms there (568 M instructions), 0.24 so; 1738^3
 // (138 000 000 edges) 13.0 and 4.6; 85^3 0.025 and 0.020.  Blocks of 8 warps wait for their slowest
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 6) k_mc_emit(QGrid g1, QBatch
 // the bins and their loads.
 //
 // A radix sort of all keys (7 or 8 passes over 24 B, flags, scan, scatter) took the weld with its
-// corner remap 0.14 ms at 30 000 edges, 0.83 at 3 700 000, 24.1 at 138 000 000 (0.03, 0.20 and 6.6 so,
+// corner remap 0.14 ms at 30 000 edges, 0.83 at 4 160 000, 24.1 at 138 000 000 (0.03, 0.20 and 6.6 so,
 // 1.1 of the last the remap).  A warp sorting each bin of 8 to 32 in registers instead of the
 // comparisons: 0.57 and 18.4.
 constexpr int kWeldT = 1024;
@@ -622,7 +622,7 @@ __global__ void k_remap(unsigned *__restrict__ tri, size_t n3, const unsigned *_
 // is passed over; a warp's vertices have about the same x and y and mostly agree on that.  Cells are
 // taken 0.01 A wider than they are: coordinates and cell numbers are rounded, by 0.004 A at most.
 //
-// Bound by instruction issue: 3 700 000 vertices in 0.17 ms (148 M warp instructions at 2.9 a cycle),
+// Bound by instruction issue: 3 540 000 vertices in 0.17 ms (148 M warp instructions at 2.9 a cycle),
 // 138 000 000 in 5.8; all 27 cells one by one took 0.30 (270 M) and 10.5, cell by cell in the order
 // of closeness 0.27 and 9.8, for each lane wants other cells then.
 __device__ __forceinline__ int closest_atom(const QGrid &g, const float4 *__restrict__ atoms, const uint2 *__restrict__ cells,
@@ -697,7 +697,7 @@ __global__ void k_closest_batch(QBatch b, const float *__restrict__ vq, const un
 // blocks before it, which have read theirs when they publish their counts, and never past its own.
 // Bound by memory, 24 B a triangle, and by the look-back that
 // orders the blocks: 1024 triangles each took 2.7 ms for 277 000 000, 2048 2.1, 4096 1.9; a flag per
-// triangle, a scan of the flags and a copy 5.2.  7 400 000: 0.19 -> 0.07 ms.
+// triangle, a scan of the flags and a copy 5.2.  8 310 000: 0.19 -> 0.07 ms.
 constexpr int kFiltT = 512, kFiltN = 8, kFiltTile = kFiltN * kFiltT;
 template <bool BATCH>
 __global__ void __launch_bounds__(kFiltT) k_tri_filter(QBatch b, const unsigned *tri, unsigned nt,
@@ -782,7 +782,7 @@ __global__ void k_csr_scatter(const unsigned *__restrict__ tri, size_t n3, uint2
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n3) return;
     const unsigned v = tri[q];
-    // offset and position with one 64-bit atomic: 22 000 000 corners 0.16 ms, 0.20 with a load more
+    // offset and position with one 64-bit atomic: 24 900 000 corners 0.16 ms, 0.20 with a load more
     const unsigned long long old = atomicAdd((unsigned long long *)&start[v], 1ull << 32);
     occ[(unsigned)old + (unsigned)(old >> 32)] = (unsigned)q;
 }

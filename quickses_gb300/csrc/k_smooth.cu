@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(128) k_gs_lists(const float *__restrict__ vq, 
 // The vertices of more than 8 corners: a warp each, a corner per lane, sorted by counting the
 // smaller ones; a hash table finds the entries that name a vertex again; their lists go to the
 // neighbour table at twice the vertex's offset.  At 0.2 A, where the surface runs through grid
-// points, a tenth of the vertices have 9 to 27 corners: 370 000 of 3 700 000 in 0.225 ms (each entry
+// points, a tenth of the vertices have 9 to 28 corners: 336 000 of 3 540 000 in 0.225 ms (each entry
 // compared with all before it: 0.286).
 __global__ void __launch_bounds__(256) k_gs_lists_long(const unsigned *__restrict__ tri, unsigned *__restrict__ occ,
                                                        const uint2 *__restrict__ start, unsigned *__restrict__ nbr,
@@ -852,7 +852,7 @@ cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax,
     // safe - a CTA only waits for slabs taken before its own, by CTAs that were running when
     // they took them - but its CTAs can then take the SMs the side stream's kernels wait for.)
     // With one CTA to an SM anyway, and slabs enough to keep most SMs busy, 18 worker warps instead of
-    // 14: 3 700 000 vertices 5.43 -> 5.35 ms, 3 900 000 at 0.3 A 5.80 -> 5.64, three passes over 650 000
+    // 14: 3 540 000 vertices 5.43 -> 5.35 ms, 5 550 000 at 0.3 A 5.80 -> 5.64, three passes over 548 000
     // 2.70 -> 2.61 (22 warps 5.38, 5.69 and 2.61).  Two CTAs fit an SM with 512 threads only: 16 frames
     // 1.25 ms, with 640 1.35.
     int dev = 0, sms = 0;
