@@ -537,8 +537,8 @@ QSES_API int qses_compute_batch(qses_context *ctx, const qses_request *reqs, uns
         const std::vector<unsigned> &ids = grp.second;
         size_t at = 0;
         while (at < ids.size()) {
-            // One pass takes at most as many molecules as their grids' positions and a molecule
-            // number fit 64 bits: it bounds the pass by the size of the grids in it.
+            // Largest prefix whose positions with a molecule number above them fit 64 bits, as
+            // the weld of crowded meshes sorts them (launch_weld_sorted_batch).
             size_t end = at;
             int kb = 0;
             while (end < ids.size()) {

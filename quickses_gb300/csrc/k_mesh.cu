@@ -12,6 +12,7 @@
 //  k_tri_filter   drop triangles with a repeated index (CudaSurf.cu:820-829)
 //  k_csr_*        neighbour lists in triangle order (getNeighboorsVertices,
 //                 SmoothMesh.cpp:45-123) for the Gauss-Seidel dataflow (k_smooth.cu)
+#include <algorithm>
 #include <cfloat>
 #include <cstdlib>
 #include <cstring>
@@ -20,6 +21,7 @@
 
 #include "kernels.h"
 #include "mc_tables.h"
+#include "prims.h"
 
 namespace qses {
 
@@ -451,6 +453,22 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 6) k_mc_emit(QGrid g1, QBatch
 constexpr int kWeldT = 1024;
 constexpr unsigned kWeldCap = 4096;  // bins at most, of either sort
 constexpr unsigned long long kWeldFirst = 1ull << 63;  // the first of equal keys: the vertex
+// What k_weld takes on itself.  A CTA needs some 8 ns for a key of its layer and 0.11 ns for a
+// comparison within its bins, all CTAs together a 300th of that.
+struct WeldLimits {
+    // A layer of more comparisons than this, and than 256 for each key, is heavy: were all so, they would
+    // take as long as the sort.
+    static constexpr unsigned long long kHeavy = 393216;
+    unsigned keys;                  // of a layer and the one before it
+    unsigned long long pairs, all;  // comparisons of a layer; of the heavy ones together
+    __device__ __forceinline__ explicit WeldLimits(unsigned ne)
+        : keys(16384u + ne / 32), pairs(kHeavy + ne), all(20000000ull + 32ull * ne) {
+        if (ne < kWeldSortMin) keys = ~0u, pairs = all = ~0ull;  // cannot crowd a layer
+    }
+    static __device__ __forceinline__ bool heavy(unsigned long long work, unsigned n) {
+        return work > kHeavy && work > 256ull * n;
+    }
+};
 constexpr unsigned kWeldX = 4096;       // x ranges of a layer at most: quanta, for voxels up to 4 A
 // Quantised x of grid plane i, as edge_key has it for the edges in the plane.
 __device__ __forceinline__ unsigned plane_quantum(const QGrid &g, int i) {
@@ -458,12 +476,23 @@ __device__ __forceinline__ unsigned plane_quantum(const QGrid &g, int i) {
     if (g.off[0] | g.off[1] | g.off[2]) p = __fadd_rn(p, __fmul_rn((float)g.off[0], g.dx));
     return (unsigned)(quantum(p) - (int)g.bx);
 }
-// In place: exclusive sums of x[0, n), by the whole block; the total is returned.
+// In place: exclusive sums of x[0, n), by the whole block; the total is returned.  squares (may be
+// null, zeroed): the sum of the squares.
 template <int NT>
-__device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, unsigned *s_tmp) {
+__device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, unsigned *s_tmp,
+                                                    unsigned long long *squares = nullptr) {
     const unsigned per = (n + NT - 1) / NT, lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
     unsigned sum = 0, total;
-    for (unsigned k = lo; k < hi; k++) sum += x[k];
+    unsigned long long sq = 0;
+    for (unsigned k = lo; k < hi; k++) {
+        sum += x[k];
+        if (squares) sq += (unsigned long long)x[k] * x[k];
+    }
+    if (squares) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if ((threadIdx.x & 31) == 0 && sq) atomicAdd(squares, sq);
+    }
     unsigned run = block_excl_scan<NT>(sum, total, s_tmp);
     for (unsigned k = lo; k < hi; k++) {
         const unsigned c = x[k];
@@ -474,6 +503,14 @@ __device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, uns
     return total;
 }
 
+// A mesh may crowd a layer, though: a face normal to x has all its edges in one or two of them, one
+// normal to y and a fibre along z put a plane's into few y ranges, and a layer's work is one CTA's and
+// grows with the square of a bin's keys.  A layer that would take longer than sorting all keys does
+// (WeldLimits) gives up and says so in total->y, and the caller sorts them (launch_weld_sorted), which
+// takes 0.12 ms and 0.17 ns a key whatever the shape.  What the other layers did is lost then, and
+// bounded by the same limits.  A flat sheet of 40 000 atoms at 0.4 A (530 000 edges) normal to x takes
+// 0.33 ms, 31.2 with bins alone and 0.23 if it were sorted at once; one of 1 000 000 (18 000 000 edges)
+// normal to y 5.1, 28.9 and 3.2.
 template <bool BATCH>
 __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned cap,
                                                     const unsigned long long *__restrict__ vkey,
@@ -482,10 +519,13 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
                                                     unsigned *sslot, unsigned *__restrict__ vmap,
                                                     float *__restrict__ vq, unsigned *__restrict__ vmol,
                                                     unsigned *__restrict__ vtx_off, uint2 *__restrict__ total,
-                                                    unsigned long long *status, unsigned *ticket, int *err) {
+                                                    unsigned long long *status, unsigned *ticket,
+                                                    unsigned long long *work, int *err) {
     extern __shared__ unsigned s_bin[];  // 2 x (2 cap + 2) and kWeldX / 2
     __shared__ unsigned s_tmp[kWeldT / 32], s_tile, s_pushed, s_before;
+    __shared__ unsigned long long s_work, s_all;
     if (threadIdx.x == 0) {
+        s_work = 0;
         s_tile = atomicAdd(ticket, 1u);  // layers in the order CTAs start, so that every wait ends
         s_pushed = 0;
     }
@@ -494,8 +534,12 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
     const QGrid &g = BATCH ? b.mols[m].g : g1;
     const unsigned i = BATCH ? tile - __ldg(b.layer_off + m) : tile, E = (unsigned)g.Gc + 1;
     const uint2 *rows = rowBase + (BATCH ? b.mols[m].row_off : 0u);
-    const unsigned s1 = rows[(size_t)i * E].y, s0 = i ? rows[(size_t)(i - 1) * E].y : s1;
-    const unsigned s2 = i + 1 < E ? rows[(size_t)(i + 1) * E].y : BATCH ? __ldg(edge_off + m + 1) : ne;
+    const unsigned s1 = rows[(size_t)i * E].y;
+    unsigned s0 = i ? rows[(size_t)(i - 1) * E].y : s1;
+    unsigned s2 = i + 1 < E ? rows[(size_t)(i + 1) * E].y : BATCH ? __ldg(edge_off + m + 1) : ne;
+    const WeldLimits limits(ne);
+    bool crowded = s2 - s0 > limits.keys;
+    if (crowded) s0 = s2 = s1;
     const unsigned X0 = plane_quantum(g, (int)i), X1 = plane_quantum(g, (int)i + 1);
     const unsigned Rq = (unsigned)g.Rq;
     unsigned *cur = s_bin, *uniq = s_bin + 2 * cap + 2;
@@ -550,7 +594,17 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
     }
     if (below) atomicAdd(&s_pushed, below);
     __syncthreads();
-    const unsigned n = block_excl_sums<kWeldT>(cur, nbin, s_tmp);
+    unsigned n = block_excl_sums<kWeldT>(cur, nbin, s_tmp, &s_work);
+    if (limits.heavy(s_work, n)) {  // seldom; the sum passes its limit for the last to add to it, if not before
+        if (threadIdx.x == 0) s_all = atomicAdd(work, s_work) + s_work;
+        __syncthreads();
+        crowded |= s_all > limits.all;
+    }
+    crowded |= s_work > limits.pairs;
+    if (crowded) {
+        s0 = s2 = s1;
+        n = 0;
+    }
     // scatter: the layer's keys to [base, base + n) (the ones before it are the slots before s1 less
     // those pushed up into this layer), bin after bin; cur[k] becomes the end of bin k
     const unsigned base = s1 - s_pushed;
@@ -579,12 +633,13 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
     __syncthreads();
     const unsigned distinct = block_excl_sums<kWeldT>(uniq, nbin, s_tmp);
     if (threadIdx.x < 32) {
-        const unsigned before = (unsigned)look_back(status, tile, distinct, err);
+        const unsigned long long sum = look_back(status, tile, distinct | (crowded ? 1ull << 32 : 0ull), err);
+        const unsigned before = (unsigned)sum;
         if (threadIdx.x == 0) {
             s_before = before;
             if (BATCH && i == 0) vtx_off[m] = before;
             if (tile == layers - 1) {
-                *total = make_uint2(before + distinct, 0u);
+                *total = make_uint2(before + distinct, (unsigned)(sum >> 32) + crowded);
                 if (BATCH) vtx_off[b.n_mol] = before + distinct;
             }
         }
@@ -609,6 +664,47 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
     }
 }
 
+// The weld by sorting all keys, for meshes that crowd a few layers: the sorted keys' first ones
+// marked, numbered by a scan, and sent to their slots.  Batch: the keys are put together anew with
+// the molecule above its positions, which sorts the molecules one after another (bits: of a position).
+__global__ void k_weld_tag(QBatch b, unsigned long long *__restrict__ vkey, const unsigned *__restrict__ edge_off,
+                           unsigned n, int bits) {
+    const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const unsigned m = qses_find(edge_off, b.n_mol, s);
+    const unsigned long long R = (unsigned long long)b.mols[m].g.Rq, key = vkey[s];
+    vkey[s] = (unsigned long long)m << bits | (((key >> 42) * R + ((key >> 21) & 0x1fffffu)) * R + (key & 0x1fffffu));
+}
+__global__ void k_weld_flags(const unsigned long long *__restrict__ skey, unsigned n, uint2 *__restrict__ flags) {
+    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) flags[p] = make_uint2(p == 0 || skey[p] != skey[p - 1] ? 1u : 0u, 0u);
+}
+template <bool BATCH>
+__global__ void k_weld_number(QGrid g1, QBatch b, const unsigned long long *__restrict__ skey,
+                              const unsigned *__restrict__ sslot, const uint2 *__restrict__ excl, unsigned n, int bits,
+                              unsigned *__restrict__ vmap, float *__restrict__ vq, unsigned *__restrict__ vmol) {
+    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const unsigned long long key = skey[p];
+    const bool first = p == 0 || key != skey[p - 1];
+    const unsigned rank = excl[p].x - (first ? 0u : 1u);
+    vmap[sslot[p]] = rank;
+    if (!first) return;
+    const unsigned m = BATCH ? (unsigned)(key >> bits) : 0u;
+    const QGrid &g = BATCH ? b.mols[m].g : g1;
+    unsigned long long x, y, z;
+    if (BATCH) {
+        const unsigned long long at = key & ((1ull << bits) - 1ull), R = (unsigned long long)g.Rq;
+        x = at / (R * R), y = at / R % R, z = at % R;
+        vmol[rank] = m;
+    } else {
+        x = key >> 42, y = (key >> 21) & 0x1fffffu, z = key & 0x1fffffu;
+    }
+    vq[3ull * rank] = __fmul_rn((float)((long long)x + g.bx), QSES_WELD_TOL);
+    vq[3ull * rank + 1] = __fmul_rn((float)((long long)y + g.by), QSES_WELD_TOL);
+    vq[3ull * rank + 2] = __fmul_rn((float)((long long)z + g.bz), QSES_WELD_TOL);
+}
+
 // out[m] = excl[at[m]] for at[m] < n, else the scan total: the first scanned element of
 // each molecule's range gives that molecule's offset in the compacted output.
 __global__ void k_gather_offsets(const uint2 *__restrict__ excl, const unsigned *__restrict__ at, unsigned n_mol,
@@ -624,13 +720,17 @@ __global__ void k_gather_offsets(const uint2 *__restrict__ excl, const unsigned 
 
 // Corners from edge slots to vertices.  Bound by the gathers, so each thread has four under way:
 // 832 000 000 corners in 1.1 ms, one to a thread took 3.2.
-__global__ void k_remap(unsigned *__restrict__ tri, size_t n3, const unsigned *__restrict__ vmap) {
+// crowded (may be null): set if the weld gave up; the slots then stay.
+__global__ void k_remap(unsigned *__restrict__ tri, size_t n3, const unsigned *__restrict__ vmap,
+                        const unsigned *__restrict__ crowded) {
     const size_t q = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const bool keep = crowded && __ldg(crowded);
     if (q + 4 <= n3) {
         uint4 t = *(const uint4 *)(tri + q);
+        if (keep) return;
         t.x = __ldg(vmap + t.x), t.y = __ldg(vmap + t.y), t.z = __ldg(vmap + t.z), t.w = __ldg(vmap + t.w);
         *(uint4 *)(tri + q) = t;
-    } else {
+    } else if (!keep) {
         for (size_t e = q; e < n3; e++) tri[e] = vmap[tri[e]];
     }
 }
@@ -883,7 +983,8 @@ static cudaError_t weld_with(const QGrid &g, const QBatch &b, const unsigned lon
     if (e == cudaSuccess) e = cudaMemsetAsync(tmp, 0, weld_tmp_bytes(layers), s);
     if (e != cudaSuccess) return e;
     k_weld<BATCH><<<layers, kWeldT, smem, s>>>(g, b, cap, vkey, rowBase, ne, layers, edge_off, skey, sslot, vmap, vq, vmol,
-                                               vtx_off, total, (unsigned long long *)((char *)tmp + 256), (unsigned *)tmp, err);
+                                               vtx_off, total, (unsigned long long *)((char *)tmp + 256), (unsigned *)tmp,
+                                               (unsigned long long *)((char *)tmp + 128), err);
     return cudaGetLastError();
 }
 cudaError_t launch_weld(const QGrid &g, const unsigned long long *vkey, const uint2 *rowBase, unsigned ne,
@@ -899,6 +1000,43 @@ cudaError_t launch_weld_batch(const QBatch &b, unsigned layers, const unsigned l
     return weld_with<true>(QGrid{}, b, vkey, rowBase, ne, layers, edge_off, skey, sslot, vmap, vq, vmol, vtx_off, total, tmp,
                            err, s);
 }
+template <bool BATCH>
+static cudaError_t weld_sorted_with(const QGrid &g, const QBatch &b, unsigned long long *vkey, unsigned long long *skey,
+                                    unsigned *sslot, unsigned ne, const unsigned *edge_off, int bits, unsigned *vmap,
+                                    float *vq, unsigned *vmol, unsigned *vtx_off, uint2 *total, int *err,
+                                    cudaStream_t s, int *launches) {
+    // Positions come last, so their memory is the sort's and the scan's workspace until then.  An even
+    // number of passes ends where it began: the other key buffer then holds the marks.
+    const int key_bits = BATCH ? bits + bits_for(b.n_mol - 1) : 63, even = (key_bits + 15) / 16 * 16;
+    if (ne < kWeldSortMin || key_bits > 64 ||
+        12ull * ne < std::max(radix_sort_tmp_bytes<unsigned long long>(ne, even), scan_u2_tmp_bytes(ne)))
+        return cudaErrorInvalidValue;
+    if (BATCH) k_weld_tag<<<nblk(ne, 256), 256, 0, s>>>(b, vkey, edge_off, ne, bits);
+    int alt = 0;
+    cudaError_t e = radix_sort<unsigned long long>(vkey, skey, sslot, vmap, ne, even, true, vq, err, s, launches, &alt);
+    if (e != cudaSuccess) return e;
+    uint2 *flags = (uint2 *)skey;
+    k_weld_flags<<<nblk(ne, 256), 256, 0, s>>>(vkey, ne, flags);
+    e = scan_u2(flags, flags, ne, total, vq, err, s, launches);
+    if (e != cudaSuccess) return e;
+    k_weld_number<BATCH><<<nblk(ne, 256), 256, 0, s>>>(g, b, vkey, sslot, flags, ne, bits, vmap, vq, vmol);
+    if (BATCH) launch_gather_offsets(flags, edge_off, b.n_mol, ne, total, vtx_off, nullptr, s);
+    *launches += BATCH ? 4 : 2;
+    return cudaGetLastError();
+}
+cudaError_t launch_weld_sorted(const QGrid &g, unsigned long long *vkey, unsigned long long *skey, unsigned *sslot,
+                               unsigned ne, unsigned *vmap, float *vq, uint2 *total, int *err, cudaStream_t s,
+                               int *launches) {
+    return weld_sorted_with<false>(g, QBatch{}, vkey, skey, sslot, ne, nullptr, 0, vmap, vq, nullptr, nullptr, total, err, s,
+                                   launches);
+}
+cudaError_t launch_weld_sorted_batch(const QBatch &b, unsigned long long *vkey, unsigned long long *skey, unsigned *sslot,
+                                     unsigned ne, const unsigned *edge_off, int bits, unsigned *vmap, float *vq,
+                                     unsigned *vmol, unsigned *vtx_off, uint2 *total, int *err, cudaStream_t s,
+                                     int *launches) {
+    return weld_sorted_with<true>(QGrid{}, b, vkey, skey, sslot, ne, edge_off, bits, vmap, vq, vmol, vtx_off, total, err, s,
+                                  launches);
+}
 void launch_gather_offsets(const uint2 *excl, const unsigned *at, unsigned n_mol, unsigned n, const uint2 *total,
                            unsigned *outx, unsigned *outy, cudaStream_t s) {
     k_gather_offsets<<<nblk(n_mol + 1, 256), 256, 0, s>>>(excl, at, n_mol, n, total, outx, outy);
@@ -908,8 +1046,8 @@ void launch_closest_batch(const QBatch &b, const float *vq, const unsigned *vmol
                           cudaStream_t s) {
     k_closest_batch<<<nblk(nv, 128), 128, 0, s>>>(b, vq, vmol, nv, atoms, cells, sorted_to_input, asorted, ainput);
 }
-void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s) {
-    k_remap<<<nblk((n3 + 3) / 4, 256), 256, 0, s>>>(tri, n3, vmap);
+void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, const unsigned *crowded, cudaStream_t s) {
+    k_remap<<<nblk((n3 + 3) / 4, 256), 256, 0, s>>>(tri, n3, vmap, crowded);
 }
 void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *atoms, const uint2 *cells,
                     const unsigned *sorted_to_input, int *asorted, int *ainput, cudaStream_t s) {

@@ -100,14 +100,17 @@ cudaError_t scan_u2(const uint2 *in, uint2 *out, unsigned n, uint2 *d_total, voi
 
 // ------------------------------------------------------------ radix sort
 constexpr int kRsT = 256, kRsW = kRsT / 32;
-constexpr int kRsI = 16;  // keys per thread: the tile is staged in shared memory before it is written out
+// Keys per thread: the tile is staged in shared memory before it is written out, so 64-bit keys take
+// fewer (static shared memory stays under 48 KB).
+template <typename K> constexpr int kRsItems = sizeof(K) == 8 ? 12 : 16;
 
-__global__ void __launch_bounds__(256) k_rs_hist(const unsigned *keys, unsigned n, int npass, unsigned *hist) {
-    __shared__ unsigned sh[4 * 256];
+template <typename K>
+__global__ void __launch_bounds__(256) k_rs_hist(const K *keys, unsigned n, int npass, unsigned *hist) {
+    __shared__ unsigned sh[sizeof(K) * 256];
     for (int q = threadIdx.x; q < npass * 256; q += 256) sh[q] = 0;
     __syncthreads();
     for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < n; idx += (size_t)gridDim.x * 256) {
-        const unsigned k = keys[idx];
+        const K k = keys[idx];
         for (int p = 0; p < npass; p++) atomicAdd(&sh[p * 256 + (unsigned)((k >> (8 * p)) & 255)], 1u);
     }
     __syncthreads();
@@ -115,19 +118,20 @@ __global__ void __launch_bounds__(256) k_rs_hist(const unsigned *keys, unsigned 
         if (sh[q]) atomicAdd(&hist[q], sh[q]);
 }
 
-// One onesweep pass over a tile of kRsT x kRsI keys: stable ranks by warp-level digit
+// One onesweep pass over a tile of kRsT x kRsItems keys: stable ranks by warp-level digit
 // matching, the tile's offset per digit by decoupled look-back over tiles, then the tile is
 // reordered by digit in shared memory so each digit's run is written out contiguously.
-__global__ void __launch_bounds__(kRsT) k_rs_pass(const unsigned *__restrict__ kin, unsigned *__restrict__ kout,
+template <typename K>
+__global__ void __launch_bounds__(kRsT) k_rs_pass(const K *__restrict__ kin, K *__restrict__ kout,
                                                   const unsigned *__restrict__ vin, unsigned *__restrict__ vout,
                                                   unsigned n, int shift, const unsigned *__restrict__ hist,
                                                   unsigned long long *status, unsigned *ticket, int *err) {
-    constexpr int I = kRsI, TILE = kRsT * I;
+    constexpr int I = kRsItems<K>, TILE = kRsT * I;
     __shared__ unsigned s_wc[kRsW][256];
     __shared__ unsigned s_base[256], s_lstart[256];
     __shared__ unsigned s_tmp[kRsT / 32];
     __shared__ unsigned s_tile;
-    __shared__ unsigned s_key[TILE];
+    __shared__ K s_key[TILE];
     __shared__ unsigned s_val[TILE];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = atomicAdd(ticket, 1u);
@@ -137,7 +141,8 @@ __global__ void __launch_bounds__(kRsT) k_rs_pass(const unsigned *__restrict__ k
     const size_t tbase = (size_t)tile * TILE;
     const size_t wbase = tbase + (size_t)warp * (32 * I);
 
-    unsigned key[I], val[I], dig[I], rank[I];
+    K key[I];
+    unsigned val[I], dig[I], rank[I];
 #pragma unroll
     for (int it = 0; it < I; it++) {
         size_t idx = wbase + (size_t)it * 32 + lane;
@@ -204,7 +209,7 @@ __global__ void __launch_bounds__(kRsT) k_rs_pass(const unsigned *__restrict__ k
     __syncthreads();
     // ltot keys of this tile, digit-sorted: consecutive threads write consecutive addresses.
     for (unsigned q = tid; q < ltot; q += kRsT) {
-        const unsigned k = s_key[q];
+        const K k = s_key[q];
         const unsigned dd = (unsigned)((k >> shift) & 255);
         const unsigned pos = s_base[dd] + (q - s_lstart[dd]);
         if (pos < n) {
@@ -214,43 +219,43 @@ __global__ void __launch_bounds__(kRsT) k_rs_pass(const unsigned *__restrict__ k
     }
 }
 
-size_t radix_sort_tmp_bytes(unsigned n, int bits) {
+template <typename K> size_t radix_sort_tmp_bytes(unsigned n, int bits) {
     int npass = (bits + 7) / 8;
-    size_t tiles = (n + kRsT * kRsI - 1) / (kRsT * kRsI);
+    size_t tiles = ((size_t)n + kRsT * kRsItems<K> - 1) / (kRsT * kRsItems<K>);
     return 256 + (size_t)(npass > 0 ? npass : 1) * 256 * (sizeof(unsigned) + tiles * sizeof(unsigned long long));
 }
 
-cudaError_t radix_sort(unsigned *keys, unsigned *keys_alt, unsigned *vals, unsigned *vals_alt, unsigned n, int bits,
-                       bool identity, void *tmp, int *d_err, cudaStream_t s, int *launches, int *in_alt,
-                       const unsigned *keys_in) {
+template <typename K>
+cudaError_t radix_sort(K *keys, K *keys_alt, unsigned *vals, unsigned *vals_alt, unsigned n, int bits, bool identity,
+                       void *tmp, int *d_err, cudaStream_t s, int *launches, int *in_alt, const K *keys_in) {
     *in_alt = 0;
     int npass = (bits + 7) / 8;
-    if (npass > 4) npass = 4;
+    if (npass > (int)sizeof(K)) npass = (int)sizeof(K);
     if (n == 0) return cudaSuccess;
     if (npass == 0) npass = 1;  // still materialise the values (identity case)
-    constexpr unsigned kTile = kRsT * kRsI;
-    unsigned tiles = (n + kTile - 1) / kTile;
+    constexpr unsigned kTile = kRsT * kRsItems<K>;
+    unsigned tiles = (unsigned)(((size_t)n + kTile - 1) / kTile);
     unsigned *ticket = (unsigned *)tmp;
     unsigned *hist = (unsigned *)((char *)tmp + 256);
     unsigned long long *status = (unsigned long long *)((char *)hist + (size_t)npass * 256 * sizeof(unsigned));
-    cudaError_t e = cudaMemsetAsync(tmp, 0, radix_sort_tmp_bytes(n, bits), s);  // every pass's at once
+    cudaError_t e = cudaMemsetAsync(tmp, 0, radix_sort_tmp_bytes<K>(n, bits), s);  // every pass's at once
     if (e != cudaSuccess) return e;
     unsigned hblocks = (n + 255) / 256;
     if (hblocks > 1216) hblocks = 1216;
-    const unsigned *first = keys_in ? keys_in : keys;
-    k_rs_hist<<<hblocks, 256, 0, s>>>(first, n, npass, hist);
+    const K *first = keys_in ? keys_in : keys;
+    k_rs_hist<K><<<hblocks, 256, 0, s>>>(first, n, npass, hist);
     if (launches) (*launches)++;
-    const unsigned *src = first;
-    unsigned *dst = keys_alt, *other = keys;  // passes after the first ping-pong between keys_alt and keys
+    const K *src = first;
+    K *dst = keys_alt, *other = keys;  // passes after the first ping-pong between keys_alt and keys
     unsigned *vsrc = identity ? nullptr : vals, *vdst = vals_alt;
     for (int p = 0; p < npass; p++) {
-        k_rs_pass<<<tiles, kRsT, 0, s>>>(src, dst, vsrc, vdst, n, 8 * p, hist + p * 256,
+        k_rs_pass<K><<<tiles, kRsT, 0, s>>>(src, dst, vsrc, vdst, n, 8 * p, hist + p * 256,
                                          status + (size_t)p * tiles * 256, ticket + p, d_err);
         if (launches) (*launches)++;
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         src = dst;
-        unsigned *tk = other; other = dst; dst = tk;
+        K *tk = other; other = dst; dst = tk;
         unsigned *written = vdst;
         vdst = (written == vals_alt) ? vals : vals_alt;
         vsrc = written;
@@ -258,5 +263,13 @@ cudaError_t radix_sort(unsigned *keys, unsigned *keys_alt, unsigned *vals, unsig
     *in_alt = (npass & 1);
     return cudaSuccess;
 }
+
+template size_t radix_sort_tmp_bytes<unsigned>(unsigned, int);
+template size_t radix_sort_tmp_bytes<unsigned long long>(unsigned, int);
+template cudaError_t radix_sort<unsigned>(unsigned *, unsigned *, unsigned *, unsigned *, unsigned, int, bool, void *,
+                                          int *, cudaStream_t, int *, int *, const unsigned *);
+template cudaError_t radix_sort<unsigned long long>(unsigned long long *, unsigned long long *, unsigned *, unsigned *,
+                                                    unsigned, int, bool, void *, int *, cudaStream_t, int *, int *,
+                                                    const unsigned long long *);
 
 }  // namespace qses

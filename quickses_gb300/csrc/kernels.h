@@ -32,12 +32,18 @@ cudaError_t launch_mc_emit(const QGrid &g, const unsigned *sign, const unsigned 
                            const unsigned *words, const uint2 *rowBase, unsigned *tri, unsigned long long *vkey,
                            cudaStream_t s);
 // Vertex ids (vmap, per edge slot), welded positions and their count from the edge keys in owner
-// row order (rowBase: the scanned row counts).  skey, sslot: scratch, one entry per edge.
+// row order (rowBase: the scanned row counts).  skey, sslot: scratch, one entry per edge.  total->y:
+// not 0 if the mesh crowds a layer (k_mesh.cu); the results are then launch_weld_sorted's, which
+// overwrites vkey, and until it has run launch_remap leaves the corners alone (crowded: &total->y).
 size_t weld_tmp_bytes(unsigned layers);
 cudaError_t launch_weld(const QGrid &g, const unsigned long long *vkey, const uint2 *rowBase, unsigned ne,
                         unsigned long long *skey, unsigned *sslot, unsigned *vmap, float *vq, uint2 *total, void *tmp,
                         int *err, cudaStream_t s);
-void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, cudaStream_t s);
+constexpr unsigned kWeldSortMin = 4096;  // edges
+cudaError_t launch_weld_sorted(const QGrid &g, unsigned long long *vkey, unsigned long long *skey, unsigned *sslot,
+                               unsigned ne, unsigned *vmap, float *vq, uint2 *total, int *err, cudaStream_t s,
+                               int *launches);
+void launch_remap(unsigned *tri, size_t n3, const unsigned *vmap, const unsigned *crowded, cudaStream_t s);
 void launch_closest(const QGrid &g, const float *vq, unsigned nv, const float4 *atoms, const uint2 *cells,
                     const unsigned *sorted_to_input, int *asorted, int *ainput, cudaStream_t s);
 // Triangles without a repeated corner, in order, to out (which may be tri); their number to *total.
@@ -135,6 +141,11 @@ cudaError_t launch_weld_batch(const QBatch &b, unsigned layers, const unsigned l
                               unsigned ne, const unsigned *edge_off, unsigned long long *skey, unsigned *sslot,
                               unsigned *vmap, float *vq, unsigned *vmol, unsigned *vtx_off, uint2 *total, void *tmp, int *err,
                               cudaStream_t s);
+// bits: of the largest position among the molecules' (with the molecules' numbers at most 64)
+cudaError_t launch_weld_sorted_batch(const QBatch &b, unsigned long long *vkey, unsigned long long *skey, unsigned *sslot,
+                                     unsigned ne, const unsigned *edge_off, int bits, unsigned *vmap, float *vq,
+                                     unsigned *vmol, unsigned *vtx_off, uint2 *total, int *err, cudaStream_t s,
+                                     int *launches);
 void launch_gather_offsets(const uint2 *excl, const unsigned *at, unsigned n_mol, unsigned n, const uint2 *total,
                            unsigned *outx, unsigned *outy, cudaStream_t s);
 void launch_closest_batch(const QBatch &b, const float *vq, const unsigned *vmol, unsigned nv, const float4 *atoms,

@@ -566,7 +566,7 @@ static int enqueue_mesh(qses_context *ctx, const MeshSeg &b, SegOut &o) {
     if (b.ne > 0) {
         QCHK(launch_weld(b.g, b.vk, b.rows, b.ne, b.vk2, b.vv, b.vmap, b.vq, b.tot, b.tmp, b.err, s));
         ctx->launches++;
-        launch_remap(b.tri, b.n3, b.vmap, s);
+        launch_remap(b.tri, b.n3, b.vmap, &b.tot->y, s);
         ctx->launches++;
         QCHK(cudaMemcpyAsync(b.h_out, b.tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
     }
@@ -834,6 +834,14 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     if (NE > 0) {
         QCHK(cudaStreamSynchronize(s));
         memcpy(&tot, ctx->h_small, sizeof(tot));
+        if (tot.y) {  // a crowded layer
+            QCHK(launch_weld_sorted(g, b.vk, b.vk2, b.vv, NE, vmap, vq, a.tot, d_err, s, &ctx->launches));
+            launch_remap(tri, n3, vmap, nullptr, s);
+            ctx->launches++;
+            QCHK(cudaMemcpyAsync(ctx->h_small, a.tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
+            QCHK(cudaStreamSynchronize(s));
+            memcpy(&tot, ctx->h_small, sizeof(tot));
+        }
         nv = tot.x;
     }
     ctx->tick(3);

@@ -154,7 +154,7 @@ static int enqueue_batch_mesh(qses_context *ctx, const BatchMeshSeg &m, SegOut &
         QCHK(launch_weld_batch(m.b, m.layers, m.vk, m.rows, m.ne, m.edge_off, m.vk2, m.vv, m.vmap, m.vq, m.vmol, m.vtx_off,
                                m.tot, m.tmp, m.err, s));
         ctx->launches++;
-        launch_remap(m.tri, m.n3, m.vmap, s);
+        launch_remap(m.tri, m.n3, m.vmap, &m.tot->y, s);
         ctx->launches++;
     } else {
         QCHK(cudaMemsetAsync(m.vtx_off, 0, 4ull * (nm + 1), s));
@@ -482,6 +482,20 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     ctx->tick(2);
     QCHK_RC(run_segment(ctx, kSegBatchMesh, mb, ob, enqueue_batch_mesh));
     QCHK(cudaStreamSynchronize(s));
+    if (NE > 0 && hsm[1]) {  // a crowded layer
+        int bits = 0;
+        for (unsigned m = 0; m < nm; m++) {
+            const unsigned long long Rq = (unsigned long long)items[m].g.Rq;
+            bits = std::max(bits, bits_for(Rq * Rq * Rq - 1));
+        }
+        QCHK(launch_weld_sorted_batch(b, mb.vk, mb.vk2, mb.vv, NE, d_edge_off, bits, vmap, vq, vmol, d_vtx_off, a.tot,
+                                      d_err, s, &ctx->launches));
+        launch_remap(tri, n3, vmap, nullptr, s);
+        ctx->launches++;
+        QCHK(cudaMemcpyAsync(ctx->h_small, a.tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
+        QCHK(cudaMemcpyAsync(ctx->h_stage, d_vtx_off, 4ull * (nm + 1), cudaMemcpyDeviceToHost, s));
+        QCHK(cudaStreamSynchronize(s));
+    }
     ctx->tick(3);
     std::vector<unsigned> vtx_off(nm + 1);
     memcpy(vtx_off.data(), ctx->h_stage, 4ull * (nm + 1));

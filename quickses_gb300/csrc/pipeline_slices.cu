@@ -231,16 +231,23 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                 // ---- triangles and edge keys; weld; the last triangle's own vertices out
                 SCHK(launch_mc_emit(b, sign_mask, codes, lut, in_mask, rows, tri, wb.vk, s));
                 SCHK(launch_weld(b, wb.vk, rows, NE, wb.vk2, wb.vv, vmap, vq, tot, wb.tmp, d_err, s));
-                launch_remap(tri, n3k, vmap, s);
+                launch_remap(tri, n3k, vmap, &tot->y, s);
                 ctx->launches += 3;
                 SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
                 SCHK(cudaStreamSynchronize(s));
+                if (h_tot->y) {  // a crowded layer
+                    SCHK(launch_weld_sorted(b, wb.vk, wb.vk2, wb.vv, NE, vmap, vq, tot, d_err, s, &ctx->launches));
+                    launch_remap(tri, n3k, vmap, nullptr, s);
+                    ctx->launches++;
+                    SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
+                    SCHK(cudaStreamSynchronize(s));
+                }
                 const unsigned V = h_tot->x;
                 SCHK(cudaMemsetAsync(used, 0, 8ull * (V + 1), s));
                 k_mark_used<<<blocks(n3k, 256), 256, 0, s>>>(tri, n3k, used);
                 SCHK(scan_u2(used, excl, V, tot, tmpb, d_err, s, &ctx->launches));
                 k_compact_vertices<<<blocks(V, 256), 256, 0, s>>>(used, excl, V, vq, vq2, vmap2);
-                launch_remap(tri, n3k, vmap2, s);
+                launch_remap(tri, n3k, vmap2, nullptr, s);
                 ctx->launches += 3;
                 SCHK(cudaMemcpyAsync(h_tot, tot, sizeof(uint2), cudaMemcpyDeviceToHost, s));
                 SCHK(cudaStreamSynchronize(s));
