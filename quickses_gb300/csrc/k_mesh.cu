@@ -477,10 +477,9 @@ __device__ __forceinline__ unsigned plane_quantum(const QGrid &g, int i) {
     return (unsigned)(quantum(p) - (int)g.bx);
 }
 // In place: exclusive sums of x[0, n), by the whole block; the total is returned.  squares (may be
-// null, zeroed): the sum of the squares.
+// null, zeroed): the sum of the squares in units of 64, what a thread has over a multiple dropped.
 template <int NT>
-__device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, unsigned *s_tmp,
-                                                    unsigned long long *squares = nullptr) {
+__device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, unsigned *s_tmp, unsigned *squares = nullptr) {
     const unsigned per = (n + NT - 1) / NT, lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
     unsigned sum = 0, total;
     unsigned long long sq = 0;
@@ -489,9 +488,9 @@ __device__ __forceinline__ unsigned block_excl_sums(unsigned *x, unsigned n, uns
         if (squares) sq += (unsigned long long)x[k] * x[k];
     }
     if (squares) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if ((threadIdx.x & 31) == 0 && sq) atomicAdd(squares, sq);
+        // a warp's share ends at 2^32 pairs: no overflow, and above every limit
+        const unsigned warp = warp_sum((unsigned)min(sq >> 6, 0x3ffffffull));
+        if ((threadIdx.x & 31) == 0 && warp) atomicAdd(squares, min(warp, 0x3ffffffu));
     }
     unsigned run = block_excl_scan<NT>(sum, total, s_tmp);
     for (unsigned k = lo; k < hi; k++) {
@@ -523,9 +522,10 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
                                                     unsigned long long *work, int *err) {
     extern __shared__ unsigned s_bin[];  // 2 x (2 cap + 2) and kWeldX / 2
     __shared__ unsigned s_tmp[kWeldT / 32], s_tile, s_pushed, s_before;
-    __shared__ unsigned long long s_work, s_all;
+    __shared__ unsigned s_squares;
+    __shared__ unsigned long long s_all;
     if (threadIdx.x == 0) {
-        s_work = 0;
+        s_squares = 0;
         s_tile = atomicAdd(ticket, 1u);  // layers in the order CTAs start, so that every wait ends
         s_pushed = 0;
     }
@@ -594,13 +594,14 @@ __global__ void __launch_bounds__(kWeldT, 2) k_weld(QGrid g1, QBatch b, unsigned
     }
     if (below) atomicAdd(&s_pushed, below);
     __syncthreads();
-    unsigned n = block_excl_sums<kWeldT>(cur, nbin, s_tmp, &s_work);
-    if (limits.heavy(s_work, n)) {  // seldom; the sum passes its limit for the last to add to it, if not before
-        if (threadIdx.x == 0) s_all = atomicAdd(work, s_work) + s_work;
+    unsigned n = block_excl_sums<kWeldT>(cur, nbin, s_tmp, &s_squares);
+    const unsigned long long pairs = 64ull * s_squares;
+    if (limits.heavy(pairs, n)) {  // seldom; the sum passes its limit for the last to add to it, if not before
+        if (threadIdx.x == 0) s_all = atomicAdd(work, pairs) + pairs;
         __syncthreads();
         crowded |= s_all > limits.all;
     }
-    crowded |= s_work > limits.pairs;
+    crowded |= pairs > limits.pairs;
     if (crowded) {
         s0 = s2 = s1;
         n = 0;
