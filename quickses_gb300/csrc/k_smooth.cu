@@ -126,6 +126,9 @@ __device__ __forceinline__ void red_ext(unsigned *ext, unsigned u, bool go) {
     asm volatile("{\n\t.reg .pred g;\n\tsetp.ne.u32 g, %2, 0;\n\t@g red.relaxed.gpu.global.add.u32 [%0], %1;\n\t}" ::"l"(ext + (u >> 2)),
                  "r"(0u - (1u << (8u * (u & 3u)))), "r"((unsigned)go) : "memory");
 }
+__device__ __forceinline__ void add_ext(unsigned *word, unsigned x) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(word), "r"(x) : "memory");
+}
 // This lane's entry of a list (what past-the-end entries read otherwise).
 __device__ __forceinline__ unsigned ld_entry(const unsigned *p, bool go, unsigned other) {
     unsigned x = other;
@@ -579,9 +582,16 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 q.w = fstamp;
                 st_pos(pos4 + a + k, q);
             }
-            if (pass + 1 < passes)
-                for (unsigned v = a + threadIdx.x; v < b; v += T) ((unsigned char *)ext)[v] = ext0[v];
-            else if (out)
+            if (pass + 1 < passes) {
+                // What the next pass starts with, added to counters that are at zero: other slabs count
+                // down the neighbouring bytes of a word at the slab's ends, by atomics of whole words too.
+                const unsigned *from = (const unsigned *)ext0;
+                for (unsigned w = a / 4 + threadIdx.x; 4 * w < b; w += T) {
+                    const unsigned below = 4 * w < a ? (1u << (8 * (a - 4 * w))) - 1u : 0u;
+                    const unsigned upto = 4 * w + 4 > b ? (1u << (8 * (b - 4 * w))) - 1u : 0xffffffffu;
+                    add_ext(ext + w, __ldg(from + w) & upto & ~below);
+                }
+            } else if (out)
                 for (unsigned k = threadIdx.x; k < 3 * len; k += T) out[3ull * a + k] = ((const float *)(rec + k / 3))[k % 3];
         } else if (stats && threadIdx.x == 0) {
             atomicAdd(stats + 1, 1ull);  // unfinished slabs
