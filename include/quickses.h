@@ -301,9 +301,12 @@ QSES_API int qses_host_timeline(qses_context *ctx, double *ms, int max);
  * waits for a hand-off from a lower slab that never comes, with its wait limited to
  * spin_cycles clock cycles (1e6 .. 4e9); *kernel_status receives the status the kernel wrote
  * (QSES_ERR_TIMEOUT: the wait gave up and every CTA returned).  Returns QSES_OK when the
- * kernel ran and the context is still usable. */
+ * kernel ran and the context is still usable.
+ * qses_debug_smoothing_wait: the cycles without any progress after which a wait of the
+ * smoothing gives up in later calls on ctx (1e6 .. 4e9; 0: the default, 4e9). */
 QSES_API void qses_debug_fail_reservations(unsigned n);
 QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int *kernel_status);
+QSES_API int qses_debug_smoothing_wait(qses_context *ctx, long long spin_cycles);
 
 /* ------------------------------------------------------------------ CUDA graphs */
 

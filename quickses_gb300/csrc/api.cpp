@@ -837,6 +837,12 @@ QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int
     return QSES_OK;
 }
 
+QSES_API int qses_debug_smoothing_wait(qses_context *ctx, long long spin_cycles) {
+    if (!ctx || (spin_cycles != 0 && (spin_cycles < 1000000ll || spin_cycles > qses::kGsSpin))) return QSES_ERR_INVALID_ARG;
+    ctx->gs_spin = spin_cycles ? spin_cycles : qses::kGsSpin;
+    return QSES_OK;
+}
+
 QSES_API int qses_host_timeline(qses_context *ctx, double *ms, int max) {
     if (!ctx || !ms) return 0;
     int k = 0;

@@ -181,15 +181,41 @@ __device__ __forceinline__ float add4(float s, float4 q) {
     return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, q.x), q.y), q.z), q.w);
 }
 
+// A wait's clock.  It runs out spin_cycles after the last sign of progress: one that the waiter sees
+// itself (restart) or an item taken from the counter since, by a CTA that has finished another.  So
+// a wait behind a long queue of slabs lasts while they are being done, however slowly, and ends
+// when none is.
+struct GsClock {
+    long long since;
+    unsigned taken;  // what the counter had at the last look
+    __device__ __forceinline__ explicit GsClock(unsigned item) {
+        since = clock64();
+        taken = item + 1;
+    }
+    __device__ __forceinline__ void restart() { since = clock64(); }
+    __device__ __forceinline__ bool out(const unsigned *next_slab, long long spin_cycles) {
+        const long long now = clock64();
+        if (now - since <= spin_cycles) return false;
+        unsigned k;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(k) : "l"(next_slab) : "memory");
+        const bool none = k == taken;
+        taken = k;
+        since = now;
+        return none;
+    }
+};
+
 // Waits until slab p and the slabs of all its higher neighbours have had `pass` passes; false if
 // that takes too long.
-__device__ __forceinline__ bool gs_wait_pass(const GsOrder &ord, unsigned p, unsigned pass, long long spin_cycles) {
-    const long long since = clock64();
-    for (unsigned j = p; j <= ord.far[p]; j++)
+__device__ __forceinline__ bool gs_wait_pass(const GsOrder &ord, unsigned p, unsigned pass, GsClock clock,
+                                             const unsigned *next_slab, long long spin_cycles) {
+    for (unsigned j = p; j <= ord.far[p]; j++) {
         while (ld_acquire_u32(&ord.done[j]) < pass) {
-            if (clock64() - since > spin_cycles) return false;
+            if (clock.out(next_slab, spin_cycles)) return false;
             __nanosleep(200);
         }
+        clock.restart();
+    }
     return true;
 }
 
@@ -239,7 +265,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
               long long spin_cycles, unsigned long long *stats) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ GsQueue s_q;
-    __shared__ unsigned s_slab, s_pass;
+    __shared__ unsigned s_slab, s_pass, s_item;
     // Per worker warp: the neighbours' coordinates, one row per component, summed in list order
     __shared__ __align__(16) float s_row[kGsThreadsMax / 32][3 * kGsRow];
     __shared__ unsigned s_void[32];  // target of touch_l1
@@ -266,11 +292,12 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
         if (threadIdx.x == 0) {
             const unsigned k = atomicAdd(next_slab, 1u);
             s_slab = 0xffffffffu;
+            s_item = k;
             if (k < Q * passes && !s_q.stop) {
                 const GsItem it = gs_item(k, Q, passes, lag);
                 s_slab = __ldg(order + it.place);
                 s_pass = it.pass;
-                if (it.pass && !gs_wait_pass(ord, s_slab, it.pass, spin_cycles)) {
+                if (it.pass && !gs_wait_pass(ord, s_slab, it.pass, GsClock(k), next_slab, spin_cycles)) {
                     raise_error(err, QSES_ERR_TIMEOUT);
                     s_q.stop = 1;
                     s_slab = 0xffffffffu;
@@ -311,7 +338,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
             // watches 32 vertices at a time: the bytes of those still waiting; a byte at zero means
             // that every neighbour in a lower slab has been updated.
             unsigned idle_ns = 0, done_seen = 0;
-            long long last = clock64();
+            GsClock clock(s_item);
             for (;;) {
                 const unsigned d = *v_done;
                 if (__any_sync(0xffffffffu, d >= len || *v_stop)) break;
@@ -346,10 +373,9 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 any = __any_sync(0xffffffffu, any);
                 left = __any_sync(0xffffffffu, left);
                 if (!left) break;  // nobody here waits for a lower slab any more
-                const long long now = clock64();
-                if (any || d != done_seen) last = now;
+                if (any || d != done_seen) clock.restart();
                 done_seen = d;
-                if (now - last > spin_cycles) {
+                if (__any_sync(0xffffffffu, clock.out(next_slab, spin_cycles))) {
                     if (lane == 0) {
                         raise_error(err, QSES_ERR_TIMEOUT);
                         *v_stop = 1;
@@ -362,15 +388,14 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
             // The workers' own wait for a vertex ends with the slab or an error; it is watched here
             // once no arrival is expected any more.
             if (warp == 0) {
-                long long since = clock64();
+                clock.restart();
                 unsigned seen = *v_done;
                 while (true) {
                     const unsigned d = *v_done;
                     if (__any_sync(0xffffffffu, d >= len || *v_stop)) break;
-                    const long long now = clock64();
-                    if (d != seen) since = now;
+                    if (d != seen) clock.restart();
                     seen = d;
-                    if (now - since > spin_cycles) {
+                    if (__any_sync(0xffffffffu, clock.out(next_slab, spin_cycles))) {
                         if (lane == 0) {
                             raise_error(err, QSES_ERR_TIMEOUT);
                             *v_stop = 1;

@@ -83,6 +83,7 @@ cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax,
                            const unsigned char *ext0, unsigned passes, unsigned stamp, const GsOrder &ord, int *err,
                            float *out, long long spin_cycles, unsigned long long *stats, cudaStream_t s);
 int gs_slab_max_blocks(int device, unsigned S, int threads);
+constexpr long long kGsSpin = 4000000000ll;  // cycles without progress after which a wait gives up
 
 // Gauss-Seidel launch shape: threads per slab CTA and the slab size aimed at (vertices);
 // the result does not depend on it, only the time does.  The cache flags name policies of an

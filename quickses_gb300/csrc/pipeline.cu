@@ -444,7 +444,8 @@ bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool
 
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
                   const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
-                  const unsigned *h_table, int *d_err, unsigned long long *stats, cudaEvent_t before_writeback, float *h_out,
+                  const unsigned *h_table, int *d_err, unsigned long long *stats, long long spin_cycles,
+                  cudaEvent_t before_writeback, float *h_out,
                   const std::function<int()> &beside) {
     cudaStream_t s = ctx->stream;
     float4 *pos4 = sb.pos4;
@@ -482,7 +483,7 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
             QCHK(launch_gs_slab(pos4, v0, v1, L.smax, gb.table + (size_t)w * L.table_words, L.qcap, gb.next_slab, L.ctas,
                                 sh.threads, sb.deg, sb.nbr, sb.word0, sb.pack, sb.ext, (const unsigned char *)sb.ext0,
                                 together ? (unsigned)passes : 1u, (unsigned)pass + 1u, gb.ord, d_err,
-                                together || pass == passes - 1 ? h_out : nullptr, 4000000000ll,
+                                together || pass == passes - 1 ? h_out : nullptr, spin_cycles,
                                 ctx->profiling ? stats : nullptr, s));
             ctx->launches++;
         }
@@ -594,6 +595,7 @@ struct FinishSeg {
     GsBuffers gb;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
     unsigned long long *stats;
+    long long spin;        // wait limit of the smoothing
     unsigned long long n3;
     unsigned nv, nt;
     int passes, keep_all, fork, late;  // late: the side stream starts behind the neighbour lists
@@ -659,7 +661,7 @@ static int enqueue_finish(qses_context *ctx, const FinishSeg &c, SegOut &o) {
     if (smooth) {
         // the closest-atom pass on the side stream reads the welded positions in vq
         const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table,
-                                     c.err, c.stats, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices,
+                                     c.err, c.stats, c.spin, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices,
                                      c.late ? std::function<int()>(beside) : nullptr);
         if (rc) return rc;
     }
@@ -883,6 +885,7 @@ int run_pipeline(qses_context *ctx, const qses_params &p, const float *d_xyz, co
     c.sb = sb;
     c.scratch = vmap;  // free after the weld
     c.stats = (unsigned long long *)((char *)ctx->small + 256);
+    c.spin = ctx->gs_spin;
     c.n3 = n3;
     c.nv = nv;
     c.nt = T;

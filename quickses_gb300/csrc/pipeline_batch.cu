@@ -186,6 +186,7 @@ struct BatchFinishSeg {
     unsigned *scratch;     // one word per vertex
     GsBuffers gb;
     const unsigned *h_table;  // pinned slab tables; the copy node reads them when the segment runs
+    long long spin;           // wait limit of the smoothing
     unsigned long long n3;
     unsigned nv, nt;
     int passes, fork, late, pad_;  // late: the side stream starts behind the neighbour lists
@@ -242,7 +243,7 @@ static int enqueue_batch_finish(qses_context *ctx, const BatchFinishSeg &c, SegO
     if (smooth) {
         // the closest-atom pass on the side stream reads the welded positions in vq
         const int rc = run_smoothing(ctx, c.sh, c.gl, c.passes, c.vq, c.nv, c.tri, c.n3, c.sb, c.scratch, c.gb, c.h_table,
-                                     c.err, nullptr, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices,
+                                     c.err, nullptr, c.spin, c.fork ? ctx->ev_join : nullptr, (float *)h_vertices,
                                      c.late ? std::function<int()>(beside) : nullptr);
         if (rc) return rc;
     }
@@ -539,6 +540,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     }
     c.sb = sb;
     c.scratch = vmap;  // free after the weld
+    c.spin = ctx->gs_spin;
     c.n3 = n3;
     c.nv = nv;
     c.nt = T;

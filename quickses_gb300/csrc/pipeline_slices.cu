@@ -266,7 +266,7 @@ int run_pipeline_slices(qses_context *ctx, const qses_params &p, const float *d_
                     const int brc = gs_buffers(ctx, plan, gb);
                     if (brc != QSES_OK) return brc;
                     const int src = run_smoothing(ctx, sh, plan.L, p.smooth_passes, vq2, nv, tri, n3k, sb, vmap, gb,
-                                                  ctx->h_gs, d_err, stats);
+                                                  ctx->h_gs, d_err, stats, ctx->gs_spin);
                     if (src != QSES_OK) return src;
                 }
                 unsigned nt = T1;

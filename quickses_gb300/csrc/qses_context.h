@@ -146,6 +146,7 @@ struct qses_context {
     unsigned long long last_d2h = 0;  // device-to-host bytes of the last qses_compute
     qses::GsShape gs_force{0, 0, 0, 0};  // autotuner: forced smoothing shape (threads 0 = none)
     qses::GsShape gs_used;            // shape of the last smoothing run
+    long long gs_spin = qses::kGsSpin;  // wait limit of the smoothing (qses_debug_smoothing_wait)
     int edt_force = -1;               // autotuner: forced refine tile shape (-1 = none)
     int edt_used = 0;
     unsigned long long diag[10] = {0};  // smoothing diagnostics: slabs, slab size, max/idle/total rounds
@@ -225,7 +226,7 @@ bool take_weld_or_smooth(Arena &a, unsigned ne, unsigned layers, size_t n3, bool
 // beside (may be null): enqueues other streams' work, once the lists are done.
 int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int passes, float *vq, unsigned nv,
                   const unsigned *tri, size_t n3, const SmoothBuffers &sb, unsigned *scratch, const GsBuffers &gb,
-                  const unsigned *h_table, int *d_err, unsigned long long *stats,
+                  const unsigned *h_table, int *d_err, unsigned long long *stats, long long spin_cycles,
                   cudaEvent_t before_writeback = nullptr, float *h_out = nullptr,
                   const std::function<int()> &beside = nullptr);
 bool side_work_late(int device, int ctas, unsigned slabs);
