@@ -204,11 +204,13 @@ def run_gpu(args):
             dm = step()
         torch.cuda.synchronize()
         # per-stage times on a separate profiled call (events on the context stream)
-        ctx.set_profiling(True)
+        ctx.set_profiling(2)
         step()
         stages = ctx.stage_times()
+        ctx.set_profiling(1)  # with the cycle counts, which slow the smoothing down
+        step()
         diag = ctx.diagnostics()
-        ctx.set_profiling(False)
+        ctx.set_profiling(0)
         launches = ctx.last_launch_count()
         torch.cuda.synchronize()
         if world > 1:
@@ -341,10 +343,10 @@ def time_config(ctx, stream, wl, flush, args):
             e1.record(stream)
             e1.synchronize()
             times.append(e0.elapsed_time(e1))
-        ctx.set_profiling(True)
+        ctx.set_profiling(2)
         ctx.compute_device(d_xyz.data_ptr(), d_rad.data_ptr(), n, voxel=wl.voxel, smooth=wl.smooth)
         stages = ctx.stage_times()
-        ctx.set_profiling(False)
+        ctx.set_profiling(0)
     torch.cuda.synchronize()
     lib = L.lib()
     pr = L.Params()
@@ -610,11 +612,11 @@ def run_batch_form(args):
         tune = ctx.autotune_batch(reqs)  # launch-shape tuning, before the warm-up
         for _ in range(args.warmup):
             _raw_batch(lib, L, ctx, rr, n)
-        ctx.set_profiling(True)
+        ctx.set_profiling(2)
         _raw_batch(lib, L, ctx, rr, n)
         stages = ctx.stage_times()
         launches = ctx.last_launch_count()
-        ctx.set_profiling(False)
+        ctx.set_profiling(0)
         times, timelines = [], []
         clk.mark()
         for _ in range(args.steps):

@@ -268,7 +268,8 @@ QSES_API const char *qses_status_string(int status);
 QSES_API const char *qses_last_error(qses_context *ctx);
 
 /* Per-stage device times (ms, CUDA events on the context stream) of the last call when
- * profiling is on.  Returns the number of stages written. */
+ * profiling is on (1; 2: without the smoothing's cycle counts of qses_diagnostics, which make
+ * that stage slower).  Returns the number of stages written. */
 QSES_API int qses_set_profiling(qses_context *ctx, int on);
 QSES_API int qses_stage_times(qses_context *ctx, float *ms, const char **names, int max);
 /* Number of kernels the last call launched. */
@@ -277,11 +278,13 @@ QSES_API int qses_last_launch_count(qses_context *ctx);
  * pre-filter count so it can start while the smoothing pass runs). */
 QSES_API unsigned long long qses_last_download_bytes(qses_context *ctx);
 /* Smoothing diagnostics of the last call: [0] slabs, [1] vertices per slab, [2] most
- * boundary polls of one slab, [3] slabs that did not finish, [6] vertices updated (summed
- * over passes); [2], [3] and [6] are counted on calls made with profiling on
- * (qses_set_profiling) and are 0 otherwise.  [4], [5] and [7]-[9] held clock cycles of parts of
- * an update; clock reads lengthen the dependency chain, so they are no longer taken and read 0.
- * Returns the number of values written. */
+ * boundary polls of one slab, [3] slabs that did not finish, [4] clock cycles spent in
+ * vertex updates, [5] in releasing successors, [6] vertices updated (summed over passes), [7]
+ * cycles until a vertex's neighbour ids arrived, [8] then until their positions arrived, [9] in
+ * the position store and its fence (summed over warps, of which each updates one or two
+ * vertices at a time); [2]-[9] are counted on calls made with profiling on
+ * (qses_set_profiling; [4], [5] and [7]-[9] only with 1) and are 0 otherwise.  Returns the
+ * number of values written. */
 QSES_API int qses_diagnostics(qses_context *ctx, unsigned long long *out, int max);
 
 /* Host timeline of the last pipeline run on ctx (ms; for a batch call, its last batch):

@@ -225,6 +225,8 @@ class Context:
         return order, keys
 
     def set_profiling(self, on=True):
+        """Stage times and smoothing diagnostics of later calls: 1 (True) with the clock cycles of an
+        update's parts, which slow the smoothing down, 2 without, 0 (False) off."""
         self._lib.qses_set_profiling(self._h, int(on))
 
     def stage_times(self):

@@ -623,8 +623,8 @@ QSES_API int qses_autotune(qses_context *ctx, const qses_params *p, const qses_f
     const int nc = qses::gs_shape_candidates(cand, 128);
     qses::GsShape best = cand[0];
     float best_ms = -1.0f;
-    const bool prof = ctx->profiling;
-    ctx->profiling = true;
+    const int prof = ctx->profiling;
+    ctx->profiling = qses_context::kProfileStages;
     unsigned nv = 0;
     if (n > 1 && p->smooth_passes > 0) {
         for (int c = 0; c < nc && rc == QSES_OK; c++) {
@@ -739,7 +739,7 @@ QSES_API const char *qses_last_error(qses_context *ctx) { return ctx ? ctx->last
 
 QSES_API int qses_set_profiling(qses_context *ctx, int on) {
     if (!ctx) return QSES_ERR_INVALID_ARG;
-    ctx->profiling = on != 0;
+    ctx->profiling = on == 2 ? qses_context::kProfileStages : on ? qses_context::kProfileAll : qses_context::kProfileOff;
     return QSES_OK;
 }
 
@@ -827,7 +827,7 @@ QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int
     if (e == cudaSuccess) e = cudaMemcpyAsync(pos, pos_h, sizeof(pos_h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = qses::launch_gs_slab(pos, 0, 4, 2, table, 2, next_slab, 2, 512, start, nbr, word0, pack, ext, nullptr, 1u, 1u,
-                                 qses::GsOrder{}, err, nullptr, spin_cycles, nullptr, s);
+                                 qses::GsOrder{}, err, nullptr, spin_cycles, nullptr, false, s);
     int h_err = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -134,7 +134,7 @@ int main(int argc, const char **argv) {
         fprintf(stderr, "QuickSES: %s\n", qses_status_string(rc));
         return 1;
     }
-    qses_set_profiling(ctx, times ? 1 : 0);
+    qses_set_profiling(ctx, times ? 2 : 0);
     qses_params p;
     qses_params_default(&p);
     p.voxel = voxel;

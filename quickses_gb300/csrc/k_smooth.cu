@@ -247,6 +247,17 @@ __device__ __forceinline__ GsItem gs_item(unsigned n, unsigned Q, unsigned passe
     return {(unsigned)(lo - (unsigned long long)lag * pass), pass};
 }
 
+// What a warp spends its steps on, in clock cycles.
+struct GsCycles {
+    unsigned long long update = 0, release = 0, ids = 0, position = 0, fence = 0;
+};
+// The clock once x is there.
+__device__ __forceinline__ long long clock_behind(unsigned x) {
+    asm volatile("{\n\t.reg .b32 t;\n\tmov.b32 t, %0;\n\t}" ::"r"(x) : "memory");
+    return clock64();
+}
+__device__ __forceinline__ long long clock_behind(float x) { return clock_behind(__float_as_uint(x)); }
+
 // Persistent CTAs take the wave's slabs from a counter, in the table's order (a slab only
 // waits for slabs taken before it, by CTAs that were running when they took them, so every
 // wait ends without a co-residency guarantee).  Per slab the first two warps watch the release
@@ -254,9 +265,12 @@ __device__ __forceinline__ GsItem gs_item(unsigned n, unsigned Q, unsigned passe
 // slabs still to come), the other warps update vertices.
 // Table: Q, the Q + 1 slab bounds in id order (qcap + 1 slots), then the Q slab ids in the
 // order they are taken.
+// COUNT: the clock cycles of an update's parts are added up too (stats not null), which lengthens every
+// step; a kernel of its own, for calls that ask for them.
 // out (may be null): host memory that the last pass's positions go to as each slab is done, 3 floats
 // a vertex.  Behind the kernel the copy of 44 MB took 0.22 ms of 8.2, that of 16 trajectory frames 0.16
 // of 3.34.
+template <bool COUNT>
 __global__ void __launch_bounds__(kGsThreadsMax, 1)
     k_gs_flow(float4 *pos4, unsigned v0, unsigned nv, unsigned smax, const unsigned *__restrict__ table, unsigned qcap,
               unsigned *next_slab, const uint2 *__restrict__ start, const unsigned *__restrict__ nbr,
@@ -283,6 +297,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
     const unsigned lag = passes > 1 ? *ord.lag : 1u;
     const unsigned v_scratch = (unsigned)__cvta_generic_to_shared(&s_void[lane]);
     unsigned long long polls = 0;
+    GsCycles cyc;  // COUNT
     if (threadIdx.x == 0) {
         s_q.stop = 0;
         rec[smax] = make_float4(-0.0f, -0.0f, -0.0f, 0.0f);
@@ -425,6 +440,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
             // release nothing and keep their vertex.  No branch: the step is one basic block (a branch
             // in it, taken or not, cost it 80-110 cycles), with predicated accesses instead.
             auto step = [&](bool &odd, bool &surplus) {
+                const long long c0 = COUNT ? clock64() : 0, c1 = COUNT ? clock_behind(code) : 0;
                 const float2 fr = s_rcp[(word >> 9) & 15u];
                 float4 q = ld_rec(rec_s + 16 * min(code & 0x1fffffffu, smax));
                 touch_l1(v_scratch, packs + 16 * (code & 0xffffu) + ((code >> 29) & 1u) * 8, (code >> 30) == 1u);
@@ -432,6 +448,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 // Neighbours in other slabs: positions of this pass below (a release may overtake its
                 // position), of the last one above.
                 ld_pos_if(q, pos4 + (code & 0x1fffffffu), (int)code < 0);
+                const long long c2 = COUNT ? clock_behind(q.x) : 0;
                 const bool stale = (code >> 30) == 2u && __float_as_uint(q.w) != stamp;
                 row[lane] = q.x; row[kGsRow + lane] = q.y; row[2 * kGsRow + lane] = q.z;
                 __syncwarp();
@@ -439,9 +456,12 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 const float4 q0 = crow[0], q1 = crow[1], q2 = crow[2], q3 = crow[3];
                 const float sum = add4(add4(add4(add4(0.0f, q0), q1), q2), q3);
                 odd = ((__ballot_sync(0xffffffffu, stale || gs_tiny(sum)) >> half) & 0xffffu) != 0u;
-                st_comp(comp + 16 * i, gs_div(sum, fr.x, fr.y), hl < 3 && act && !odd);
+                const float at = gs_div(sum, fr.x, fr.y);
+                const long long c3 = COUNT ? clock_behind(at) : 0;
+                st_comp(comp + 16 * i, at, hl < 3 && act && !odd);
                 __syncwarp();
                 fence_cta();  // release: the position before the counters
+                const long long c4 = COUNT ? clock64() : 0;
                 const unsigned k = code & 0xffffu, old = dec_rec(rec_s + 16 * k, (code >> 29) == kGsSucc && !odd);
                 const bool now = (old & 0x7fu) == 1u;
                 const unsigned ready = (__ballot_sync(0xffffffffu, now) >> half) & 0xffffu;
@@ -463,6 +483,10 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 code = ld_entry(packs + 16 * i + hl, act && !odd && !(word & kGsLong), odd ? code : smax);
                 gs_fill(ring_s, slot, k, now && lane != f);
                 surplus = !act && (int)(qt.y - qt.x) > 0;  // more vertices ready than warps wait for, and a half free
+                if (COUNT) {
+                    cyc.ids += c1 - c0, cyc.position += c2 - c1, cyc.fence += c4 - c3, cyc.update += c4 - c0;
+                    cyc.release += clock_behind((unsigned)surplus) - c4;
+                }
             };
             for (;;) {
                 // Nothing at hand: wait for a vertex (the ring's slot of this warp's ticket).
@@ -512,11 +536,14 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                                 n = 2 * (start[a + vi + 1].x - e);
                             }
                         }
+                        const long long c0 = COUNT ? clock64() : 0;
                         float sum = 0.0f;
                         unsigned first = smax;
                         for (unsigned base = 0; base < n; base += 32) {
                             const unsigned cd = ld_entry(ids + base + lane, base + lane < n, smax);
                             if (base == 0) first = cd;
+                            const long long ca = COUNT ? clock_behind(cd) : 0;
+                            if (COUNT && base == 0) cyc.ids += ca - c0;
                             float4 q = ld_rec(rec_s + 16 * min(cd & 0x1fffffffu, smax));
                             const float4 *up = pos4 + (cd & 0x1fffffffu);
                             ld_pos_if(q, up, (int)cd < 0);
@@ -530,15 +557,20 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                                 }
                                 ld_pos_if(q, up, stale);
                             }
+                            if (COUNT && base == 0) cyc.position += clock_behind(q.x) - ca;
                             __syncwarp();  // the rows are rewritten
                             row[lane] = q.x; row[kGsRow + lane] = q.y; row[2 * kGsRow + lane] = q.z;
                             __syncwarp();
                             const float4 *all = (const float4 *)(row + kGsRow * min(hl, 2u));
                             for (int j = 0; j < 8; j++) sum = add4(sum, all[j]);
                         }
-                        st_comp(comp + 16 * vi, __fdiv_rn(sum, (float)(int)n), lane < 3);
+                        const float at = __fdiv_rn(sum, (float)(int)n);
+                        const long long c3 = COUNT ? clock_behind(at) : 0;
+                        st_comp(comp + 16 * vi, at, lane < 3);
                         __syncwarp();
                         fence_cta();  // release: the position before the counters
+                        const long long c4 = COUNT ? clock64() : 0;
+                        if (COUNT) cyc.fence += c4 - c3, cyc.update += c4 - c0;
                         float4 r = ld_rec(rec_s + 16 * vi);
                         r.w = fstamp;
                         unsigned next = kGsEmpty, nw = 0;
@@ -558,6 +590,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                             st_pos(pos4 + a + vi, r, (cd >> 29) == kGsFar);
                             red_ext(ext, cd & 0x1fffffffu, (cd >> 29) == kGsFar);
                         }
+                        if (COUNT) cyc.release += clock_behind(next) - c4;
                         if (half == h) {
                             done++;
                             act = next != kGsEmpty;
@@ -628,6 +661,13 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
         }
     }  // next slab
     if (stats && threadIdx.x == 0) atomicMax(stats, polls);
+    if (COUNT && stats && lane == 0 && warp >= kGsRecvWarps) {
+        atomicAdd(stats + 2, cyc.update);
+        atomicAdd(stats + 3, cyc.release);
+        atomicAdd(stats + 5, cyc.ids);
+        atomicAdd(stats + 6, cyc.position);
+        atomicAdd(stats + 7, cyc.fence);
+    }
 }
 
 // Where a vertex's lists end up, and the counts that make its word.
@@ -875,10 +915,11 @@ cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax,
                            unsigned qcap, unsigned *next_slab, int P, int threads,
                            const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
                            const unsigned char *ext0, unsigned passes, unsigned stamp, const GsOrder &ord, int *err,
-                           float *out, long long spin_cycles, unsigned long long *stats, cudaStream_t s) {
+                           float *out, long long spin_cycles, unsigned long long *stats, bool cycles, cudaStream_t s) {
     if (smax == 0 || smax > kGsSlabCap) return cudaErrorInvalidValue;
     const size_t smem = gs_slab_smem(smax);
-    const void *fn = (const void *)k_gs_flow;
+    // the same registers per thread at most, so as many blocks fit with COUNT
+    const void *fn = stats && cycles ? (const void *)k_gs_flow<true> : (const void *)k_gs_flow<false>;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs_slab_smem(kGsSlabCap));
     void *args[] = {&pos, &v0, &nv, &smax, (void *)&table, &qcap, &next_slab, (void *)&start, (void *)&nbr,
                     (void *)&word0, (void *)&pack, &ext, (void *)&ext0, &passes, &stamp, (void *)&ord, &out, &err,
@@ -921,7 +962,7 @@ void gs_l2_window(int device, cudaStream_t s, const void *p, size_t bytes) {
 }
 
 int gs_slab_max_blocks(int device, unsigned S, int threads) {
-    const void *fn = (const void *)k_gs_flow;
+    const void *fn = (const void *)k_gs_flow<false>;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs_slab_smem(kGsSlabCap));
     int per_sm = 0, sms = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads >= 1024 ? 1024 : 512, gs_slab_smem(S));

@@ -76,12 +76,13 @@ void launch_from_float4(const float4 *v4, unsigned nv, float *v3, cudaStream_t s
 // vertices), taken by P persistent CTAs from *next_slab (zeroed).  passes > 1: that many passes,
 // each following the one before through the slabs (ext0: the release counters a pass starts with).
 // stamp: written to w of every position updated, one more for each pass (another value than any
-// position holds before).  threads: 512 or 1024 per slab CTA.
+// position holds before).  threads: 512 or 1024 per slab CTA.  cycles: those of an update's parts too
+// (stats[2], [3] and [5]-[7]), which makes it slower.
 cudaError_t launch_gs_slab(float4 *pos, unsigned v0, unsigned nv, unsigned smax, const unsigned *table,
                            unsigned qcap, unsigned *next_slab, int P, int threads,
                            const uint2 *start, const unsigned *nbr, const unsigned *word0, const uint4 *pack, unsigned *ext,
                            const unsigned char *ext0, unsigned passes, unsigned stamp, const GsOrder &ord, int *err,
-                           float *out, long long spin_cycles, unsigned long long *stats, cudaStream_t s);
+                           float *out, long long spin_cycles, unsigned long long *stats, bool cycles, cudaStream_t s);
 int gs_slab_max_blocks(int device, unsigned S, int threads);
 constexpr long long kGsSpin = 4000000000ll;  // cycles without progress after which a wait gives up
 

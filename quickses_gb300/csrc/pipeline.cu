@@ -484,7 +484,7 @@ int run_smoothing(qses_context *ctx, const GsShape &sh, const GsLaunch &L, int p
                                 sh.threads, sb.deg, sb.nbr, sb.word0, sb.pack, sb.ext, (const unsigned char *)sb.ext0,
                                 together ? (unsigned)passes : 1u, (unsigned)pass + 1u, gb.ord, d_err,
                                 together || pass == passes - 1 ? h_out : nullptr, spin_cycles,
-                                ctx->profiling ? stats : nullptr, s));
+                                ctx->profiling ? stats : nullptr, ctx->profiling == qses_context::kProfileAll, s));
             ctx->launches++;
         }
     }

@@ -139,7 +139,8 @@ struct qses_context {
     void *h_stage = nullptr;          // pinned staging for batch uploads (grows)
     size_t h_stage_cap = 0;
     std::string last_error;
-    bool profiling = false;
+    enum { kProfileOff = 0, kProfileAll, kProfileStages };  // kProfileStages: without the smoothing's cycle counts
+    int profiling = kProfileOff;
     std::vector<std::pair<const char *, cudaEvent_t>> marks;
     std::vector<std::pair<const char *, float>> times;
     int launches = 0;
