@@ -381,7 +381,9 @@ QSES_API int qses_grid_info_for(const qses_float3 *atoms, const float *radii, un
 QSES_API int qses_debug_codes(qses_context *ctx, uint8_t *codes, size_t bytes);
 /* Cell-sorted atom order of the last call: sorted_to_input[n], cell hash per sorted atom. */
 QSES_API int qses_debug_atom_order(qses_context *ctx, uint32_t *sorted_to_input, uint32_t *hash, unsigned n);
-/* Slab plan of the smoothing pass, for tests (no reference counterpart, no GPU needed): nv
+/* A slab plan, for tests (no reference counterpart, no GPU needed), as cache_flags ask for it;
+ * the plan that a smoothing pass gets is qses_debug_smoothing_plan's, whose slabs hold at most
+ * 11 904 vertices and may be more than there are CTAs.  nv
  * vertices, molecules' vertex ranges mol_off (nm + 1 entries; NULL = one molecule) and
  * depth estimates, smoothing shape (threads, target, cache_flags, wave as
  * qses_set_smoothing_shape) and
@@ -391,6 +393,9 @@ QSES_API int qses_debug_atom_order(qses_context *ctx, uint32_t *sorted_to_input,
 QSES_API int qses_debug_slab_plan(unsigned nv, const unsigned *mol_off, const int *depth, unsigned nm, int threads,
                                   unsigned target, unsigned cache_flags, unsigned wave, int pmax, unsigned *launch,
                                   unsigned *table, size_t cap);
+QSES_API int qses_debug_smoothing_plan(unsigned nv, const unsigned *mol_off, const int *depth, unsigned nm, int threads,
+                                       unsigned target, unsigned wave, int pmax, unsigned *launch, unsigned *table,
+                                       size_t cap);
 
 /* --------------------------------------------------------- synthetic molecules */
 QSES_API int qses_synth_ball(unsigned N, uint64_t seed, float density, float min_dist, float *xyz,

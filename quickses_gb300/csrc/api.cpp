@@ -443,6 +443,17 @@ QSES_API void qses_mesh_release(qses_mesh *m) {
 
 namespace {
 
+// A plan's launch values and slab tables, for tests.
+int plan_out(const qses::GsPlan &pl, unsigned *launch, unsigned *table, size_t cap) {
+    const unsigned v[6] = {(unsigned)pl.L.ctas, pl.L.smax, pl.L.qcap, pl.L.wsize, pl.L.waves, pl.L.table_words};
+    memcpy(launch, v, sizeof(v));
+    if (table) {
+        if (cap < pl.table.size()) return QSES_ERR_INVALID_ARG;
+        memcpy(table, pl.table.data(), 4 * pl.table.size());
+    }
+    return QSES_OK;
+}
+
 // Host bounds + reference sizing of one request (the device path reads the same bounds
 // with k_atom_minmax: min/max/max-radius are exact either way).
 int size_request(const qses_request &r, QGrid &g) {
@@ -773,14 +784,17 @@ QSES_API int qses_debug_slab_plan(unsigned nv, const unsigned *mol_off, const in
     qses::GsPlan pl;
     const int rc =
         qses::gs_plan_for(pmax, qses::GsShape{threads, target, cache_flags, wave}, nv, mol_off, depth, nm, pl);
-    if (rc != QSES_OK) return rc;
-    const unsigned v[6] = {(unsigned)pl.L.ctas, pl.L.smax, pl.L.qcap, pl.L.wsize, pl.L.waves, pl.L.table_words};
-    memcpy(launch, v, sizeof(v));
-    if (table) {
-        if (cap < pl.table.size()) return QSES_ERR_INVALID_ARG;
-        memcpy(table, pl.table.data(), 4 * pl.table.size());
-    }
-    return QSES_OK;
+    return rc != QSES_OK ? rc : plan_out(pl, launch, table, cap);
+}
+
+QSES_API int qses_debug_smoothing_plan(unsigned nv, const unsigned *mol_off, const int *depth, unsigned nm, int threads,
+                                       unsigned target, unsigned wave, int pmax, unsigned *launch, unsigned *table,
+                                       size_t cap) {
+    if (!launch || (nm > 1 && !mol_off)) return QSES_ERR_INVALID_ARG;
+    qses::GsPlan pl;
+    const int rc =
+        qses::gs_plan_resident(pmax, qses::GsShape{threads, target, 0, wave}, nv, mol_off, depth, nm, pl);
+    return rc != QSES_OK ? rc : plan_out(pl, launch, table, cap);
 }
 
 QSES_API void qses_debug_fail_reservations(unsigned n) { qses::g_fail_reserves.store(n); }

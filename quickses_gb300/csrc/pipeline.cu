@@ -251,24 +251,34 @@ static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 static unsigned ceil_div(unsigned long long a, unsigned long long b) { return (unsigned)((a + b - 1) / b); }
 
+// Every slab's state is in shared memory: at most kGsSlabCap vertices, and smaller targets fit more
+// CTAs per SM.
+static GsShape gs_resident_shape(GsShape sh) {
+    sh.flags |= kGsSmemPos;
+    sh.cap = kGsSlabCap;
+    return sh;
+}
+
 int gs_plan(int device, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
             GsPlan &pl) {
-    // every slab's state is in shared memory: at most kGsSlabCap vertices, and smaller targets fit
-    // more CTAs per SM
-    GsShape in = sh;
-    in.flags |= kGsSmemPos;
-    in.cap = kGsSlabCap;
-    const int pmax = std::min(gs_slab_max_blocks(device, std::min(std::max(in.target, 256u), in.cap), in.threads), 1024);
+    const unsigned S = std::min(std::max(sh.target, 256u), kGsSlabCap);
+    const int pmax = std::min(gs_slab_max_blocks(device, S, sh.threads), 1024);
     if (pmax < 1) return QSES_ERR_NO_DEVICE;
-    return gs_plan_for(pmax, in, nv, mol_off, mol_depth, nm, pl);
+    return gs_plan_resident(pmax, sh, nv, mol_off, mol_depth, nm, pl);
+}
+
+int gs_plan_resident(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth,
+                     unsigned nm, GsPlan &pl) {
+    return gs_plan_for(pmax, gs_resident_shape(sh), nv, mol_off, mol_depth, nm, pl);
 }
 
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
                 GsPlan &pl) {
     pl = GsPlan();
     if (pmax < 1 || nv == 0) return QSES_ERR_INVALID_ARG;
-    // with the slab's positions in shared memory (kGsSmemPos) slabs hold at most 8192
-    // vertices and a molecule may have more slabs than there are resident CTAs
+    // With the slabs' state in shared memory (kGsSmemPos, as gs_plan_resident has it) a molecule may have
+    // more slabs than there are resident CTAs.  The other split, and the limits without a cap, are
+    // those of kernels that kept it elsewhere; qses_debug_slab_plan still shows them.
     const bool spos = (sh.flags & kGsSmemPos) != 0;
     const unsigned Smax = sh.cap ? sh.cap : spos ? kGsSmemPosMaxVerts : kGsSlabMaxVerts;
     const unsigned t = std::min(std::max(sh.target, 256u), Smax);

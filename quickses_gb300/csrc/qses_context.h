@@ -238,6 +238,9 @@ bool side_work_late(int device, int ctas, unsigned slabs);
 int gs_plan(int device, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
             GsPlan &pl);
 // The same for at most pmax resident slab CTAs (no device query).
+int gs_plan_resident(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth,
+                     unsigned nm, GsPlan &pl);
+// The split itself, by the shape's flags and cap.
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
                 GsPlan &pl);
 // All items share `passes`.  Results in ctx->batch.
