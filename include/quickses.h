@@ -190,8 +190,9 @@ QSES_API void qses_set_pinned_cache(unsigned long long bytes);
 
 /* Picks the smoothing launch shape (threads per slab CTA, slab size aimed at) for meshes of
  * this size, and the refine tile shape for grids of this size, by running the molecule once
- * per candidate shape (`repeats` times each) and keeping the fastest; later calls of this process on meshes of the same size class (log2
- * of the vertex count) use it.  The mesh is identical for every shape: the update order is
+ * per candidate shape (`repeats` times each) and keeping the fastest; later calls of this
+ * process on meshes of the same size class (log2 of the vertex count) use it, with as many
+ * passes: one, or several.  The mesh is identical for every shape: the update order is
  * fixed by the vertex ids.  No reference counterpart (QuickSES hard-codes its launches). */
 QSES_API int qses_autotune(qses_context *ctx, const qses_params *p, const qses_float3 *atoms, const float *radii,
                            unsigned n, int repeats, int *threads_out, unsigned *target_out, unsigned *flags_out,
@@ -216,7 +217,8 @@ QSES_API int qses_set_smoothing_shape(qses_context *ctx, int threads, unsigned t
  * (batch = 1), replacing what the autotuner recorded; contexts with a fixed shape keep it.
  * No reference counterpart.  Lets a server use a shape that shares the SMs between lanes. */
 QSES_API int qses_set_default_smoothing_shape(int batch, int threads, unsigned target, unsigned cache_flags);
-/* The same for the batch form, timing whole qses_compute_batch calls on `reqs`. */
+/* The same for the batch form, timing whole qses_compute_batch calls on `reqs`; later batches
+ * use it whose largest molecule is of the same size class, too. */
 QSES_API int qses_autotune_batch(qses_context *ctx, const qses_request *reqs, unsigned count, int repeats,
                                  int *threads_out, unsigned *target_out, unsigned *flags_out, float *ms_out);
 

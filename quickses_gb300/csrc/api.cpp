@@ -701,7 +701,7 @@ QSES_API int qses_autotune(qses_context *ctx, const qses_params *p, const qses_f
     ctx->profiling = prof;
     if (rc) return rc;
     if (field_shape_out) *field_shape_out = best_edt;
-    if (nv > 0) qses::gs_shape_record(nv, false, best);
+    if (nv > 0) qses::gs_shape_record(nv, false, nv, p->smooth_passes, best);
     if (threads_out) *threads_out = best.threads;
     if (target_out) *target_out = best.target;
     if (flags_out) *flags_out = best.flags;
@@ -716,7 +716,8 @@ QSES_API int qses_autotune_batch(qses_context *ctx, const qses_request *reqs, un
     const int nc = qses::gs_shape_candidates(cand, 128);
     qses::GsShape best = cand[0];
     double best_s = -1.0;
-    unsigned long long nv = 0;
+    unsigned long long nv[2] = {0, 0};  // of the requests with one pass, with several
+    unsigned biggest[2] = {0, 0};
     std::vector<qses_mesh> out(count ? count : 1);
     int rc = QSES_OK;
     for (int c = 0; c < nc && rc == QSES_OK; c++) {
@@ -725,9 +726,13 @@ QSES_API int qses_autotune_batch(qses_context *ctx, const qses_request *reqs, un
             const auto t0 = std::chrono::steady_clock::now();
             rc = qses_compute_batch(ctx, reqs, count, out.data(), nullptr);
             const double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-            nv = 0;
+            nv[0] = nv[1] = biggest[0] = biggest[1] = 0;
             for (unsigned i = 0; i < count; i++) {
-                nv += out[i].n_vertices;
+                const int several = reqs[i].smooth_passes > 1;
+                if (reqs[i].smooth_passes > 0) {
+                    nv[several] += out[i].n_vertices;
+                    biggest[several] = std::max(biggest[several], out[i].n_vertices);
+                }
                 qses_mesh_release(&out[i]);
             }
             if (rc == QSES_OK && (best_s < 0 || dt < best_s)) {
@@ -738,7 +743,10 @@ QSES_API int qses_autotune_batch(qses_context *ctx, const qses_request *reqs, un
     }
     ctx->gs_force = qses::GsShape{0, 0, 0, 0};
     if (rc) return rc;
-    if (nv > 0) qses::gs_shape_record((unsigned)std::min<unsigned long long>(nv, 0xffffffffull), true, best);
+    for (int several = 0; several < 2; several++)
+        if (nv[several] > 0)
+            qses::gs_shape_record((unsigned)std::min<unsigned long long>(nv[several], 0xffffffffull), true, biggest[several],
+                                  several ? 2 : 1, best);
     if (threads_out) *threads_out = best.threads;
     if (target_out) *target_out = best.target;
     if (flags_out) *flags_out = best.flags;

@@ -110,8 +110,8 @@ void gs_l2_window(int device, cudaStream_t s, const void *p, size_t bytes);
 // Tuned shape for a mesh of nv vertices (batch: many molecules), or the default; biggest: the
 // vertices of the largest molecule.
 GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes);
-void gs_shape_record(unsigned nv, bool batch, GsShape s);
-void gs_shape_record_all(bool batch, GsShape s);  // every mesh-size class
+void gs_shape_record(unsigned nv, bool batch, unsigned biggest, int passes, GsShape s);
+void gs_shape_record_all(bool batch, GsShape s);  // for every such call
 int gs_shape_candidates(GsShape *out, int max);
 // Tuned refine tile shape (launch_edt `shape`) for grids of G voxels per axis, or 0.
 int edt_shape(int G);

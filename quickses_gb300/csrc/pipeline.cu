@@ -125,18 +125,25 @@ void fill_lut(const QGrid &g, float *lut) {
 
 // ------------------------------------------------------------------ tuning
 
-// Process-wide Gauss-Seidel shapes per (mode, log2 of the vertex count), filled by the
-// autotuner (qses_autotune*); absent entries use the default shape.
+// Process-wide Gauss-Seidel shapes, filled by the autotuner (qses_autotune*); absent entries use the
+// default shape.  What shape is best depends on what the default's rule depends on, so those are
+// the key: one molecule or a batch, one pass or several, log2 of the vertex count and of the
+// largest molecule's.
 static std::mutex g_tune_mu;
-static GsShape g_tune[2][33];
-static bool g_tuned[2][33];
+struct TunedShape {
+    GsShape shape;
+    bool set = false;
+};
+static TunedShape g_tune[2][2][33][33];
 
-static int tune_bucket(unsigned nv) { return bits_for(nv); }
+static TunedShape &tuned_shape(unsigned nv, bool batch, unsigned biggest, int passes) {
+    return g_tune[batch][passes > 1][bits_for(nv)][bits_for(batch ? biggest : nv)];
+}
 
 GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    const int b = tune_bucket(nv);
-    if (g_tuned[batch][b]) return g_tune[batch][b];
+    const TunedShape &tuned = tuned_shape(nv, batch, biggest, passes);
+    if (tuned.set) return tuned.shape;
     // Untuned.  A molecule of V vertices passes through V / target slabs one after another, each
     // crossing adding a hand-off to the chain of updates, while a slab that is too large queues its
     // ready vertices for one SM: 6.5 sqrt(V) was within 4 % of the best of seven targets for balls and
@@ -151,19 +158,16 @@ GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes) {
     return GsShape{512, nv > 8000000u ? kGsSlabTwo : std::min(std::max(t, 256u), kGsSlabCap), 0, 0};
 }
 
-void gs_shape_record(unsigned nv, bool batch, GsShape sh) {
+void gs_shape_record(unsigned nv, bool batch, unsigned biggest, int passes, GsShape sh) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    const int b = tune_bucket(nv);
-    g_tune[batch][b] = sh;
-    g_tuned[batch][b] = true;
+    tuned_shape(nv, batch, biggest, passes) = {sh, true};
 }
 
 void gs_shape_record_all(bool batch, GsShape sh) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    for (int b = 0; b < 33; b++) {
-        g_tune[batch][b] = sh;
-        g_tuned[batch][b] = true;
-    }
+    for (auto &several : g_tune[batch])
+        for (auto &row : several)
+            for (TunedShape &t : row) t = {sh, true};
 }
 
 static int g_edt_tune[2][16];  // [tuned?][log2 G]
