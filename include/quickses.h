@@ -312,6 +312,10 @@ QSES_API int qses_host_timeline(qses_context *ctx, double *ms, int max);
 QSES_API void qses_debug_fail_reservations(unsigned n);
 QSES_API int qses_debug_wait_limit(qses_context *ctx, long long spin_cycles, int *kernel_status);
 QSES_API int qses_debug_smoothing_wait(qses_context *ctx, long long spin_cycles);
+/* Device bytes that a server counts for a request (no GPU needed): what it needs, which the
+ * server's whole budget has to cover, and what a lane reserves for it, which counts towards
+ * the lane's share. */
+QSES_API int qses_debug_request_bytes(const qses_request *req, unsigned long long *need, unsigned long long *reserved);
 
 /* ------------------------------------------------------------------ CUDA graphs */
 

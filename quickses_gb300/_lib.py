@@ -113,6 +113,8 @@ SIGNATURES = {
     "qses_set_graphs": (ctypes.c_int, [_VP, ctypes.c_int]),
     "qses_debug_fail_reservations": (None, [ctypes.c_uint]),
     "qses_debug_wait_limit": (ctypes.c_int, [_VP, ctypes.c_longlong, ctypes.POINTER(ctypes.c_int)]),
+    "qses_debug_request_bytes": (ctypes.c_int, [ctypes.POINTER(Request), ctypes.POINTER(ctypes.c_ulonglong),
+                                                ctypes.POINTER(ctypes.c_ulonglong)]),
     "qses_debug_smoothing_wait": (ctypes.c_int, [_VP, ctypes.c_longlong]),
     "qses_host_timeline": (ctypes.c_int, [_VP, ctypes.POINTER(ctypes.c_double), ctypes.c_int]),
     "qses_debug_slab_plan": (ctypes.c_int, [ctypes.c_uint, _VP, _VP, ctypes.c_uint, ctypes.c_int, ctypes.c_uint,

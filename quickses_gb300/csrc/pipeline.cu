@@ -213,7 +213,7 @@ int Arena::reserve(size_t bytes) {
     if (base) cudaFree(base);
     base = nullptr;
     cap = 0;
-    size_t want = bytes + bytes / 4 + (1 << 20);
+    const size_t want = grown(bytes);
     if (cudaMalloc(&base, want) != cudaSuccess) {
         cudaGetLastError();
         base = nullptr;

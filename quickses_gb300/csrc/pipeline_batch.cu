@@ -60,6 +60,23 @@ static int stage_reserve(qses_context *ctx, size_t bytes) {
     return QSES_OK;
 }
 
+static size_t batch_desc_bytes(unsigned nm) {
+    return a256(sizeof(QMol) * nm) + 10 * a256(4ull * (nm + 1)) + a256(1024ull * nm);
+}
+static size_t batch_field_tmp(unsigned n, size_t cells, size_t rows) {
+    return std::max(radix_sort_tmp_bytes(n, bits_for(cells ? cells - 1 : 0)), scan_u2_tmp_bytes((unsigned)rows));
+}
+size_t batch_field_bytes(unsigned nm, unsigned n, size_t cells, size_t words, size_t codes, size_t rows) {
+    return batch_desc_bytes(nm) + a256(16ull * n) + 4 * a256(4ull * n) + a256(16ull * n) + a256(8 * cells) +
+           3 * a256(4 * words) + a256(codes) + a256(8 * rows) + 2 * a256(64) + a256(batch_field_tmp(n, cells, rows)) + 8192;
+}
+size_t batch_mesh_bytes(unsigned ne, unsigned nt, unsigned layers, bool smooth) {
+    const size_t n3 = 3ull * nt;
+    // the filter works in place unless the smoothing reads the triangles beside it
+    return (smooth ? 2 : 1) * a256(4 * n3 + 4) + 4 * a256(4ull * ne + 4) + a256(12ull * ne + 12) +
+           a256(weld_or_smooth_bytes(ne, layers, n3, smooth)) + a256(tri_filter_tmp_bytes(nt)) + 4096;
+}
+
 // ---- segment 1: descriptors and atoms up, atoms sorted into cells, field, row counts
 struct BatchFieldSeg {
     unsigned long long mem;  // free counters of the buffers it uses
@@ -320,7 +337,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
     const unsigned N = (unsigned)atoms_tot;
 
     // ---- pinned staging: descriptor block then atoms, one copy each
-    const size_t desc_bytes = a256(sizeof(QMol) * nm) + 10 * a256(4ull * (nm + 1)) + a256(1024ull * nm);
+    const size_t desc_bytes = batch_desc_bytes(nm);
     const size_t atom_bytes = 16ull * N;
     if (stage_reserve(ctx, desc_bytes + atom_bytes + 256) != QSES_OK)
         return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "pinned batch staging");
@@ -356,9 +373,8 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
 
     // ---- field workspace
     const int cell_bits = bits_for(cell_tot ? cell_tot - 1 : 0);
-    const size_t tmpA = std::max(radix_sort_tmp_bytes(N, cell_bits), scan_u2_tmp_bytes((unsigned)rows));
-    const size_t needA = desc_bytes + a256(16ull * N) + 4 * a256(4ull * N) + a256(16ull * N) + a256(8 * cell_tot) +
-                         3 * a256(4 * mask_tot) + a256(code_tot) + a256(8 * rows) + 2 * a256(64) + a256(tmpA) + 8192;
+    const size_t tmpA = batch_field_tmp(N, cell_tot, rows);
+    const size_t needA = batch_field_bytes(nm, N, cell_tot, mask_tot, code_tot, rows);
     if (ctx->field.reserve(needA) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "batch field workspace");
     Arena &A = ctx->field;
     BatchFieldSeg a;
@@ -434,9 +450,7 @@ int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int pas
 
     // ---- mesh workspace
     const size_t n3 = 3ull * T;
-    // the filter works in place unless the smoothing reads the triangles beside it
-    const size_t needB = (passes > 0 ? 2 : 1) * a256(4 * n3 + 4) + 4 * a256(4ull * NE + 4) + a256(12ull * NE + 12) +
-                         a256(weld_or_smooth_bytes(NE, layer_off[nm], n3, passes > 0)) + a256(tri_filter_tmp_bytes(T)) + 4096;
+    const size_t needB = batch_mesh_bytes(NE, T, layer_off[nm], passes > 0);
     if (ctx->mesh_ws.reserve(needB) != QSES_OK) return ctx->fail(QSES_ERR_OUT_OF_MEMORY, "batch mesh workspace");
     Arena &B = ctx->mesh_ws;
     unsigned *tri = (unsigned *)B.take(4 * n3 + 4);

@@ -25,6 +25,7 @@ struct Arena {
     int reserve(size_t bytes);  // resets the bump pointer; grows (and invalidates) if needed
     void *take(size_t bytes);   // 256-byte aligned; null when out of room
     void release();
+    static size_t grown(size_t bytes) { return bytes + bytes / 4 + (1 << 20); }  // what it takes for that many
 };
 
 // Device-resident result of the last call (pointers into the context arenas).
@@ -243,6 +244,10 @@ int gs_plan_resident(int pmax, const GsShape &sh, unsigned nv, const unsigned *m
 // The split itself, by the shape's flags and cap.
 int gs_plan_for(int pmax, const GsShape &sh, unsigned nv, const unsigned *mol_off, const int *mol_depth, unsigned nm,
                 GsPlan &pl);
+// Workspaces of a batch: of atoms, cells, voxel words and owner rows; of edges, pre-filter triangles
+// and owner planes.
+size_t batch_field_bytes(unsigned nm, unsigned n, size_t cells, size_t words, size_t codes, size_t rows);
+size_t batch_mesh_bytes(unsigned ne, unsigned nt, unsigned layers, bool smooth);
 // All items share `passes`.  Results in ctx->batch.
 int run_batch(qses_context *ctx, const BatchItem *items, unsigned count, int passes);
 }

@@ -40,16 +40,33 @@ struct Job {
     Clock::time_point t_submit, t_start, t_done;
 };
 
-// Device bytes a request needs while it runs (field workspace + a surface-sized mesh
-// workspace), from its grid alone; used only for admission.
-unsigned long long estimate_bytes(const QGrid &g, unsigned n) {
-    const double G = g.G;
-    // codes (one byte per padded voxel, and as much again in reserve), three masks, cells
-    const double field = 2.0 * G * G * (double)g.Gp + 3.0 * G * G * g.W * 4.0 + 8.0 * (double)g.gnb * g.gnb * g.gnb +
-                         48.0 * n + 8.0 * (g.Gc + 1.0) * (g.Gc + 1.0);
-    const double edges = 12.0 * G * G;  // active edges of a globular surface, generous
-    const double mesh = edges * 220.0;  // every mesh array per edge (keys, slots, CSR, positions)
-    return (unsigned long long)(field + mesh) + (1ull << 20);
+// Device bytes of a request while it runs (field workspace + a surface-sized mesh workspace), from its
+// grid alone, for admission: what it needs, and what a context reserves for that.
+struct RequestBytes {
+    unsigned long long need, reserved;
+};
+RequestBytes request_bytes(const QGrid &g, unsigned n, int passes) {
+    const size_t G = (size_t)g.G, E = (size_t)g.Gc + 1;
+    const size_t field = qses::batch_field_bytes(1, n, (size_t)g.gnb * g.gnb * g.gnb, G * G * g.W, G * G * g.Gp, E * E);
+    // active edges of a globular surface, generous; two triangles an edge
+    const unsigned edges = (unsigned)std::min<size_t>(12 * G * G, 1u << 30);
+    const size_t mesh = qses::batch_mesh_bytes(edges, 2 * edges, (unsigned)E, passes > 0);
+    return {field + mesh, qses::Arena::grown(field) + qses::Arena::grown(mesh)};
+}
+
+// Host bounds and the reference's grid of a request's atoms.
+int request_grid(const float *xyz, const float *r, unsigned n, float voxel, QGrid &g) {
+    // bounds start at atom 0, as the device min/max pass starts from its first atom
+    float mn[3] = {xyz[0], xyz[1], xyz[2]}, mx[3] = {xyz[0], xyz[1], xyz[2]}, maxR = r[0];
+    for (unsigned a = 1; a < n; a++) {
+        for (int q = 0; q < 3; q++) {
+            mn[q] = std::min(mn[q], xyz[3ull * a + q]);
+            mx[q] = std::max(mx[q], xyz[3ull * a + q]);
+        }
+        maxR = std::max(maxR, r[a]);
+    }
+    qses_grid_info gi;
+    return qses::grid_from_bounds(mn, mx, maxR, n, voxel, g, &gi, nullptr);
 }
 
 }  // namespace
@@ -177,22 +194,13 @@ QSES_API int qses_server_submit(qses_server *s, const qses_request *req, unsigne
     memset(&j->mesh, 0, sizeof(j->mesh));
     j->t_submit = Clock::now();
     if (req->n > 1) {
-        qses_grid_info gi;
         QGrid g;
-        // bounds start at atom 0, as the device min/max pass starts from its first atom
-        float mn[3] = {j->xyz[0], j->xyz[1], j->xyz[2]}, mx[3] = {j->xyz[0], j->xyz[1], j->xyz[2]}, maxR = j->r[0];
-        for (unsigned a = 1; a < req->n; a++) {
-            for (int q = 0; q < 3; q++) {
-                mn[q] = std::min(mn[q], j->xyz[3ull * a + q]);
-                mx[q] = std::max(mx[q], j->xyz[3ull * a + q]);
-            }
-            maxR = std::max(maxR, j->r[a]);
-        }
-        int rc = qses::grid_from_bounds(mn, mx, maxR, req->n, req->voxel, g, &gi, nullptr);
+        const int rc = request_grid(j->xyz.data(), j->r.data(), req->n, req->voxel, g);
         if (rc != QSES_OK) return rc;  // rejected at admission, never queued
-        j->est_bytes = estimate_bytes(g, req->n);
+        const RequestBytes bytes = request_bytes(g, req->n, req->smooth_passes);
+        j->est_bytes = bytes.reserved;
         j->voxels = (unsigned long long)g.G * g.G * g.G;
-        if (j->est_bytes > s->cfg.memory_budget) return QSES_ERR_OUT_OF_MEMORY;
+        if (bytes.need > s->cfg.memory_budget) return QSES_ERR_OUT_OF_MEMORY;
     }
     std::lock_guard<std::mutex> lock(s->mu);
     if (s->stopping) return QSES_ERR_INVALID_ARG;
@@ -201,6 +209,18 @@ QSES_API int qses_server_submit(qses_server *s, const qses_request *req, unsigne
     s->pending.push_back(j.get());
     s->jobs.emplace(j->ticket, std::move(j));
     s->cv_work.notify_one();
+    return QSES_OK;
+}
+
+QSES_API int qses_debug_request_bytes(const qses_request *req, unsigned long long *need, unsigned long long *reserved) {
+    if (!req || !need || !reserved || req->n < 2 || !req->atoms || !req->radii || !(req->voxel > 0.0f))
+        return QSES_ERR_INVALID_ARG;
+    QGrid g;
+    const int rc = request_grid((const float *)req->atoms, req->radii, req->n, req->voxel, g);
+    if (rc != QSES_OK) return rc;
+    const RequestBytes bytes = request_bytes(g, req->n, req->smooth_passes);
+    *need = bytes.need;
+    *reserved = bytes.reserved;
     return QSES_OK;
 }
 
