@@ -430,10 +430,9 @@ __device__ __forceinline__ void z_word(unsigned a, unsigned c, unsigned d, int R
         z_planes<true>(a, c, d, R, out);
 }
 
-// Shared-memory layout of one refine tile for a window of R voxels: the halo rows' outside
-// words (only without precomputed z distances), their z distances, the y-pass rows, and the
-// tile's in/out words.  Sized per launch, so a smaller window (a larger voxel) fits more CTAs
-// per SM; the largest layout (R = QSES_RMAX, no z distances) bounds every other.
+// Shared-memory layout of one refine tile for a window of R voxels: the halo rows' z distances, the
+// y-pass rows, and the tile's in/out words.  Sized per launch, so a smaller window (a larger voxel)
+// fits more CTAs per SM; the largest layout (R = QSES_RMAX) bounds every other.
 struct EdtLayout {
     size_t h_off, in_off, ot_off, bytes;
 };

@@ -1,4 +1,4 @@
-// Marching cubes, vertex weld, closest atom, degenerate filter and Laplacian smoothing.
+// Marching cubes, vertex weld, closest atom, degenerate filter and the neighbour lists' corners.
 //
 //  k_mc_count     per (x, y) row of cells: triangle count and active-edge count
 //                 (countVertexPerCell, MarchingCubes.cu:571-658, single-slice cell range),
@@ -7,7 +7,8 @@
 //                 active edge (generateTriangleVerticesSMEM + groupVertices,
 //                 MarchingCubes.cu:736-862).  The sign of 32 voxels is one word, so cube
 //                 indices and edge activity are bit ops.
-//  k_weld         unique quantised positions in lexicographic order (CudaSurf.cu:444-457)
+//  k_weld         unique quantised positions in lexicographic order (CudaSurf.cu:444-457), plane by
+//                 plane; k_weld_number and the radix sort for meshes that crowd a plane
 //  k_closest      closest atom per welded vertex (closestAtomPerVertex, Kernels.cu:547-604)
 //  k_tri_filter   drop triangles with a repeated index (CudaSurf.cu:820-829)
 //  k_csr_*        neighbour lists in triangle order (getNeighboorsVertices,
@@ -103,10 +104,6 @@ __device__ __forceinline__ unsigned grp_incl_scan(unsigned v, int sub, int Lg) {
     return v;
 }
 
-// One owner row (i, j) of a molecule's grid per group of Lg lanes; every lane of the warp
-// calls this (groups whose row is past the end pass valid = false and write nothing).  Bound by
-// instruction issue: 664^3 0.112 ms, 0.101 with the rows' addresses worked out once and words
-// without a change of sign passed over; 1738^3 1.44 and 1.27.
 // Bits [a, b) of a 32-bit word, the bounds clamped to [0, 32].
 __device__ __forceinline__ unsigned bits_in(int a, int b) {
     a = max(a, 0);
@@ -186,17 +183,16 @@ __device__ __forceinline__ void mc_count_row(const QGrid &g, long long row, bool
     if (valid && sub == 0) rowCount[row] = make_uint2(carry >> 16, carry & 0xffffu);
 }
 
-template <bool FULL>
 __global__ void __launch_bounds__(256, 4) k_mc_count(QGrid g, const unsigned *__restrict__ sign,
                                                      uint2 *__restrict__ rowCount, unsigned *__restrict__ words, int lanes) {
     __shared__ unsigned long long s_tab[256];
     s_tab[threadIdx.x] = c_mc[threadIdx.x];
     __syncthreads();
-    const int E = g.Gc + 1, Lg = FULL ? 32 : lanes;
+    const int E = g.Gc + 1, Lg = lanes;
     const long long first = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (32 / Lg), nrow = (long long)E * E;
     if (first >= nrow) return;  // the whole warp
     const long long row = first + (threadIdx.x & 31) / Lg;
-    mc_count_row<FULL>(g, row, row < nrow, Lg, sign, s_tab, rowCount, words);
+    mc_count_row<false>(g, row, row < nrow, Lg, sign, s_tab, rowCount, words);
 }
 
 // Batch form: rows are numbered molecule after molecule, so one scan over all rows gives
@@ -928,10 +924,7 @@ void launch_mc_count(const QGrid &g, const unsigned *sign, uint2 *rowCount, unsi
     // Narrow groups put more rows in flight per warp: 664^3 grid 0.248 ms with whole-warp rows, 0.127
     // with 2 lanes; 502^3 0.105 and 0.074.
     const int L = (g.Gc + 32) / 32 >= 8 ? 2 : mc_lanes(g.Gc);
-    if (L == 32)
-        k_mc_count<true><<<nblk(rows, 8), 256, 0, s>>>(g, sign, rowCount, words, 32);
-    else
-        k_mc_count<false><<<nblk(rows, 8 * (32 / L)), 256, 0, s>>>(g, sign, rowCount, words, L);
+    k_mc_count<<<nblk(rows, 8 * (32 / L)), 256, 0, s>>>(g, sign, rowCount, words, L);
 }
 void launch_mc_count_batch(const QBatch &b, unsigned units, const unsigned *sign, uint2 *rowCount, unsigned *words,
                            cudaStream_t s) {

@@ -95,7 +95,7 @@ struct GsShape {
     int threads = 512;
     unsigned target = 16384;
     unsigned flags = 0;
-    unsigned wave = 0;   // most vertices per slab-kernel launch (0: all that fit on the GPU)
+    unsigned wave = 0;   // most vertices per slab-kernel launch (0: the whole mesh)
     unsigned cap = 0;    // largest slab (0: 8192 with kGsSmemPos, else 25 000)
 };
 constexpr unsigned kGsPersistL2 = 4;    // host side: keep the positions in persisting L2 lines
@@ -113,7 +113,7 @@ GsShape gs_shape(unsigned nv, bool batch, unsigned biggest, int passes);
 void gs_shape_record(unsigned nv, bool batch, unsigned biggest, int passes, GsShape s);
 void gs_shape_record_all(bool batch, GsShape s);  // for every such call
 int gs_shape_candidates(GsShape *out, int max);
-// Tuned refine tile shape (launch_edt `shape`) for grids of G voxels per axis, or 0.
+// Tuned refine tile shape (launch_edt `shape`) for grids of G voxels per axis, or the default.
 int edt_shape(int G);
 void edt_shape_record(int G, int shape);
 constexpr int kEdtShapes = 4;
@@ -154,6 +154,6 @@ void launch_closest_batch(const QBatch &b, const float *vq, const unsigned *vmol
                           const uint2 *cells, const unsigned *sorted_to_input, int *asorted, int *ainput,
                           cudaStream_t s);
 cudaError_t launch_tri_filter_batch(const QBatch &b, const unsigned *tri, unsigned nt, unsigned *out, unsigned *kept_off,
-                                    uint2 *total, void *tmp, int *err, cudaStream_t s);  // 8 B of shared memory per vertex, 16-bit slab offsets
+                                    uint2 *total, void *tmp, int *err, cudaStream_t s);
 
 }  // namespace qses

@@ -15,7 +15,7 @@
 //     molecule's vertices contiguously in its own order;
 //   * Gauss-Seidel runs as one dataflow over all molecules (no dependency crosses a
 //     molecule, so each molecule is smoothed exactly as alone, and the critical path is the
-//     deepest molecule, not the sum), in waves of at most 152 x 25 000 vertices.
+//     deepest molecule, not the sum).
 // Per-molecule arithmetic is the single-molecule path's: the same tile bodies, the same
 // row body, the same keys and the same update order.
 #include <algorithm>
