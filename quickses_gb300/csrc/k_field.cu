@@ -25,6 +25,7 @@ __device__ __forceinline__ unsigned enc_f(float f) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// A coordinate or radius that is not a number bounds nothing, as on the host and in the reference.
 // 200 000 atoms 5 us; with the atomics of every warp in global memory 26.
 __global__ void k_atom_minmax(const float *__restrict__ xyz, const float *__restrict__ r, unsigned n,
                               unsigned *mm /* 7, zeroed: complements of min xyz; max xyz, max r (order-preserving encodings) */) {
@@ -32,11 +33,14 @@ __global__ void k_atom_minmax(const float *__restrict__ xyz, const float *__rest
     for (size_t a = (size_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (size_t)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            unsigned e = enc_f(xyz[3 * a + c]);
+            const float x = xyz[3 * a + c];
+            if (x != x) continue;
+            const unsigned e = enc_f(x);
             lo[c] = min(lo[c], e);
             hi[c] = max(hi[c], e);
         }
-        hi[3] = max(hi[3], enc_f(r[a]));
+        const float rad = r[a];
+        if (rad == rad) hi[3] = max(hi[3], enc_f(rad));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {

@@ -12,10 +12,11 @@
 
 namespace qses {
 
+// Cells beyond the grid's, which the bounds rule out for atoms that are somewhere, are clamped: the
+// cell table has no others.
 __device__ __forceinline__ unsigned atom_key(const QGrid &g, const float *__restrict__ xyz, unsigned a) {
-    const int cx = (int)((xyz[3 * a] - g.ox) / g.cell);
-    const int cy = (int)((xyz[3 * a + 1] - g.oy) / g.cell);
-    const int cz = (int)((xyz[3 * a + 2] - g.oz) / g.cell);
+    auto cell = [&](float p, float o) { return min(max((int)((p - o) / g.cell), 0), g.gnb - 1); };
+    const int cx = cell(xyz[3 * a], g.ox), cy = cell(xyz[3 * a + 1], g.oy), cz = cell(xyz[3 * a + 2], g.oz);
     return (unsigned)(g.gnb * g.gnb * cx + g.gnb * cy + cz);
 }
 __global__ void k_atom_hash(QGrid g, const float *__restrict__ xyz, unsigned n, unsigned *__restrict__ key) {
@@ -63,11 +64,7 @@ __global__ void k_atom_hash_batch(QBatch b, const float *__restrict__ xyz, unsig
     unsigned a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n) return;
     const unsigned m = qses_find(b.atom_off, b.n_mol, a);
-    const QGrid g = b.mols[m].g;
-    const int cx = (int)((xyz[3 * a] - g.ox) / g.cell);
-    const int cy = (int)((xyz[3 * a + 1] - g.oy) / g.cell);
-    const int cz = (int)((xyz[3 * a + 2] - g.oz) / g.cell);
-    key[a] = b.mols[m].cell_off + (unsigned)(g.gnb * g.gnb * cx + g.gnb * cy + cz);
+    key[a] = b.mols[m].cell_off + atom_key(b.mols[m].g, xyz, a);
 }
 
 void launch_atom_hash(const QGrid &g, const float *xyz, unsigned n, unsigned *key, cudaStream_t s) {
