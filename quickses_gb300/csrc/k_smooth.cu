@@ -184,7 +184,7 @@ __device__ __forceinline__ float add4(float s, float4 q) {
 // A wait's clock.  It runs out spin_cycles after the last sign of progress: one that the waiter sees
 // itself (restart) or an item taken from the counter since, by a CTA that has finished another.  So
 // a wait behind a long queue of slabs lasts while they are being done, however slowly, and ends
-// when none is.
+// when none is, or at its next look after another wait has run out.
 struct GsClock {
     long long since;
     unsigned taken;  // what the counter had at the last look
@@ -193,7 +193,7 @@ struct GsClock {
         taken = item + 1;
     }
     __device__ __forceinline__ void restart() { since = clock64(); }
-    __device__ __forceinline__ bool out(const unsigned *next_slab, long long spin_cycles) {
+    __device__ __forceinline__ bool out(const unsigned *next_slab, long long spin_cycles, const int *err) {
         const long long now = clock64();
         if (now - since <= spin_cycles) return false;
         unsigned k;
@@ -201,17 +201,17 @@ struct GsClock {
         const bool none = k == taken;
         taken = k;
         since = now;
-        return none;
+        return none || *(const volatile int *)err != 0;
     }
 };
 
 // Waits until slab p and the slabs of all its higher neighbours have had `pass` passes; false if
 // that takes too long.
 __device__ __forceinline__ bool gs_wait_pass(const GsOrder &ord, unsigned p, unsigned pass, GsClock clock,
-                                             const unsigned *next_slab, long long spin_cycles) {
+                                             const unsigned *next_slab, long long spin_cycles, const int *err) {
     for (unsigned j = p; j <= ord.far[p]; j++) {
         while (ld_acquire_u32(&ord.done[j]) < pass) {
-            if (clock.out(next_slab, spin_cycles)) return false;
+            if (clock.out(next_slab, spin_cycles, err)) return false;
             __nanosleep(200);
         }
         clock.restart();
@@ -305,14 +305,15 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
     if (threadIdx.x < 16) s_rcp[threadIdx.x] = make_float2(2.0f * threadIdx.x, __frcp_rn(2.0f * threadIdx.x));
     for (;;) {
         if (threadIdx.x == 0) {
-            const unsigned k = atomicAdd(next_slab, 1u);
+            // a CTA whose wait ran out takes nothing more, or the others would see progress
+            const unsigned k = s_q.stop ? 0xffffffffu : atomicAdd(next_slab, 1u);
             s_slab = 0xffffffffu;
             s_item = k;
-            if (k < Q * passes && !s_q.stop) {
+            if (k < Q * passes) {
                 const GsItem it = gs_item(k, Q, passes, lag);
                 s_slab = __ldg(order + it.place);
                 s_pass = it.pass;
-                if (it.pass && !gs_wait_pass(ord, s_slab, it.pass, GsClock(k), next_slab, spin_cycles)) {
+                if (it.pass && !gs_wait_pass(ord, s_slab, it.pass, GsClock(k), next_slab, spin_cycles, err)) {
                     raise_error(err, QSES_ERR_TIMEOUT);
                     s_q.stop = 1;
                     s_slab = 0xffffffffu;
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                 if (!left) break;  // nobody here waits for a lower slab any more
                 if (any || d != done_seen) clock.restart();
                 done_seen = d;
-                if (__any_sync(0xffffffffu, clock.out(next_slab, spin_cycles))) {
+                if (__any_sync(0xffffffffu, clock.out(next_slab, spin_cycles, err))) {
                     if (lane == 0) {
                         raise_error(err, QSES_ERR_TIMEOUT);
                         *v_stop = 1;
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(kGsThreadsMax, 1)
                     if (__any_sync(0xffffffffu, d >= len || *v_stop)) break;
                     if (d != seen) clock.restart();
                     seen = d;
-                    if (__any_sync(0xffffffffu, clock.out(next_slab, spin_cycles))) {
+                    if (__any_sync(0xffffffffu, clock.out(next_slab, spin_cycles, err))) {
                         if (lane == 0) {
                             raise_error(err, QSES_ERR_TIMEOUT);
                             *v_stop = 1;
