@@ -27,6 +27,13 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// A request that comes in a burst (kBurst behind the one before it), alone in the queue and while another
+// lane runs, waits kGather for company, so that requests which arrive together run as one batch.
+// Calls take little more than a millisecond, and without it idle lanes would pick such requests up one
+// by one: of three that come within 0.1 ms, two lanes made three batches in one run of eight.  It costs 1 % of the
+// median latency at 200 requests/s (0.90 ms), 3 % at 1 000; a burst of 1 ms and 0.25 ms of waiting 4 and 13 %.
+constexpr std::chrono::microseconds kBurst(250), kGather(150);
+
 struct Job {
     unsigned long long ticket = 0;
     std::vector<float> xyz, r;
@@ -37,6 +44,7 @@ struct Job {
     qses_mesh mesh;
     bool done = false;
     bool claimed = false;  // a qses_server_wait is waiting for (or has taken) this result
+    bool burst = false;    // came at most kBurst after the request before it
     Clock::time_point t_submit, t_start, t_done;
 };
 
@@ -74,10 +82,11 @@ int request_grid(const float *xyz, const float *r, unsigned n, float voxel, QGri
 struct qses_server {
     qses_server_config cfg;
     std::mutex mu;
-    std::condition_variable cv_work, cv_done;
+    std::condition_variable cv_work, cv_more, cv_done;  // cv_more: lanes that have one request
     std::deque<Job *> pending;
     std::unordered_map<unsigned long long, std::unique_ptr<Job>> jobs;
     unsigned long long next_ticket = 1;
+    Clock::time_point last_submit;
     bool stopping = false;
     std::vector<std::thread> workers;
     std::vector<qses_context *> ctxs;
@@ -97,6 +106,10 @@ void qses_server::lane_loop(int lane) {
             std::unique_lock<std::mutex> lock(mu);
             cv_work.wait(lock, [&] { return stopping || !pending.empty(); });
             if (stopping && pending.empty()) return;
+            if (pending.size() == 1 && pending.front()->burst && inflight_lanes > 0 && cfg.max_batch > 1 && !stopping) {
+                cv_more.wait_for(lock, kGather, [&] { return stopping || pending.size() != 1; });
+                if (pending.empty()) continue;  // another lane's by now, or cancelled
+            }
             unsigned long long bytes = 0, vox = 0;
             while (!pending.empty() && batch.size() < cfg.max_batch) {
                 Job *j = pending.front();
@@ -206,9 +219,12 @@ QSES_API int qses_server_submit(qses_server *s, const qses_request *req, unsigne
     if (s->stopping) return QSES_ERR_INVALID_ARG;
     j->ticket = s->next_ticket++;
     *ticket = j->ticket;
+    j->burst = j->t_submit - s->last_submit <= kBurst;
+    s->last_submit = j->t_submit;
     s->pending.push_back(j.get());
     s->jobs.emplace(j->ticket, std::move(j));
     s->cv_work.notify_one();
+    s->cv_more.notify_all();
     return QSES_OK;
 }
 
@@ -292,6 +308,7 @@ QSES_API int qses_server_destroy(qses_server *s) {
         s->stopping = true;
     }
     s->cv_work.notify_all();
+    s->cv_more.notify_all();
     for (auto &t : s->workers) t.join();
     for (auto &kv : s->jobs) qses_mesh_release(&kv.second->mesh);  // results never collected
     for (auto *c : s->ctxs) qses_context_destroy(c);
